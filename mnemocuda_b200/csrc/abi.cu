@@ -15,6 +15,7 @@ void gemm_init();
 void moe_fused_init();
 void router_static_init();
 void support_init();
+void attn_int8_init();
 
 namespace {
 int g_status = MB200_OK;
@@ -83,6 +84,7 @@ void cuda_kernels_init(void)
     gemm_init();
     moe_fused_init();
     support_init();
+    attn_int8_init();
     router_static_init();
     (void)device_sms();
     (void)device_error_word();

@@ -28,6 +28,9 @@ int pdl_enabled();
 bool stream_matvec_q8_0(const void *w, const float *x, float *y, int n_rows, int n_cols, cudaStream_t s);
 bool stream_matvec_q5k(const void *w, const float *x, float *y, int n_rows, int n_cols, cudaStream_t s);
 bool stream_matvec_q3k(const void *w, const float *x, float *y, int n_rows, int n_cols, cudaStream_t s);
+// attention over the INT8 cache on tensor cores (attn_int8.cu); false = shape or alignment it does not take
+bool attn_int8_tc(const float *q, const void *k, const void *v, const float *ks, const float *vs, float *out, int n_heads_q,
+                  int n_kv_heads, int gqa, int seq_len, float scale, cudaStream_t stream);
 
 namespace {
 
@@ -268,138 +271,7 @@ __global__ void __launch_bounds__(128) int8_kv_kernel(const float *in_a, const f
     }
 }
 
-// ---- attention over the INT8 cache ----
-// One CTA per (group of HPB query heads that share a KV head, chunk of positions): the group's heads
-// share every K / V byte read.
-// Each warp walks positions of the chunk with an online softmax per query head, lanes over head
-// dimensions (4 consecutive int8 per lane per 128 dims); the warps' and chunks' partial (m, l, acc)
-// are merged by the last CTA of the KV head to arrive (ticket in the workspace).
-constexpr int kI8Warps = 8;
-constexpr int kI8MaxGqa = 8;    // query heads per CTA (registers: q and the running sums of each)
-constexpr int kI8Groups = 64;   // head groups per launch
-constexpr int kI8Slots = 512;   // (group, chunk) pairs per launch
-
-struct I8Work {  // library-resident workspace: 512 slots x 8 query heads x (128 + 2) floats (2.1 MB per device)
-    float part[kI8Slots * kI8MaxGqa * 128];
-    float ml[kI8Slots * kI8MaxGqa * 2];
-    int tickets[kI8Groups];
-};
-__device__ I8Work g_i8;
-
-template <int GQA>
-__global__ void __launch_bounds__(kI8Warps * 32) attn_int8_kernel(const float *q, const int8_t *__restrict__ kv_k,
-                                                                  const int8_t *__restrict__ kv_v, const float *k_scales,
-                                                                  const float *v_scales, float *out, int n_kv_heads,
-                                                                  int seq_len, float scale, int chunks, int gqa_ratio)
-{
-    pdl_enter();
-    __shared__ float s_acc[kI8Warps][GQA][128];
-    __shared__ float s_ml[kI8Warps][GQA][2];
-    __shared__ int s_last;
-    // group blockIdx.x = query heads [GQA * blockIdx.x, GQA * (blockIdx.x + 1)), all on KV head kvh
-    const int grp = blockIdx.x, kvh = grp * GQA / gqa_ratio, chunk = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t stride = (size_t)n_kv_heads * 128;
-    float qv[GQA][4], acc[GQA][4], m[GQA], l[GQA];
-#pragma unroll
-    for (int h = 0; h < GQA; h++) {
-        const float4 t = __ldcg(reinterpret_cast<const float4 *>(q + ((size_t)grp * GQA + h) * 128) + lane);
-        qv[h][0] = t.x * scale; qv[h][1] = t.y * scale; qv[h][2] = t.z * scale; qv[h][3] = t.w * scale;
-        acc[h][0] = acc[h][1] = acc[h][2] = acc[h][3] = 0.0f;
-        m[h] = -INFINITY;
-        l[h] = 0.0f;
-    }
-    const int per = (seq_len + chunks - 1) / chunks;
-    const int p0 = chunk * per, p1 = min(seq_len, p0 + per);
-    for (int p = p0 + warp; p < p1; p += kI8Warps) {
-        const unsigned kb = __ldcg(reinterpret_cast<const unsigned *>(kv_k + (size_t)p * stride + (size_t)kvh * 128) + lane);
-        const unsigned vb = __ldcg(reinterpret_cast<const unsigned *>(kv_v + (size_t)p * stride + (size_t)kvh * 128) + lane);
-        const float ks = __ldcg(k_scales + (size_t)p * n_kv_heads + kvh), vs = __ldcg(v_scales + (size_t)p * n_kv_heads + kvh);
-        float kf[4], vf[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            kf[i] = (float)(int)(signed char)((kb >> (8 * i)) & 0xFF) * ks;
-            vf[i] = (float)(int)(signed char)((vb >> (8 * i)) & 0xFF) * vs;
-        }
-#pragma unroll
-        for (int h = 0; h < GQA; h++) {
-            float s = qv[h][0] * kf[0] + qv[h][1] * kf[1] + qv[h][2] * kf[2] + qv[h][3] * kf[3];
-            s = warp_sum(s);
-            const float mn = fmaxf(m[h], s), r = __expf(m[h] - mn), pw = __expf(s - mn);
-#pragma unroll
-            for (int i = 0; i < 4; i++) acc[h][i] = acc[h][i] * r + pw * vf[i];
-            l[h] = l[h] * r + pw;
-            m[h] = mn;
-        }
-    }
-#pragma unroll
-    for (int h = 0; h < GQA; h++) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) s_acc[warp][h][4 * lane + i] = acc[h][i];
-        if (lane == 0) {
-            s_ml[warp][h][0] = m[h];
-            s_ml[warp][h][1] = l[h];
-        }
-    }
-    __syncthreads();
-    // the CTA's partial for this chunk
-    float *part = g_i8.part + ((size_t)(grp * chunks + chunk) * kI8MaxGqa) * 128;
-    float *ml = g_i8.ml + ((size_t)(grp * chunks + chunk) * kI8MaxGqa) * 2;
-    for (int i = threadIdx.x; i < GQA * 128; i += blockDim.x) {
-        const int h = i >> 7, d = i & 127;
-        float M = -INFINITY;
-        for (int w2 = 0; w2 < kI8Warps; w2++) M = fmaxf(M, s_ml[w2][h][0]);
-        float o = 0.0f, L = 0.0f;
-        for (int w2 = 0; w2 < kI8Warps; w2++) {
-            const float f = s_ml[w2][h][0] == -INFINITY ? 0.0f : __expf(s_ml[w2][h][0] - M);
-            o += s_acc[w2][h][d] * f;
-            L += s_ml[w2][h][1] * f;
-        }
-        part[i] = o;
-        if (d == 0) {
-            ml[2 * h] = M;
-            ml[2 * h + 1] = L;
-        }
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(&g_i8.tickets[grp], 1) == chunks - 1;
-    __syncthreads();
-    if (!s_last) return;
-    __threadfence();
-    for (int i = threadIdx.x; i < GQA * 128; i += blockDim.x) {
-        const int h = i >> 7;
-        // eight chunks' loads in flight at a time (one chunk after the other would be a chain of L2 round trips)
-        float M = -INFINITY;
-        for (int c0 = 0; c0 < chunks; c0 += 8) {
-            float mv[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++)
-                mv[u] = c0 + u < chunks ? __ldcg(g_i8.ml + ((size_t)(grp * chunks + c0 + u) * kI8MaxGqa + h) * 2) : -INFINITY;
-#pragma unroll
-            for (int u = 0; u < 8; u++) M = fmaxf(M, mv[u]);
-        }
-        float o = 0.0f, L = 0.0f;
-        for (int c0 = 0; c0 < chunks; c0 += 8) {
-            float mv[8], lv[8], pv[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const size_t b = (size_t)(grp * chunks + min(c0 + u, chunks - 1)) * kI8MaxGqa;
-                mv[u] = __ldcg(g_i8.ml + (b + h) * 2);
-                lv[u] = __ldcg(g_i8.ml + (b + h) * 2 + 1);
-                pv[u] = __ldcg(g_i8.part + b * 128 + i);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const float f = (c0 + u >= chunks || mv[u] == -INFINITY) ? 0.0f : __expf(mv[u] - M);
-                o += pv[u] * f;
-                L += lv[u] * f;
-            }
-        }
-        out[((size_t)grp * GQA) * 128 + i] = L > 0.0f ? o / L : 0.0f;
-    }
-    if (threadIdx.x == 0) g_i8.tickets[grp] = 0;  // ready for the next launch
-}
-
+// ---- attention over the INT8 cache: head_dim 128 runs in attn_int8.cu, the rest here ----
 // Any head_dim / ratio: one CTA per query head, a warp per position (reference's shape of work).
 __global__ void __launch_bounds__(256) attn_int8_generic_kernel(const float *q, const int8_t *__restrict__ kv_k,
                                                                const int8_t *__restrict__ kv_v, const float *k_scales,
@@ -455,20 +327,6 @@ __global__ void __launch_bounds__(256) attn_int8_generic_kernel(const float *q, 
         for (int w2 = 0; w2 < 8; w2++) o += ms[w2] == -INFINITY ? 0.0f : gsm[w2 * head_dim + d] * expf(ms[w2] - M);
         out[(size_t)head * head_dim + d] = L > 0.0f ? o / L : 0.0f;
     }
-}
-
-template <int GQA>
-void launch_attn_int8(const float *q, const void *kv_k, const void *kv_v, const float *ks, const float *vs, float *out,
-                      int n_heads_q, int n_kv_heads, int gqa_ratio, int seq_len, float scale, cudaStream_t stream)
-{
-    const int groups = n_heads_q / GQA;
-    int chunks = 2 * device_sms() / groups;  // two CTAs per SM
-    if (chunks > kI8Slots / groups) chunks = kI8Slots / groups;
-    if (chunks < 1) chunks = 1;
-    if (chunks > (seq_len + kI8Warps - 1) / kI8Warps) chunks = (seq_len + kI8Warps - 1) / kI8Warps;
-    launch_k(attn_int8_kernel<GQA>, dim3(groups, chunks), dim3(kI8Warps * 32), 0, stream, q,
-             static_cast<const int8_t *>(kv_k), static_cast<const int8_t *>(kv_v), ks, vs, out, n_kv_heads, seq_len, scale,
-             chunks, gqa_ratio);
 }
 
 }  // namespace
@@ -538,12 +396,8 @@ void cuda_attention_int8kv(const float *q, const void *kv_k, const void *kv_v, c
         set_status(MB200_ERR_UNSUPPORTED, "cuda_attention_int8kv");
         return;
     }
-    const bool fast = head_dim == 128 && n_heads_q == n_kv_heads * gqa_ratio;
-    if (fast && gqa_ratio % 8 == 0 && n_heads_q / 8 <= kI8Groups) {
-        launch_attn_int8<8>(q, kv_k, kv_v, k_scales, v_scales, out, n_heads_q, n_kv_heads, gqa_ratio, seq_len, scale, stream);
-    } else if (fast && gqa_ratio % 4 == 0 && n_heads_q / 4 <= kI8Groups) {
-        launch_attn_int8<4>(q, kv_k, kv_v, k_scales, v_scales, out, n_heads_q, n_kv_heads, gqa_ratio, seq_len, scale, stream);
-    } else {
+    if (head_dim != 128 ||
+        !attn_int8_tc(q, kv_k, kv_v, k_scales, v_scales, out, n_heads_q, n_kv_heads, gqa_ratio, seq_len, scale, stream)) {
         const size_t smem = ((size_t)8 * head_dim + 16) * sizeof(float);
         launch_k(attn_int8_generic_kernel, dim3(n_heads_q), dim3(256), smem, stream, q, static_cast<const int8_t *>(kv_k),
                  static_cast<const int8_t *>(kv_v), k_scales, v_scales, out, head_dim, n_kv_heads, seq_len, gqa_ratio,

@@ -1,0 +1,52 @@
+"""The tensor-core attention over the INT8 cache at the edges of its tiles, chunks and head blocks, and the sampler
+beyond the vocabulary size whose candidates all fit one list per thread (both against the C oracle)."""
+import numpy as np
+import pytest
+import torch
+
+from mnemocuda_b200 import synth
+from oracle import oracle
+from tests.gpu_util import dev, host
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K():
+    from mnemocuda_b200 import kernels
+    kernels.mb200_init()
+    return kernels
+
+
+# one chunk / one cluster / several clusters; a position past a tile and past a chunk; 1, 3, 16 and 20 heads per KV head
+@pytest.mark.parametrize("nh,nkv,S", [(4, 4, 16), (16, 1, 17), (64, 4, 128), (64, 4, 129), (12, 4, 255), (20, 1, 1025),
+                                      (40, 2, 2049), (32, 8, 4097)])
+@pytest.mark.parametrize("spread", [1.0, 1e6])
+def test_int8_attention_edges(K, nh, nkv, S, spread):
+    """spread: V scales that differ by that factor from position to position (they are folded into fp16 operands)."""
+    rng = np.random.default_rng(S + nh)
+    k8 = rng.integers(-127, 128, (S, nkv, 128), dtype=np.int8)
+    v8 = rng.integers(-127, 128, (S, nkv, 128), dtype=np.int8)
+    ks = ((0.5 + rng.random((S, nkv))) / 127).astype(np.float32)
+    vs = (spread ** -rng.random((S, nkv)) / 127).astype(np.float32)
+    q = synth.normal_f32(4100 + S, nh * 128)
+    want = oracle.attention_int8kv(q, k8, v8, ks, vs, nh, 128, nkv, S, nh // nkv, 128 ** -0.5).reshape(nh, 128).astype(np.float64)
+    out = torch.full((nh * 128,), float("nan"), device="cuda")
+    for _ in range(2):  # twice: the tickets must be back at zero
+        out.fill_(float("nan"))
+        K.cuda_attention_int8kv(dev(q), dev(k8), dev(v8), dev(ks), dev(vs), out, nh, 128, nkv, S, nh // nkv, 128 ** -0.5)
+        got = host(out).reshape(nh, 128).astype(np.float64)
+        rel = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
+        assert rel.max() <= 2e-5, rel.max()
+
+
+@pytest.mark.parametrize("V", [7, 256, 2049, 262144, 300001])
+def test_sample_top_p_sizes(K, V):
+    logits = (synth.normal_f32(4200 + V, V) * 2.0).astype(np.float32)
+    d_l, res = dev(logits), torch.full((1,), -1, dtype=torch.int32, device="cuda")
+    seeds = [int(s) for s in np.random.default_rng(V).integers(1, 2 ** 63, 12)]
+    miss = 0
+    for seed in seeds:
+        K.cuda_sample_token(d_l, V, 0.8, 0.9, seed, res)
+        miss += int(res.item()) != oracle.sample_top_p(logits, 0.8, 0.9, seed)
+    assert miss <= 1, miss  # a cut or draw within float rounding of a boundary
