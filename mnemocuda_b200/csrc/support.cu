@@ -680,11 +680,19 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ l
     int bi = 0;
     // candidates are compared by their index in the whole vocabulary (index_offset + i), so that a row shard
     // orders ties as the whole vector would; bi stays shard-local until the end
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float v = __ldcg(logits + i);
-        if (argmax_better(v, i + index_offset, bv, bi + index_offset)) {
-            bv = v;
-            bi = i;
+    // eight loads in flight: at the vocabulary's size a thread has five, and one at a time they were five round trips
+    const int step = gridDim.x * blockDim.x;
+    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 8 * step) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = i0 + u * step < n ? __ldcg(logits + i0 + u * step) : -INFINITY;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int i = i0 + u * step;
+            if (i < n && argmax_better(v[u], i + index_offset, bv, bi + index_offset)) {
+                bv = v[u];
+                bi = i;
+            }
         }
     }
     bi += index_offset;
@@ -740,41 +748,97 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ l
 // candidates and walks them with the reference's arithmetic (float sums in descending order). Among equal
 // probabilities the smaller token id is preferred; the sum of all p is added in another order than the
 // reference's, so a cut that falls within rounding of top_p * sum can come out one candidate apart.
+//
+// All latency (600 KB of logits): what counts is the length of the dependent chain. A candidate is one 64-bit key
+// {bits of p, ~id}, ordered as the preference is (p >= 0). The sort starts from the classes' sorted runs of eight and
+// keeps them in registers: strides below 8 inside a thread, below 256 by shuffles, and only six steps through shared
+// memory. The walk's three float sums over the nucleus are prefixes of one and the same sequence, so ONE serial chain
+// of additions leaves all of them and the two searches run on all threads. (Sort in shared memory with 66 barriers,
+// three serial walks by one thread, scan loads one at a time: 60-72 us per token at 151936, now 28.)
 constexpr int kSampleClasses = 256, kSampleKeep = 8, kSampleCands = kSampleClasses * kSampleKeep;
 constexpr int kSampleCtas = kSampleClasses / 8;
+constexpr int kSampleThreads = 1024;
+constexpr int kSampleSmem = kSampleThreads * kSampleKeep * 8 + kSampleCands * 8;
 __device__ float g_sample_pair[2];
-__device__ float g_sample_p[kSampleCands];
-__device__ int g_sample_id[kSampleCands];
+__device__ __align__(16) unsigned long long g_sample_key[kSampleCands];
 __device__ float g_sample_sum[kSampleCtas];
 __device__ int g_sample_ticket;
 
-__device__ __forceinline__ bool cand_better(float p, int id, float bp, int bid)
+__device__ __forceinline__ unsigned long long cand_key(float p, int id)  // 0 = no candidate
 {
-    return p > bp || (p == bp && id >= 0 && (bid < 0 || id < bid));
+    return id < 0 ? 0ull : (static_cast<unsigned long long>(__float_as_uint(p)) << 32) | (~static_cast<unsigned>(id));
+}
+__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k)
+{
+    const unsigned hi = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(k >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(k >> 32) == hi ? static_cast<unsigned>(k) : 0u);
+    return (static_cast<unsigned long long>(hi) << 32) | lo;
+}
+__device__ __forceinline__ void sample_barrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }  // the sort's threads
+// Descending bitonic sort of 2048 keys, eight consecutive ones per thread (256 threads). On entry every thread's
+// eight are sorted: descending in even threads, ascending in odd ones. xch: 2048 keys of shared memory.
+__device__ __forceinline__ void sort_keys(unsigned long long (&v)[kSampleKeep], unsigned long long *xch, int tid)
+{
+#pragma unroll 1
+    for (int size = 16; size <= kSampleCands; size <<= 1) {
+        const bool desc = ((tid * kSampleKeep) & size) == 0;
+#pragma unroll 1
+        for (int d = size >> 4; d > 0; d >>= 1) {  // stride 8 d: the same position of thread tid ^ d
+            const bool keep_max = ((tid & d) == 0) == desc;
+            if (d >= 32) {
+#pragma unroll
+                for (int q = 0; q < kSampleKeep; q++) xch[q * 256 + tid] = v[q];
+                sample_barrier();
+            }
+#pragma unroll
+            for (int q = 0; q < kSampleKeep; q++) {
+                const unsigned long long o = d >= 32 ? xch[q * 256 + (tid ^ d)] : __shfl_xor_sync(0xffffffffu, v[q], d);
+                if ((o > v[q]) == keep_max) v[q] = o;
+            }
+            if (d >= 32) sample_barrier();
+        }
+#pragma unroll
+        for (int s = 4; s > 0; s >>= 1)
+#pragma unroll
+            for (int q = 0; q < kSampleKeep; q++)
+                if ((q & s) == 0 && (v[q + s] > v[q]) == desc) {
+                    const unsigned long long o = v[q];
+                    v[q] = v[q + s];
+                    v[q + s] = o;
+                }
+    }
 }
 
-__global__ void __launch_bounds__(256) sample_top_p_kernel(const float *__restrict__ logits, int n, float temperature,
-                                                           float top_p, unsigned long long seed, int *result)
+__global__ void __launch_bounds__(kSampleThreads) sample_top_p_kernel(const float *__restrict__ logits, int n, float temperature,
+                                                                      float top_p, unsigned long long seed, int *result)
 {
     pdl_enter();
-    __shared__ float sp[256 * kSampleKeep];
-    __shared__ int si[256 * kSampleKeep];
-    __shared__ float ssum[8];
-    __shared__ int is_last;
+    extern __shared__ __align__(16) unsigned long long keys[];  // [1024 x 8] candidates of the scan, later the sort's
+    float *sp = reinterpret_cast<float *>(keys + kSampleThreads * kSampleKeep), *cum = sp + kSampleCands;
+    __shared__ float ssum[32];
+    __shared__ int is_last, s_len, s_nucleus, s_pick;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float mx = __ldcg(&g_sample_pair[0]);
     const float inv_t = 1.0f / temperature;
-    // ---- scan: thread (jj = tid / 8, k = tid % 8) takes i = 256 (jj + 32 m) + 8 blockIdx.x + k ----
+    // ---- scan: thread (jj = tid / 8, k = tid % 8) takes i = 256 (jj + 128 m) + 8 blockIdx.x + k; its first eight are its
+    // list as they come (that is all of them up to 262144 logits), later ones replace the list's smallest ----
     const int k = tid & 7, jj = tid >> 3;
-    float vp[kSampleKeep];
+    constexpr int kStep = 256 * (kSampleThreads / 8);
+    float vp[kSampleKeep], lg[kSampleKeep];
     int vi[kSampleKeep];
+    const int first = 256 * jj + 8 * blockIdx.x + k;
+#pragma unroll
+    for (int q = 0; q < kSampleKeep; q++) lg[q] = first + q * kStep < n ? __ldcg(logits + first + q * kStep) : 0.0f;
+    float sum = 0.0f;
 #pragma unroll
     for (int q = 0; q < kSampleKeep; q++) {
-        vp[q] = -1.0f;
-        vi[q] = -1;
+        const int i = first + q * kStep;
+        const bool in = i < n;
+        vp[q] = in ? expf((lg[q] - mx) * inv_t) : -1.0f;
+        vi[q] = in ? i : -1;
+        if (in) sum += vp[q];
     }
-    float sum = 0.0f;
-    for (int i = 256 * jj + 8 * blockIdx.x + k; i < n; i += 256 * 32) {
+    for (int i = first + kSampleKeep * kStep; i < n; i += kStep) {
         const float p = expf((__ldcg(logits + i) - mx) * inv_t);
         sum += p;
         int mi = 0;
@@ -788,129 +852,129 @@ __global__ void __launch_bounds__(256) sample_top_p_kernel(const float *__restri
                 vi[q] = i;
             }
     }
-    // lists to shared memory, class-major: class k holds 32 threads x 8 = 256 candidates
+    // lists to shared memory, class-major: class k holds 128 threads x 8 = 1024 candidates, 256 for each of four warps
 #pragma unroll
-    for (int q = 0; q < kSampleKeep; q++) {
-        sp[(k * 32 + jj) * kSampleKeep + q] = vp[q];
-        si[(k * 32 + jj) * kSampleKeep + q] = vi[q];
-    }
+    for (int q = 0; q < kSampleKeep; q++) keys[(k * kSampleKeep + q) * 128 + jj] = cand_key(vp[q], vi[q]);
     sum = warp_sum(sum);
     if (lane == 0) ssum[warp] = sum;
     __syncthreads();
-    // ---- warp w keeps the eight best of class w: eight rounds of a warp-wide maximum ----
+    // ---- warp (class c, quarter): the eight best of its 256, by rounds of a warp-wide maximum; then one warp per class
+    // the eight best of the four quarters' ----
     {
-        float cp[kSampleKeep];
-        int ci[kSampleKeep];
+        const int c = warp >> 2, quarter = warp & 3;
+        unsigned long long v[kSampleKeep], mine = 0;
 #pragma unroll
-        for (int q = 0; q < kSampleKeep; q++) {
-            cp[q] = sp[(warp * 32 + lane) * kSampleKeep + q];
-            ci[q] = si[(warp * 32 + lane) * kSampleKeep + q];
-        }
+        for (int q = 0; q < kSampleKeep; q++) v[q] = keys[(c * kSampleKeep + q) * 128 + quarter * 32 + lane];
+#pragma unroll 1
         for (int round = 0; round < kSampleKeep; round++) {
-            float bp = -1.0f;
-            int bi = -1;
+            unsigned long long best = v[0];
+#pragma unroll
+            for (int q = 1; q < kSampleKeep; q++) best = v[q] > best ? v[q] : best;
+            best = warp_max_key(best);
+            if (lane == round) mine = best;
 #pragma unroll
             for (int q = 0; q < kSampleKeep; q++)
-                if (cand_better(cp[q], ci[q], bp, bi)) {
-                    bp = cp[q];
-                    bi = ci[q];
-                }
-            float wp = bp;
-            int wi = bi;
+                if (v[q] == best) v[q] = 0;  // keys are unique: the winner's owner retires it
+        }
+        __syncthreads();
+        if (lane < kSampleKeep) keys[warp * kSampleKeep + lane] = mine;
+        __syncthreads();
+        if (warp < 8) {
+            unsigned long long key = keys[warp * 32 + lane];
+            mine = 0;
+#pragma unroll 1
+            for (int round = 0; round < kSampleKeep; round++) {
+                const unsigned long long best = warp_max_key(key);
+                if (lane == round) mine = best;
+                if (key == best) key = 0;
+            }
+            if (lane < kSampleKeep) g_sample_key[(8 * blockIdx.x + warp) * kSampleKeep + lane] = mine;
+        }
+        if (warp == 8) {
+            const float s = warp_sum(ssum[lane]);
+            if (lane == 0) g_sample_sum[blockIdx.x] = s;
+        }
+    }
+    __syncthreads();
+    if (tid == 0) {  // one fence for the CTA: the barrier orders the other threads' stores before it
+        __threadfence();
+        is_last = (atomicAdd(&g_sample_ticket, 1) == static_cast<int>(gridDim.x) - 1);
+        __threadfence();
+    }
+    __syncthreads();
+    if (!is_last || tid >= 256) return;
+    // ---- last CTA, 256 threads: sort the candidates (probability descending, token id ascending), walk them ----
+    unsigned long long v[kSampleKeep];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float op = __shfl_xor_sync(0xffffffffu, wp, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, wi, o);
-                if (cand_better(op, oi, wp, wi)) {
-                    wp = op;
-                    wi = oi;
-                }
-            }
-            if (wi >= 0 && wi == bi) {  // the winner's owner retires it
+    for (int q = 0; q < kSampleKeep; q++) v[q] = __ldcg(&g_sample_key[tid * kSampleKeep + ((tid & 1) ? kSampleKeep - 1 - q : q)]);
+    if (tid < kSampleCtas) ssum[tid] = __ldcg(&g_sample_sum[tid]);
+    sort_keys(v, keys, tid);
 #pragma unroll
-                for (int q = 0; q < kSampleKeep; q++)
-                    if (ci[q] == wi) {
-                        cp[q] = -1.0f;
-                        ci[q] = -1;
-                    }
-            }
-            if (lane == 0) {
-                const int c = (8 * blockIdx.x + warp) * kSampleKeep + round;
-                g_sample_p[c] = wi >= 0 ? wp : -1.0f;
-                g_sample_id[c] = wi;
-            }
-        }
-    }
+    for (int q = 0; q < kSampleKeep; q++) sp[tid * kSampleKeep + q] = __uint_as_float(static_cast<unsigned>(v[q] >> 32));
     if (tid == 0) {
-        float s = 0.0f;
-        for (int w = 0; w < 8; w++) s += ssum[w];
-        g_sample_sum[blockIdx.x] = s;
+        s_nucleus = kSampleCands;
+        s_pick = kSampleCands;
     }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) is_last = (atomicAdd(&g_sample_ticket, 1) == static_cast<int>(gridDim.x) - 1);
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    // ---- last CTA: sort the candidates (probability descending, token id ascending), walk them ----
-    for (int c = tid; c < kSampleCands; c += 256) {
-        sp[c] = __ldcg(&g_sample_p[c]);
-        si[c] = __ldcg(&g_sample_id[c]);
-    }
-    __syncthreads();
-    for (int size = 2; size <= kSampleCands; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int t = tid; t < kSampleCands / 2; t += 256) {
-                const int lo = 2 * t - (t & (stride - 1));
-                const int hi = lo + stride;
-                const bool desc = ((lo & size) == 0);
-                const bool hi_first = cand_better(sp[hi], si[hi], sp[lo], si[lo]);
-                if (hi_first == desc) {
-                    const float tp = sp[lo];
-                    const int ti = si[lo];
-                    sp[lo] = sp[hi];
-                    si[lo] = si[hi];
-                    sp[hi] = tp;
-                    si[hi] = ti;
-                }
-            }
-            __syncthreads();
-        }
-    }
-    if (tid == 0) {
-        float total = 0.0f;
-        for (int c = 0; c < static_cast<int>(gridDim.x); c++) total += __ldcg(&g_sample_sum[c]);
-        unsigned long long rs0 = seed, rs1 = seed ^ 0xDEADBEEFCAFEBABEULL;
-        for (int w = 0; w < 4; w++) {  // three warm-up rounds and the draw
-            const unsigned long long t = rs0 ^ (rs0 << 23);
-            rs0 = rs1;
-            rs1 = t ^ rs1 ^ (t >> 17) ^ (rs1 >> 26);
-        }
-        const float r = static_cast<float>((rs0 + rs1) >> 11) * (1.0f / 9007199254740992.0f);
-        const float mass = top_p * total;
-        float cumul = 0.0f;
-        int nucleus = 0;
-        for (int c = 0; c < kSampleCands; c++) {
-            if (sp[c] <= 0.0f) break;
-            cumul += sp[c];
-            nucleus = c + 1;
-            if (cumul >= mass) break;
-        }
-        float nsum = 0.0f;
-        for (int c = 0; c < nucleus; c++) nsum += sp[c];
-        const float target = r * nsum;
+    sample_barrier();
+    float total = 0.0f;
+    for (int c = 0; c < static_cast<int>(gridDim.x); c++) total += ssum[c];
+    const float mass = top_p * total;
+    if (tid == 0) {  // the running sums, in order, as far as anyone will look
         float acc = 0.0f;
-        int sampled = si[0];
-        for (int c = 0; c < nucleus; c++) {
-            acc += sp[c];
-            if (acc >= target) {
-                sampled = si[c];
-                break;
+        int c = 0;
+        float4 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) x[u] = *reinterpret_cast<const float4 *>(sp + 4 * u);
+        while (c < kSampleCands && acc < mass && x[0].x > 0.0f) {
+            float4 y[4];  // the next sixteen are fetched while these are added
+            const int nx = min(c + 16, kSampleCands - 16);
+#pragma unroll
+            for (int u = 0; u < 4; u++) y[u] = *reinterpret_cast<const float4 *>(sp + nx + 4 * u);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                x[u].x = acc += x[u].x;
+                x[u].y = acc += x[u].y;
+                x[u].z = acc += x[u].z;
+                x[u].w = acc += x[u].w;
+                *reinterpret_cast<float4 *>(cum + c + 4 * u) = x[u];
+                x[u] = y[u];
             }
+            c += 16;
         }
-        *result = sampled;
-        g_sample_ticket = 0;
+        s_len = c;
     }
+    sample_barrier();
+    const int len = s_len;
+    // the nucleus ends after the first candidate that reaches the mass, or before the first of probability zero
+    for (int c = tid; c < len; c += 256) {
+        if (sp[c] <= 0.0f)
+            atomicMin(&s_nucleus, c);
+        else if (cum[c] >= mass)
+            atomicMin(&s_nucleus, c + 1);
+    }
+    if (tid == 0) atomicMin(&s_nucleus, len);  // everything before len was walked, nothing after it counts
+    sample_barrier();
+    const int nucleus = s_nucleus;
+    unsigned long long rs0 = seed, rs1 = seed ^ 0xDEADBEEFCAFEBABEULL;
+#pragma unroll
+    for (int w = 0; w < 4; w++) {  // three warm-up rounds and the draw
+        const unsigned long long t = rs0 ^ (rs0 << 23);
+        rs0 = rs1;
+        rs1 = t ^ rs1 ^ (t >> 17) ^ (rs1 >> 26);
+    }
+    const float r = static_cast<float>((rs0 + rs1) >> 11) * (1.0f / 9007199254740992.0f);
+    const float target = nucleus > 0 ? r * cum[nucleus - 1] : 0.0f;
+    for (int c = tid; c < nucleus; c += 256)
+        if (cum[c] >= target) {
+            atomicMin(&s_pick, c);
+            break;
+        }
+    sample_barrier();
+    const int pick = s_pick < nucleus ? s_pick : 0;
+#pragma unroll
+    for (int q = 0; q < kSampleKeep; q++)
+        if (tid * kSampleKeep + q == pick) *result = v[q] ? static_cast<int>(~static_cast<unsigned>(v[q])) : -1;
+    if (tid == 0) g_sample_ticket = 0;
 }
 
 // The best of the shards' (value, index) pairs, by the same order as above; writes the token and advances the position.
@@ -994,9 +1058,20 @@ float *sample_pair_addr()
     return addr[dev];
 }
 
+// The sampling kernel's shared-memory opt-in, once per device.
+void sample_attr()
+{
+    static bool done[kMaxDevices] = {false};
+    const int dev = current_device();
+    if (done[dev]) return;
+    cudaFuncSetAttribute(sample_top_p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmem);
+    done[dev] = true;
+}
+
 void support_init()
 {
     attn_attr();
+    sample_attr();
     (void)static_attn();
     (void)sample_pair_addr();
 }
@@ -1073,14 +1148,14 @@ void launch_embed_q4k(const void *table, float *out, const int *token_ptr, int t
 
 void launch_argmax(const float *logits, int n, int *result, int *pos_ptr, cudaStream_t stream)
 {
-    int ctas = (n + 2047) / 2048;  // eight logits per thread
+    int ctas = (n + 1023) / 1024;  // four logits per thread, up to the number of slots
     ctas = ctas < 1 ? 1 : (ctas > kArgmaxCtas ? kArgmaxCtas : ctas);
     launch_k(argmax_kernel, dim3(ctas), dim3(256), 0, stream, logits, n, result, pos_ptr, static_cast<float *>(nullptr), 0);
 }
 
 void launch_argmax_pair(const float *logits, int n, int index_offset, float *pair_out, cudaStream_t stream)
 {
-    int ctas = (n + 2047) / 2048;
+    int ctas = (n + 1023) / 1024;
     ctas = ctas < 1 ? 1 : (ctas > kArgmaxCtas ? kArgmaxCtas : ctas);
     launch_k(argmax_kernel, dim3(ctas), dim3(256), 0, stream, logits, n, static_cast<int *>(nullptr),
              static_cast<int *>(nullptr), pair_out, index_offset);
@@ -1227,7 +1302,8 @@ void cuda_sample_token(const float *logits, int vocab_size, float temperature, f
             return;
         }
         launch_argmax_pair(logits, vocab_size, 0, pair, stream);  // the maximum, for exp(l - max)
-        launch_k(sample_top_p_kernel, dim3(kSampleCtas), dim3(256), 0, stream, logits, vocab_size, temperature, top_p,
+        sample_attr();
+        launch_k(sample_top_p_kernel, dim3(kSampleCtas), dim3(kSampleThreads), kSampleSmem, stream, logits, vocab_size, temperature, top_p,
                  rng_state, d_result);
         MB200_CHECK_LAUNCH("cuda_sample_token");
         return;
