@@ -12,6 +12,7 @@ void q6k_init();
 void pair_init();
 void other_types_init();
 void gemm_init();
+void grouped_init();
 void moe_fused_init();
 void router_static_init();
 void support_init();
@@ -82,6 +83,7 @@ void cuda_kernels_init(void)
     pair_init();
     other_types_init();
     gemm_init();
+    grouped_init();
     moe_fused_init();
     support_init();
     attn_int8_init();

@@ -1,0 +1,113 @@
+// Weights -> pairs of fp16 (hi, lo) for the tensor cores, in packed fp16 arithmetic.
+//
+// A weight of a sub-block is w = s * n - b with n a small integer and s = d * scale, b = dmin * min of the sub-block
+// (Q6_K: w = s * (q - 32)). With a unit u, a power of two chosen per sub-block so that no |w| of it exceeds 2048 u,
+// s1 = s and b1 = b rounded to multiples of u make hi = s1 * n - b1 an integer multiple of u of at most 11 bits: one
+// HFMA2 computes it EXACTLY for two weights. lo = (s - s1) * n - (b - b1), the rest, is at most about 8 u and is rounded
+// to fp16 once: hi + lo is w to 2^-18 of the sub-block's largest weight or better. Two instructions per two weights
+// for both halves, where converting an fp32 weight, converting back, subtracting and converting the remainder took
+// ten (the producers of the grouped GEMM were issue-bound on exactly that).
+//
+// What is left is getting n out of the packed bits, on the integer pipe, which has half the FMA pipe's rate. A nibble shifted
+// to bits 6..9 of a 16-bit half and OR-ed with 0x4C00 is 16 + n: one shift and one LOP3 for two weights, no byte permute and
+// no subtraction, because the 16 goes into the addend exactly (16 s1 + b1 is a multiple of u below 2^11 u as well). The two
+// weights are then bytes 0 and 2 (1 and 3) of a word: inside every four columns the order is 0, 2, 1, 3, and the
+// activations are laid out the same way (k_order).
+#pragma once
+#include <cuda_fp16.h>
+
+#include "common.cuh"
+
+namespace mb200 {
+
+__device__ __forceinline__ uint32_t dup_half(float v)
+{
+    const __half2 h = __float2half2_rn(v);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+__device__ __forceinline__ uint32_t hadd2(uint32_t a, uint32_t b)
+{
+    const __half2 r = __hadd2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
+__device__ __forceinline__ uint32_t hmul2(uint32_t a, uint32_t b)
+{
+    const __half2 r = __hmul2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
+__device__ __forceinline__ uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c)
+{
+    const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b),
+                              *reinterpret_cast<const __half2 *>(&c));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
+// 1.5 * 2^23 * u with u = 2^(exponent of t - DROP): adding and subtracting it rounds to a multiple of u
+template <int DROP>
+__device__ __forceinline__ float round_magic(float t)
+{
+    return __uint_as_float((__float_as_uint(t) & 0x7F800000u) + (static_cast<uint32_t>(23 - DROP) << 23) + 0x00400000u);
+}
+
+// Position of column k in the operand layout: columns 1 and 2 of every four change places.
+__host__ __device__ constexpr int k_order(int k) { return (k & ~3) | ((k & 1) << 1) | ((k >> 1) & 1); }
+
+// d * v for an integer v of at most 23 bits: v in the mantissa of 2^23, one FMA (c = -2^23 d) instead of a conversion
+__device__ __forceinline__ float mul_small(float d, float c, uint32_t v) { return fmaf(d, __uint_as_float(0x4B000000u | v), c); }
+
+// One Q4_K sub-block's scale and min as the packed factors of hi and lo for operands 16 + n.
+struct SplitQ4 {
+    uint32_t s1, c1, rs, cr;
+    __device__ __forceinline__ void set(float s, float b)
+    {
+        const float M = round_magic<10>(fmaf(16.0f, fabsf(s), fabsf(b)));  // 16 |s| + |b| < 2^11 u
+        const float s1f = (s + M) - M, b1f = (b + M) - M, rsf = s - s1f;
+        s1 = dup_half(s1f);
+        rs = dup_half(rsf);
+        c1 = dup_half(fmaf(-16.0f, s1f, -b1f));
+        cr = dup_half(fmaf(-16.0f, rsf, b1f - b));
+    }
+};
+// 32 weights whose nibbles are the low (HIGH = false) or high nibbles of 8 words, two per register in k_order
+template <bool HIGH>
+__device__ __forceinline__ void split_q4(const uint32_t (&w)[8], const SplitQ4 &f, uint32_t (&hi)[16], uint32_t (&lo)[16])
+{
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t v0 = ((HIGH ? w[i] << 2 : w[i] << 6) & 0x03C003C0u) | 0x4C004C00u;
+        const uint32_t v1 = ((HIGH ? w[i] >> 6 : w[i] >> 2) & 0x03C003C0u) | 0x4C004C00u;
+        hi[2 * i] = hfma2(v0, f.s1, f.c1);
+        lo[2 * i] = hfma2(v0, f.rs, f.cr);
+        hi[2 * i + 1] = hfma2(v1, f.s1, f.c1);
+        lo[2 * i + 1] = hfma2(v1, f.rs, f.cr);
+    }
+}
+
+struct SplitQ6 {
+    uint32_t s1, rs;
+    __device__ __forceinline__ void set(float s)
+    {
+        const float M = round_magic<5>(fabsf(s));  // |s (q - 32)| <= 2^11 u
+        const float s1f = (s + M) - M;
+        s1 = dup_half(s1f);
+        rs = dup_half(s - s1f);
+    }
+};
+// 32 weights q - 32: q = the nibble of `l` at bit 4 (LHI = false: at bit 0) | two bits of `h` at bit HB, << 4, of each byte.
+// q goes to bits 4..9 of a half: 64 + q. The first 16 weights have scale f[0], the others f[1].
+template <bool LHI, int HB>
+__device__ __forceinline__ void split_q6(const uint32_t *l, const uint32_t *h, const SplitQ6 (&f)[2], uint32_t (&hi)[16],
+                                         uint32_t (&lo)[16])
+{
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t h0 = ((h[i] << (8 - HB)) & 0x03000300u) | 0x54005400u, h1 = ((h[i] >> HB) & 0x03000300u) | 0x54005400u;
+        const uint32_t q0 = ((LHI ? l[i] : l[i] << 4) & 0x00F000F0u) | h0, q1 = ((LHI ? l[i] >> 8 : l[i] >> 4) & 0x00F000F0u) | h1;
+        const uint32_t v0 = hadd2(q0, 0xD600D600u), v1 = hadd2(q1, 0xD600D600u);  // - 96
+        hi[2 * i] = hmul2(v0, f[i >> 2].s1);
+        lo[2 * i] = hmul2(v0, f[i >> 2].rs);
+        hi[2 * i + 1] = hmul2(v1, f[i >> 2].s1);
+        lo[2 * i + 1] = hmul2(v1, f[i >> 2].rs);
+    }
+}
+
+}  // namespace mb200

@@ -19,20 +19,25 @@
 //   * the 16 producer warps read the accumulator back with tcgen05.ld and store out[t][n]
 //     (coalesced over n).
 // 4-stage ring (48 KB per stage); every mbarrier wait is bounded; TMEM is always released.
-//
-// Split-precision variants (template parameter HL) for the grouped per-expert form, where two GEMMs are
-// chained and one fp16 rounding per operand per GEMM would add up to more than 1e-3 on some token rows:
-//   HL = 1: every weight is written as hi = fp16(w) and lo = fp16(w - hi), and the stage is multiplied
-//           twice into the same TMEM accumulator (D += A_hi B, D += A_lo B): weights carry ~22 bits;
-//   HL = 2: the activations come as hi and lo halves too (two TMA tiles): D += A_hi B_hi + A_lo B_hi + A_hi B_lo.
-// The tensor pipe has the time: the grouped form is bound by the weight stream.
-#include <cuda.h>
-
 #include <cstdio>
 
-#include "common.cuh"
+#include "tcgen.cuh"
 
 namespace mb200 {
+
+EncodeTiledFn encode_tiled()
+{
+    static EncodeTiledFn fn = nullptr;
+    if (!fn) {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<EncodeTiledFn>(p);
+    }
+    return fn;
+}
+
 namespace {
 
 constexpr int kBN = 128;   // weight rows per CTA (UMMA M)
@@ -54,100 +59,6 @@ struct Cfg {
     static constexpr uint32_t kIdesc =
         (1u << 4) | (static_cast<uint32_t>(BT >> 3) << 17) | (static_cast<uint32_t>(kBN >> 4) << 24);
 };
-
-// ---- tcgen05 / TMA wrappers ---------------------------------------------------
-__device__ __forceinline__ void tmem_alloc(uint32_t *dst_smem, uint32_t ncols)
-{
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(dst_smem)),
-                 "r"(ncols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols)
-{
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void proxy_fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                         uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        :
-        : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// A operand in tensor memory (128 lanes = rows, two fp16 per 32-bit column), B operand through a shared-memory descriptor.
-__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                            uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        :
-        : "r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// 32 consecutive 32-bit columns of this thread's TMEM lane (lane = 32 * (warp % 4) + lane id)
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32])
-{
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-        :
-        : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-          "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-          "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t *bar)
-{
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, "
-        "[%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tma_load_2d(void *dst_smem, const CUtensorMap *map, int x, int y, uint64_t *bar)
-{
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            smem_u32(dst_smem)),
-        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, rows of 128 bytes, 8-row
-// groups 1024 bytes apart (SBO); the tile base is 1024-byte aligned (base offset 0).
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr)
-{
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);  // start address, 16-byte units
-    d |= static_cast<uint64_t>(1) << 16;                  // leading-dimension offset: unused for swizzled K-major
-    d |= static_cast<uint64_t>(1024 >> 4) << 32;          // stride-dimension offset
-    d |= static_cast<uint64_t>(1) << 46;                  // descriptor version (sm_100)
-    d |= static_cast<uint64_t>(2) << 61;                  // SWIZZLE_128B
-    return d;
-}
 
 #ifdef MB200_TRACE
 __device__ long long g_gemm_trace[256];
@@ -273,7 +184,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
     constexpr int kATotal = C::kATotal, kBTotal = C::kBTotal;
     constexpr uint32_t kIdesc = C::kIdesc;
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    uint8_t *smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);  // not through an integer: stays a shared-memory pointer
     uint8_t *stage_base = smem;                                    // kStages x (A 16 KB | B 32 KB), 1024-byte aligned
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + kStages * kStageBytes);
     uint64_t *empty = full + kStages;
@@ -336,43 +247,28 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_const
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            int s = 0, ph = 0;
-            for (int kb = 0; kb < n_kb; kb++) {
-                if (!mbar_wait(&full[s], ph)) {
-                    *abort_flag = 1;
-                    break;
-                }
-                tc_fence_after();
-                if (kb >= 16 && kb < 24) GSTAMP(32 + (kb - 16) * 2);
-                if (kb == 0) GSTAMP(4);
-                if (kb == 8) GSTAMP(5);
-                if (kb == n_kb - 1) GSTAMP(6);
-                const uint32_t a_addr = smem_u32(stage_base + s * kStageBytes);
-                const uint64_t da = smem_desc_sw128(a_addr), db = smem_desc_sw128(a_addr + kATotal);
+        // ---------------- MMA issuer: the warp runs converged (tcgen.cuh) ----------------
+        const uint32_t leader = elect_lane(), tm = warp_uniform(tmem_base), s0 = warp_uniform(smem_u32(stage_base));
+        int s = 0, ph = 0;
+        for (int kb = 0; kb < n_kb; kb++) {
+            if (!mbar_wait(&full[s], ph)) *abort_flag = 1;
+            if (__any_sync(0xffffffffu, *abort_flag)) break;
+            tc_fence_after();
+            const uint32_t a_addr = s0 + s * kStageBytes;
+            const uint64_t da = smem_desc_sw128(a_addr), db = smem_desc_sw128(a_addr + kATotal);
+            if (leader) {
 #pragma unroll
                 for (int kk = 0; kk < kBK / 16; kk++)  // 16 fp16 = 32 bytes = 2 descriptor units per K step
-                    umma_f16(tmem_base, da + 2 * kk, db + 2 * kk, kIdesc, (kb | kk) != 0);
-                if (HL) {  // the lo halves of the weights against the same activations
-                    const uint64_t dal = smem_desc_sw128(a_addr + kABytes);
-#pragma unroll
-                    for (int kk = 0; kk < kBK / 16; kk++) umma_f16(tmem_base, dal + 2 * kk, db + 2 * kk, kIdesc, 1u);
-                }
-                if (HL == 2) {  // the hi halves of the weights against the lo halves of the activations
-                    const uint64_t dbl = smem_desc_sw128(a_addr + kATotal + kBBytes);
-#pragma unroll
-                    for (int kk = 0; kk < kBK / 16; kk++) umma_f16(tmem_base, da + 2 * kk, dbl + 2 * kk, kIdesc, 1u);
-                }
+                    umma_f16(tm, da + 2 * kk, db + 2 * kk, kIdesc, (kb | kk) != 0);
                 umma_commit(&empty[s]);  // the stage may be refilled once these MMAs have read it
-                if (kb >= 16 && kb < 24) GSTAMP(33 + (kb - 16) * 2);
-                if (++s == kStages) {
-                    s = 0;
-                    ph ^= 1;
-                }
             }
-            umma_commit(acc_full);  // all MMAs done: the accumulator is complete
+            __syncwarp();
+            if (++s == kStages) {
+                s = 0;
+                ph ^= 1;
+            }
         }
+        if (leader) umma_commit(acc_full);  // all MMAs done: the accumulator is complete
     } else {
         // ---------------- dequant producers: weights -> fp16, swizzled K-major ----------------
         const int dt = tid - 64;        // 0..511
@@ -497,7 +393,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_atm_kernel(const __grid_c
                                                                  const __grid_constant__ GemmParams P)
 {
     extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    uint8_t *smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);  // not through an integer: stays a shared-memory pointer
     // one ring: stage s holds the weights of a chunk in TMEM and its activations in shared memory
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + kAtmBStages * kAtmBBytes);
     uint64_t *empty = full + kAtmBStages;
@@ -542,29 +438,30 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_atm_kernel(const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {  // ---- MMA issuer ----
-            int s = 0, ph = 0;
-            for (int kb = 0; kb < n_kb; kb++) {
-                if (!mbar_wait(&full[s], ph)) {
-                    *abort_flag = 1;
-                    break;
-                }
-                tc_fence_after();
-                const uint64_t db = smem_desc_sw128(smem_u32(smem + s * kAtmBBytes));
-                const uint32_t ta = tmem_a0 + s * (kAtmSlabs * kAtmACols);
+        // ---- MMA issuer: the warp runs converged (tcgen.cuh) ----
+        const uint32_t leader = elect_lane(), tm = warp_uniform(tmem_base), b0 = warp_uniform(smem_u32(smem));
+        int s = 0, ph = 0;
+        for (int kb = 0; kb < n_kb; kb++) {
+            if (!mbar_wait(&full[s], ph)) *abort_flag = 1;
+            if (__any_sync(0xffffffffu, *abort_flag)) break;
+            tc_fence_after();
+            const uint64_t db = smem_desc_sw128(b0 + s * kAtmBBytes);
+            const uint32_t ta = tm + kAtmAccCols + s * (kAtmSlabs * kAtmACols);
+            if (leader) {
 #pragma unroll
                 for (int kk = 0; kk < kBK / 16; kk++)  // 16 fp16 of K = 8 operand columns = 2 descriptor units
 #pragma unroll
                     for (int sl = 0; sl < kAtmSlabs; sl++)
-                        umma_f16_ta(tmem_base + sl * kAtmBT, ta + sl * kAtmACols + 8 * kk, db + 2 * kk, kAtmIdesc, (kb | kk) != 0);
+                        umma_f16_ta(tm + sl * kAtmBT, ta + sl * kAtmACols + 8 * kk, db + 2 * kk, kAtmIdesc, (kb | kk) != 0);
                 umma_commit(&empty[s]);
-                if (++s == kAtmBStages) {
-                    s = 0;
-                    ph ^= 1;
-                }
             }
-            umma_commit(acc_full);
+            __syncwarp();
+            if (++s == kAtmBStages) {
+                s = 0;
+                ph ^= 1;
+            }
         }
+        if (leader) umma_commit(acc_full);
     } else {
         // ---- producers: lane quarter q = warp % 4 (a warp may only touch TMEM lanes 32 q ..), idx = (warp - 2) / 4,
         // slab = idx % slabs, group par = idx / slabs: the thread owns row 128 slab + 32 q + lane of the tile and
@@ -634,6 +531,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_atm_kernel(const __grid_c
                 }
                 tc_fence_after();  // the MMAs that read this stage are complete: the overwrite is ordered after them
                 tmem_st32(tmem_a0 + lane_addr + (s * kAtmSlabs + slab) * kAtmACols, pk);
+                tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&full[s]);
@@ -666,23 +564,6 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_atm_kernel(const __grid_c
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem_base, kAtmTmemCols);
     if (tid == 0 && *abort_flag) atomicExch(P.err, MB200_ERR_TIMEOUT);
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled()
-{
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    }
-    return fn;
 }
 
 // X: fp16 [rows_x][K] row-major. Launches gemm_tc_kernel<BT> over grid (weight tiles [x experts], token tiles).
@@ -770,162 +651,6 @@ int launch_gemm(const void *w, const void *x_f16, float *out, int M, int N, int 
     return launch_gemm_bt<256>(P, x_f16, M, dim3((N + kBN - 1) / kBN, (M + 255) / 256), stream, where);
 }
 
-// ---- grouped per-expert form: the MoE block for a batch of tokens (prefill) ----------------------
-// Routed (token, slot) pairs are sorted by expert; each expert's tokens then form a contiguous
-// slice of the gathered activations and one grouped launch runs every expert's GEMM on its slice.
-constexpr int kGroupBT = 64;
-
-struct SortOut {
-    int *cnt, *off, *row_of_pair, *pair_of_row;
-};
-
-// One block of 1024 threads, deterministic layout: the rows of an expert hold its pairs in pair order.
-// Pairs with id < 0 (empty slots) or id >= n_experts get row -1.
-// Counts: a shared-memory histogram (the order of the additions does not matter). Placement: the pairs are taken
-// 1024 at a time, one per thread; within a warp a pair's rank among the pairs of the same expert comes from
-// __match_any_sync, and the warps add their counts to the expert's running total one after the other, so a pair's
-// row is offset + (pairs of that expert in earlier chunks and earlier warps) + rank. (Up to 256 experts the warps
-// post their counts in a table instead of taking turns.)
-__global__ void moe_sort_kernel(const int *__restrict__ ids, int n_pairs, int n_experts, int cap, SortOut o, int *err)
-{
-    __shared__ int s_off[1025];
-    __shared__ int s_run[1024];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int e = tid; e < 1024; e += blockDim.x) s_run[e] = 0;
-    __syncthreads();
-    for (int p = tid; p < n_pairs; p += blockDim.x) {
-        const int id = ids[p];
-        if (id >= 0 && id < n_experts) atomicAdd(&s_run[id], 1);
-    }
-    __syncthreads();
-    if (tid < n_experts) {
-        const int c = s_run[tid];
-        o.cnt[tid] = c;
-        s_off[tid + 1] = c;
-        if (c > cap) atomicExch(err, MB200_ERR_UNSUPPORTED);  // more tokens on one expert than the launch was sized for
-    }
-    if (tid == 0) s_off[0] = 0;
-    __syncthreads();
-    if (tid == 0)
-        for (int i = 0; i < n_experts; i++) s_off[i + 1] += s_off[i];
-    __syncthreads();
-    if (tid < n_experts) o.off[tid] = s_off[tid];
-    if (tid == 0) o.off[n_experts] = s_off[n_experts];
-    for (int e = tid; e < 1024; e += blockDim.x) s_run[e] = 0;
-    __syncthreads();
-    const int n_warps = blockDim.x >> 5;
-    constexpr int kTabExperts = 256;
-    __shared__ int s_tab[32][kTabExperts];  // up to 256 experts: pairs of expert e seen by warp w in the current chunk
-    const bool tabbed = n_experts <= kTabExperts;
-    for (int p0 = 0; p0 < n_pairs; p0 += blockDim.x) {
-        const int p = p0 + tid;
-        const int id = p < n_pairs ? ids[p] : -1;
-        const bool valid = id >= 0 && id < n_experts;
-        // lanes with the same expert (invalid pairs form a group of their own that is not counted)
-        const unsigned same = __match_any_sync(0xffffffffu, valid ? id : -1);
-        const int rank = __popc(same & ((1u << lane) - 1u));
-        int base = 0;
-        if (tabbed) {
-            // three barriers per chunk: every warp posts its counts, every pair adds up the warps before its own
-            for (int i = tid; i < 32 * n_experts; i += blockDim.x) s_tab[i / n_experts][i % n_experts] = 0;
-            __syncthreads();
-            if (valid && rank == 0) s_tab[warp][id] = __popc(same);
-            __syncthreads();
-            if (valid) {
-                base = s_run[id];
-                for (int w = 0; w < warp; w++) base += s_tab[w][id];
-            }
-            __syncthreads();
-            if (valid && rank == 0) atomicAdd(&s_run[id], __popc(same));  // integer adds: the order does not matter
-        } else {
-            for (int w = 0; w < n_warps; w++) {  // the warps take turns
-                if (warp == w && valid) {
-                    base = s_run[id];
-                    __syncwarp(same);
-                    if (rank == 0) s_run[id] = base + __popc(same);
-                }
-                __syncthreads();
-            }
-        }
-        if (p < n_pairs) {
-            if (valid) {
-                const int r = s_off[id] + base + rank;
-                o.row_of_pair[p] = r;
-                o.pair_of_row[r] = p;
-            } else {
-                o.row_of_pair[p] = -1;
-            }
-        }
-    }
-}
-
-// Xs[row] = X[token of the pair in that row]; one block per row, 16-byte copies
-__global__ void moe_gather_kernel(const uint4 *__restrict__ x, uint4 *__restrict__ xs, const int *__restrict__ pair_of_row,
-                                  const int *__restrict__ off, int n_experts, int k, int vec_per_row)
-{
-    const int row = blockIdx.x;
-    if (row >= off[n_experts]) return;
-    const int t = pair_of_row[row] / k;
-    for (int i = threadIdx.x; i < vec_per_row; i += blockDim.x) xs[(size_t)row * vec_per_row + i] = x[(size_t)t * vec_per_row + i];
-}
-
-// act16[row][j] = fp16(silu(gate) * up * 2^-4): the 2^-4 keeps SwiGLU outputs inside fp16's range
-// (they reach ~2.5e4 with the benchmark's weights); the combine step multiplies it back exactly.
-constexpr float kActScale = 1.0f / 16.0f;
-// The activation keeps ~22 bits as two fp16 arrays: act_hi = fp16(a), act_lo = fp16(a - act_hi).
-__global__ void moe_swiglu_rows_kernel(const float *__restrict__ gu, __half *__restrict__ act_hi,
-                                       __half *__restrict__ act_lo, const int *__restrict__ off, int n_experts, int EFF)
-{
-    const int row = blockIdx.x;
-    if (row >= off[n_experts]) return;
-    const float *g = gu + (size_t)row * 2 * EFF;
-    for (int j = threadIdx.x; j < EFF; j += blockDim.x) {
-        const float gv = g[j];
-        const float a = gv / (1.0f + expf(-gv)) * g[EFF + j] * kActScale;
-        const __half hi = __float2half_rn(a);
-        act_hi[(size_t)row * EFF + j] = hi;
-        act_lo[(size_t)row * EFF + j] = __float2half_rn(a - __half2float(hi));
-    }
-}
-
-// y[t] = (residual ? residual[t] : 0) + sum over slots, in slot order, of w * down-output of that pair
-__global__ void moe_combine_kernel(const float *__restrict__ dn, const int *__restrict__ row_of_pair,
-                                   const float *__restrict__ wts, const float *__restrict__ residual,
-                                   float *__restrict__ y, int k, int H)
-{
-    const int t = blockIdx.x;
-    for (int j = threadIdx.x; j < H; j += blockDim.x) {
-        float acc = 0.0f;
-        for (int s = 0; s < k; s++) {
-            const int row = row_of_pair[t * k + s];
-            if (row >= 0) acc = fmaf(wts[t * k + s] * (1.0f / kActScale), dn[(size_t)row * H + j], acc);
-        }
-        y[(size_t)t * H + j] = (residual ? residual[(size_t)t * H + j] : 0.0f) + acc;
-    }
-}
-
-inline size_t align_up(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
-
-struct Workspace {
-    size_t cnt, off, row_of_pair, pair_of_row, xs, gu, act, dn, total;
-};
-Workspace workspace_layout(int M, int k, int H, int EFF, int n_experts)
-{
-    const size_t P = (size_t)M * k;
-    Workspace w;
-    size_t o = 0;
-    w.cnt = o;          o = align_up(o + sizeof(int) * n_experts);
-    w.off = o;          o = align_up(o + sizeof(int) * (n_experts + 1));
-    w.row_of_pair = o;  o = align_up(o + sizeof(int) * P);
-    w.pair_of_row = o;  o = align_up(o + sizeof(int) * P);
-    w.xs = o;           o = align_up(o + 2 * P * H);
-    w.gu = o;           o = align_up(o + 4 * P * 2 * EFF);
-    w.act = o;          o = align_up(o + 2 * 2 * P * EFF);  // hi halves [P][EFF], then lo halves [P][EFF]
-    w.dn = o;           o = align_up(o + 4 * P * H);
-    w.total = o;
-    return w;
-}
-
 }  // namespace
 
 void gemm_init()
@@ -950,78 +675,6 @@ int mb200_gemm_q4k_f16(const void *w, const void *x_f16, float *out, int M, int 
 int mb200_gemm_q6k_f16(const void *w, const void *x_f16, float *out, int M, int N, int K, cudaStream_t stream)
 {
     return launch_gemm(w, x_f16, out, M, N, K, 1, stream, "mb200_gemm_q6k_f16");
-}
-
-size_t mb200_moe_prefill_workspace_bytes(int M, int k, int H, int EFF, int n_experts)
-{
-    if (M < 1 || k < 1 || H < 1 || EFF < 1 || n_experts < 1) return 0;
-    return workspace_layout(M, k, H, EFF, n_experts).total;
-}
-
-int mb200_moe_prefill(const void *experts, size_t expert_stride, size_t gate_sz, size_t up_sz, int down_type,
-                      int n_experts, int k, int H, int EFF, const void *x_f16, const int *ids, const float *wts,
-                      const float *residual, float *y, int M, int max_tokens_per_expert, void *workspace,
-                      cudaStream_t stream)
-{
-    const char *where = "mb200_moe_prefill";
-    if (!experts || !x_f16 || !ids || !wts || !y || !workspace || M < 1 || k < 1 || k > 16 || n_experts < 1 ||
-        n_experts > 1024)
-        return MB200_ERR_ARG;
-    if (H % 256 != 0 || EFF % 256 != 0 || (down_type != 12 && down_type != 14)) return MB200_ERR_UNSUPPORTED;
-    if ((reinterpret_cast<uintptr_t>(experts) & 15) || (expert_stride & 15) || (gate_sz & 15) ||
-        (reinterpret_cast<uintptr_t>(x_f16) & 15) || (reinterpret_cast<uintptr_t>(workspace) & 255))
-        return MB200_ERR_ARG;
-    if (gate_sz != up_sz || gate_sz != (size_t)EFF * (H / 256) * kQ4KBlock) return MB200_ERR_ARG;
-    const int P = M * k;
-    const int cap = (max_tokens_per_expert > 0 && max_tokens_per_expert < M) ? max_tokens_per_expert : M;
-    const Workspace L = workspace_layout(M, k, H, EFF, n_experts);
-    uint8_t *ws = static_cast<uint8_t *>(workspace);
-    SortOut so{reinterpret_cast<int *>(ws + L.cnt), reinterpret_cast<int *>(ws + L.off),
-               reinterpret_cast<int *>(ws + L.row_of_pair), reinterpret_cast<int *>(ws + L.pair_of_row)};
-    __half *xs = reinterpret_cast<__half *>(ws + L.xs);
-    float *gu = reinterpret_cast<float *>(ws + L.gu);
-    __half *act = reinterpret_cast<__half *>(ws + L.act);
-    float *dn = reinterpret_cast<float *>(ws + L.dn);
-
-    moe_sort_kernel<<<1, 1024, 0, stream>>>(ids, P, n_experts, cap, so, device_error_word());
-    moe_gather_kernel<<<P, 128, 0, stream>>>(static_cast<const uint4 *>(x_f16), reinterpret_cast<uint4 *>(xs),
-                                             so.pair_of_row, so.off, n_experts, k, H / 8);
-    const int token_tiles = (cap + kGroupBT - 1) / kGroupBT;
-
-    GemmParams G{};  // gate and up are adjacent Q4_K matrices of a blob: one [2*EFF x H] matrix
-    G.w = static_cast<const uint8_t *>(experts);
-    G.out = gu;
-    G.M = P;
-    G.N = 2 * EFF;
-    G.K = H;
-    G.q6 = 0;
-    G.seg_off = so.off;
-    G.seg_cnt = so.cnt;
-    G.tiles_per_expert = (2 * EFF + kBN - 1) / kBN;
-    G.expert_stride = expert_stride;
-    // weights as hi + lo fp16 (x is fp16 already): the gate / up values keep fp32 accuracy
-    int rc = launch_gemm_bt<kGroupBT, 1>(G, xs, P, dim3(n_experts * G.tiles_per_expert, token_tiles), stream, where);
-    if (rc != MB200_OK) return rc;
-
-    moe_swiglu_rows_kernel<<<P, 256, 0, stream>>>(gu, act, act + (size_t)P * EFF, so.off, n_experts, EFF);
-
-    GemmParams D{};
-    D.w = static_cast<const uint8_t *>(experts) + gate_sz + up_sz;
-    D.out = dn;
-    D.M = P;
-    D.N = H;
-    D.K = EFF;
-    D.q6 = down_type == 14;
-    D.seg_off = so.off;
-    D.seg_cnt = so.cnt;
-    D.tiles_per_expert = (H + kBN - 1) / kBN;
-    D.expert_stride = expert_stride;
-    D.x_lo_row0 = P;  // the tensor map covers [2 P][EFF]: hi rows, then lo rows
-    rc = launch_gemm_bt<kGroupBT, 2>(D, act, 2 * P, dim3(n_experts * D.tiles_per_expert, token_tiles), stream, where);
-    if (rc != MB200_OK) return rc;
-
-    moe_combine_kernel<<<M, 256, 0, stream>>>(dn, so.row_of_pair, wts, residual, y, k, H);
-    return cudaGetLastError() == cudaSuccess ? MB200_OK : MB200_ERR_LAUNCH;
 }
 
 }  // extern "C"
