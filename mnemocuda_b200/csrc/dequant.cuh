@@ -110,4 +110,50 @@ __device__ __forceinline__ void split_q6(const uint32_t *l, const uint32_t *h, c
     }
 }
 
+// ---- Q6_K blocks in shared memory ----
+// A block is 210 bytes at a 2-byte alignment: no tensor map fits it and 16-byte copies would have to carry up to 14 bytes of
+// skew. A warp copies the 53 aligned words that hold it (two words per lane; the last word's spare bytes share it with valid
+// ones); a row's thread then reads its words, which start 0 or 2 bytes into the first (`skew`).
+__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src)  // 4 bytes, shared <- global, both 4-byte aligned
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_arrive(uint64_t *bar)  // one arrival when this thread's copies so far have landed
+{
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void copy_q6k_row(uint32_t dst_lane, const uint8_t *blk, int lane)  // dst_lane: the row's slot + 4 lane
+{
+    const uint8_t *a = reinterpret_cast<const uint8_t *>(reinterpret_cast<uintptr_t>(blk) & ~static_cast<uintptr_t>(3)) + 4 * lane;
+    cp_async4(dst_lane, a);
+    if (lane < 53 - 32) cp_async4(dst_lane + 128, a + 128);
+}
+struct RawQ6 {  // half a block: 128 weights
+    uint32_t ql[16], qh[8], sc[2];
+    float d;
+    __device__ __forceinline__ void load(const uint8_t *row, uint32_t skew, int half)
+    {
+        const uint32_t sel = skew ? 0x5432u : 0x3210u;
+        const uint32_t *wp = reinterpret_cast<const uint32_t *>(row);
+        uint32_t prev = wp[16 * half];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const uint32_t nx = wp[16 * half + i + 1];
+            ql[i] = __byte_perm(prev, nx, sel);
+            prev = nx;
+        }
+        prev = wp[32 + 8 * half];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const uint32_t nx = wp[32 + 8 * half + i + 1];
+            qh[i] = __byte_perm(prev, nx, sel);
+            prev = nx;
+        }
+        const uint32_t a = wp[48 + 2 * half], b = wp[49 + 2 * half], c = wp[50 + 2 * half];
+        sc[0] = __byte_perm(a, b, sel);
+        sc[1] = __byte_perm(b, c, sel);
+        d = __half2float(__ushort_as_half(static_cast<unsigned short>(skew ? wp[52] >> 16 : wp[52])));
+    }
+};
+
 }  // namespace mb200

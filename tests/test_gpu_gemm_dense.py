@@ -1,0 +1,46 @@
+"""The dense GEMM in each of its forms -- K split over a cluster, 64 / 128 / 256-token tiles, two CTAs on one tile -- at sizes
+around their edges: rows past the last tile, an odd number of row tiles, K of one block and of a count the splits do not divide,
+Q6_K tensors on an odd 2-byte address. Every token row against the C oracle."""
+import numpy as np
+import pytest
+import torch
+
+from mnemocuda_b200 import synth
+from oracle import oracle
+from tests.gpu_util import dev, host
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def K():
+    from mnemocuda_b200 import kernels
+    kernels.mb200_init()
+    return kernels
+
+
+@pytest.mark.parametrize("kind", ["q4k", "q6k"])
+@pytest.mark.parametrize("M,N,Kd", [(1, 1, 256), (9, 130, 2816), (65, 257, 4352), (63, 128, 8192), (100, 1377, 2048),
+                                    (129, 2050, 512), (257, 8100, 256), (511, 8191, 768), (770, 5121, 256)])
+def test_every_form(K, kind, M, N, Kd):
+    gen, ref, call = ((synth.q4k_matrix, oracle.gemm_q4k_f16, K.mb200_gemm_q4k_f16) if kind == "q4k" else
+                      (synth.q6k_matrix, oracle.gemm_q6k_f16, K.mb200_gemm_q6k_f16))
+    w = gen(2700 + N, N, Kd)
+    x = synth.normal_f16(2701 + M, M * Kd).reshape(M, Kd)
+    want = ref(w, x, M, N, Kd).astype(np.float64)
+    pad = 2 if kind == "q6k" else 16
+    buf = torch.zeros(w.size + 32, dtype=torch.uint8, device="cuda")
+    d_w = buf[pad:pad + w.size]
+    d_w.copy_(dev(w))
+    guard = torch.full((M * N + 64,), 7.0, device="cuda")
+    out = guard[:M * N].view(M, N)
+    for pdl in (False, True):
+        before = K.mb200_set_pdl(pdl)
+        out.fill_(float("nan"))
+        call(d_w, dev(x), out, M, N, Kd)
+        got = host(out).astype(np.float64)
+        K.mb200_set_pdl(before)
+        rel = np.linalg.norm(got - want, axis=1) / np.maximum(np.linalg.norm(want, axis=1), 1e-30)
+        assert rel.max() <= 1e-3, (pdl, rel.max())
+    assert bool((guard[M * N:] == 7.0).all())
+    assert K.mb200_device_error() == 0
