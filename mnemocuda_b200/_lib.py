@@ -11,6 +11,7 @@ import re
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libmnemo_b200.so")
+NATIVE_PATH = os.path.join(_HERE, "_native.so")  # the compiled binding over it
 HEADER_PATH = os.path.join(_HERE, "..", "include", "mnemo_b200.h")
 
 _vp, _i, _f, _sz, _u64 = C.c_void_p, C.c_int, C.c_float, C.c_size_t, C.c_uint64
@@ -133,3 +134,18 @@ def lib() -> C.CDLL:
         fn.argtypes = args
     _lib = handle
     return _lib
+
+
+class _NotBuilt:
+    """Stands in for the binding in a tree that has not been built: importing works, calling says what is missing."""
+
+    def __getattr__(self, name):
+        raise ImportError(f"{NATIVE_PATH} is missing: build it with `python -m mnemocuda_b200.build`. "
+                          "There is no CPU or PyTorch fallback for these kernels.")
+
+
+def native():
+    if not (os.path.exists(NATIVE_PATH) and os.path.exists(LIB_PATH)):
+        return _NotBuilt()
+    from . import _native
+    return _native

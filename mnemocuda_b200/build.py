@@ -6,12 +6,16 @@ from __future__ import annotations
 
 import glob
 import os
+import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libmnemo_b200.so")
+NATIVE = os.path.join(HERE, "_native.so")  # Python binding of the library (csrc/binding.cpp)
+BINDING = os.path.join(CSRC, "binding.cpp")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -26,7 +30,9 @@ def sources() -> list[str]:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(NATIVE):
+        return True
+    if os.path.getmtime(BINDING) > os.path.getmtime(NATIVE):
         return True
     t = os.path.getmtime(LIB)
     deps = sources() + glob.glob(os.path.join(CSRC, "*.cuh")) + [
@@ -59,6 +65,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
         objs = list(pool.map(compile_one, sources()))
     subprocess.check_call([nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", LIB, *objs, "-lcudart"],
                           env=env)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(nvcc) or "/usr/local/cuda/bin/nvcc")))
+    subprocess.check_call([os.environ.get("HOST_CXX", "g++"), "-O2", "-std=c++20", "-fPIC", "-shared",
+                           "-I" + os.path.join(cuda, "include"), "-I" + sysconfig.get_paths()["include"], BINDING, "-o", NATIVE,
+                           "-L" + HERE, "-l:libmnemo_b200.so", "-L" + os.path.join(cuda, "lib64"), "-lcudart",
+                           "-Wl,-rpath,$ORIGIN"], env=env)  # found beside the library, wherever the tree lies
     return LIB
 
 
