@@ -683,3 +683,6 @@ __device__ __noinline__ void merge_head(int b, int hq, int nc, int chunks, const
     cta_sync();
 }
 
+}  // namespace
+}  // namespace persist
+}  // namespace mb200
