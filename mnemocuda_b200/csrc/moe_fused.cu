@@ -304,15 +304,8 @@ __device__ __forceinline__ void split_store(const float4 t, int c0, int lane, in
     if (F::kSumCols == 16) sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     const float sc = amax * (1.0f / 127.0f);
     const float inv = amax > 0.0f ? 127.0f / amax : 0.0f;
-    uint32_t p1 = 0, p2 = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float a = rintf(v[i] * inv);
-        const float r = fmaf(-a, sc, v[i]);
-        const float b = fminf(fmaxf(rintf(r * inv * 254.0f), -127.0f), 127.0f);
-        p1 |= (static_cast<uint32_t>(__float2int_rn(a)) & 0xFFu) << (8 * i);
-        p2 |= (static_cast<uint32_t>(__float2int_rn(b)) & 0xFFu) << (8 * i);
-    }
+    uint32_t p1, p2;
+    stream::split_levels(v, sc, inv, p1, p2);
     const int idx = F::xword(c0) * pitch + F::xslot(c0);
     q1[idx] = p1;
     q2[idx] = p2;
