@@ -447,6 +447,9 @@ int mb200_decode_begin(const mb200_decode_model *m, void *workspace, const int *
                        cudaStream_t stream);
 int mb200_decode_layer(const mb200_decode_model *m, int layer, void *workspace, const int *d_pos,
                        cudaStream_t stream);
+/* Layers first .. first + count - 1, one kernel launch for all of them where the shape allows it. */
+int mb200_decode_layers(const mb200_decode_model *m, int first, int count, void *workspace, const int *d_pos,
+                        cudaStream_t stream);
 int mb200_decode_finish(const mb200_decode_model *m, void *workspace, float *d_logits, int *d_token, int *d_pos,
                         cudaStream_t stream);
 /* The layer in three pieces for a model sharded over devices (this replaces the reference's layer-range split,

@@ -85,6 +85,7 @@ SIGNATURES = {
     "mb200_decode_step": (_i, [_vp, _vp, _vp, _vp, _vp, _vp]),
     "mb200_decode_begin": (_i, [_vp, _vp, _vp, _vp, _vp]),
     "mb200_decode_layer": (_i, [_vp, _i, _vp, _vp, _vp]),
+    "mb200_decode_layers": (_i, [_vp, _i, _i, _vp, _vp, _vp]),
     "mb200_decode_finish": (_i, [_vp, _vp, _vp, _vp, _vp, _vp]),
     "mb200_comm_buffer_bytes": (_sz, [_i, _sz]),
     "mb200_comm_alloc": (_i, [_i, _sz, _vp, _vp]),

@@ -16,6 +16,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "persist.cuh"
 #include "support.cuh"
 
 namespace mb200 {
@@ -23,14 +24,31 @@ void qkv_q4k_q6k(const void *wq, float *q, int q_rows, const void *wk, float *k,
                  const float *x, int n_cols, const float *norm_w, float norm_eps, cudaStream_t stream, const char *where);
 void q4k_matvec2(const void *wa, float *ya, int rows_a, const void *wb, float *yb, int rows_b, const float *x,
                  int n_cols, cudaStream_t stream, const char *where, const float *norm_w, float norm_eps);
+int moe_fused_mode();
 
 namespace {
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 struct Workspace {
-    size_t hidden, normed, q, k, v, attn, rope, ids, wts, act, scratch, attn_ws, zero, total;
+    size_t hidden, normed, q, k, v, attn, rope, ids, wts, act, scratch, attn_ws, zero, persist, total;
 };
+
+// The model's shape for the persistent kernel
+void persist_shape(const mb200_decode_model &m, persist::Params &P)
+{
+    P.H = m.hidden;
+    P.EFF = m.moe_inter;
+    P.QD = m.n_heads * m.head_dim;
+    P.KD = m.n_kv_heads * m.head_dim;
+    P.n_heads = m.n_heads;
+    P.n_kv = m.n_kv_heads;
+    P.gqa = m.n_heads / m.n_kv_heads;
+    P.n_experts = m.n_experts;
+    P.k = m.top_k;
+    P.eps = m.rms_eps;
+    P.scale = 1.0f / sqrtf(static_cast<float>(m.head_dim));
+}
 
 Workspace layout(const mb200_decode_model &m)
 {
@@ -45,6 +63,11 @@ Workspace layout(const mb200_decode_model &m)
     // counters first: the caller zeroes the workspace once, these must start at zero
     w.scratch = take(mb200_router_scratch_bytes(m.n_experts));
     w.attn_ws = take(attn_workspace_bytes(m.n_kv_heads, m.n_heads / (m.n_kv_heads > 0 ? m.n_kv_heads : 1)));
+    {
+        static thread_local persist::Params P;
+        persist_shape(m, P);
+        w.persist = take(persist::scratch(P, nullptr));
+    }
     w.zero = take(H * 4);  // stays zero: the "residual" of a rank that must not add one
     w.hidden = take(H * 4);
     w.normed = take(H * 4);
@@ -195,6 +218,77 @@ int run_layer(const mb200_decode_model &m, const mb200_layer_weights &L, uint8_t
     return run_moe(m, L, ws, W, true, B.hidden, s);
 }
 
+// Layers [first, first + count) in one launch; MB200_ERR_UNSUPPORTED (nothing ran) for what the persistent kernel does not cover:
+// sharded models, other weight types or alignments, shapes outside its plan.
+int run_persist(const mb200_decode_model &m, int first, int count, uint8_t *ws, const Workspace &W, const int *d_pos, cudaStream_t s)
+{
+    if (moe_fused_mode() != 2 || m.n_heads_total > 0 || m.o_rows > 0 || m.expert_lo != 0 ||
+        (m.expert_cnt > 0 && m.expert_cnt < m.n_experts) || count > persist::kMaxLayers)
+        return MB200_ERR_UNSUPPORTED;
+    static thread_local persist::Params P;  // too big for a stack
+    auto ok16 = [](const void *p) { return p && (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    for (int l = 0; l < count; l++) {
+        const mb200_layer_weights &L = m.layers[first + l];
+        const bool own = L.expert_stride != 0;
+        const size_t stride = own ? L.expert_stride : m.expert_stride, gate = own ? L.gate_sz : m.gate_sz, up = own ? L.up_sz : m.up_sz;
+        const int down = own ? L.down_type : m.down_type;
+        if (L.wq_type != 12 || L.wk_type != 12 || L.wo_type != 12 || (L.wv_type != 12 && L.wv_type != 14) || (down != 12 && down != 14))
+            return MB200_ERR_UNSUPPORTED;
+        if (!ok16(L.wq) || !ok16(L.wk) || !L.wv || !ok16(L.wo) || !ok16(L.experts) || !ok16(L.router) || !ok16(L.attn_norm) ||
+            !ok16(L.ffn_norm) || !ok16(L.kv_k) || !ok16(L.kv_v))
+            return MB200_ERR_UNSUPPORTED;
+        if ((L.wv_type == 12 && !ok16(L.wv)) || (reinterpret_cast<uintptr_t>(L.wv) & 1) || (stride & 15) || (gate & 15) ||
+            ((gate + up) & (down == 12 ? 15 : 1)) || gate > 0x7fffffff || gate + up > 0x7fffffff)
+            return MB200_ERR_UNSUPPORTED;
+        persist::Layer &D = P.L[l];
+        D.attn_norm = L.attn_norm;
+        D.q_norm = L.q_norm;
+        D.k_norm = L.k_norm;
+        D.ffn_norm = L.ffn_norm;
+        D.router = L.router;
+        D.wq = static_cast<const uint8_t *>(L.wq);
+        D.wk = static_cast<const uint8_t *>(L.wk);
+        D.wv = static_cast<const uint8_t *>(L.wv);
+        D.wo = static_cast<const uint8_t *>(L.wo);
+        D.experts = static_cast<const uint8_t *>(L.experts);
+        D.kv_k = static_cast<__half *>(L.kv_k);
+        D.kv_v = static_cast<__half *>(L.kv_v);
+        D.estride = stride;
+        D.up_off = static_cast<uint32_t>(gate);
+        D.down_off = static_cast<uint32_t>(gate + up);
+        D.v_q6 = L.wv_type == 14;
+        D.down_q6 = down == 14;
+    }
+    persist_shape(m, P);
+    persist::scratch(P, ws + W.persist);
+    const Bufs B = bufs(m, ws, W);
+    P.n_layers = count;
+    P.cos_t = B.cos_t;
+    P.sin_t = B.sin_t;
+    P.pos = d_pos;
+    P.hidden = B.hidden;
+    if (!persist::plan(P)) return MB200_ERR_UNSUPPORTED;
+    return persist::launch(P, s);
+}
+
+// Layers in as few launches as the kernels allow
+int run_layers(const mb200_decode_model &m, int first, int count, uint8_t *ws, const Workspace &W, const int *d_pos, cudaStream_t s)
+{
+    while (count > 0) {
+        const int n = count < persist::kMaxLayers ? count : persist::kMaxLayers;
+        int rc = run_persist(m, first, n, ws, W, d_pos, s);
+        // not covered, or refused (fewer SMs available than the grid needs): nothing ran
+        if (rc == MB200_ERR_UNSUPPORTED || rc == MB200_ERR_LAUNCH) {
+            rc = MB200_OK;
+            for (int l = first; l < first + n && rc == MB200_OK; l++) rc = run_layer(m, m.layers[l], ws, W, d_pos, s);
+        }
+        if (rc != MB200_OK) return rc;
+        first += n;
+        count -= n;
+    }
+    return MB200_OK;
+}
+
 }  // namespace
 }  // namespace mb200
 
@@ -240,9 +334,16 @@ int mb200_decode_layer(const mb200_decode_model *m, int layer, void *workspace, 
 {
     int rc = check_model(m);
     if (rc != MB200_OK) return rc;
-    if (!workspace || !d_pos || layer < 0 || layer >= m->n_layers) return MB200_ERR_ARG;
+    return mb200_decode_layers(m, layer, 1, workspace, d_pos, stream);
+}
+
+int mb200_decode_layers(const mb200_decode_model *m, int first, int count, void *workspace, const int *d_pos, cudaStream_t stream)
+{
+    int rc = check_model(m);
+    if (rc != MB200_OK) return rc;
+    if (!workspace || !d_pos || first < 0 || count < 1 || first > m->n_layers - count) return MB200_ERR_ARG;
     mb200_clear_status();
-    rc = run_layer(*m, m->layers[layer], static_cast<uint8_t *>(workspace), layout(*m), d_pos, stream);
+    rc = run_layers(*m, first, count, static_cast<uint8_t *>(workspace), layout(*m), d_pos, stream);
     if (rc != MB200_OK) return rc;
     if (cudaGetLastError() != cudaSuccess) return MB200_ERR_LAUNCH;
     return mb200_last_status();
@@ -373,8 +474,7 @@ int mb200_decode_step(const mb200_decode_model *m, void *workspace, int *d_token
 {
     int rc = mb200_decode_begin(m, workspace, d_token, d_pos, stream);
     if (rc != MB200_OK) return rc;
-    for (int l = 0; l < m->n_layers; l++)
-        if ((rc = mb200_decode_layer(m, l, workspace, d_pos, stream)) != MB200_OK) return rc;
+    if ((rc = mb200_decode_layers(m, 0, m->n_layers, workspace, d_pos, stream)) != MB200_OK) return rc;
     return mb200_decode_finish(m, workspace, d_logits, d_token, d_pos, stream);
 }
 

@@ -2,7 +2,6 @@
 // src/forward.c:604-1117):
 //   Q, K, V of RMSNorm(hidden) | q/k norm + RoPE + KV store + attention partials | merge of the partials | O + residual |
 //   router logits of RMSNorm(hidden) | top-k, gate / up + SwiGLU of the routed experts | down, weighted sum + residual
-// and, with the last three alone, the MoE block.
 //
 // At batch 1 a layer streams 49 MB (30B-A3B shape) or 157 MB (235B-A22B shape), 7.6 / 24 us at the copy rate; as five to seven
 // kernels it took 68 / 104 us, because every kernel paid for its launch, for instructions fetched cold, for staging its input
@@ -18,9 +17,8 @@
 //     which is all of most operations), and K / V rows of the cache before q exists;
 //   * the input vector of an operation is split by every CTA into two int8 levels as it arrives.
 //
-// The top-k a CTA does for itself by counting: the rank of an expert is how many logits are larger. The MoE block returns ids,
-// weights and activations in the reference's slots, which follow from its replace-the-minimum walk: slots_of() has the closed
-// form (see topk.cuh), evaluated while the first weights are on their way. Equal logits where it matters take the walk itself.
+// The top-k a CTA does for itself by counting: the rank of an expert is how many logits are larger. Only where equal logits
+// straddle the boundary does the reference's replace-the-minimum walk decide, and is then run.
 //
 // The code of a layer is run once per layer: what counts is that it stays in the instruction caches (with everything inlined it
 // was 270 KB, and a layer took longer than the separate kernels). So every step is a function, one copy each, whose arguments
@@ -33,6 +31,7 @@
 
 #include <cstdio>
 
+#include "comm.cuh"
 #include "q4k_policy.cuh"
 #include "q6k_policy.cuh"
 
@@ -60,19 +59,27 @@ struct Misc {
     unsigned long long launch;
     float red[2][kWarps];
     float am[kWarps][16], al[kWarps][16];  // attention: running maximum / sum per warp and head
+    float res[kWarps][16];                 // residual of a warp's rows of the O projection
     float part[kMaxK][kMaxDownRows];
     uint32_t key[kMaxExperts];             // ordered logits
-    int arrival[kMaxExperts], byrank[kMaxExperts];
-    int top_id[kMaxK + 1], slot_of_rank[kMaxK];
+    int top_id[kMaxK + 1];
     uint32_t top_key[kMaxK + 1];
-    int sid[kMaxK], slot[kMaxK];
     float swt[kMaxK];
-    int accepted, tie, abort_flag;
+    int abort_flag;
+    int xc, off_row, off_ring, ring_bytes;  // copies of the launch's geometry for the steps
+    int own[kWarps][12];                    // a warp's shares, see Own
 };
+enum Own { oQ0, oQn, oQm, oO0, oOn, oG0, oGn, oD0, oDn };
+// Shared memory: Misc, the staged vector (and the attention's fragments, the merge), the router row, the warps' rings.
+constexpr int kX = (static_cast<int>(sizeof(Misc)) + 127) & ~127;
+__device__ __forceinline__ Misc &misc() { return *reinterpret_cast<Misc *>(smem); }
+__device__ __forceinline__ uint8_t *ring() { return smem + misc().off_ring + (threadIdx.x >> 5) * misc().ring_bytes; }
+__device__ __forceinline__ uint64_t *ring_bars() { return misc().bars[threadIdx.x >> 5]; }
+__device__ __forceinline__ volatile int *gave_up() { return &misc().abort_flag; }
 
 __device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kWork) : "memory"); }
 // Every thread: true = somebody in the CTA has given up (the same answer for all of them). A barrier of the CTA.
-__device__ __forceinline__ bool cta_aborted(const volatile int *flag)
+__device__ __forceinline__ bool cta_aborted()
 {
     uint32_t r;
     asm volatile(
@@ -81,17 +88,18 @@ __device__ __forceinline__ bool cta_aborted(const volatile int *flag)
         "barrier.cta.red.or.pred p, 1, %2, q;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(r)
-        : "r"(static_cast<uint32_t>(*flag)), "n"(kWork)
+        : "r"(static_cast<uint32_t>(*gave_up())), "n"(kWork)
         : "memory");
     return r != 0;
 }
 
-__device__ __noinline__ void wait_slow(uint64_t *bar, uint32_t parity, volatile int *abort_flag)
+// (Not left early when somebody gives up: copies in flight are always waited for.)
+__device__ __noinline__ void wait_slow(uint64_t *bar, uint32_t parity)
 {
 #pragma unroll 1
     for (uint32_t i = 0; i < kWaitBudget; i++)
-        if (*abort_flag || mbar_try_wait(bar, parity)) return;
-    *abort_flag = 1;
+        if (mbar_try_wait(bar, parity)) return;
+    *gave_up() = 1;
 }
 
 // ---- cells ----
@@ -106,19 +114,19 @@ __device__ __forceinline__ void st_cells2(uint2 *p, float a, float b, uint32_t t
     asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(p), "r"(__float_as_uint(a)), "r"(tag), "r"(__float_as_uint(b)) : "memory");
 }
 // One cell, bounded wait (0 and the abort flag if it does not come).
-__device__ __forceinline__ float wait_value(const uint2 *p, uint32_t tag, volatile int *abort_flag)
+__device__ __forceinline__ float wait_value(const uint2 *p, uint32_t tag)
 {
 #pragma unroll 1
     for (uint32_t i = 0; i < kPolls; i++) {
         const uint2 c = ld_cell(p);
         if (c.y == tag) return __uint_as_float(c.x);
-        if (*abort_flag) return 0.0f;
+        if (*gave_up()) return 0.0f;
     }
-    *abort_flag = 1;
+    *gave_up() = 1;
     return 0.0f;
 }
 // Four cells, 32 apart (a head's values of a lane), all requested at once.
-__device__ __forceinline__ void wait_values4(const uint2 *p, uint32_t tag, volatile int *abort_flag, float (&v)[4])
+__device__ __forceinline__ void wait_values4(const uint2 *p, uint32_t tag, float (&v)[4])
 {
 #pragma unroll 1
     for (uint32_t i = 0;; i++) {
@@ -129,8 +137,8 @@ __device__ __forceinline__ void wait_values4(const uint2 *p, uint32_t tag, volat
             v[u] = __uint_as_float(c.x);
             ok = ok && c.y == tag;
         }
-        if (ok || *abort_flag) return;
-        if (i == kPolls) *abort_flag = 1;
+        if (ok || *gave_up()) return;
+        if (i == kPolls) *gave_up() = 1;
     }
 }
 
@@ -141,8 +149,8 @@ __device__ __forceinline__ int chunk_at(int j)
     const int b = (j >> 3) & 3;
     return j ^ (b ^ (b << 1));
 }
-__device__ __forceinline__ float *x_scale(int xc) { return reinterpret_cast<float *>(smem + 2 * xc); }
-__device__ __forceinline__ float *x_sum(int xc) { return reinterpret_cast<float *>(smem + 2 * xc + xc / 8); }
+__device__ __forceinline__ float *x_scale(int xc) { return reinterpret_cast<float *>(smem + kX + 2 * xc); }
+__device__ __forceinline__ float *x_sum(int xc) { return reinterpret_cast<float *>(smem + kX + 2 * xc + xc / 8); }
 __device__ __forceinline__ void stage_quad(int xc, const float4 t, int c0, int lane)
 {
     const float v[4] = {t.x, t.y, t.z, t.w};
@@ -167,8 +175,8 @@ __device__ __forceinline__ void stage_quad(int xc, const float4 t, int c0, int l
     const uint32_t p1 = __byte_perm(__byte_perm(a[0], a[1], 0x0040), __byte_perm(a[2], a[3], 0x0040), 0x5410);
     const uint32_t p2 = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
     const int at = chunk_at(c0 >> 4) * 16 + (c0 & 12);
-    *reinterpret_cast<uint32_t *>(smem + at) = p1;
-    *reinterpret_cast<uint32_t *>(smem + xc + at) = p2;
+    *reinterpret_cast<uint32_t *>(smem + kX + at) = p1;
+    *reinterpret_cast<uint32_t *>(smem + kX + xc + at) = p2;
     if ((lane & 7) == 0) x_scale(xc)[c0 >> 5] = sc;
     if ((lane & 3) == 0) x_sum(xc)[c0 >> 4] = sum;
 }
@@ -178,7 +186,7 @@ __device__ __forceinline__ void load_x(Q4::XRegs &r, int xc, int col, int g)
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         const int at = chunk_at(j + i) * 16;
-        const uint4 a = *reinterpret_cast<const uint4 *>(smem + at), b = *reinterpret_cast<const uint4 *>(smem + xc + at);
+        const uint4 a = *reinterpret_cast<const uint4 *>(smem + kX + at), b = *reinterpret_cast<const uint4 *>(smem + kX + xc + at);
         r.q1[4 * i] = a.x; r.q1[4 * i + 1] = a.y; r.q1[4 * i + 2] = a.z; r.q1[4 * i + 3] = a.w;
         r.q2[4 * i] = b.x; r.q2[4 * i + 1] = b.y; r.q2[4 * i + 2] = b.z; r.q2[4 * i + 3] = b.w;
     }
@@ -195,7 +203,7 @@ __device__ __forceinline__ void load_x(Q6::XRegs &r, int xc, int col, int sub)
 #pragma unroll
     for (int g = 0; g < 4; g++) {
         const int j = j0 + 2 * g, at = chunk_at(j) * 16;
-        const uint4 a = *reinterpret_cast<const uint4 *>(smem + at), b = *reinterpret_cast<const uint4 *>(smem + xc + at);
+        const uint4 a = *reinterpret_cast<const uint4 *>(smem + kX + at), b = *reinterpret_cast<const uint4 *>(smem + kX + xc + at);
         r.q1[4 * g] = a.x; r.q1[4 * g + 1] = a.y; r.q1[4 * g + 2] = a.z; r.q1[4 * g + 3] = a.w;
         r.q2[4 * g] = b.x; r.q2[4 * g + 1] = b.y; r.q2[4 * g + 2] = b.z; r.q2[4 * g + 3] = b.w;
         r.k[g] = x_scale(xc)[j >> 1] * (1.0f / 254.0f);
@@ -205,13 +213,11 @@ __device__ __forceinline__ void load_x(Q6::XRegs &r, int xc, int col, int sub)
 
 // Stages K columns (every thread of the CTA calls it; K a multiple of 256): src holds floats, or cells if tag != 0. norm_w:
 // RMS-normalised with it. logit_cell: the row of shared memory at off_row times the (normalised) vector goes there with
-// logit_tag, before the splitting starts. With either of them K <= 8192: the whole vector in registers. Returns whether the CTA
+// the tag, before the splitting starts. With either of them K <= 8192: the whole vector in registers. Returns whether the CTA
 // has given up.
-__device__ __noinline__ bool stage_vec(const void *src, uint32_t tag, int K, const float *norm_w, float eps, int off_row,
-                                       uint2 *logit_cell, uint32_t logit_tag, int xc, int off_misc)
+__device__ __noinline__ bool stage_vec(const void *src, uint32_t tag, int K, const float *norm_w, float eps, uint2 *logit_cell)
 {
-    Misc &M = *reinterpret_cast<Misc *>(smem + off_misc);
-    volatile int *abort_flag = &M.abort_flag;
+    Misc &M = misc();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool whole = norm_w || logit_cell;
 #pragma unroll 1
@@ -223,22 +229,32 @@ __device__ __noinline__ bool stage_vec(const void *src, uint32_t tag, int K, con
                 g[u] = base + u * kWork * 4 < K ? __ldg(reinterpret_cast<const float4 *>(norm_w + base + u * kWork * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         if (tag) {
+            uint32_t todo = 0;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+                todo |= (base + u * kWork * 4 < K ? 1u : 0u) << u;
+            }
 #pragma unroll 1
-            for (uint32_t i = 0;; i++) {
-                bool ok = true;
+            for (uint32_t i = 0; todo; i++) {  // what has not come is asked for again
+                uint4 a[4], b[4];
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
-                    uint4 a = make_uint4(0, tag, 0, tag), b = a;
-                    if (base + u * kWork * 4 < K) {
+                    a[u] = b[u] = make_uint4(0, 0, 0, 0);
+                    if (todo >> u & 1) {
                         const uint2 *p = static_cast<const uint2 *>(src) + base + u * kWork * 4;
-                        a = ld_cells2(p);
-                        b = ld_cells2(p + 2);
+                        a[u] = ld_cells2(p);
+                        b[u] = ld_cells2(p + 2);
                     }
-                    ok = ok && a.y == tag && a.w == tag && b.y == tag && b.w == tag;
-                    v[u] = make_float4(__uint_as_float(a.x), __uint_as_float(a.z), __uint_as_float(b.x), __uint_as_float(b.z));
                 }
-                if (ok || *abort_flag) break;
-                if (i == kPolls) *abort_flag = 1;
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (a[u].y == tag && a[u].w == tag && b[u].y == tag && b[u].w == tag) {
+                        v[u] = make_float4(__uint_as_float(a[u].x), __uint_as_float(a[u].z), __uint_as_float(b[u].x), __uint_as_float(b[u].z));
+                        todo &= ~(1u << u);
+                    }
+                if (*gave_up()) break;
+                if (i == kPolls) *gave_up() = 1;
             }
             __syncwarp();
         } else {
@@ -260,7 +276,7 @@ __device__ __noinline__ bool stage_vec(const void *src, uint32_t tag, int K, con
 #pragma unroll
                 for (int u = 0; u < 4; u++)
                     if (base + u * kWork * 4 < K) {
-                        const float4 r = *reinterpret_cast<const float4 *>(smem + off_row + (base + u * kWork * 4) * 4);
+                        const float4 r = *reinterpret_cast<const float4 *>(smem + M.off_row + (base + u * kWork * 4) * 4);
                         dot = fmaf(v[u].x, r.x, fmaf(v[u].y, r.y, fmaf(v[u].z, r.z, fmaf(v[u].w, r.w, dot))));
                     }
             }
@@ -282,7 +298,7 @@ __device__ __noinline__ bool stage_vec(const void *src, uint32_t tag, int K, con
                 float d = 0.0f;
 #pragma unroll
                 for (int w = 0; w < kWarps; w++) d += M.red[1][w];
-                st_cell(logit_cell, d * scale, logit_tag);
+                st_cell(logit_cell, d * scale, tag);
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) { v[u].x *= scale; v[u].y *= scale; v[u].z *= scale; v[u].w *= scale; }
@@ -291,18 +307,18 @@ __device__ __noinline__ bool stage_vec(const void *src, uint32_t tag, int K, con
         for (int u = 0; u < 4; u++) {
             const int c0 = base + u * kWork * 4;
             if (c0 - lane * 4 >= K) break;  // warp-uniform: a warp covers 128 columns
-            stage_quad(xc, v[u], c0, lane);
+            stage_quad(M.xc, v[u], c0, lane);
         }
         if (whole) break;
     }
-    return cta_aborted(abort_flag);
+    return cta_aborted();
 }
 
 // ---- a warp's private ring: it issues its own copies and consumes them, so one "full" barrier per stage is all it takes.
 // `parity`: per stage, the parity of its next completion. ----
-__device__ __forceinline__ void ring_wait(uint64_t *bars, int s, uint32_t &parity, volatile int *abort_flag)
+__device__ __forceinline__ void ring_wait(uint64_t *bars, int s, uint32_t &parity)
 {
-    if (!mbar_try_wait(&bars[s], (parity >> s) & 1)) wait_slow(&bars[s], (parity >> s) & 1, abort_flag);
+    if (!mbar_try_wait(&bars[s], (parity >> s) & 1)) wait_slow(&bars[s], (parity >> s) & 1);
     parity ^= 1u << s;
     __syncwarp();
 }
@@ -320,9 +336,11 @@ __device__ __forceinline__ void issue_unit(const uint8_t *w, int row, int rows, 
     bulk_g2s(dst, reinterpret_cast<const void *>(a0), bytes, bar);
 }
 // Requests the first units, a lane each; returns the mask of stages in flight.
-__device__ __noinline__ uint32_t prefetch(const uint8_t *w, int r0, int n, uint32_t row_bytes, int ur, uint8_t *buf, int ring_bytes,
-                                          uint64_t *bars)
+__device__ __noinline__ uint32_t prefetch(const uint8_t *w, int r0, int n, uint32_t row_bytes, int ur)
 {
+    uint8_t *buf = ring();
+    uint64_t *bars = ring_bars();
+    const int ring_bytes = misc().ring_bytes;
     const uint32_t sb = stage_bytes_of(ur * row_bytes);
     const int lane = threadIdx.x & 31;
     const int stages = min(kStages, ring_bytes / static_cast<int>(sb)), count = min(stages, n > 0 ? (n + ur - 1) / ur : 0);
@@ -334,8 +352,11 @@ __device__ __noinline__ uint32_t prefetch(const uint8_t *w, int r0, int n, uint3
 // dst[row] = value (+ add[row - r0]), as a cell if tag != 0. Returns the ring's parities.
 template <class F, int RU>
 __device__ __noinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, int r0, int n, void *dst, uint32_t tag, const float *add, int xcol,
-                                        int xc, uint8_t *buf, int ring_bytes, uint64_t *bars, uint32_t parity, volatile int *abort_flag)
+                                        uint32_t parity)
 {
+    uint8_t *buf = ring();
+    uint64_t *bars = ring_bars();
+    const int ring_bytes = misc().ring_bytes, xc = misc().xc;
     const int lane = threadIdx.x & 31, q = lane >> 2, sub = lane & 3;
     const int v = 1 << lv, rpp = 8 >> lv, cq = q & (v - 1), rq = q >> lv, W = 4 << lv;
     const int groups = (bpr + v - 1) >> lv, ur = RU * rpp;
@@ -345,7 +366,7 @@ __device__ __noinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, int r
     int s = 0;
 #pragma unroll 1
     for (int r = 0; r < n; r += ur) {
-        ring_wait(bars, s, parity, abort_flag);
+        ring_wait(bars, s, parity);
         uint32_t skew = 0;
         if (F::kBlockBytes % 16) skew = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(w) + (size_t)(r0 + r) * row_bytes) & 15u;
         const uint8_t *base = buf + s * sb + skew + rq * row_bytes;
@@ -433,9 +454,11 @@ __device__ __noinline__ float4 norm_rope(float4 v, const float *w, float eps, co
 }
 
 // K / V rows of a tile of 16 positions, a row per lane
-__device__ __forceinline__ void load_kv(const __half *kv_k, const __half *kv_v, int tile, int pos, int n_kv, int kvh, uint8_t *buf, uint64_t *bar)
+__device__ __forceinline__ void load_kv(const __half *kv_k, const __half *kv_v, int tile, int pos, int n_kv, int kvh)
 {
     const int lane = threadIdx.x & 31;
+    uint8_t *buf = ring();
+    uint64_t *bar = ring_bars();
     if (lane == 0) mbar_expect_tx(bar, 32 * 256);
     __syncwarp();
     const int p = min(tile * 16 + (lane & 15), pos);
@@ -448,9 +471,10 @@ __device__ __forceinline__ void load_kv(const __half *kv_k, const __half *kv_v, 
 // and, with store, writes them to the cache. Returns the ring's parities.
 __device__ __noinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_kv, int kvh, __half *kv_k, __half *kv_v, bool store,
                                             const uint2 *c_k, const uint2 *c_v, uint32_t tag, const float *k_norm, float eps,
-                                            const float *cos_t, const float *sin_t, uint8_t *buf, uint32_t parity, int off_misc)
+                                            const float *cos_t, const float *sin_t, uint32_t parity)
 {
-    Misc &M = *reinterpret_cast<Misc *>(smem + off_misc);
+    uint8_t *buf = ring();
+    Misc &M = misc();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     uint64_t *bars = M.bars[warp];
     float O[16][4];
@@ -462,11 +486,11 @@ __device__ __noinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_kv,
     const uint32_t va = vbase + ((lane & 7) + ((lane >> 3) & 1) * 8) * kKvPitch + (lane >> 4) * 16;
 #pragma unroll 1
     for (;;) {
-        ring_wait(bars, 0, parity, &M.abort_flag);
+        ring_wait(bars, 0, parity);
         if (tile == (pos >> 4)) {
             float kv[4], vv[4];
-            wait_values4(c_k + kvh * 128 + lane, tag, &M.abort_flag, kv);
-            wait_values4(c_v + kvh * 128 + lane, tag, &M.abort_flag, vv);
+            wait_values4(c_k + kvh * 128 + lane, tag, kv);
+            wait_values4(c_v + kvh * 128 + lane, tag, vv);
             __syncwarp();
             const float4 kr = norm_rope(make_float4(kv[0], kv[1], kv[2], kv[3]), k_norm, eps, cos_t, sin_t);
             const float kn[4] = {kr.x, kr.y, kr.z, kr.w};
@@ -492,7 +516,7 @@ __device__ __noinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_kv,
             for (int e = 0; e < 4; e++) S[n][e] = T[n][e] = 0.0f;
 #pragma unroll
         for (int jj = 0; jj < 4; jj++) {
-            const uint8_t *f = smem + (2 * jj * 32 + lane) * 16;
+            const uint8_t *f = smem + kX + (2 * jj * 32 + lane) * 16;
             const uint4 h0 = *reinterpret_cast<const uint4 *>(f), h1 = *reinterpret_cast<const uint4 *>(f + 512);
             const uint4 lo0 = *reinterpret_cast<const uint4 *>(f + 4096), lo1 = *reinterpret_cast<const uint4 *>(f + 4096 + 512);
 #pragma unroll
@@ -554,7 +578,7 @@ __device__ __noinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_kv,
         tile += kWarps;
         if (tile >= t1) break;
         __syncwarp();
-        load_kv(kv_k, kv_v, tile, pos, n_kv, kvh, buf, &bars[0]);
+        load_kv(kv_k, kv_v, tile, pos, n_kv, kvh);
     }
 #pragma unroll
     for (int o = 1; o <= 2; o <<= 1) {
@@ -579,13 +603,13 @@ __device__ __noinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_kv,
 
 // Warp h (< nh) brings query head h0 + h into the fragments (hi + lo halves of q * scale * log2 e); the others' rows are zero.
 __device__ __noinline__ void q_fragments(const uint2 *c_q, uint32_t tag, bool live, const float *q_norm, float eps, const float *cos_t,
-                                         const float *sin_t, float sc, int off_misc)
+                                         const float *sin_t, float sc)
 {
-    Misc &M = *reinterpret_cast<Misc *>(smem + off_misc);
+    Misc &M = misc();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float v[4] = {0.f, 0.f, 0.f, 0.f};
     if (live) {
-        wait_values4(c_q + lane, tag, &M.abort_flag, v);
+        wait_values4(c_q + lane, tag, v);
         __syncwarp();
         const float4 r = norm_rope(make_float4(v[0], v[1], v[2], v[3]), q_norm, eps, cos_t, sin_t);
         v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
@@ -596,15 +620,15 @@ __device__ __noinline__ void q_fragments(const uint2 *c_q, uint32_t tag, bool li
         const int at = ((d >> 4) * 32 + (warp & 7) * 4 + ((kk & 7) >> 1)) * 16 + ((warp >> 3) + 2 * (kk >> 3)) * 4 + (kk & 1) * 2;
         const float s = v[i] * sc;
         const __half hi = __float2half_rn(s);
-        *reinterpret_cast<__half *>(smem + at) = hi;
-        *reinterpret_cast<__half *>(smem + 4096 + at) = __float2half_rn(s - __half2float(hi));
+        *reinterpret_cast<__half *>(smem + kX + at) = hi;
+        *reinterpret_cast<__half *>(smem + kX + 4096 + at) = __float2half_rn(s - __half2float(hi));
     }
 }
 
 // The CTA's partial of nw warps: one head per warp, four dims per lane, into the cells of slot `slot`.
-__device__ __noinline__ void attn_partial(int nw, uint2 *c_part, uint2 *c_ml, int slot, uint32_t tag, int off_misc, int off_ring, int ring_bytes)
+__device__ __noinline__ void attn_partial(int nw, uint2 *c_part, uint2 *c_ml, int slot, uint32_t tag)
 {
-    Misc &M = *reinterpret_cast<Misc *>(smem + off_misc);
+    Misc &M = misc();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float m = -INFINITY, s = 0.0f;
 #pragma unroll 1
@@ -613,7 +637,7 @@ __device__ __noinline__ void attn_partial(int nw, uint2 *c_part, uint2 *c_ml, in
 #pragma unroll 1
     for (int w = 0; w < nw; w++) {
         const float f = exp2f(M.am[w][warp] - m);
-        const float4 o = *reinterpret_cast<const float4 *>(smem + off_ring + w * ring_bytes + (warp * kPitch + 4 * lane) * 4);
+        const float4 o = *reinterpret_cast<const float4 *>(smem + M.off_ring + w * M.ring_bytes + (warp * kPitch + 4 * lane) * 4);
         s = fmaf(M.al[w][warp], f, s);
         a.x = fmaf(o.x, f, a.x); a.y = fmaf(o.y, f, a.y); a.z = fmaf(o.z, f, a.z); a.w = fmaf(o.w, f, a.w);
     }
@@ -624,10 +648,9 @@ __device__ __noinline__ void attn_partial(int nw, uint2 *c_part, uint2 *c_ml, in
 }
 
 // Merges the nc chunks' partials of one head (hq of head block b): the CTA's warps over the chunks; cells of the result.
-__device__ __noinline__ void merge_head(int b, int hq, int nc, int chunks, const uint2 *c_part, const uint2 *c_ml, uint2 *dst, uint32_t tag, int off_misc)
+__device__ __noinline__ void merge_head(int b, int hq, int nc, int chunks, const uint2 *c_part, const uint2 *c_ml, uint2 *dst, uint32_t tag)
 {
-    Misc &M = *reinterpret_cast<Misc *>(smem + off_misc);
-    volatile int *abort_flag = &M.abort_flag;
+    Misc &M = misc();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     float m = -INFINITY, s = 0.0f;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -645,8 +668,8 @@ __device__ __noinline__ void merge_head(int b, int hq, int nc, int chunks, const
                 o1[u] = ld_cells2(c_part + slot * 128 + 4 * lane + 2);
                 ok = ok && ms[u].y == tag && ms[u].w == tag && o0[u].y == tag && o0[u].w == tag && o1[u].y == tag && o1[u].w == tag;
             }
-            if (ok || *abort_flag) break;
-            if (i == kPolls) *abort_flag = 1;
+            if (ok || *gave_up()) break;
+            if (i == kPolls) *gave_up() = 1;
         }
         __syncwarp();
 #pragma unroll
@@ -661,7 +684,7 @@ __device__ __noinline__ void merge_head(int b, int hq, int nc, int chunks, const
             m = mn;
         }
     }
-    float *buf = reinterpret_cast<float *>(smem);  // [16][128]
+    float *buf = reinterpret_cast<float *>(smem + kX);  // [16][128]
     *reinterpret_cast<float4 *>(buf + warp * 128 + 4 * lane) = a;
     if (lane == 0) {
         M.red[0][warp] = m;
@@ -683,6 +706,453 @@ __device__ __noinline__ void merge_head(int b, int hq, int nc, int chunks, const
     cta_sync();
 }
 
+// ---- selection ----
+__device__ __forceinline__ uint32_t ordered(float v)
+{
+    const uint32_t b = __float_as_uint(v + 0.0f);  // -0 counts as 0
+    return b ^ ((b >> 31) ? 0xFFFFFFFFu : 0x80000000u);
+}
+__device__ __forceinline__ float unordered(uint32_t k) { return __uint_as_float(k ^ ((k >> 31) ? 0x80000000u : 0xFFFFFFFFu)); }
+
+// One thread: the reference's walk (n <= 32 k: nothing is dropped before the merge) over the logits in (e % 32, e / 32) order,
+// replacing the first minimum when strictly greater.
+__device__ __noinline__ void walk(int n, int k)
+{
+    Misc &M = misc();
+#pragma unroll 1
+    for (int i = 0; i < k; i++) {
+        M.top_id[i] = 0;
+        M.top_key[i] = 0;
+    }
+#pragma unroll 1
+    for (int l = 0; l < 32; l++)
+#pragma unroll 1
+        for (int e = l; e < n; e += 32) {
+            int at = 0;
+#pragma unroll 1
+            for (int i = 1; i < k; i++)
+                if (M.top_key[i] < M.top_key[at]) at = i;
+            if (M.key[e] > M.top_key[at]) {
+                M.top_key[at] = M.key[e];
+                M.top_id[at] = e;
+            }
+        }
+}
+
+// The k largest of n logits (every thread of the CTA calls it): lane i < k of every warp returns the i-th expert, the weights go
+// to M.swt (visible after the next barrier of the CTA). -1: the CTA has given up.
+__device__ __noinline__ int select_experts(const uint2 *cells, uint32_t tag, int n, int k)
+{
+    Misc &M = misc();
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid < kMaxExperts) M.key[tid] = tid < n ? ordered(wait_value(cells + tid, tag)) : 0;
+    if (cta_aborted()) return -1;
+    {
+        const int e = tid >> 1, half = (n + 1) >> 1, lo = (tid & 1) ? half : 0, hi = (tid & 1) ? n : half;
+        if (e - (lane >> 1) < n) {  // warp-uniform
+            const uint32_t me = M.key[e];
+            int rank = 0;
+#pragma unroll 8
+            for (int i = lo; i < hi; i++) rank += (M.key[i] > me || (M.key[i] == me && i < e)) ? 1 : 0;
+            rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+            if (rank <= k && e < n && !(tid & 1)) {
+                M.top_id[rank] = e;
+                M.top_key[rank] = me;
+            }
+        }
+    }
+    cta_sync();
+    if (n > k && M.top_key[k - 1] == M.top_key[k]) {  // the same for the whole CTA
+        cta_sync();
+        if (tid == 0) walk(n, k);
+        cta_sync();
+    }
+    const int id = M.top_id[lane < k ? lane : 0];
+    const float v = lane < k ? unordered(M.top_key[lane]) : -INFINITY;
+    float mx = v;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float e = lane < k ? expf(v - mx) : 0.0f;
+    const float sum = warp_sum(e);
+    if (tid < k) M.swt[tid] = e / sum;
+    return id;
+}
+
+// ---- gate / up: items [i0, i0 + n), item i = a pass of gate rows and the same up rows of the i / ipe-th routed expert ----
+__device__ __forceinline__ void issue_pair(const uint8_t *experts, size_t estride, uint32_t up_off, int id, uint32_t row_off, uint32_t half,
+                                           uint8_t *dst, uint64_t *bar)
+{
+    const uint8_t *src = experts + (size_t)id * estride + row_off;
+    mbar_expect_tx(bar, 2 * half);
+    bulk_g2s(dst, src, half, bar);
+    bulk_g2s(dst + half, src + up_off, half, bar);
+}
+// id: lane i holds the i-th routed expert. Writes SwiGLU's result as cells act[slot * EFF + row].
+__device__ __noinline__ uint32_t gate_up(const uint8_t *experts, size_t estride, uint32_t up_off, int id, int i0, int n, int ipe, uint32_t magic,
+                                         int bpr, int lv, int EFF, uint2 *act, uint32_t tag, uint32_t parity)
+{
+    uint8_t *buf = ring();
+    uint64_t *bars = ring_bars();
+    const int ring_bytes = misc().ring_bytes, xc = misc().xc;
+    const int lane = threadIdx.x & 31, q = lane >> 2, sub = lane & 3;
+    const int v = 1 << lv, rpp = 8 >> lv, cq = q & (v - 1), rq = q >> lv, W = 4 << lv;
+    const int groups = (bpr + v - 1) >> lv;
+    const uint32_t row_bytes = bpr * kQ4KBlock, half = rpp * row_bytes, sb = 2 * half;
+    const int stages = min(kStages, ring_bytes / static_cast<int>(sb));
+    {
+        const int i = i0 + lane, slot = __umulhi(i, magic);
+        const int ex = __shfl_sync(0xffffffffu, id, slot & 31);
+        if (lane < min(stages, n)) issue_pair(experts, estride, up_off, ex, (i - slot * ipe) * half, half, buf + lane * sb, &bars[lane]);
+        __syncwarp();
+    }
+    Q4::XRegs xr;
+    int s = 0;
+#pragma unroll 1
+    for (int i = i0; i < i0 + n; i++) {
+        ring_wait(bars, s, parity);
+        const uint8_t *base = buf + s * sb + rq * row_bytes;
+        float acc[2] = {0.0f, 0.0f};
+#pragma unroll 1
+        for (int c = 0; c < groups; c++) {
+            const int col = (c << lv) + cq;
+            const bool in = col < bpr;  // a ragged last group
+            const int at = in ? col : 0;
+            if (groups > 1 || i == i0) load_x(xr, xc, at, sub);
+            const float g = Q4::block_dot(base + at * kQ4KBlock, sub, xr);
+            const float u = Q4::block_dot(base + half + at * kQ4KBlock, sub, xr);
+            acc[0] += in ? g : 0.0f;
+            acc[1] += in ? u : 0.0f;
+        }
+        __syncwarp();
+        {
+            const int j = i + stages, slot = __umulhi(j, magic);
+            const int ex = __shfl_sync(0xffffffffu, id, slot & 31);
+            if (lane == 0 && j < i0 + n) issue_pair(experts, estride, up_off, ex, (j - slot * ipe) * half, half, buf + s * sb, &bars[s]);
+        }
+        int which;
+        const float g = stream::packed_sum<2, false>(acc, W, lane, which);
+        const float u = __shfl_xor_sync(0xffffffffu, g, W >> 1);  // which = 1 in the upper half of a row's lanes
+        if ((lane & (W - 1)) == 0) {
+            const int slot = __umulhi(i, magic);
+            st_cell(act + slot * EFF + (i - slot * ipe) * rpp + rq, g / (1.0f + expf(-g)) * u, tag);
+        }
+        if (++s == stages) s = 0;
+    }
+    return parity;
+}
+
+__global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant__ Params P)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x, grid = gridDim.x;
+    Misc &M = misc();
+    if (tid < kWarps * kStages) mbar_init(&M.bars[0][0] + tid, 1);
+    if (tid == kWork - 1) {
+        mbar_init(&M.row_bar, 1);
+        M.abort_flag = 0;
+        M.xc = P.xc;
+        M.off_row = P.off_row;
+        M.off_ring = P.off_ring;
+        M.ring_bytes = P.ring_bytes;
+    }
+    // What a warp does in every layer; kept in shared memory (registers would be saved and restored around every step)
+    const volatile int *own = M.own[warp];
+    if (lane == 0) {
+        int *o = M.own[warp];
+        const int gid = warp * grid + cta;
+        int i0, n, m = 0;
+        share(P.sq, gid, i0, n);  // rows of one of the three matrices behind the first norm
+        if (gid >= P.sk.w0) { m = 1; share(P.sk, gid, i0, n); }
+        if (gid >= P.sv.w0) { m = 2; share(P.sv, gid, i0, n); }
+        o[oQ0] = i0 << (3 - P.mH.lv);
+        o[oQn] = n << (3 - P.mH.lv);
+        o[oQm] = m;
+        share(P.so, gid, i0, n);
+        o[oO0] = i0 << (3 - P.mQ.lv);
+        o[oOn] = n << (3 - P.mQ.lv);
+        share(P.sg, gid, i0, n);
+        o[oG0] = i0;
+        o[oGn] = n;
+        // down: the CTA's rows, shared by the warps of a slot
+        const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid), R1 = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid);
+        const int wps = kWarps / P.k, slot = warp / wps, part = warp - slot * wps, per = (R1 - R0 + wps - 1) / wps;
+        o[oD0] = R0 + part * per;
+        o[oDn] = slot < P.k ? max(0, min(per, R1 - R0 - part * per)) : 0;
+    }
+    mbar_fence_init();
+    __syncthreads();
+    auto prefetch_qkv = [&](int l) {
+        const Layer &L = P.L[l];
+        const int qm = own[oQm];
+        const bool q6 = qm == 2 && L.v_q6;
+        const uint8_t *w = qm == 0 ? L.wq : qm == 1 ? L.wk : L.wv;
+        return prefetch(w, own[oQ0], own[oQn], P.mH.bpr * (q6 ? kQ6KBlock : kQ4KBlock), (q6 ? 1 : 2) << (3 - P.mH.lv));
+    };
+    auto request_row = [&](int l) {
+        mbar_expect_tx(&M.row_bar, P.H * 4);
+        bulk_g2s(smem + P.off_row, P.L[l].router + (size_t)blockIdx.x * P.H, P.H * 4, &M.row_bar);
+    };
+    uint32_t parity = 0;
+    uint32_t pend = prefetch_qkv(0);  // stages in flight while the CTA may still give up
+    const bool has_row = cta < P.n_experts;
+    int row_pend = has_row ? 0 : -1;  // parity of the router row on its way
+    if (has_row && tid == 0) request_row(0);
+    if (P.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (tid == 0) {
+        // arrivals of the launches before this one (nobody of this launch arrives before every CTA has read it: the last layer
+        // needs the activations of all of them); the quotient by a multiplication, a 64-bit division is a hundred instructions
+        unsigned long long c;
+        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(P.ctr) : "memory");
+        unsigned long long n = static_cast<unsigned long long>(__ull2double_rz(c) * P.inv_grid);
+        const long long r = static_cast<long long>(c - n * grid);
+        if (r < 0) n--;
+        if (r >= grid) n++;
+        M.launch = n;
+    }
+    __syncthreads();
+    uint32_t tag = static_cast<uint32_t>(M.launch) * 128u;
+    const int pos = __ldcg(P.pos);
+    bool ok = true;
+
+#pragma unroll 1
+    for (int l = 0; l < P.n_layers; l++) {
+        const Layer &L = P.L[l];
+        tag++;
+        // ---- Q, K, V ----
+        ok = !stage_vec(l == 0 ? static_cast<const void *>(P.hidden) : P.c_h0, l == 0 ? 0 : tag - 1, P.H, L.attn_norm, P.eps, nullptr);
+        if (!ok) break;
+        {
+            const int qm = own[oQm];
+            uint2 *dst = qm == 0 ? P.c_q : qm == 1 ? P.c_k : P.c_v;
+            const uint8_t *w = qm == 0 ? L.wq : qm == 1 ? L.wk : L.wv;
+            if (qm == 2 && L.v_q6)
+                parity = matvec<Q6, 1>(w, P.mH.bpr, P.mH.lv, own[oQ0], own[oQn], dst, tag, nullptr, 0, parity);
+            else
+                parity = matvec<Q4, 2>(w, P.mH.bpr, P.mH.lv, own[oQ0], own[oQn], dst, tag, nullptr, 0, parity);
+            pend = 0;
+        }
+        // ---- attention of this CTA's positions ----
+        const int tpc = ((pos >> 4) + P.chunks) / P.chunks, nc = ((pos >> 4) + tpc) / tpc;  // tiles of 16 positions per chunk, chunks
+        {
+            const int ab = cta / P.chunks, ac = cta - ab * P.chunks;  // head block and chunk
+            if (ab < P.n_kv * P.qblocks && ac < nc) {
+                const int kvh = ab / P.qblocks, qb = ab - kvh * P.qblocks;
+                const int tile0 = ac * tpc + warp, tile1 = min((ac + 1) * tpc, (pos >> 4) + 1);
+                if (tile0 < tile1) {
+                    load_kv(L.kv_k, L.kv_v, tile0, pos, P.n_kv, kvh);
+                    pend = 1;
+                }
+                cta_sync();  // the staged vector has been read
+                const int nh = min(16, P.gqa - qb * 16);
+                q_fragments(P.c_q + (kvh * P.gqa + qb * 16 + warp) * 128, tag, warp < nh, L.q_norm, P.eps, P.cos_t, P.sin_t, P.scale * kLog2e);
+                ok = !cta_aborted();
+                if (!ok) break;
+                if (tile0 < tile1)
+                    parity = attn_tiles(tile0, tile1, pos, P.n_kv, kvh, L.kv_k, L.kv_v, qb == 0, P.c_k, P.c_v, tag, L.k_norm, P.eps, P.cos_t,
+                                        P.sin_t, parity);
+                pend = 0;
+                cta_sync();
+                attn_partial(min(kWarps, tile1 - ac * tpc), P.c_part, P.c_ml, ab * P.chunks + ac, tag);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the ring was written and read as plain memory
+            }
+        }
+        cta_sync();
+        // ---- O projection + residual ----
+        pend = prefetch(L.wo, own[oO0], own[oOn], P.mQ.bpr * kQ4KBlock, 2 << (3 - P.mQ.lv));
+        if (lane < own[oOn]) M.res[warp][lane] = l == 0 ? __ldcg(P.hidden + own[oO0] + lane) : wait_value(P.c_h0 + own[oO0] + lane, tag - 1);
+        if (cta < P.n_heads) {
+            const int kv = cta / P.gqa, hq = cta - kv * P.gqa;
+            merge_head(kv * P.qblocks + (hq >> 4), hq & 15, nc, P.chunks, P.c_part, P.c_ml, P.c_attn + cta * 128, tag);
+        }
+        ok = !stage_vec(P.c_attn, tag, P.QD, nullptr, 0.0f, nullptr);
+        if (!ok) break;
+        parity = matvec<Q4, 2>(L.wo, P.mQ.bpr, P.mQ.lv, own[oO0], own[oOn], P.c_h1, tag, M.res[warp], 0, parity);
+        pend = 0;
+        // ---- router logit of this CTA's expert; the normalised vector stays staged for gate / up ----
+        if (has_row && !mbar_try_wait(&M.row_bar, l & 1)) wait_slow(&M.row_bar, l & 1);
+        row_pend = -1;
+        cta_sync();  // the staged vector has been read
+        ok = !stage_vec(P.c_h1, tag, P.H, L.ffn_norm, P.eps, has_row ? P.c_logit + cta : nullptr);
+        if (!ok) break;
+        if (has_row && l + 1 < P.n_layers) {
+            row_pend = (l + 1) & 1;
+            if (tid == 0) request_row(l + 1);
+        }
+        const int id = select_experts(P.c_logit, tag, P.n_experts, P.k);
+        ok = id >= 0;
+        if (!ok) break;
+        // ---- experts ----
+        parity = gate_up(L.experts, L.estride, L.up_off, id, own[oG0], own[oGn], P.ipe, P.ipe_magic, P.mH.bpr, P.mH.lv, P.EFF, P.c_act, tag, parity);
+        const int slot = warp / (kWarps / P.k), R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid),
+                  rows = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid) - R0;
+        const uint8_t *down = L.experts + (size_t)__shfl_sync(0xffffffffu, id, slot & 31) * L.estride + L.down_off;
+        pend = prefetch(down, own[oD0], own[oDn], P.mE.bpr * (L.down_q6 ? kQ6KBlock : kQ4KBlock), (L.down_q6 ? 1 : 2) << (3 - P.mE.lv));
+        const float res = tid < rows ? wait_value(P.c_h1 + R0 + tid, tag) : 0.0f;
+        cta_sync();  // the staged vector has been read
+        ok = !stage_vec(P.c_act, tag, P.k * P.EFF, nullptr, 0.0f, nullptr);
+        if (!ok) break;
+        {
+            float *dst = M.part[slot < P.k ? slot : 0] - R0;
+            if (L.down_q6)
+                parity = matvec<Q6, 1>(down, P.mE.bpr, P.mE.lv, own[oD0], own[oDn], dst, 0, nullptr, slot * P.mE.bpr, parity);
+            else
+                parity = matvec<Q4, 2>(down, P.mE.bpr, P.mE.lv, own[oD0], own[oDn], dst, 0, nullptr, slot * P.mE.bpr, parity);
+            pend = 0;
+        }
+        const bool more = l + 1 < P.n_layers;
+        if (more) pend = prefetch_qkv(l + 1);
+        cta_sync();
+        if (tid < rows) {
+            float y = 0.0f;
+#pragma unroll 1
+            for (int i = 0; i < P.k; i++) y = fmaf(M.swt[i], M.part[i][tid], y);
+            if (more)
+                st_cell(P.c_h0 + R0 + tid, res + y, tag);
+            else
+                P.hidden[R0 + tid] = res + y;
+        }
+    }
+    if (P.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!ok) {  // given up: leave after the copies in flight
+        if (tid == 0) atomicExch(P.err, MB200_ERR_TIMEOUT);
+#pragma unroll 1
+        for (int s = 0; s < kStages; s++)
+            if (pend >> s & 1) mbar_wait(&M.bars[warp][s], (parity >> s) & 1);
+        if (row_pend >= 0) mbar_wait(&M.row_bar, row_pend);
+    }
+    __syncthreads();
+    if (tid == 0) asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(P.ctr) : "memory");
+}
+
+Split split(int w0, int nw, int passes) { return Split{w0, nw, passes / nw, passes % nw}; }
+Map map_of(int cols)
+{
+    Map m{cols / 256, 0};
+    while (m.lv < 3 && !(m.bpr >> m.lv & 1)) m.lv++;
+    if (m.lv < 2 && m.bpr >= 8) m.lv = 3;  // a ragged last group costs less than single blocks side by side
+    return m;
+}
+int stage_rows(const Map &m, bool q6) { return (q6 ? 1 : 2) << (3 - m.lv); }
+int stage_of(const Map &m, bool q6) { return stage_bytes_of(stage_rows(m, q6) * m.bpr * (q6 ? kQ6KBlock : kQ4KBlock)); }
+constexpr int kSmemBytes = 227 * 1024;
+
 }  // namespace
+
+size_t scratch(Params &P, uint8_t *base)
+{
+    size_t o = 256;
+    if (base) P.ctr = reinterpret_cast<unsigned long long *>(base);
+    auto take = [&](uint2 *&p, size_t n) {
+        if (base) p = reinterpret_cast<uint2 *>(base + o);
+        o += (n * sizeof(uint2) + 255) & ~static_cast<size_t>(255);
+    };
+    const size_t grid = device_sms();
+    take(P.c_q, P.QD);
+    take(P.c_k, P.KD);
+    take(P.c_v, P.KD);
+    take(P.c_part, grid * 16 * 128);
+    take(P.c_ml, grid * 16 * 2);
+    take(P.c_attn, P.QD);
+    take(P.c_h1, P.H);
+    take(P.c_act, (size_t)P.k * P.EFF);
+    take(P.c_h0, P.H);
+    take(P.c_logit, P.n_experts);
+    return o;
+}
+
+bool plan(Params &P)
+{
+    const int grid = device_sms();
+    if (P.H % 256 || P.EFF % 256 || P.QD % 256 || P.H < 256 || P.EFF < 256 || P.QD < 256 || P.H > 8192) return false;
+    if (P.k < 1 || P.k > kMaxK || P.n_experts < P.k || P.n_experts > min(grid, kMaxExperts) || P.n_experts > 32 * P.k) return false;
+    if (P.n_layers < 1 || P.n_layers > kMaxLayers) return false;
+    P.qblocks = (P.gqa + 15) / 16;
+    const int blocks = P.n_kv * P.qblocks;
+    if (blocks > grid || P.n_heads > grid) return false;
+    P.chunks = grid / blocks;
+    P.mH = map_of(P.H);
+    P.mQ = map_of(P.QD);
+    P.mE = map_of(P.EFF);
+    const int warps = kWarps * grid, rpp = 8 >> P.mH.lv, rppQ = 8 >> P.mQ.lv;
+    // the O projection and the down projection must have rows for every CTA: what tells a writer that all have read
+    if (P.H / rppQ < grid) return false;
+    if ((P.H / rppQ + warps - 1) / warps * rppQ > 16 || P.H / grid + 1 > kMaxDownRows) return false;
+    P.so = split(0, warps, P.H / rppQ);
+    // Q, K, V: warps by what the rows cost (Q6_K: 1.46 times the bytes and more arithmetic per byte)
+    const double cq = P.QD, ck = P.KD, cv = P.KD * (P.L[0].v_q6 ? 1.8 : 1.0), sum = cq + ck + cv;
+    int wk = static_cast<int>(warps * ck / sum), wv = static_cast<int>(warps * cv / sum);
+    wk = wk < 1 ? 1 : wk;
+    wv = wv < 1 ? 1 : wv;
+    P.sq = split(0, warps - wk - wv, P.QD / rpp);
+    P.sk = split(warps - wk - wv, wk, P.KD / rpp);
+    P.sv = split(warps - wv, wv, P.KD / rpp);
+    P.ipe = P.EFF / rpp;
+    P.ipe_magic = static_cast<uint32_t>((1ull << 32) / P.ipe) + 1;
+    P.sg = split(0, warps, P.k * P.ipe);
+    P.xc = P.H > P.QD ? P.H : P.QD;
+    if (P.k * P.EFF > P.xc) P.xc = P.k * P.EFF;
+    if (P.xc < 4096) P.xc = 4096;  // the attention's fragments and the merge use the same 8 KB
+    auto up = [](int v) { return (v + 127) & ~127; };
+    P.off_row = up(kX + 2 * P.xc + P.xc / 8 + P.xc / 4);
+    P.off_ring = up(P.off_row + P.H * 4);
+    P.ring_bytes = ((kSmemBytes - P.off_ring) / kWarps) & ~127;
+    bool v6 = false, d4 = false, d6 = false;
+    for (int l = 0; l < P.n_layers; l++) {
+        v6 = v6 || P.L[l].v_q6;
+        d6 = d6 || P.L[l].down_q6;
+        d4 = d4 || !P.L[l].down_q6;
+    }
+    int need = 32 * kKvPitch;
+    auto fit = [&](int b) { need = b > need ? b : need; };
+    fit(stage_of(P.mH, false));
+    fit(stage_of(P.mQ, false));
+    fit(2 * rpp * P.mH.bpr * kQ4KBlock);
+    if (v6) fit(stage_of(P.mH, true));
+    if (d4) fit(stage_of(P.mE, false));
+    if (d6) fit(stage_of(P.mE, true));
+    return need <= P.ring_bytes;
+}
+
+int launch(Params &P, cudaStream_t stream)
+{
+    static bool done[kMaxDevices] = {false};
+    static int pdl_ok = 1;  // cleared if the driver refuses cooperative + programmatic serialization together
+    const int dev = current_device(), grid = device_sms();
+    if (!done[dev]) {
+        if (cudaFuncSetAttribute(persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) != cudaSuccess) {
+            cudaGetLastError();
+            return MB200_ERR_LAUNCH;
+        }
+        done[dev] = true;
+    }
+    P.inv_grid = 1.0 / grid;
+    P.err = device_error_word();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kWork);
+    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeCooperative;  // the CTAs wait for one another: all must be resident
+    attr[0].val.cooperative = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    P.pdl = (pdl_enabled() && pdl_ok) ? 1 : 0;
+    cfg.numAttrs = P.pdl ? 2 : 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, persist_kernel, P);
+    if (e != cudaSuccess && P.pdl) {
+        cudaGetLastError();
+        pdl_ok = 0;
+        P.pdl = 0;
+        cfg.numAttrs = 1;
+        e = cudaLaunchKernelEx(&cfg, persist_kernel, P);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return MB200_ERR_LAUNCH;
+    }
+    return MB200_OK;
+}
+
 }  // namespace persist
 }  // namespace mb200

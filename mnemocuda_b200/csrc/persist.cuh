@@ -4,7 +4,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "comm.cuh"
 
 namespace mb200 {
 namespace persist {
@@ -32,36 +31,32 @@ struct Map {
 };
 
 struct Params {
-    int n_layers, attn;  // attn = 0: the MoE block alone (one layer)
-    int H, EFF, QD, KD, n_heads, n_kv, gqa, qblocks, chunks, n_experts, k, expert_lo, expert_cnt;
+    int n_layers;
+    int H, EFF, QD, KD, n_heads, n_kv, gqa, qblocks, chunks, n_experts, k;
     float eps, scale;
     const float *cos_t, *sin_t;
     const int *pos;
-    float *hidden;             // attn = 1: before the first layer, after the last one
-    const float *x, *residual; // attn = 0
-    float *y, *act;
-    // Exchange buffers of {value, tag} cells: what one CTA computes and the others need (attn = 1; the logits always)
+    float *hidden;  // before the first layer, after the last one
+    // Exchange buffers of {value, tag} cells: what one CTA computes and the others need
     uint2 *c_q, *c_k, *c_v, *c_part, *c_ml, *c_attn, *c_h1, *c_act, *c_h0, *c_logit;
-    int *ids_out;              // attn = 0: the selection in the reference's slot order
-    float *wts_out;
-    unsigned long long *ctr;   // arrivals, only grows: one per CTA and launch
+    unsigned long long *ctr;  // arrivals, only grows: one per CTA and launch
     double inv_grid;
     int *err;
     int pdl;
-    PushDesc push;  // world > 0: the block of one rank of an expert-sharded model, all-reduced over the ranks
     // geometry
-    Map mH, mQ, mE;            // rows of H, QD and EFF columns
-    Split sq, sk, sv, so;      // passes of the four projections
-    int xc, off_row, off_misc, off_ring, ring_bytes;  // columns of the staged vector; byte offsets in shared memory
+    Map mH, mQ, mE;         // rows of H, QD and EFF columns
+    Split sq, sk, sv, so, sg;  // passes of the four projections; gate / up items
+    uint32_t ipe, ipe_magic;   // gate / up items per expert, 2^32 / ipe rounded up
+    int xc, off_row, off_ring, ring_bytes;  // columns of the staged vector; byte offsets in shared memory
     Layer L[kMaxLayers];
 };
 
 // Fills in the geometry of P for its shape; false = a shape this kernel does not take.
 bool plan(Params &P);
 int launch(Params &P, cudaStream_t stream);  // MB200_OK or an error status
-void init();
-// Cells of the exchange buffers (attn = 1) in the order of Params; returns the bytes, fills the pointers in if base is given.
-size_t cells(Params &P, uint8_t *base);
+// Bytes of the exchange buffers and the counter for a shape (H, EFF, QD, KD, n_heads, n_experts, k set); fills the pointers in if
+// base is given. Zeroed once by the owner.
+size_t scratch(Params &P, uint8_t *base);
 
 }  // namespace persist
 }  // namespace mb200

@@ -377,8 +377,12 @@ class ResidentModel:
                      "mb200_decode_step")
             return
         self.begin(stream)
-        for l in range(self.cfg.n_layers):
-            self.layer(l, stream)
+        if self.world == 1:
+            K._check(_lib.lib().mb200_decode_layers(C.byref(self.desc), 0, self.cfg.n_layers, self.workspace.data_ptr(),
+                                                    self.pos.data_ptr(), self._st(stream)), "mb200_decode_layers")
+        else:
+            for l in range(self.cfg.n_layers):
+                self.layer(l, stream)
         self.finish(advance, stream)
 
     def capture(self, steps: int = 1, advance: bool = True) -> torch.cuda.CUDAGraph:
