@@ -41,17 +41,32 @@ int pdl_enabled();
 namespace persist {
 namespace {
 
-constexpr int kWarps = 16, kWork = kWarps * 32;
+constexpr int kWarps = 8, kWork = kWarps * 32;
 constexpr int kStages = 5;         // ring stages per warp at most
 constexpr int kPitch = 132;        // floats between heads of a warp's attention result
 constexpr int kKvPitch = 272;      // bytes between K / V rows in shared memory
 constexpr int kMaxDownRows = 64;   // rows of the hidden vector per CTA
-constexpr int kMaxK = 16;
+constexpr int kMaxK = kWarps;    // a warp per slot, or several
 constexpr int kMaxExperts = 256;   // two threads per expert
 constexpr uint32_t kPolls = 1u << 19;  // a fraction of a second
 constexpr float kLog2e = 1.4426950408889634f;
 
 extern __shared__ __align__(1024) uint8_t smem[];
+
+// Read anew by every step (volatile): what follows from it is then not computed once, ahead of the loop over the layers, and kept
+// in registers -- or in local memory -- all along.
+__device__ __forceinline__ int thread_id()
+{
+    int t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    return t;
+}
+__device__ __forceinline__ int cta_id()
+{
+    int t;
+    asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(t));
+    return t;
+}
 
 struct Misc {
     uint64_t bars[kWarps][kStages];
@@ -66,15 +81,17 @@ struct Misc {
     uint32_t top_key[kMaxK + 1];
     float swt[kMaxK];
     int abort_flag;
-    int xc, off_row, off_ring, ring_bytes;  // copies of the launch's geometry for the steps
-    int own[kWarps][12];                    // a warp's shares, see Own
+    Head head;                              // the launch's parameters, read from here by every step (see thread_id)
+    int2 own[kWarps][4];                    // a warp's rows of each operation: first, count (gate / up: items)
+    int own_qm[kWarps];                     // which of Q, K, V
 };
-enum Own { oQ0, oQn, oQm, oO0, oOn, oG0, oGn, oD0, oDn };
+enum Op { kQKV, kO, kExperts, kDown };
 // Shared memory: Misc, the staged vector (and the attention's fragments, the merge), the router row, the warps' rings.
 constexpr int kX = (static_cast<int>(sizeof(Misc)) + 127) & ~127;
 __device__ __forceinline__ Misc &misc() { return *reinterpret_cast<Misc *>(smem); }
-__device__ __forceinline__ uint8_t *ring() { return smem + misc().off_ring + (threadIdx.x >> 5) * misc().ring_bytes; }
-__device__ __forceinline__ uint64_t *ring_bars() { return misc().bars[threadIdx.x >> 5]; }
+__device__ __forceinline__ const volatile Head &head() { return misc().head; }
+__device__ __forceinline__ uint8_t *ring() { return smem + head().off_ring + (thread_id() >> 5) * head().ring_bytes; }
+__device__ __forceinline__ uint64_t *ring_bars() { return misc().bars[thread_id() >> 5]; }
 __device__ __forceinline__ volatile int *gave_up() { return &misc().abort_flag; }
 
 __device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kWork) : "memory"); }
@@ -94,12 +111,15 @@ __device__ __forceinline__ bool cta_aborted()
 }
 
 // (Not left early when somebody gives up: copies in flight are always waited for.)
-__device__ __noinline__ void wait_slow(uint64_t *bar, uint32_t parity)
+__device__ __forceinline__ void wait_copy(uint64_t *bar, uint32_t parity)
 {
+    uint32_t i = 0;
 #pragma unroll 1
-    for (uint32_t i = 0; i < kWaitBudget; i++)
-        if (mbar_try_wait(bar, parity)) return;
-    *gave_up() = 1;
+    while (!mbar_try_wait(bar, parity))
+        if (++i == kWaitBudget) {
+            *gave_up() = 1;
+            break;
+        }
 }
 
 // ---- cells ----
@@ -213,13 +233,14 @@ __device__ __forceinline__ void load_x(Q6::XRegs &r, int xc, int col, int sub)
 
 // Stages K columns (every thread of the CTA calls it; K a multiple of 256): src holds floats, or cells if tag != 0. norm_w:
 // RMS-normalised with it. logit_cell: the row of shared memory at off_row times the (normalised) vector goes there with
-// the tag, before the splitting starts. With either of them K <= 8192: the whole vector in registers. Returns whether the CTA
+// the tag, before the splitting starts. With either of them K <= 16 kWork: the whole vector in registers. Returns whether the CTA
 // has given up.
-__device__ __noinline__ bool stage_vec(const void *src, uint32_t tag, int K, const float *norm_w, float eps, uint2 *logit_cell)
+__device__ __forceinline__ bool stage_vec(const void *src, uint32_t tag, int K, const float *norm_w, float eps, uint2 *logit_cell)
 {
     Misc &M = misc();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = thread_id(), lane = tid & 31, warp = tid >> 5;
     const bool whole = norm_w || logit_cell;
+    const int xc = head().xc;
 #pragma unroll 1
     for (int base = tid * 4; base < K || whole; base += kWork * 16) {
         float4 v[4], g[4];
@@ -276,7 +297,7 @@ __device__ __noinline__ bool stage_vec(const void *src, uint32_t tag, int K, con
 #pragma unroll
                 for (int u = 0; u < 4; u++)
                     if (base + u * kWork * 4 < K) {
-                        const float4 r = *reinterpret_cast<const float4 *>(smem + M.off_row + (base + u * kWork * 4) * 4);
+                        const float4 r = *reinterpret_cast<const float4 *>(smem + head().off_row + (base + u * kWork * 4) * 4);
                         dot = fmaf(v[u].x, r.x, fmaf(v[u].y, r.y, fmaf(v[u].z, r.z, fmaf(v[u].w, r.w, dot))));
                     }
             }
@@ -307,7 +328,7 @@ __device__ __noinline__ bool stage_vec(const void *src, uint32_t tag, int K, con
         for (int u = 0; u < 4; u++) {
             const int c0 = base + u * kWork * 4;
             if (c0 - lane * 4 >= K) break;  // warp-uniform: a warp covers 128 columns
-            stage_quad(M.xc, v[u], c0, lane);
+            stage_quad(xc, v[u], c0, lane);
         }
         if (whole) break;
     }
@@ -318,7 +339,7 @@ __device__ __noinline__ bool stage_vec(const void *src, uint32_t tag, int K, con
 // `parity`: per stage, the parity of its next completion. ----
 __device__ __forceinline__ void ring_wait(uint64_t *bars, int s, uint32_t &parity)
 {
-    if (!mbar_try_wait(&bars[s], (parity >> s) & 1)) wait_slow(&bars[s], (parity >> s) & 1);
+    wait_copy(&bars[s], (parity >> s) & 1);
     parity ^= 1u << s;
     __syncwarp();
 }
@@ -336,13 +357,13 @@ __device__ __forceinline__ void issue_unit(const uint8_t *w, int row, int rows, 
     bulk_g2s(dst, reinterpret_cast<const void *>(a0), bytes, bar);
 }
 // Requests the first units, a lane each; returns the mask of stages in flight.
-__device__ __noinline__ uint32_t prefetch(const uint8_t *w, int r0, int n, uint32_t row_bytes, int ur)
+__device__ __forceinline__ uint32_t prefetch(const uint8_t *w, int r0, int n, uint32_t row_bytes, int ur)
 {
     uint8_t *buf = ring();
     uint64_t *bars = ring_bars();
-    const int ring_bytes = misc().ring_bytes;
+    const int ring_bytes = head().ring_bytes;
     const uint32_t sb = stage_bytes_of(ur * row_bytes);
-    const int lane = threadIdx.x & 31;
+    const int lane = thread_id() & 31;
     const int stages = min(kStages, ring_bytes / static_cast<int>(sb)), count = min(stages, n > 0 ? (n + ur - 1) / ur : 0);
     if (lane < count) issue_unit(w, r0 + lane * ur, min(ur, n - lane * ur), row_bytes, buf + lane * sb, &bars[lane]);
     __syncwarp();
@@ -351,13 +372,13 @@ __device__ __noinline__ uint32_t prefetch(const uint8_t *w, int r0, int n, uint3
 // Those rows (first units requested by prefetch() with the same arguments) times the staged vector from super-block xcol on:
 // dst[row] = value (+ add[row - r0]), as a cell if tag != 0. Returns the ring's parities.
 template <class F, int RU>
-__device__ __noinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, int r0, int n, void *dst, uint32_t tag, const float *add, int xcol,
+__device__ __forceinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, int r0, int n, void *dst, uint32_t tag, const float *add, int xcol,
                                         uint32_t parity)
 {
     uint8_t *buf = ring();
     uint64_t *bars = ring_bars();
-    const int ring_bytes = misc().ring_bytes, xc = misc().xc;
-    const int lane = threadIdx.x & 31, q = lane >> 2, sub = lane & 3;
+    const int ring_bytes = head().ring_bytes, xc = head().xc;
+    const int lane = thread_id() & 31, q = lane >> 2, sub = lane & 3;
     const int v = 1 << lv, rpp = 8 >> lv, cq = q & (v - 1), rq = q >> lv, W = 4 << lv;
     const int groups = (bpr + v - 1) >> lv, ur = RU * rpp;
     const uint32_t row_bytes = bpr * F::kBlockBytes, sb = stage_bytes_of(ur * row_bytes);
@@ -405,7 +426,7 @@ __device__ __noinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, int r
 }
 
 // Item range of work warp `gid` in a split; n = 0 if it has no part.
-__device__ __forceinline__ void share(const Split &sp, int gid, int &i0, int &n)
+__device__ __forceinline__ void share(const volatile Split &sp, int gid, int &i0, int &n)
 {
     const int i = gid - sp.w0;
     const bool in = i >= 0 && i < sp.nw;
@@ -438,9 +459,9 @@ __device__ __forceinline__ uint32_t pack2(float a, float b)
 }
 
 // A head's 128 values, four per lane at lane + 32 i: RMS norm (w may be null) and rotation.
-__device__ __noinline__ float4 norm_rope(float4 v, const float *w, float eps, const float *cos_t, const float *sin_t)
+__device__ __forceinline__ float4 norm_rope(float4 v, const float *w, float eps, const float *cos_t, const float *sin_t)
 {
-    const int lane = threadIdx.x & 31;
+    const int lane = thread_id() & 31;
     const float ss = warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
     if (w) {
         const float f = 1.0f / sqrtf(ss * (1.0f / 128.0f) + eps);
@@ -456,7 +477,7 @@ __device__ __noinline__ float4 norm_rope(float4 v, const float *w, float eps, co
 // K / V rows of a tile of 16 positions, a row per lane
 __device__ __forceinline__ void load_kv(const __half *kv_k, const __half *kv_v, int tile, int pos, int n_kv, int kvh)
 {
-    const int lane = threadIdx.x & 31;
+    const int lane = thread_id() & 31;
     uint8_t *buf = ring();
     uint64_t *bar = ring_bars();
     if (lane == 0) mbar_expect_tx(bar, 32 * 256);
@@ -465,17 +486,17 @@ __device__ __forceinline__ void load_kv(const __half *kv_k, const __half *kv_v, 
     bulk_g2s(buf + lane * kKvPitch, (lane < 16 ? kv_k : kv_v) + ((size_t)p * n_kv + kvh) * 128, 256, bar);
 }
 
-// This warp's tiles (tile, tile + 16, ... < t1; the first has been requested into the ring) for the 16 query heads whose
+// This warp's tiles (tile, tile + kWarps, ... < t1; the first has been requested into the ring) for the 16 query heads whose
 // fragments are in shared memory at 0 (hi halves) and 4096 (lo): leaves the unnormalised result [16][kPitch] in the ring, the
 // running maxima (log2 domain) and sums in M.am / M.al. The tile of the newest position takes its K and V from the projections
 // and, with store, writes them to the cache. Returns the ring's parities.
-__device__ __noinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_kv, int kvh, __half *kv_k, __half *kv_v, bool store,
+__device__ __forceinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_kv, int kvh, __half *kv_k, __half *kv_v, bool store,
                                             const uint2 *c_k, const uint2 *c_v, uint32_t tag, const float *k_norm, float eps,
                                             const float *cos_t, const float *sin_t, uint32_t parity)
 {
     uint8_t *buf = ring();
     Misc &M = misc();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int lane = thread_id() & 31, warp = thread_id() >> 5, g = lane >> 2, t = lane & 3;
     uint64_t *bars = M.bars[warp];
     float O[16][4];
 #pragma unroll
@@ -514,7 +535,7 @@ __device__ __noinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_kv,
         for (int n = 0; n < 2; n++)
 #pragma unroll
             for (int e = 0; e < 4; e++) S[n][e] = T[n][e] = 0.0f;
-#pragma unroll
+#pragma unroll 1
         for (int jj = 0; jj < 4; jj++) {
             const uint8_t *f = smem + kX + (2 * jj * 32 + lane) * 16;
             const uint4 h0 = *reinterpret_cast<const uint4 *>(f), h1 = *reinterpret_cast<const uint4 *>(f + 512);
@@ -601,57 +622,62 @@ __device__ __noinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_kv,
     return parity;
 }
 
-// Warp h (< nh) brings query head h0 + h into the fragments (hi + lo halves of q * scale * log2 e); the others' rows are zero.
-__device__ __noinline__ void q_fragments(const uint2 *c_q, uint32_t tag, bool live, const float *q_norm, float eps, const float *cos_t,
+// The warps bring nh query heads (128 cells each) into the fragments (hi + lo halves of q * scale * log2 e); the other rows are zero.
+__device__ __forceinline__ void q_fragments(const uint2 *c_q, uint32_t tag, int nh, const float *q_norm, float eps, const float *cos_t,
                                          const float *sin_t, float sc)
 {
-    Misc &M = misc();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (live) {
-        wait_values4(c_q + lane, tag, v);
-        __syncwarp();
-        const float4 r = norm_rope(make_float4(v[0], v[1], v[2], v[3]), q_norm, eps, cos_t, sin_t);
-        v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
-    }
+    const int lane = thread_id() & 31;
+#pragma unroll 1
+    for (int h = thread_id() >> 5; h < 16; h += kWarps) {
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (h < nh) {
+            wait_values4(c_q + h * 128 + lane, tag, v);
+            __syncwarp();
+            const float4 r = norm_rope(make_float4(v[0], v[1], v[2], v[3]), q_norm, eps, cos_t, sin_t);
+            v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
+        }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int d = lane + 32 * i, kk = d & 15;
-        const int at = ((d >> 4) * 32 + (warp & 7) * 4 + ((kk & 7) >> 1)) * 16 + ((warp >> 3) + 2 * (kk >> 3)) * 4 + (kk & 1) * 2;
-        const float s = v[i] * sc;
-        const __half hi = __float2half_rn(s);
-        *reinterpret_cast<__half *>(smem + kX + at) = hi;
-        *reinterpret_cast<__half *>(smem + kX + 4096 + at) = __float2half_rn(s - __half2float(hi));
+        for (int i = 0; i < 4; i++) {
+            const int d = lane + 32 * i, kk = d & 15;
+            const int at = ((d >> 4) * 32 + (h & 7) * 4 + ((kk & 7) >> 1)) * 16 + ((h >> 3) + 2 * (kk >> 3)) * 4 + (kk & 1) * 2;
+            const float s = v[i] * sc;
+            const __half hi = __float2half_rn(s);
+            *reinterpret_cast<__half *>(smem + kX + at) = hi;
+            *reinterpret_cast<__half *>(smem + kX + 4096 + at) = __float2half_rn(s - __half2float(hi));
+        }
     }
 }
 
 // The CTA's partial of nw warps: one head per warp, four dims per lane, into the cells of slot `slot`.
-__device__ __noinline__ void attn_partial(int nw, uint2 *c_part, uint2 *c_ml, int slot, uint32_t tag)
+__device__ __forceinline__ void attn_partial(int nw, int nh, uint2 *c_part, uint2 *c_ml, int slot, uint32_t tag)
 {
     Misc &M = misc();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float m = -INFINITY, s = 0.0f;
+    const int lane = thread_id() & 31;
 #pragma unroll 1
-    for (int w = 0; w < nw; w++) m = fmaxf(m, M.am[w][warp]);
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int h = thread_id() >> 5; h < nh; h += kWarps) {
+        float m = -INFINITY, s = 0.0f;
 #pragma unroll 1
-    for (int w = 0; w < nw; w++) {
-        const float f = exp2f(M.am[w][warp] - m);
-        const float4 o = *reinterpret_cast<const float4 *>(smem + M.off_ring + w * M.ring_bytes + (warp * kPitch + 4 * lane) * 4);
-        s = fmaf(M.al[w][warp], f, s);
-        a.x = fmaf(o.x, f, a.x); a.y = fmaf(o.y, f, a.y); a.z = fmaf(o.z, f, a.z); a.w = fmaf(o.w, f, a.w);
+        for (int w = 0; w < nw; w++) m = fmaxf(m, M.am[w][h]);
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+        for (int w = 0; w < nw; w++) {
+            const float f = exp2f(M.am[w][h] - m);
+            const float4 o = *reinterpret_cast<const float4 *>(smem + head().off_ring + w * head().ring_bytes + (h * kPitch + 4 * lane) * 4);
+            s = fmaf(M.al[w][h], f, s);
+            a.x = fmaf(o.x, f, a.x); a.y = fmaf(o.y, f, a.y); a.z = fmaf(o.z, f, a.z); a.w = fmaf(o.w, f, a.w);
+        }
+        uint2 *p = c_part + ((size_t)slot * 16 + h) * 128 + 4 * lane;
+        st_cells2(p, a.x, a.y, tag);
+        st_cells2(p + 2, a.z, a.w, tag);
+        if (lane == 0) st_cells2(c_ml + ((size_t)slot * 16 + h) * 2, m, s, tag);
     }
-    uint2 *p = c_part + ((size_t)slot * 16 + warp) * 128 + 4 * lane;
-    st_cells2(p, a.x, a.y, tag);
-    st_cells2(p + 2, a.z, a.w, tag);
-    if (lane == 0) st_cells2(c_ml + ((size_t)slot * 16 + warp) * 2, m, s, tag);
 }
 
 // Merges the nc chunks' partials of one head (hq of head block b): the CTA's warps over the chunks; cells of the result.
-__device__ __noinline__ void merge_head(int b, int hq, int nc, int chunks, const uint2 *c_part, const uint2 *c_ml, uint2 *dst, uint32_t tag)
+__device__ __forceinline__ void merge_head(int b, int hq, int nc, int chunks, const uint2 *c_part, const uint2 *c_ml, uint2 *dst, uint32_t tag)
 {
     Misc &M = misc();
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = thread_id(), lane = tid & 31, warp = tid >> 5;
     float m = -INFINITY, s = 0.0f;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
@@ -741,15 +767,17 @@ __device__ __noinline__ void walk(int n, int k)
 
 // The k largest of n logits (every thread of the CTA calls it): lane i < k of every warp returns the i-th expert, the weights go
 // to M.swt (visible after the next barrier of the CTA). -1: the CTA has given up.
-__device__ __noinline__ int select_experts(const uint2 *cells, uint32_t tag, int n, int k)
+__device__ __forceinline__ int select_experts(const uint2 *cells, uint32_t tag, int n, int k)
 {
     Misc &M = misc();
-    const int tid = threadIdx.x, lane = tid & 31;
+    const int tid = thread_id(), lane = tid & 31;
+    static_assert(kWork >= kMaxExperts, "a thread per logit");
     if (tid < kMaxExperts) M.key[tid] = tid < n ? ordered(wait_value(cells + tid, tag)) : 0;
     if (cta_aborted()) return -1;
     {
-        const int e = tid >> 1, half = (n + 1) >> 1, lo = (tid & 1) ? half : 0, hi = (tid & 1) ? n : half;
-        if (e - (lane >> 1) < n) {  // warp-uniform
+        const int half = (n + 1) >> 1, lo = (tid & 1) ? half : 0, hi = (tid & 1) ? n : half;
+#pragma unroll 1
+        for (int e = tid >> 1; e - (lane >> 1) < n; e += kWork / 2) {  // warp-uniform; two threads per expert
             const uint32_t me = M.key[e];
             int rank = 0;
 #pragma unroll 8
@@ -788,13 +816,13 @@ __device__ __forceinline__ void issue_pair(const uint8_t *experts, size_t estrid
     bulk_g2s(dst + half, src + up_off, half, bar);
 }
 // id: lane i holds the i-th routed expert. Writes SwiGLU's result as cells act[slot * EFF + row].
-__device__ __noinline__ uint32_t gate_up(const uint8_t *experts, size_t estride, uint32_t up_off, int id, int i0, int n, int ipe, uint32_t magic,
+__device__ __forceinline__ uint32_t gate_up(const uint8_t *experts, size_t estride, uint32_t up_off, int id, int i0, int n, int ipe, uint32_t magic,
                                          int bpr, int lv, int EFF, uint2 *act, uint32_t tag, uint32_t parity)
 {
     uint8_t *buf = ring();
     uint64_t *bars = ring_bars();
-    const int ring_bytes = misc().ring_bytes, xc = misc().xc;
-    const int lane = threadIdx.x & 31, q = lane >> 2, sub = lane & 3;
+    const int ring_bytes = head().ring_bytes, xc = head().xc;
+    const int lane = thread_id() & 31, q = lane >> 2, sub = lane & 3;
     const int v = 1 << lv, rpp = 8 >> lv, cq = q & (v - 1), rq = q >> lv, W = 4 << lv;
     const int groups = (bpr + v - 1) >> lv;
     const uint32_t row_bytes = bpr * kQ4KBlock, half = rpp * row_bytes, sb = 2 * half;
@@ -841,175 +869,227 @@ __device__ __noinline__ uint32_t gate_up(const uint8_t *experts, size_t estride,
     return parity;
 }
 
-__global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant__ Params P)
+__global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant__ Params params)
 {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cta = blockIdx.x, grid = gridDim.x;
+    const int tid = thread_id(), lane = tid & 31, warp = tid >> 5, cta = cta_id(), grid = gridDim.x;
     Misc &M = misc();
+    const volatile Head &P = M.head;
+    {
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(static_cast<const Head *>(&params));
+        for (int i = tid; i < static_cast<int>(sizeof(Head) / 4); i += kWork) reinterpret_cast<uint32_t *>(&M.head)[i] = src[i];
+    }
     if (tid < kWarps * kStages) mbar_init(&M.bars[0][0] + tid, 1);
     if (tid == kWork - 1) {
         mbar_init(&M.row_bar, 1);
         M.abort_flag = 0;
-        M.xc = P.xc;
-        M.off_row = P.off_row;
-        M.off_ring = P.off_ring;
-        M.ring_bytes = P.ring_bytes;
     }
-    // What a warp does in every layer; kept in shared memory (registers would be saved and restored around every step)
-    const volatile int *own = M.own[warp];
+    __syncthreads();
+    // What a warp does in every layer, in shared memory: it is looked up once per operation
     if (lane == 0) {
-        int *o = M.own[warp];
         const int gid = warp * grid + cta;
         int i0, n, m = 0;
         share(P.sq, gid, i0, n);  // rows of one of the three matrices behind the first norm
         if (gid >= P.sk.w0) { m = 1; share(P.sk, gid, i0, n); }
         if (gid >= P.sv.w0) { m = 2; share(P.sv, gid, i0, n); }
-        o[oQ0] = i0 << (3 - P.mH.lv);
-        o[oQn] = n << (3 - P.mH.lv);
-        o[oQm] = m;
+        M.own[warp][kQKV] = make_int2(i0 << (3 - P.mH.lv), n << (3 - P.mH.lv));
+        M.own_qm[warp] = m;
         share(P.so, gid, i0, n);
-        o[oO0] = i0 << (3 - P.mQ.lv);
-        o[oOn] = n << (3 - P.mQ.lv);
+        M.own[warp][kO] = make_int2(i0 << (3 - P.mQ.lv), n << (3 - P.mQ.lv));
         share(P.sg, gid, i0, n);
-        o[oG0] = i0;
-        o[oGn] = n;
+        M.own[warp][kExperts] = make_int2(i0, n);
         // down: the CTA's rows, shared by the warps of a slot
         const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid), R1 = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid);
         const int wps = kWarps / P.k, slot = warp / wps, part = warp - slot * wps, per = (R1 - R0 + wps - 1) / wps;
-        o[oD0] = R0 + part * per;
-        o[oDn] = slot < P.k ? max(0, min(per, R1 - R0 - part * per)) : 0;
+        M.own[warp][kDown] = make_int2(R0 + part * per, slot < P.k ? max(0, min(per, R1 - R0 - part * per)) : 0);
     }
     mbar_fence_init();
     __syncthreads();
-    auto prefetch_qkv = [&](int l) {
-        const Layer &L = P.L[l];
-        const int qm = own[oQm];
-        const bool q6 = qm == 2 && L.v_q6;
-        const uint8_t *w = qm == 0 ? L.wq : qm == 1 ? L.wk : L.wv;
-        return prefetch(w, own[oQ0], own[oQn], P.mH.bpr * (q6 ? kQ6KBlock : kQ4KBlock), (q6 ? 1 : 2) << (3 - P.mH.lv));
-    };
+    const bool has_row = cta < P.n_experts;
     auto request_row = [&](int l) {
         mbar_expect_tx(&M.row_bar, P.H * 4);
-        bulk_g2s(smem + P.off_row, P.L[l].router + (size_t)blockIdx.x * P.H, P.H * 4, &M.row_bar);
+        bulk_g2s(smem + P.off_row, params.L[l].router + (size_t)cta_id() * P.H, P.H * 4, &M.row_bar);
     };
-    uint32_t parity = 0;
-    uint32_t pend = prefetch_qkv(0);  // stages in flight while the CTA may still give up
-    const bool has_row = cta < P.n_experts;
     int row_pend = has_row ? 0 : -1;  // parity of the router row on its way
     if (has_row && tid == 0) request_row(0);
-    if (P.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (tid == 0) {
-        // arrivals of the launches before this one (nobody of this launch arrives before every CTA has read it: the last layer
-        // needs the activations of all of them); the quotient by a multiplication, a 64-bit division is a hundred instructions
-        unsigned long long c;
-        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(P.ctr) : "memory");
-        unsigned long long n = static_cast<unsigned long long>(__ull2double_rz(c) * P.inv_grid);
-        const long long r = static_cast<long long>(c - n * grid);
-        if (r < 0) n--;
-        if (r >= grid) n++;
-        M.launch = n;
-    }
-    __syncthreads();
-    uint32_t tag = static_cast<uint32_t>(M.launch) * 128u;
-    const int pos = __ldcg(P.pos);
-    bool ok = true;
 
+    uint32_t parity = 0, pend = 0, tag = 0;  // pend: stages in flight while the CTA may still give up
+    int pos = 0, nc = 0, id = 0;             // nc: chunks of positions; id: lane i holds the i-th routed expert
+    float res = 0.0f;                        // residual of this thread's row of the down projection
+    bool ok = true;
+    // One pass of the loop: an operation (there is one copy of every step's code), preceded by the request for its weights. The
+    // pass before the first only requests.
 #pragma unroll 1
-    for (int l = 0; l < P.n_layers; l++) {
-        const Layer &L = P.L[l];
-        tag++;
-        // ---- Q, K, V ----
-        ok = !stage_vec(l == 0 ? static_cast<const void *>(P.hidden) : P.c_h0, l == 0 ? 0 : tag - 1, P.H, L.attn_norm, P.eps, nullptr);
-        if (!ok) break;
-        {
-            const int qm = own[oQm];
-            uint2 *dst = qm == 0 ? P.c_q : qm == 1 ? P.c_k : P.c_v;
-            const uint8_t *w = qm == 0 ? L.wq : qm == 1 ? L.wk : L.wv;
-            if (qm == 2 && L.v_q6)
-                parity = matvec<Q6, 1>(w, P.mH.bpr, P.mH.lv, own[oQ0], own[oQn], dst, tag, nullptr, 0, parity);
-            else
-                parity = matvec<Q4, 2>(w, P.mH.bpr, P.mH.lv, own[oQ0], own[oQn], dst, tag, nullptr, 0, parity);
-            pend = 0;
-        }
-        // ---- attention of this CTA's positions ----
-        const int tpc = ((pos >> 4) + P.chunks) / P.chunks, nc = ((pos >> 4) + tpc) / tpc;  // tiles of 16 positions per chunk, chunks
-        {
-            const int ab = cta / P.chunks, ac = cta - ab * P.chunks;  // head block and chunk
-            if (ab < P.n_kv * P.qblocks && ac < nc) {
-                const int kvh = ab / P.qblocks, qb = ab - kvh * P.qblocks;
-                const int tile0 = ac * tpc + warp, tile1 = min((ac + 1) * tpc, (pos >> 4) + 1);
-                if (tile0 < tile1) {
-                    load_kv(L.kv_k, L.kv_v, tile0, pos, P.n_kv, kvh);
-                    pend = 1;
+    for (int it = -1, l = 0, op = kDown;; it++) {
+        const int tid = thread_id(), lane = tid & 31, warp = tid >> 5, cta = cta_id();
+        if (it >= 0) {
+            const Layer &L = params.L[l];
+            // ---- the input vector ----
+            {
+                const void *src = P.c_act;
+                const float *norm_w = nullptr;
+                uint32_t t = tag;
+                int K = P.k * P.EFF;
+                uint2 *logit = nullptr;
+                if (op == kQKV) {
+                    src = l == 0 ? static_cast<const void *>(P.hidden) : P.c_h0;
+                    t = l == 0 ? 0 : tag - 1;
+                    norm_w = L.attn_norm;
+                    K = P.H;
+                } else if (op == kO) {
+                    src = P.c_attn;
+                    K = P.QD;
+                } else if (op == kExperts) {  // the router logit of this CTA's expert on the way
+                    src = P.c_h1;
+                    norm_w = L.ffn_norm;
+                    K = P.H;
+                    logit = has_row ? P.c_logit + cta : nullptr;
+                    if (has_row) wait_copy(&M.row_bar, l & 1);
+                    row_pend = -1;
                 }
-                cta_sync();  // the staged vector has been read
-                const int nh = min(16, P.gqa - qb * 16);
-                q_fragments(P.c_q + (kvh * P.gqa + qb * 16 + warp) * 128, tag, warp < nh, L.q_norm, P.eps, P.cos_t, P.sin_t, P.scale * kLog2e);
-                ok = !cta_aborted();
+                ok = !stage_vec(src, t, K, norm_w, P.eps, logit);
                 if (!ok) break;
-                if (tile0 < tile1)
-                    parity = attn_tiles(tile0, tile1, pos, P.n_kv, kvh, L.kv_k, L.kv_v, qb == 0, P.c_k, P.c_v, tag, L.k_norm, P.eps, P.cos_t,
-                                        P.sin_t, parity);
+            }
+            // ---- its rows ----
+            if (op == kExperts) {
+                if (has_row && l + 1 < P.n_layers) {
+                    row_pend = (l + 1) & 1;
+                    if (tid == 0) request_row(l + 1);
+                }
+                id = select_experts(P.c_logit, tag, P.n_experts, P.k);
+                ok = id >= 0;
+                if (!ok) break;
+                const int2 own = M.own[warp][kExperts];
+                parity = gate_up(L.experts, L.estride, L.up_off, id, own.x, own.y, P.ipe, P.ipe_magic, P.mH.bpr, P.mH.lv, P.EFF, P.c_act, tag,
+                                 parity);
+            } else {
+                const int2 own = M.own[warp][op];
+                const int qm = M.own_qm[warp], slot = warp / (kWarps / P.k);
+                const uint8_t *w = qm == 0 ? L.wq : qm == 1 ? L.wk : L.wv;
+                void *dst = qm == 0 ? P.c_q : qm == 1 ? P.c_k : P.c_v;
+                const float *add = nullptr;
+                uint32_t t = tag;
+                bool q6 = qm == 2 && L.v_q6;
+                int bpr = P.mH.bpr, lv = P.mH.lv, xcol = 0;
+                if (op == kO) {
+                    w = L.wo;
+                    dst = P.c_h1;
+                    add = M.res[warp];
+                    q6 = false;
+                    bpr = P.mQ.bpr;
+                    lv = P.mQ.lv;
+                } else if (op == kDown) {
+                    w = L.experts + (size_t)__shfl_sync(0xffffffffu, id, slot & 31) * L.estride + L.down_off;
+                    dst = M.part[slot < P.k ? slot : 0] - static_cast<int>(static_cast<unsigned>(P.H) * cta / grid);
+                    t = 0;
+                    q6 = L.down_q6;
+                    bpr = P.mE.bpr;
+                    lv = P.mE.lv;
+                    xcol = slot * bpr;
+                }
+                if (q6)
+                    parity = matvec<Q6, 2>(w, bpr, lv, own.x, own.y, dst, t, add, xcol, parity);
+                else
+                    parity = matvec<Q4, 4>(w, bpr, lv, own.x, own.y, dst, t, add, xcol, parity);
                 pend = 0;
-                cta_sync();
-                attn_partial(min(kWarps, tile1 - ac * tpc), P.c_part, P.c_ml, ab * P.chunks + ac, tag);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the ring was written and read as plain memory
+            }
+            // ---- attention of this CTA's positions ----
+            if (op == kQKV) {
+                const int tpc = ((pos >> 4) + P.chunks) / P.chunks;  // tiles of 16 positions per chunk
+                nc = ((pos >> 4) + tpc) / tpc;
+                const int ab = cta / P.chunks, ac = cta - ab * P.chunks;  // head block and chunk
+                if (ab < P.n_kv * P.qblocks && ac < nc) {
+                    const int kvh = ab / P.qblocks, qb = ab - kvh * P.qblocks;
+                    const int tile0 = ac * tpc + warp, tile1 = min((ac + 1) * tpc, (pos >> 4) + 1);
+                    if (tile0 < tile1) {
+                        load_kv(L.kv_k, L.kv_v, tile0, pos, P.n_kv, kvh);
+                        pend = 1;
+                    }
+                    cta_sync();  // the staged vector has been read
+                    const int nh = min(16, P.gqa - qb * 16);
+                    q_fragments(P.c_q + (kvh * P.gqa + qb * 16) * 128, tag, nh, L.q_norm, P.eps, P.cos_t, P.sin_t,
+                                P.scale * kLog2e);
+                    ok = !cta_aborted();
+                    if (!ok) break;
+                    if (tile0 < tile1)
+                        parity = attn_tiles(tile0, tile1, pos, P.n_kv, kvh, L.kv_k, L.kv_v, qb == 0, P.c_k, P.c_v, tag, L.k_norm, P.eps,
+                                            P.cos_t, P.sin_t, parity);
+                    pend = 0;
+                    cta_sync();
+                    attn_partial(min(kWarps, tile1 - ac * tpc), nh, P.c_part, P.c_ml, ab * P.chunks + ac, tag);
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the ring was written and read as plain memory
+                }
+            }
+            cta_sync();  // the staged vector and the ring have been read
+        }
+        // ---- the next operation's weights; gate / up requests its own: they depend on the routing ----
+        const int next = (op + 1) & 3, ln = l + (op == kDown && it >= 0 ? 1 : 0);
+        if (ln < P.n_layers && next != kExperts) {
+            const Layer &L = params.L[ln];
+            const int2 own = M.own[warp][next];
+            const int qm = M.own_qm[warp];
+            const uint8_t *w = qm == 0 ? L.wq : qm == 1 ? L.wk : L.wv;
+            bool q6 = qm == 2 && L.v_q6;
+            int bpr = P.mH.bpr, lv = P.mH.lv;
+            if (next == kO) {
+                w = L.wo;
+                q6 = false;
+                bpr = P.mQ.bpr;
+                lv = P.mQ.lv;
+            } else if (next == kDown) {
+                w = L.experts + (size_t)__shfl_sync(0xffffffffu, id, (warp / (kWarps / P.k)) & 31) * L.estride + L.down_off;
+                q6 = L.down_q6;
+                bpr = P.mE.bpr;
+                lv = P.mE.lv;
+            }
+            pend = prefetch(w, own.x, own.y, bpr * (q6 ? kQ6KBlock : kQ4KBlock), (q6 ? 2 : 4) << (3 - lv));
+        }
+        if (it < 0) {
+            if (P.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
+            if (tid == 0) {
+                // arrivals of the launches before this one (nobody of this launch arrives before every CTA has read it: the last
+                // layer needs the activations of all of them); the quotient by a multiplication, a 64-bit division is a hundred
+                // instructions
+                unsigned long long c;
+                asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(P.ctr) : "memory");
+                unsigned long long n = static_cast<unsigned long long>(__ull2double_rz(c) * P.inv_grid);
+                const long long r = static_cast<long long>(c - n * grid);
+                if (r < 0) n--;
+                if (r >= grid) n++;
+                M.launch = n;
+            }
+            __syncthreads();
+            tag = static_cast<uint32_t>(M.launch) * 128u + 1u;
+            pos = __ldcg(P.pos);
+        } else if (op == kQKV) {
+            const int2 own = M.own[warp][kO];
+            if (lane < own.y) M.res[warp][lane] = l == 0 ? __ldcg(P.hidden + own.x + lane) : wait_value(P.c_h0 + own.x + lane, tag - 1);
+            if (cta < P.n_heads) {
+                const int kv = cta / P.gqa, hq = cta - kv * P.gqa;
+                merge_head(kv * P.qblocks + (hq >> 4), hq & 15, nc, P.chunks, P.c_part, P.c_ml, P.c_attn + cta * 128, tag);
+            }
+        } else if (op >= kExperts) {
+            const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid),
+                      rows = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid) - R0;
+            if (tid < rows) {
+                if (op == kExperts) {
+                    res = wait_value(P.c_h1 + R0 + tid, tag);
+                } else {
+                    float y = 0.0f;
+#pragma unroll 4
+                    for (int i = 0; i < P.k; i++) y = fmaf(M.swt[i], M.part[i][tid], y);
+                    if (ln < P.n_layers)
+                        st_cell(P.c_h0 + R0 + tid, res + y, tag);
+                    else
+                        P.hidden[R0 + tid] = res + y;
+                }
+            }
+            if (op == kDown) {
+                if (ln == P.n_layers) break;
+                tag++;
             }
         }
-        cta_sync();
-        // ---- O projection + residual ----
-        pend = prefetch(L.wo, own[oO0], own[oOn], P.mQ.bpr * kQ4KBlock, 2 << (3 - P.mQ.lv));
-        if (lane < own[oOn]) M.res[warp][lane] = l == 0 ? __ldcg(P.hidden + own[oO0] + lane) : wait_value(P.c_h0 + own[oO0] + lane, tag - 1);
-        if (cta < P.n_heads) {
-            const int kv = cta / P.gqa, hq = cta - kv * P.gqa;
-            merge_head(kv * P.qblocks + (hq >> 4), hq & 15, nc, P.chunks, P.c_part, P.c_ml, P.c_attn + cta * 128, tag);
-        }
-        ok = !stage_vec(P.c_attn, tag, P.QD, nullptr, 0.0f, nullptr);
-        if (!ok) break;
-        parity = matvec<Q4, 2>(L.wo, P.mQ.bpr, P.mQ.lv, own[oO0], own[oOn], P.c_h1, tag, M.res[warp], 0, parity);
-        pend = 0;
-        // ---- router logit of this CTA's expert; the normalised vector stays staged for gate / up ----
-        if (has_row && !mbar_try_wait(&M.row_bar, l & 1)) wait_slow(&M.row_bar, l & 1);
-        row_pend = -1;
-        cta_sync();  // the staged vector has been read
-        ok = !stage_vec(P.c_h1, tag, P.H, L.ffn_norm, P.eps, has_row ? P.c_logit + cta : nullptr);
-        if (!ok) break;
-        if (has_row && l + 1 < P.n_layers) {
-            row_pend = (l + 1) & 1;
-            if (tid == 0) request_row(l + 1);
-        }
-        const int id = select_experts(P.c_logit, tag, P.n_experts, P.k);
-        ok = id >= 0;
-        if (!ok) break;
-        // ---- experts ----
-        parity = gate_up(L.experts, L.estride, L.up_off, id, own[oG0], own[oGn], P.ipe, P.ipe_magic, P.mH.bpr, P.mH.lv, P.EFF, P.c_act, tag, parity);
-        const int slot = warp / (kWarps / P.k), R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid),
-                  rows = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid) - R0;
-        const uint8_t *down = L.experts + (size_t)__shfl_sync(0xffffffffu, id, slot & 31) * L.estride + L.down_off;
-        pend = prefetch(down, own[oD0], own[oDn], P.mE.bpr * (L.down_q6 ? kQ6KBlock : kQ4KBlock), (L.down_q6 ? 1 : 2) << (3 - P.mE.lv));
-        const float res = tid < rows ? wait_value(P.c_h1 + R0 + tid, tag) : 0.0f;
-        cta_sync();  // the staged vector has been read
-        ok = !stage_vec(P.c_act, tag, P.k * P.EFF, nullptr, 0.0f, nullptr);
-        if (!ok) break;
-        {
-            float *dst = M.part[slot < P.k ? slot : 0] - R0;
-            if (L.down_q6)
-                parity = matvec<Q6, 1>(down, P.mE.bpr, P.mE.lv, own[oD0], own[oDn], dst, 0, nullptr, slot * P.mE.bpr, parity);
-            else
-                parity = matvec<Q4, 2>(down, P.mE.bpr, P.mE.lv, own[oD0], own[oDn], dst, 0, nullptr, slot * P.mE.bpr, parity);
-            pend = 0;
-        }
-        const bool more = l + 1 < P.n_layers;
-        if (more) pend = prefetch_qkv(l + 1);
-        cta_sync();
-        if (tid < rows) {
-            float y = 0.0f;
-#pragma unroll 1
-            for (int i = 0; i < P.k; i++) y = fmaf(M.swt[i], M.part[i][tid], y);
-            if (more)
-                st_cell(P.c_h0 + R0 + tid, res + y, tag);
-            else
-                P.hidden[R0 + tid] = res + y;
-        }
+        op = next;
+        l = ln;
     }
     if (P.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (!ok) {  // given up: leave after the copies in flight
@@ -1031,7 +1111,7 @@ Map map_of(int cols)
     if (m.lv < 2 && m.bpr >= 8) m.lv = 3;  // a ragged last group costs less than single blocks side by side
     return m;
 }
-int stage_rows(const Map &m, bool q6) { return (q6 ? 1 : 2) << (3 - m.lv); }
+int stage_rows(const Map &m, bool q6) { return (q6 ? 2 : 4) << (3 - m.lv); }
 int stage_of(const Map &m, bool q6) { return stage_bytes_of(stage_rows(m, q6) * m.bpr * (q6 ? kQ6KBlock : kQ4KBlock)); }
 constexpr int kSmemBytes = 227 * 1024;
 
@@ -1062,7 +1142,7 @@ size_t scratch(Params &P, uint8_t *base)
 bool plan(Params &P)
 {
     const int grid = device_sms();
-    if (P.H % 256 || P.EFF % 256 || P.QD % 256 || P.H < 256 || P.EFF < 256 || P.QD < 256 || P.H > 8192) return false;
+    if (P.H % 256 || P.EFF % 256 || P.QD % 256 || P.H < 256 || P.EFF < 256 || P.QD < 256 || P.H > 16 * kWork) return false;
     if (P.k < 1 || P.k > kMaxK || P.n_experts < P.k || P.n_experts > min(grid, kMaxExperts) || P.n_experts > 32 * P.k) return false;
     if (P.n_layers < 1 || P.n_layers > kMaxLayers) return false;
     P.qblocks = (P.gqa + 15) / 16;

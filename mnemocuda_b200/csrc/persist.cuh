@@ -30,7 +30,7 @@ struct Map {
     int bpr, lv;
 };
 
-struct Params {
+struct Head {
     int n_layers;
     int H, EFF, QD, KD, n_heads, n_kv, gqa, qblocks, chunks, n_experts, k;
     float eps, scale;
@@ -48,6 +48,9 @@ struct Params {
     Split sq, sk, sv, so, sg;  // passes of the four projections; gate / up items
     uint32_t ipe, ipe_magic;   // gate / up items per expert, 2^32 / ipe rounded up
     int xc, off_row, off_ring, ring_bytes;  // columns of the staged vector; byte offsets in shared memory
+};
+
+struct Params : Head {
     Layer L[kMaxLayers];
 };
 
