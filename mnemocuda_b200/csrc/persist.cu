@@ -74,9 +74,9 @@ struct Misc {
     unsigned long long launch;
     float red[2][kWarps];
     float am[kWarps][16], al[kWarps][16];  // attention: running maximum / sum per warp and head
-    float res[kWarps][16];                 // residual of a warp's rows of the O projection
+    float hid[kMaxDownRows];               // the CTA's rows of the hidden vector: it writes them in both of a layer's halves
     float part[kMaxK][kMaxDownRows];
-    uint32_t key[kMaxExperts];             // ordered logits
+    alignas(16) uint32_t key[kMaxExperts]; // ordered logits
     int top_id[kMaxK + 1];
     uint32_t top_key[kMaxK + 1];
     float swt[kMaxK];
@@ -370,9 +370,9 @@ __device__ __forceinline__ uint32_t prefetch(const uint8_t *w, int r0, int n, ui
     return (1u << count) - 1;
 }
 // Those rows (first units requested by prefetch() with the same arguments) times the staged vector from super-block xcol on:
-// dst[row] = value (+ add[row - r0]), as a cell if tag != 0. Returns the ring's parities.
+// dst[row] = value (with keep: added to keep[row], which takes the sum), as a cell if tag != 0. Returns the ring's parities.
 template <class F, int RU>
-__device__ __forceinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, int r0, int n, void *dst, uint32_t tag, const float *add, int xcol,
+__device__ __forceinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, int r0, int n, void *dst, uint32_t tag, float *keep, int xcol,
                                         uint32_t parity)
 {
     uint8_t *buf = ring();
@@ -414,7 +414,8 @@ __device__ __forceinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, in
         const float sum = stream::packed_sum<RU, false>(acc, W, lane, which);
         const int row = r + which * rpp + rq;
         if ((lane & (W / RU - 1)) == 0 && row < n) {
-            const float o = sum + (add ? add[row] : 0.0f);
+            float o = sum;
+            if (keep) keep[r0 + row] = o += keep[r0 + row];
             if (tag)
                 st_cell(static_cast<uint2 *>(dst) + r0 + row, o, tag);
             else
@@ -656,11 +657,12 @@ __device__ __forceinline__ void attn_partial(int nw, int nh, uint2 *c_part, uint
 #pragma unroll 1
     for (int h = thread_id() >> 5; h < nh; h += kWarps) {
         float m = -INFINITY, s = 0.0f;
-#pragma unroll 1
-        for (int w = 0; w < nw; w++) m = fmaxf(m, M.am[w][h]);
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) m = fmaxf(m, w < nw ? M.am[w][h] : -INFINITY);
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-        for (int w = 0; w < nw; w++) {
+#pragma unroll
+        for (int w = 0; w < kWarps; w++) {
+            if (w >= nw) break;
             const float f = exp2f(M.am[w][h] - m);
             const float4 o = *reinterpret_cast<const float4 *>(smem + head().off_ring + w * head().ring_bytes + (h * kPitch + 4 * lane) * 4);
             s = fmaf(M.al[w][h], f, s);
@@ -681,13 +683,13 @@ __device__ __forceinline__ void merge_head(int b, int hq, int nc, int chunks, co
     float m = -INFINITY, s = 0.0f;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
-    for (int c0 = warp; c0 < nc; c0 += 3 * kWarps) {
-        uint4 ms[3], o0[3], o1[3];
+    for (int c0 = warp; c0 < nc; c0 += 5 * kWarps) {
+        uint4 ms[5], o0[5], o1[5];
 #pragma unroll 1
         for (uint32_t i = 0;; i++) {
             bool ok = true;
 #pragma unroll
-            for (int u = 0; u < 3; u++) {
+            for (int u = 0; u < 5; u++) {
                 const size_t slot = ((size_t)b * chunks + min(c0 + u * kWarps, nc - 1)) * 16 + hq;
                 ms[u] = ld_cells2(c_ml + slot * 2);
                 o0[u] = ld_cells2(c_part + slot * 128 + 4 * lane);
@@ -699,7 +701,7 @@ __device__ __forceinline__ void merge_head(int b, int hq, int nc, int chunks, co
         }
         __syncwarp();
 #pragma unroll
-        for (int u = 0; u < 3; u++) {
+        for (int u = 0; u < 5; u++) {
             if (c0 + u * kWarps >= nc) break;
             const float mu = __uint_as_float(ms[u].x), mn = fmaxf(m, mu), fo = exp2f(m - mn), fn = exp2f(mu - mn);
             s = s * fo + __uint_as_float(ms[u].z) * fn;
@@ -710,7 +712,7 @@ __device__ __forceinline__ void merge_head(int b, int hq, int nc, int chunks, co
             m = mn;
         }
     }
-    float *buf = reinterpret_cast<float *>(smem + kX);  // [16][128]
+    float *buf = reinterpret_cast<float *>(smem + kX);  // [kWarps][128]
     *reinterpret_cast<float4 *>(buf + warp * 128 + 4 * lane) = a;
     if (lane == 0) {
         M.red[0][warp] = m;
@@ -719,9 +721,9 @@ __device__ __forceinline__ void merge_head(int b, int hq, int nc, int chunks, co
     cta_sync();
     if (tid < 128) {
         float mt = -INFINITY, st = 0.0f, o = 0.0f;
-#pragma unroll 1
+#pragma unroll
         for (int w = 0; w < kWarps; w++) mt = fmaxf(mt, M.red[0][w]);
-#pragma unroll 1
+#pragma unroll
         for (int w = 0; w < kWarps; w++) {
             const float f = exp2f(M.red[0][w] - mt);  // 0 for a warp without a chunk
             st = fmaf(M.red[1][w], f, st);
@@ -736,7 +738,7 @@ __device__ __forceinline__ void merge_head(int b, int hq, int nc, int chunks, co
 __device__ __forceinline__ uint32_t ordered(float v)
 {
     const uint32_t b = __float_as_uint(v + 0.0f);  // -0 counts as 0
-    return b ^ ((b >> 31) ? 0xFFFFFFFFu : 0x80000000u);
+    return min(b ^ ((b >> 31) ? 0xFFFFFFFFu : 0x80000000u), 0xFFFFFFFEu);
 }
 __device__ __forceinline__ float unordered(uint32_t k) { return __uint_as_float(k ^ ((k >> 31) ? 0x80000000u : 0xFFFFFFFFu)); }
 
@@ -775,13 +777,16 @@ __device__ __forceinline__ int select_experts(const uint2 *cells, uint32_t tag, 
     if (tid < kMaxExperts) M.key[tid] = tid < n ? ordered(wait_value(cells + tid, tag)) : 0;
     if (cta_aborted()) return -1;
     {
-        const int half = (n + 1) >> 1, lo = (tid & 1) ? half : 0, hi = (tid & 1) ? n : half;
+        const int half = ((n + 7) >> 3) * 4, lo = (tid & 1) ? half : 0, hi = lo + half;  // keys beyond n are 0
 #pragma unroll 1
         for (int e = tid >> 1; e - (lane >> 1) < n; e += kWork / 2) {  // warp-uniform; two threads per expert
             const uint32_t me = M.key[e];
             int rank = 0;
-#pragma unroll 8
-            for (int i = lo; i < hi; i++) rank += (M.key[i] > me || (M.key[i] == me && i < e)) ? 1 : 0;
+#pragma unroll 4
+            for (int i = lo; i < hi; i += 4) {  // an equal one before it counts as larger (a key is never the largest integer)
+                const uint4 o = *reinterpret_cast<const uint4 *>(&M.key[i]);
+                rank += (o.x + (i < e) > me) + (o.y + (i + 1 < e) > me) + (o.z + (i + 2 < e) > me) + (o.w + (i + 3 < e) > me);
+            }
             rank += __shfl_xor_sync(0xffffffffu, rank, 1);
             if (rank <= k && e < n && !(tid & 1)) {
                 M.top_id[rank] = e;
@@ -806,63 +811,62 @@ __device__ __forceinline__ int select_experts(const uint2 *cells, uint32_t tag, 
     return id;
 }
 
-// ---- gate / up: items [i0, i0 + n), item i = a pass of gate rows and the same up rows of the i / ipe-th routed expert ----
-__device__ __forceinline__ void issue_pair(const uint8_t *experts, size_t estride, uint32_t up_off, int id, uint32_t row_off, uint32_t half,
-                                           uint8_t *dst, uint64_t *bar)
+// ---- gate / up: items [i0, i0 + n), item i = a pass of gate rows and the same up rows of the i / ipe-th routed expert. Two items
+// a stage: their four products hide one another's latency, and one reduction serves them (a warp has 3 to 11 items). ----
+// Every lane calls it: lane 2 j + h requests half h (gate, up) of item i + j of the stage, j < 2.
+__device__ __forceinline__ void issue_items(const uint8_t *experts, size_t estride, uint32_t up_off, int id, int i, int end, int ipe, uint32_t magic,
+                                            uint32_t half, bool mine, int j, int h, uint8_t *dst, uint64_t *bar)
 {
-    const uint8_t *src = experts + (size_t)id * estride + row_off;
-    mbar_expect_tx(bar, 2 * half);
-    bulk_g2s(dst, src, half, bar);
-    bulk_g2s(dst + half, src + up_off, half, bar);
+    const int item = i + j, slot = __umulhi(item, magic);
+    const int ex = __shfl_sync(0xffffffffu, id, slot & 31);
+    const bool in = mine && item < end;
+    if (in && j == 0 && h == 0) mbar_expect_tx(bar, (i + 1 < end ? 4 : 2) * half);
+    __syncwarp();
+    if (in) bulk_g2s(dst + (2 * j + h) * half, experts + (size_t)ex * estride + (item - slot * ipe) * half + (h ? up_off : 0), half, bar);
 }
 // id: lane i holds the i-th routed expert. Writes SwiGLU's result as cells act[slot * EFF + row].
 __device__ __forceinline__ uint32_t gate_up(const uint8_t *experts, size_t estride, uint32_t up_off, int id, int i0, int n, int ipe, uint32_t magic,
-                                         int bpr, int lv, int EFF, uint2 *act, uint32_t tag, uint32_t parity)
+                                            int bpr, int lv, int EFF, uint2 *act, uint32_t tag, uint32_t parity)
 {
     uint8_t *buf = ring();
     uint64_t *bars = ring_bars();
     const int ring_bytes = head().ring_bytes, xc = head().xc;
     const int lane = thread_id() & 31, q = lane >> 2, sub = lane & 3;
     const int v = 1 << lv, rpp = 8 >> lv, cq = q & (v - 1), rq = q >> lv, W = 4 << lv;
-    const int groups = (bpr + v - 1) >> lv;
-    const uint32_t row_bytes = bpr * kQ4KBlock, half = rpp * row_bytes, sb = 2 * half;
+    const int groups = (bpr + v - 1) >> lv, end = i0 + n;
+    const uint32_t row_bytes = bpr * kQ4KBlock, half = rpp * row_bytes, sb = 4 * half;
     const int stages = min(kStages, ring_bytes / static_cast<int>(sb));
-    {
-        const int i = i0 + lane, slot = __umulhi(i, magic);
-        const int ex = __shfl_sync(0xffffffffu, id, slot & 31);
-        if (lane < min(stages, n)) issue_pair(experts, estride, up_off, ex, (i - slot * ipe) * half, half, buf + lane * sb, &bars[lane]);
-        __syncwarp();
-    }
+    const int ij = (lane >> 1) & 1, ih = lane & 1, is = lane >> 2;  // of a request: item, half, stage
+    issue_items(experts, estride, up_off, id, i0 + 2 * is, end, ipe, magic, half, is < stages, ij, ih, buf + is * sb, &bars[is < stages ? is : 0]);
     Q4::XRegs xr;
     int s = 0;
 #pragma unroll 1
-    for (int i = i0; i < i0 + n; i++) {
+    for (int i = i0; i < end; i += 2) {
         ring_wait(bars, s, parity);
         const uint8_t *base = buf + s * sb + rq * row_bytes;
-        float acc[2] = {0.0f, 0.0f};
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // gate, up of the two items
 #pragma unroll 1
         for (int c = 0; c < groups; c++) {
             const int col = (c << lv) + cq;
             const bool in = col < bpr;  // a ragged last group
             const int at = in ? col : 0;
             if (groups > 1 || i == i0) load_x(xr, xc, at, sub);
-            const float g = Q4::block_dot(base + at * kQ4KBlock, sub, xr);
-            const float u = Q4::block_dot(base + half + at * kQ4KBlock, sub, xr);
-            acc[0] += in ? g : 0.0f;
-            acc[1] += in ? u : 0.0f;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (u == 2 && i + 1 >= end) break;
+                const float d = Q4::block_dot(base + u * half + at * kQ4KBlock, sub, xr);
+                acc[u] += in ? d : 0.0f;
+            }
         }
         __syncwarp();
-        {
-            const int j = i + stages, slot = __umulhi(j, magic);
-            const int ex = __shfl_sync(0xffffffffu, id, slot & 31);
-            if (lane == 0 && j < i0 + n) issue_pair(experts, estride, up_off, ex, (j - slot * ipe) * half, half, buf + s * sb, &bars[s]);
-        }
+        issue_items(experts, estride, up_off, id, i + 2 * stages, end, ipe, magic, half, lane < 4, ij, ih, buf + s * sb, &bars[s]);
         int which;
-        const float g = stream::packed_sum<2, false>(acc, W, lane, which);
-        const float u = __shfl_xor_sync(0xffffffffu, g, W >> 1);  // which = 1 in the upper half of a row's lanes
-        if ((lane & (W - 1)) == 0) {
-            const int slot = __umulhi(i, magic);
-            st_cell(act + slot * EFF + (i - slot * ipe) * rpp + rq, g / (1.0f + expf(-g)) * u, tag);
+        const float g = stream::packed_sum<4, false>(acc, W, lane, which);
+        const float u = __shfl_xor_sync(0xffffffffu, g, W >> 2);  // which ^ 1: a quarter of the row's lanes away
+        const int item = i + (which >> 1);
+        if ((lane & (W / 4 - 1)) == 0 && !(which & 1) && item < end) {
+            const int slot = __umulhi(item, magic);
+            st_cell(act + slot * EFF + (item - slot * ipe) * rpp + rq, g / (1.0f + expf(-g)) * u, tag);
         }
         if (++s == stages) s = 0;
     }
@@ -893,13 +897,12 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
         if (gid >= P.sv.w0) { m = 2; share(P.sv, gid, i0, n); }
         M.own[warp][kQKV] = make_int2(i0 << (3 - P.mH.lv), n << (3 - P.mH.lv));
         M.own_qm[warp] = m;
-        share(P.so, gid, i0, n);
-        M.own[warp][kO] = make_int2(i0 << (3 - P.mQ.lv), n << (3 - P.mQ.lv));
         share(P.sg, gid, i0, n);
         M.own[warp][kExperts] = make_int2(i0, n);
-        // down: the CTA's rows, shared by the warps of a slot
+        // O, down: the CTA's rows of the hidden vector; down: shared by the warps of a slot
         const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid), R1 = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid);
         const int wps = kWarps / P.k, slot = warp / wps, part = warp - slot * wps, per = (R1 - R0 + wps - 1) / wps;
+        M.own[warp][kO] = make_int2(R0 + (R1 - R0) * warp / kWarps, (R1 - R0) * (warp + 1) / kWarps - (R1 - R0) * warp / kWarps);
         M.own[warp][kDown] = make_int2(R0 + part * per, slot < P.k ? max(0, min(per, R1 - R0 - part * per)) : 0);
     }
     mbar_fence_init();
@@ -914,7 +917,6 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
 
     uint32_t parity = 0, pend = 0, tag = 0;  // pend: stages in flight while the CTA may still give up
     int pos = 0, nc = 0, id = 0;             // nc: chunks of positions; id: lane i holds the i-th routed expert
-    float res = 0.0f;                        // residual of this thread's row of the down projection
     bool ok = true;
     // One pass of the loop: an operation (there is one copy of every step's code), preceded by the request for its weights. The
     // pass before the first only requests.
@@ -966,20 +968,21 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                 const int qm = M.own_qm[warp], slot = warp / (kWarps / P.k);
                 const uint8_t *w = qm == 0 ? L.wq : qm == 1 ? L.wk : L.wv;
                 void *dst = qm == 0 ? P.c_q : qm == 1 ? P.c_k : P.c_v;
-                const float *add = nullptr;
+                float *keep = nullptr;
+                const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid);
                 uint32_t t = tag;
                 bool q6 = qm == 2 && L.v_q6;
                 int bpr = P.mH.bpr, lv = P.mH.lv, xcol = 0;
                 if (op == kO) {
                     w = L.wo;
                     dst = P.c_h1;
-                    add = M.res[warp];
+                    keep = M.hid - R0;
                     q6 = false;
                     bpr = P.mQ.bpr;
                     lv = P.mQ.lv;
                 } else if (op == kDown) {
                     w = L.experts + (size_t)__shfl_sync(0xffffffffu, id, slot & 31) * L.estride + L.down_off;
-                    dst = M.part[slot < P.k ? slot : 0] - static_cast<int>(static_cast<unsigned>(P.H) * cta / grid);
+                    dst = M.part[slot < P.k ? slot : 0] - R0;
                     t = 0;
                     q6 = L.down_q6;
                     bpr = P.mE.bpr;
@@ -987,9 +990,9 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                     xcol = slot * bpr;
                 }
                 if (q6)
-                    parity = matvec<Q6, 2>(w, bpr, lv, own.x, own.y, dst, t, add, xcol, parity);
+                    parity = matvec<Q6, 2>(w, bpr, lv, own.x, own.y, dst, t, keep, xcol, parity);
                 else
-                    parity = matvec<Q4, 4>(w, bpr, lv, own.x, own.y, dst, t, add, xcol, parity);
+                    parity = matvec<Q4, 4>(w, bpr, lv, own.x, own.y, dst, t, keep, xcol, parity);
                 pend = 0;
             }
             // ---- attention of this CTA's positions ----
@@ -1060,33 +1063,30 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
             __syncthreads();
             tag = static_cast<uint32_t>(M.launch) * 128u + 1u;
             pos = __ldcg(P.pos);
+            const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid),
+                      rows = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid) - R0;
+            if (tid < rows) M.hid[tid] = __ldcg(P.hidden + R0 + tid);
         } else if (op == kQKV) {
-            const int2 own = M.own[warp][kO];
-            if (lane < own.y) M.res[warp][lane] = l == 0 ? __ldcg(P.hidden + own.x + lane) : wait_value(P.c_h0 + own.x + lane, tag - 1);
             if (cta < P.n_heads) {
                 const int kv = cta / P.gqa, hq = cta - kv * P.gqa;
                 merge_head(kv * P.qblocks + (hq >> 4), hq & 15, nc, P.chunks, P.c_part, P.c_ml, P.c_attn + cta * 128, tag);
             }
-        } else if (op >= kExperts) {
+        } else if (op == kDown) {
             const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid),
                       rows = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid) - R0;
             if (tid < rows) {
-                if (op == kExperts) {
-                    res = wait_value(P.c_h1 + R0 + tid, tag);
-                } else {
-                    float y = 0.0f;
+                float y = 0.0f;
 #pragma unroll 4
-                    for (int i = 0; i < P.k; i++) y = fmaf(M.swt[i], M.part[i][tid], y);
-                    if (ln < P.n_layers)
-                        st_cell(P.c_h0 + R0 + tid, res + y, tag);
-                    else
-                        P.hidden[R0 + tid] = res + y;
-                }
+                for (int i = 0; i < P.k; i++) y = fmaf(M.swt[i], M.part[i][tid], y);
+                y += M.hid[tid];
+                M.hid[tid] = y;
+                if (ln < P.n_layers)
+                    st_cell(P.c_h0 + R0 + tid, y, tag);
+                else
+                    P.hidden[R0 + tid] = y;
             }
-            if (op == kDown) {
-                if (ln == P.n_layers) break;
-                tag++;
-            }
+            if (ln == P.n_layers) break;
+            tag++;
         }
         op = next;
         l = ln;
@@ -1152,11 +1152,9 @@ bool plan(Params &P)
     P.mH = map_of(P.H);
     P.mQ = map_of(P.QD);
     P.mE = map_of(P.EFF);
-    const int warps = kWarps * grid, rpp = 8 >> P.mH.lv, rppQ = 8 >> P.mQ.lv;
+    const int warps = kWarps * grid, rpp = 8 >> P.mH.lv;
     // the O projection and the down projection must have rows for every CTA: what tells a writer that all have read
-    if (P.H / rppQ < grid) return false;
-    if ((P.H / rppQ + warps - 1) / warps * rppQ > 16 || P.H / grid + 1 > kMaxDownRows) return false;
-    P.so = split(0, warps, P.H / rppQ);
+    if (P.H < grid || P.H / grid + 1 > kMaxDownRows) return false;
     // Q, K, V: warps by what the rows cost (Q6_K: 1.46 times the bytes and more arithmetic per byte)
     const double cq = P.QD, ck = P.KD, cv = P.KD * (P.L[0].v_q6 ? 1.8 : 1.0), sum = cq + ck + cv;
     int wk = static_cast<int>(warps * ck / sum), wv = static_cast<int>(warps * cv / sum);
@@ -1185,7 +1183,7 @@ bool plan(Params &P)
     auto fit = [&](int b) { need = b > need ? b : need; };
     fit(stage_of(P.mH, false));
     fit(stage_of(P.mQ, false));
-    fit(2 * rpp * P.mH.bpr * kQ4KBlock);
+    fit(4 * rpp * P.mH.bpr * kQ4KBlock);
     if (v6) fit(stage_of(P.mH, true));
     if (d4) fit(stage_of(P.mE, false));
     if (d6) fit(stage_of(P.mE, true));

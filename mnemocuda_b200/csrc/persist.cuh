@@ -45,7 +45,7 @@ struct Head {
     int pdl;
     // geometry
     Map mH, mQ, mE;         // rows of H, QD and EFF columns
-    Split sq, sk, sv, so, sg;  // passes of the four projections; gate / up items
+    Split sq, sk, sv, sg;   // passes of Q, K, V; gate / up items
     uint32_t ipe, ipe_magic;   // gate / up items per expert, 2^32 / ipe rounded up
     int xc, off_row, off_ring, ring_bytes;  // columns of the staged vector; byte offsets in shared memory
 };
