@@ -910,12 +910,16 @@ inline bool prepare(Params &P, const char *where, int grid_cap, int force_ru, La
     const int mult = (P.mode == kSwiGLU || P.mode == kMoeGateUp) ? 2 : 1;  // stage rows per virtual row
     const int n_x = (P.mode == kMoeDown) ? P.n_slots : 1;
 
-    // RU: the fewest pass-times to cover the longest range; ties go to the larger RU (more independent work per warp)
+    // RU: what the longest range costs. A pass of a unit of four rows hides the most latency; on its own it takes 1.45 times, in
+    // units of two 1.17 times as long (measured over 2048 to 50000 rows of 1536 to 8192 columns, Q4_K, Q5_K, Q6_K: counting
+    // passes alone chose single rows for most tall matrices and took up to 1.6 times as long there, 57.3 us against 36.6 for
+    // 50000 x 4096 Q6_K). Units of four need three of them per warp: with fewer the ring has too few tiles to overlap.
     int ru = 1, best = 1 << 30;
-    for (int cand = 1; cand <= 4; cand *= 2) {
+    constexpr int kPassCost[3] = {58, 47, 40};
+    for (int cand = 1, i = 0; cand <= 4; cand *= 2, i++) {
         const int rows = mult * per_cta;
-        const int cost = ((rows + sweep1 * cand - 1) / (sweep1 * cand)) * cand;
-        if (cost <= best) {
+        const int units = (rows + sweep1 * cand - 1) / (sweep1 * cand), cost = units * cand * kPassCost[i];
+        if (cost <= best && (cand < 4 || units >= 3)) {
             best = cost;
             ru = cand;
         }
