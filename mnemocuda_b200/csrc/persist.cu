@@ -80,6 +80,7 @@ struct Misc {
     int top_id[kMaxK + 1];
     uint32_t top_key[kMaxK + 1];
     float swt[kMaxK];
+    float rope[128], norm[2][128];         // cosines and sines of the position; this layer's q and k norm weights
     int abort_flag;
     Head head;                              // the launch's parameters, read from here by every step (see thread_id)
     int2 own[kWarps][4];                    // a warp's rows of each operation: first, count (gate / up: items)
@@ -459,19 +460,21 @@ __device__ __forceinline__ uint32_t pack2(float a, float b)
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-// A head's 128 values, four per lane at lane + 32 i: RMS norm (w may be null) and rotation.
-__device__ __forceinline__ float4 norm_rope(float4 v, const float *w, float eps, const float *cos_t, const float *sin_t)
+// A head's 128 values, four per lane at lane + 32 i: RMS norm with the weights M.norm[which] (unless !normed) and rotation by M.rope.
+__device__ __forceinline__ float4 norm_rope(float4 v, int which, bool normed, float eps)
 {
+    const Misc &M = misc();
     const int lane = thread_id() & 31;
+    const float *w = M.norm[which];
     const float ss = warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
-    if (w) {
+    if (normed) {
         const float f = 1.0f / sqrtf(ss * (1.0f / 128.0f) + eps);
-        v.x *= f * __ldg(w + lane);
-        v.y *= f * __ldg(w + lane + 32);
-        v.z *= f * __ldg(w + lane + 64);
-        v.w *= f * __ldg(w + lane + 96);
+        v.x *= f * w[lane];
+        v.y *= f * w[lane + 32];
+        v.z *= f * w[lane + 64];
+        v.w *= f * w[lane + 96];
     }
-    const float c0 = __ldcg(cos_t + lane), c1 = __ldcg(cos_t + lane + 32), s0 = __ldcg(sin_t + lane), s1 = __ldcg(sin_t + lane + 32);
+    const float c0 = M.rope[lane], c1 = M.rope[lane + 32], s0 = M.rope[64 + lane], s1 = M.rope[96 + lane];
     return make_float4(v.x * c0 - v.z * s0, v.y * c1 - v.w * s1, v.x * s0 + v.z * c0, v.y * s1 + v.w * c1);
 }
 
@@ -492,8 +495,8 @@ __device__ __forceinline__ void load_kv(const __half *kv_k, const __half *kv_v, 
 // running maxima (log2 domain) and sums in M.am / M.al. The tile of the newest position takes its K and V from the projections
 // and, with store, writes them to the cache. Returns the ring's parities.
 __device__ __forceinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_kv, int kvh, __half *kv_k, __half *kv_v, bool store,
-                                            const uint2 *c_k, const uint2 *c_v, uint32_t tag, const float *k_norm, float eps,
-                                            const float *cos_t, const float *sin_t, uint32_t parity)
+                                            const uint2 *c_k, const uint2 *c_v, uint32_t tag, bool k_normed, float eps,
+                                            uint32_t parity)
 {
     uint8_t *buf = ring();
     Misc &M = misc();
@@ -514,7 +517,7 @@ __device__ __forceinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_
             wait_values4(c_k + kvh * 128 + lane, tag, kv);
             wait_values4(c_v + kvh * 128 + lane, tag, vv);
             __syncwarp();
-            const float4 kr = norm_rope(make_float4(kv[0], kv[1], kv[2], kv[3]), k_norm, eps, cos_t, sin_t);
+            const float4 kr = norm_rope(make_float4(kv[0], kv[1], kv[2], kv[3]), 1, k_normed, eps);
             const float kn[4] = {kr.x, kr.y, kr.z, kr.w};
             const size_t row = ((size_t)pos * n_kv + kvh) * 128;
             uint8_t *kd = buf + (pos & 15) * kKvPitch;
@@ -624,8 +627,7 @@ __device__ __forceinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_
 }
 
 // The warps bring nh query heads (128 cells each) into the fragments (hi + lo halves of q * scale * log2 e); the other rows are zero.
-__device__ __forceinline__ void q_fragments(const uint2 *c_q, uint32_t tag, int nh, const float *q_norm, float eps, const float *cos_t,
-                                         const float *sin_t, float sc)
+__device__ __forceinline__ void q_fragments(const uint2 *c_q, uint32_t tag, int nh, bool q_normed, float eps, float sc)
 {
     const int lane = thread_id() & 31;
 #pragma unroll 1
@@ -634,7 +636,7 @@ __device__ __forceinline__ void q_fragments(const uint2 *c_q, uint32_t tag, int 
         if (h < nh) {
             wait_values4(c_q + h * 128 + lane, tag, v);
             __syncwarp();
-            const float4 r = norm_rope(make_float4(v[0], v[1], v[2], v[3]), q_norm, eps, cos_t, sin_t);
+            const float4 r = norm_rope(make_float4(v[0], v[1], v[2], v[3]), 0, q_normed, eps);
             v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
         }
 #pragma unroll
@@ -948,8 +950,13 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                     if (has_row) wait_copy(&M.row_bar, l & 1);
                     row_pend = -1;
                 }
+                // the norm weights of the heads: on their way while the vector is waited for
+                const float *hw = tid < 128 ? L.q_norm : L.k_norm;
+                float hn = 0.0f;
+                if (op == kQKV && tid < 256 && hw) hn = __ldg(hw + (tid & 127));
                 ok = !stage_vec(src, t, K, norm_w, P.eps, logit);
                 if (!ok) break;
+                if (op == kQKV && tid < 256) M.norm[tid >> 7][tid & 127] = hn;
             }
             // ---- its rows ----
             if (op == kExperts) {
@@ -1009,13 +1016,12 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                     }
                     cta_sync();  // the staged vector has been read
                     const int nh = min(16, P.gqa - qb * 16);
-                    q_fragments(P.c_q + (kvh * P.gqa + qb * 16) * 128, tag, nh, L.q_norm, P.eps, P.cos_t, P.sin_t,
-                                P.scale * kLog2e);
+                    q_fragments(P.c_q + (kvh * P.gqa + qb * 16) * 128, tag, nh, L.q_norm != nullptr, P.eps, P.scale * kLog2e);
                     ok = !cta_aborted();
                     if (!ok) break;
                     if (tile0 < tile1)
-                        parity = attn_tiles(tile0, tile1, pos, P.n_kv, kvh, L.kv_k, L.kv_v, qb == 0, P.c_k, P.c_v, tag, L.k_norm, P.eps,
-                                            P.cos_t, P.sin_t, parity);
+                        parity = attn_tiles(tile0, tile1, pos, P.n_kv, kvh, L.kv_k, L.kv_v, qb == 0, P.c_k, P.c_v, tag,
+                                            L.k_norm != nullptr, P.eps, parity);
                     pend = 0;
                     cta_sync();
                     attn_partial(min(kWarps, tile1 - ac * tpc), nh, P.c_part, P.c_ml, ab * P.chunks + ac, tag);
@@ -1023,6 +1029,10 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                 }
             }
             cta_sync();  // the staged vector and the ring have been read
+            if (op == kQKV && cta < P.n_heads) {
+                const int kv = cta / P.gqa, hq = cta - kv * P.gqa;
+                merge_head(kv * P.qblocks + (hq >> 4), hq & 15, nc, P.chunks, P.c_part, P.c_ml, P.c_attn + cta * 128, tag);
+            }
         }
         // ---- the next operation's weights; gate / up requests its own: they depend on the routing ----
         const int next = (op + 1) & 3, ln = l + (op == kDown && it >= 0 ? 1 : 0);
@@ -1066,11 +1076,7 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
             const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid),
                       rows = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid) - R0;
             if (tid < rows) M.hid[tid] = __ldcg(P.hidden + R0 + tid);
-        } else if (op == kQKV) {
-            if (cta < P.n_heads) {
-                const int kv = cta / P.gqa, hq = cta - kv * P.gqa;
-                merge_head(kv * P.qblocks + (hq >> 4), hq & 15, nc, P.chunks, P.c_part, P.c_ml, P.c_attn + cta * 128, tag);
-            }
+            if (tid < 128) M.rope[tid] = __ldcg(tid < 64 ? P.cos_t + tid : P.sin_t + tid - 64);
         } else if (op == kDown) {
             const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid),
                       rows = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid) - R0;
