@@ -169,21 +169,29 @@ namespace mb200 {
 namespace {
 // x and the residual from mapped host memory into device memory: volatile loads (the host rewrites the buffer
 // between calls; nothing of it may be served from a cache), one 16-byte load per thread and round.
-__global__ void __launch_bounds__(1024) host_stage_in_kernel(const float4 *src, float4 *dst, int n4)
+// (Four loads of a thread are in flight together: a load across PCIe takes 1.5 us, in turn they took that each.)
+constexpr int kStageThreads = 256, kStageLoads = 4;
+__global__ void __launch_bounds__(kStageThreads) host_stage_in_kernel(const float4 *src, float4 *dst, int n4)
 {
-    for (int i = threadIdx.x; i < n4; i += blockDim.x) {
-        float4 v;
-        asm volatile("ld.volatile.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                     : "l"(src + i));
-        dst[i] = v;
-    }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the block's CTAs start up behind these loads
+    const int i0 = blockIdx.x * (kStageThreads * kStageLoads) + threadIdx.x;
+    float4 v[kStageLoads];
+#pragma unroll
+    for (int u = 0; u < kStageLoads; u++)
+        if (i0 + u * kStageThreads < n4)
+            asm volatile("ld.volatile.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v[u].x), "=f"(v[u].y), "=f"(v[u].z), "=f"(v[u].w)
+                         : "l"(src + i0 + u * kStageThreads));
+#pragma unroll
+    for (int u = 0; u < kStageLoads; u++)
+        if (i0 + u * kStageThreads < n4) dst[i0 + u * kStageThreads] = v[u];
 }
 
 // Last node of a host call: the kernels before it have completed (stream order), so the result rows are on their
 // way to host memory ahead of this store; the host spins on the word instead of asking the driver to wait.
 __global__ void host_signal_kernel(unsigned int *dev_counter, volatile unsigned int *host_flag)
 {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const unsigned int v = *dev_counter + 1;
     *dev_counter = v;
     __threadfence_system();
@@ -432,12 +440,23 @@ int mb200_moe_block_host(const float *router_w, const void *experts, size_t expe
         const bool plain = !host_state_ready(st) || cudaStreamIsCapturing(stream, &cap) != cudaSuccess ||
                            cap != cudaStreamCaptureStatusNone;
         auto enqueue = [&](bool signal) -> int {
-            host_stage_in_kernel<<<1, 1024, 0, stream>>>(static_cast<const float4 *>(d_in), reinterpret_cast<float4 *>(dev_io),
-                                                         2 * H / 4);
+            constexpr int per = kStageThreads * kStageLoads;
+            host_stage_in_kernel<<<(2 * H / 4 + per - 1) / per, kStageThreads, 0, stream>>>(
+                static_cast<const float4 *>(d_in), reinterpret_cast<float4 *>(dev_io), 2 * H / 4);
             const int rc = mb200_moe_block_local(router_w, experts, expert_stride, gate_sz, up_sz, down_type, n_experts,
                                                  expert_lo, cnt, k, H, EFF, dev_io, dev_io + H, static_cast<float *>(d_out),
                                                  ids, wts, act, scratch, stream);
-            if (rc == MB200_OK && signal) host_signal_kernel<<<1, 1, 0, stream>>>(st.counter, st.flag_dev);
+            if (rc == MB200_OK && signal) {
+                cudaLaunchConfig_t cfg = {};
+                cfg.gridDim = cfg.blockDim = dim3(1);
+                cfg.stream = stream;
+                cudaLaunchAttribute attr;  // launched while the block is still running, it waits for its end
+                attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+                attr.val.programmaticStreamSerializationAllowed = 1;
+                cfg.attrs = &attr;
+                cfg.numAttrs = pdl_enabled() ? 1 : 0;
+                if (cudaLaunchKernelEx(&cfg, host_signal_kernel, st.counter, st.flag_dev) != cudaSuccess) return MB200_ERR_LAUNCH;
+            }
             return rc;
         };
         if (plain) {  // no completion word, or the caller is capturing this stream itself
