@@ -84,7 +84,9 @@ struct Misc {
     int abort_flag;
     Head head;                              // the launch's parameters, read from here by every step (see thread_id)
     int2 own[kWarps][4];                    // a warp's rows of each operation: first, count (gate / up: items)
-    int own_qm[kWarps];                     // which of Q, K, V
+    int own_qm[kWarps], own_slot[kWarps];   // which of Q, K, V; slot of the down projection
+    // the CTA's rows of the hidden vector; its part of the attention (chunks in all, own head block and tiles); the head it merges
+    int R0, rows, nc, kvh, qb, part_slot, tile0, tile1, merge_block, merge_head;
 };
 enum Op { kQKV, kO, kExperts, kDown };
 // Shared memory: Misc, the staged vector (and the attention's fragments, the merge), the router row, the warps' rings.
@@ -358,14 +360,12 @@ __device__ __forceinline__ void issue_unit(const uint8_t *w, int row, int rows, 
     bulk_g2s(dst, reinterpret_cast<const void *>(a0), bytes, bar);
 }
 // Requests the first units, a lane each; returns the mask of stages in flight.
-__device__ __forceinline__ uint32_t prefetch(const uint8_t *w, int r0, int n, uint32_t row_bytes, int ur)
+__device__ __forceinline__ uint32_t prefetch(const uint8_t *w, int r0, int n, uint32_t row_bytes, int log_ur, int stages)
 {
     uint8_t *buf = ring();
     uint64_t *bars = ring_bars();
-    const int ring_bytes = head().ring_bytes;
-    const uint32_t sb = stage_bytes_of(ur * row_bytes);
-    const int lane = thread_id() & 31;
-    const int stages = min(kStages, ring_bytes / static_cast<int>(sb)), count = min(stages, n > 0 ? (n + ur - 1) / ur : 0);
+    const int lane = thread_id() & 31, ur = 1 << log_ur, count = min(stages, (n + ur - 1) >> log_ur);
+    const uint32_t sb = stage_bytes_of(row_bytes << log_ur);
     if (lane < count) issue_unit(w, r0 + lane * ur, min(ur, n - lane * ur), row_bytes, buf + lane * sb, &bars[lane]);
     __syncwarp();
     return (1u << count) - 1;
@@ -374,16 +374,15 @@ __device__ __forceinline__ uint32_t prefetch(const uint8_t *w, int r0, int n, ui
 // dst[row] = value (with keep: added to keep[row], which takes the sum), as a cell if tag != 0. Returns the ring's parities.
 template <class F, int RU>
 __device__ __forceinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, int r0, int n, void *dst, uint32_t tag, float *keep, int xcol,
-                                        uint32_t parity)
+                                        int stages, uint32_t parity)
 {
     uint8_t *buf = ring();
     uint64_t *bars = ring_bars();
-    const int ring_bytes = head().ring_bytes, xc = head().xc;
+    const int xc = head().xc;
     const int lane = thread_id() & 31, q = lane >> 2, sub = lane & 3;
     const int v = 1 << lv, rpp = 8 >> lv, cq = q & (v - 1), rq = q >> lv, W = 4 << lv;
     const int groups = (bpr + v - 1) >> lv, ur = RU * rpp;
     const uint32_t row_bytes = bpr * F::kBlockBytes, sb = stage_bytes_of(ur * row_bytes);
-    const int stages = min(kStages, ring_bytes / static_cast<int>(sb));
     typename F::XRegs xr;
     int s = 0;
 #pragma unroll 1
@@ -828,16 +827,15 @@ __device__ __forceinline__ void issue_items(const uint8_t *experts, size_t estri
 }
 // id: lane i holds the i-th routed expert. Writes SwiGLU's result as cells act[slot * EFF + row].
 __device__ __forceinline__ uint32_t gate_up(const uint8_t *experts, size_t estride, uint32_t up_off, int id, int i0, int n, int ipe, uint32_t magic,
-                                            int bpr, int lv, int EFF, uint2 *act, uint32_t tag, uint32_t parity)
+                                            int bpr, int lv, int EFF, uint2 *act, uint32_t tag, int stages, uint32_t parity)
 {
     uint8_t *buf = ring();
     uint64_t *bars = ring_bars();
-    const int ring_bytes = head().ring_bytes, xc = head().xc;
+    const int xc = head().xc;
     const int lane = thread_id() & 31, q = lane >> 2, sub = lane & 3;
     const int v = 1 << lv, rpp = 8 >> lv, cq = q & (v - 1), rq = q >> lv, W = 4 << lv;
     const int groups = (bpr + v - 1) >> lv, end = i0 + n;
     const uint32_t row_bytes = bpr * kQ4KBlock, half = rpp * row_bytes, sb = 4 * half;
-    const int stages = min(kStages, ring_bytes / static_cast<int>(sb));
     const int ij = (lane >> 1) & 1, ih = lane & 1, is = lane >> 2;  // of a request: item, half, stage
     issue_items(experts, estride, up_off, id, i0 + 2 * is, end, ipe, magic, half, is < stages, ij, ih, buf + is * sb, &bars[is < stages ? is : 0]);
     Q4::XRegs xr;
@@ -905,6 +903,9 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
         const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid), R1 = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid);
         const int wps = kWarps / P.k, slot = warp / wps, part = warp - slot * wps, per = (R1 - R0 + wps - 1) / wps;
         M.own[warp][kO] = make_int2(R0 + (R1 - R0) * warp / kWarps, (R1 - R0) * (warp + 1) / kWarps - (R1 - R0) * warp / kWarps);
+        M.own_slot[warp] = slot;
+        M.R0 = R0;
+        M.rows = R1 - R0;
         M.own[warp][kDown] = make_int2(R0 + part * per, slot < P.k ? max(0, min(per, R1 - R0 - part * per)) : 0);
     }
     mbar_fence_init();
@@ -918,7 +919,7 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
     if (has_row && tid == 0) request_row(0);
 
     uint32_t parity = 0, pend = 0, tag = 0;  // pend: stages in flight while the CTA may still give up
-    int pos = 0, nc = 0, id = 0;             // nc: chunks of positions; id: lane i holds the i-th routed expert
+    int pos = 0, id = 0;                     // id: lane i holds the i-th routed expert
     bool ok = true;
     // One pass of the loop: an operation (there is one copy of every step's code), preceded by the request for its weights. The
     // pass before the first only requests.
@@ -969,17 +970,17 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                 if (!ok) break;
                 const int2 own = M.own[warp][kExperts];
                 parity = gate_up(L.experts, L.estride, L.up_off, id, own.x, own.y, P.ipe, P.ipe_magic, P.mH.bpr, P.mH.lv, P.EFF, P.c_act, tag,
-                                 parity);
+                                 P.stages[5], parity);
             } else {
                 const int2 own = M.own[warp][op];
-                const int qm = M.own_qm[warp], slot = warp / (kWarps / P.k);
+                const int qm = M.own_qm[warp], slot = M.own_slot[warp];
                 const uint8_t *w = qm == 0 ? L.wq : qm == 1 ? L.wk : L.wv;
                 void *dst = qm == 0 ? P.c_q : qm == 1 ? P.c_k : P.c_v;
                 float *keep = nullptr;
-                const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid);
+                const int R0 = M.R0;
                 uint32_t t = tag;
                 bool q6 = qm == 2 && L.v_q6;
-                int bpr = P.mH.bpr, lv = P.mH.lv, xcol = 0;
+                int bpr = P.mH.bpr, lv = P.mH.lv, xcol = 0, kind = q6 ? 1 : 0;
                 if (op == kO) {
                     w = L.wo;
                     dst = P.c_h1;
@@ -987,6 +988,7 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                     q6 = false;
                     bpr = P.mQ.bpr;
                     lv = P.mQ.lv;
+                    kind = 2;
                 } else if (op == kDown) {
                     w = L.experts + (size_t)__shfl_sync(0xffffffffu, id, slot & 31) * L.estride + L.down_off;
                     dst = M.part[slot < P.k ? slot : 0] - R0;
@@ -994,22 +996,20 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                     q6 = L.down_q6;
                     bpr = P.mE.bpr;
                     lv = P.mE.lv;
+                    kind = q6 ? 4 : 3;
                     xcol = slot * bpr;
                 }
                 if (q6)
-                    parity = matvec<Q6, 2>(w, bpr, lv, own.x, own.y, dst, t, keep, xcol, parity);
+                    parity = matvec<Q6, 2>(w, bpr, lv, own.x, own.y, dst, t, keep, xcol, P.stages[kind], parity);
                 else
-                    parity = matvec<Q4, 4>(w, bpr, lv, own.x, own.y, dst, t, keep, xcol, parity);
+                    parity = matvec<Q4, 4>(w, bpr, lv, own.x, own.y, dst, t, keep, xcol, P.stages[kind], parity);
                 pend = 0;
             }
             // ---- attention of this CTA's positions ----
             if (op == kQKV) {
-                const int tpc = ((pos >> 4) + P.chunks) / P.chunks;  // tiles of 16 positions per chunk
-                nc = ((pos >> 4) + tpc) / tpc;
-                const int ab = cta / P.chunks, ac = cta - ab * P.chunks;  // head block and chunk
-                if (ab < P.n_kv * P.qblocks && ac < nc) {
-                    const int kvh = ab / P.qblocks, qb = ab - kvh * P.qblocks;
-                    const int tile0 = ac * tpc + warp, tile1 = min((ac + 1) * tpc, (pos >> 4) + 1);
+                const int base = M.tile0, tile1 = M.tile1, tile0 = base + warp;
+                if (base < tile1) {
+                    const int kvh = M.kvh, qb = M.qb;
                     if (tile0 < tile1) {
                         load_kv(L.kv_k, L.kv_v, tile0, pos, P.n_kv, kvh);
                         pend = 1;
@@ -1024,14 +1024,13 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                                             L.k_norm != nullptr, P.eps, parity);
                     pend = 0;
                     cta_sync();
-                    attn_partial(min(kWarps, tile1 - ac * tpc), nh, P.c_part, P.c_ml, ab * P.chunks + ac, tag);
+                    attn_partial(min(kWarps, tile1 - base), nh, P.c_part, P.c_ml, M.part_slot, tag);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the ring was written and read as plain memory
                 }
             }
             cta_sync();  // the staged vector and the ring have been read
             if (op == kQKV && cta < P.n_heads) {
-                const int kv = cta / P.gqa, hq = cta - kv * P.gqa;
-                merge_head(kv * P.qblocks + (hq >> 4), hq & 15, nc, P.chunks, P.c_part, P.c_ml, P.c_attn + cta * 128, tag);
+                merge_head(M.merge_block, M.merge_head, M.nc, P.chunks, P.c_part, P.c_ml, P.c_attn + cta * 128, tag);
             }
         }
         // ---- the next operation's weights; gate / up requests its own: they depend on the routing ----
@@ -1042,19 +1041,21 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
             const int qm = M.own_qm[warp];
             const uint8_t *w = qm == 0 ? L.wq : qm == 1 ? L.wk : L.wv;
             bool q6 = qm == 2 && L.v_q6;
-            int bpr = P.mH.bpr, lv = P.mH.lv;
+            int bpr = P.mH.bpr, lv = P.mH.lv, kind = q6 ? 1 : 0;
             if (next == kO) {
                 w = L.wo;
                 q6 = false;
                 bpr = P.mQ.bpr;
                 lv = P.mQ.lv;
+                kind = 2;
             } else if (next == kDown) {
-                w = L.experts + (size_t)__shfl_sync(0xffffffffu, id, (warp / (kWarps / P.k)) & 31) * L.estride + L.down_off;
+                w = L.experts + (size_t)__shfl_sync(0xffffffffu, id, M.own_slot[warp] & 31) * L.estride + L.down_off;
                 q6 = L.down_q6;
                 bpr = P.mE.bpr;
                 lv = P.mE.lv;
+                kind = q6 ? 4 : 3;
             }
-            pend = prefetch(w, own.x, own.y, bpr * (q6 ? kQ6KBlock : kQ4KBlock), (q6 ? 2 : 4) << (3 - lv));
+            pend = prefetch(w, own.x, own.y, bpr * (q6 ? kQ6KBlock : kQ4KBlock), (q6 ? 4 : 5) - lv, P.stages[kind]);
         }
         if (it < 0) {
             if (P.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -1073,13 +1074,23 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
             __syncthreads();
             tag = static_cast<uint32_t>(M.launch) * 128u + 1u;
             pos = __ldcg(P.pos);
-            const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid),
-                      rows = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid) - R0;
+            if (tid == 0) {
+                const int tpc = ((pos >> 4) + P.chunks) / P.chunks, ab = cta / P.chunks, ac = cta - ab * P.chunks;  // tiles per chunk; ours
+                M.nc = ((pos >> 4) + tpc) / tpc;
+                M.kvh = ab / P.qblocks;
+                M.qb = ab - M.kvh * P.qblocks;
+                M.part_slot = cta;
+                M.tile0 = ac * tpc;
+                M.tile1 = ab < P.n_kv * P.qblocks ? min((ac + 1) * tpc, (pos >> 4) + 1) : 0;
+                const int kv = cta / P.gqa, hq = cta - kv * P.gqa;
+                M.merge_block = kv * P.qblocks + (hq >> 4);
+                M.merge_head = hq & 15;
+            }
+            const int R0 = M.R0, rows = M.rows;
             if (tid < rows) M.hid[tid] = __ldcg(P.hidden + R0 + tid);
             if (tid < 128) M.rope[tid] = __ldcg(tid < 64 ? P.cos_t + tid : P.sin_t + tid - 64);
         } else if (op == kDown) {
-            const int R0 = static_cast<int>(static_cast<unsigned>(P.H) * cta / grid),
-                      rows = static_cast<int>(static_cast<unsigned>(P.H) * (cta + 1) / grid) - R0;
+            const int R0 = M.R0, rows = M.rows;
             if (tid < rows) {
                 float y = 0.0f;
 #pragma unroll 4
@@ -1185,15 +1196,14 @@ bool plan(Params &P)
         d6 = d6 || P.L[l].down_q6;
         d4 = d4 || !P.L[l].down_q6;
     }
-    int need = 32 * kKvPitch;
-    auto fit = [&](int b) { need = b > need ? b : need; };
-    fit(stage_of(P.mH, false));
-    fit(stage_of(P.mQ, false));
-    fit(4 * rpp * P.mH.bpr * kQ4KBlock);
-    if (v6) fit(stage_of(P.mH, true));
-    if (d4) fit(stage_of(P.mE, false));
-    if (d6) fit(stage_of(P.mE, true));
-    return need <= P.ring_bytes;
+    const int bytes[6] = {stage_of(P.mH, false), stage_of(P.mH, true), stage_of(P.mQ, false), stage_of(P.mE, false), stage_of(P.mE, true),
+                          4 * rpp * P.mH.bpr * kQ4KBlock};
+    const bool used[6] = {true, v6, true, d4, d6, true};
+    for (int i = 0; i < 6; i++) {
+        P.stages[i] = P.ring_bytes / bytes[i] < kStages ? P.ring_bytes / bytes[i] : kStages;
+        if (used[i] && P.stages[i] < 1) return false;
+    }
+    return 32 * kKvPitch <= P.ring_bytes && 16 * kPitch * 4 <= P.ring_bytes;
 }
 
 int launch(Params &P, cudaStream_t stream)

@@ -47,6 +47,7 @@ struct Head {
     Map mH, mQ, mE;         // rows of H, QD and EFF columns
     Split sq, sk, sv, sg;   // passes of Q, K, V; gate / up items
     uint32_t ipe, ipe_magic;   // gate / up items per expert, 2^32 / ipe rounded up
+    int stages[6];             // of a warp's ring: H Q4_K, H Q6_K, QD, EFF Q4_K, EFF Q6_K, gate / up
     int xc, off_row, off_ring, ring_bytes;  // columns of the staged vector; byte offsets in shared memory
 };
 
