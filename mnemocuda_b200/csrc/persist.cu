@@ -768,8 +768,8 @@ __device__ __noinline__ void walk(int n, int k)
         }
 }
 
-// The k largest of n logits (every thread of the CTA calls it): lane i < k of every warp returns the i-th expert, the weights go
-// to M.swt (visible after the next barrier of the CTA). -1: the CTA has given up.
+// The k largest of n logits (every thread of the CTA calls it): lane i < k of every warp returns the i-th expert, M.top_key
+// keeps their logits. -1: the CTA has given up.
 __device__ __forceinline__ int select_experts(const uint2 *cells, uint32_t tag, int n, int k)
 {
     Misc &M = misc();
@@ -801,15 +801,20 @@ __device__ __forceinline__ int select_experts(const uint2 *cells, uint32_t tag, 
         if (tid == 0) walk(n, k);
         cta_sync();
     }
-    const int id = M.top_id[lane < k ? lane : 0];
+    return M.top_id[lane < k ? lane : 0];
+}
+// One warp, later (the requests for the experts do not need them): the weights of the selected, to M.swt.
+__device__ __forceinline__ void select_weights(int k)
+{
+    Misc &M = misc();
+    const int lane = thread_id() & 31;
     const float v = lane < k ? unordered(M.top_key[lane]) : -INFINITY;
     float mx = v;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     const float e = lane < k ? expf(v - mx) : 0.0f;
     const float sum = warp_sum(e);
-    if (tid < k) M.swt[tid] = e / sum;
-    return id;
+    if (lane < k) M.swt[lane] = e / sum;
 }
 
 // ---- gate / up: items [i0, i0 + n), item i = a pass of gate rows and the same up rows of the i / ipe-th routed expert. Two items
@@ -971,6 +976,7 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                 const int2 own = M.own[warp][kExperts];
                 parity = gate_up(L.experts, L.estride, L.up_off, id, own.x, own.y, P.ipe, P.ipe_magic, P.mH.bpr, P.mH.lv, P.EFF, P.c_act, tag,
                                  P.stages[5], parity);
+                if (warp == kWarps - 1) select_weights(P.k);
             } else {
                 const int2 own = M.own[warp][op];
                 const int qm = M.own_qm[warp], slot = M.own_slot[warp];
