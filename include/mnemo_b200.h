@@ -150,9 +150,9 @@ void cuda_f32_to_int8_kv(const float *in, void *out, float *scales, int head_dim
 void cuda_f32_to_int8_kv_dual(const float *k, const float *v, void *out_k, void *out_v, float *k_scales,
                               float *v_scales, int head_dim, int n_kv_heads, cudaStream_t stream);
 /* Decode attention over the INT8 cache ([position][kv head][head_dim] int8, scales [position][kv head]).
- * Replaces src/kernels.cu:1536-1546 (kernel :1382-1480). head_dim 128 with 4 or 8 | gqa_ratio shares each
- * K / V read among the query heads of a CTA and splits the positions over the SMs (partials pass through a
- * workspace inside the library image); anything else runs one CTA per query head. */
+ * Replaces src/kernels.cu:1536-1546 (kernel :1382-1480). head_dim 128: on tensor cores, 16 query heads of a KV head share
+ * each K / V read and the positions are split over the SMs (partials pass through a workspace inside the library
+ * image); anything else runs one CTA per query head. */
 void cuda_attention_int8kv(const float *q, const void *kv_k, const void *kv_v, const float *k_scales,
                            const float *v_scales, float *out, int n_heads_q, int head_dim, int n_kv_heads,
                            int seq_len, int gqa_ratio, float scale, cudaStream_t stream);

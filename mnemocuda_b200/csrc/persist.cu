@@ -13,17 +13,25 @@
 //     and the read of the vector another one; a cell is with its reader about 1 us after it was written). A tag belongs to one
 //     layer of one launch. A cell is overwritten only by a CTA that has results of every CTA that were computed after they had
 //     read it: each operation's writers depend on all CTAs' rows of the O projection and of the down projection;
-//   * weights depend on nobody: while a warp would wait it has the first ~11 KB of its next rows on the way (180 KB per SM,
+//   * weights depend on nobody: while a warp would wait it has the first 20 KB of its next rows on the way (160 KB per SM,
 //     which is all of most operations), and K / V rows of the cache before q exists;
-//   * the input vector of an operation is split by every CTA into two int8 levels as it arrives.
+//   * the input vector of an operation is split by every CTA into two int8 levels as it arrives;
+//   * a CTA's rows of the hidden vector stay in its shared memory: it updates them in both halves of every layer.
 //
 // The top-k a CTA does for itself by counting: the rank of an expert is how many logits are larger. Only where equal logits
 // straddle the boundary does the reference's replace-the-minimum walk decide, and is then run.
 //
-// The code of a layer is run once per layer: what counts is that it stays in the instruction caches (with everything inlined it
-// was 270 KB, and a layer took longer than the separate kernels). So every step is a function, one copy each, whose arguments
-// are plain values -- a reference to the parameter block or to a struct would be read through memory, behind the weight
-// stream -- and which finds its shared memory by offsets; loops over run-time counts are not unrolled.
+// The code of a layer is run once per layer: what counts is its size (270 KB with a copy of every step per operation, 106 KB as
+// one loop over the operations) and that nothing lives in local memory, which the weight stream and 227 KB of shared memory
+// leave no L1 for. Hence eight warps with 255 registers (sixteen with 128 spilled 2 KB a thread: 2870 us instead of 1930 per token
+// below), several rows per warp in flight instead, thread_id() and cta_id() read anew by every step, and the launch's
+// parameters, divisions already done, in shared memory.
+//
+// Measured, per token: 30B shape at position 4095 (48 layers) 3240 -> 1643 us, 8 layers of the 235B shape at 8191 925 -> 629; a
+// layer is 33 / 65 us. What bounds it: seven exchanges between all SMs (a value written is with its readers 1 us later, and they
+// wait for the slowest CTA: 20 of the 33 us), then instruction issue of the products (Q6_K down: 9 us at the 235B shape,
+// where gate / up runs at the copy rate). Tried and slower: two K / V tiles in flight per warp, the selection by repeated warp
+// maxima (150 cycles a round), the next round of a wide vector requested ahead (all three: registers), units of two rows.
 //
 // Every wait is bounded: a cell or a copy that does not come raises the abort flag of the CTA and the device error word, and
 // the CTA leaves after its copies in flight.
