@@ -57,10 +57,12 @@ FUSED_TRAFFIC_BYTES = 98054912 + 3864064     # the fused routed-expert kernel al
 
 
 def _launches_per_token(cfg, world: int) -> int:
-    """Kernels of this library per decoded token: embedding + RoPE table; per layer Q/K/V (one launch), q/k-norm +
-    RoPE + KV store, attention, O projection, MoE block (one launch where the one-launch form covers the shape,
-    else router + gate/up + down), plus the exchanges of a sharded layer (two all-gathers and, where the block is not
-    one launch with its all-reduce inside, the all-reduce); lm_head + sampling."""
+    """Kernels of this library per decoded token: embedding + RoPE table; all layers in one launch on one device; a
+    sharded layer is Q/K/V (one launch), q/k-norm + RoPE + KV store, attention, O projection, MoE block (one launch where
+    the one-launch form covers the shape, else router + gate/up + down) and its exchanges (two all-gathers and, where the
+    block is not one launch with its all-reduce inside, the all-reduce); lm_head + sampling."""
+    if world == 1 and cfg.hidden <= 4096 and cfg.top_k <= 8 and cfg.n_layers <= 112:
+        return 2 + 1 + 2
     moe = 1 if (cfg.hidden % 2048 == 0 and cfg.moe_inter % 512 == 0) else 3
     per_layer = 4 + moe + ((2 if moe == 1 else 3) if world > 1 else 0)
     return 2 + per_layer * cfg.n_layers + (2 if world == 1 else 4)
