@@ -29,6 +29,7 @@ struct Q8 {
     static constexpr bool kGroup4Tail = false;
     static constexpr int kBaseAlign = 16;  // 272-byte rows of blocks; inside a block the fields sit at even offsets
     static constexpr int kTileTargetBytes = 27648;
+    static constexpr int kPairCost = 47;  // of a pass in units of two rows, against 40 in units of four
     static constexpr int kMaxCols = 16384;
     static constexpr int kXWords = 16;
     static constexpr int kSlotsPerBlock = 4;
@@ -92,6 +93,7 @@ struct Q5 {
     static constexpr bool kGroup4Tail = false;
     static constexpr int kBaseAlign = 16;
     static constexpr int kTileTargetBytes = 28160;
+    static constexpr int kPairCost = 47;  // of a pass in units of two rows, against 40 in units of four
     static constexpr int kMaxCols = 16384;
     static constexpr int kXWords = 16;
     static constexpr int kSlotsPerBlock = 4;
@@ -169,6 +171,7 @@ struct Q3 {
     static constexpr bool kGroup4Tail = false;
     static constexpr int kBaseAlign = 2;
     static constexpr int kTileTargetBytes = 28160;
+    static constexpr int kPairCost = 47;  // of a pass in units of two rows, against 40 in units of four
     static constexpr int kMaxCols = 16384;
     static constexpr int kXWords = 16;
     static constexpr int kSlotsPerBlock = 4;

@@ -27,6 +27,7 @@ struct Q4 {
     static constexpr bool kGroup4Tail = true;  // reference src/kernels.cu:124,131
     static constexpr int kBaseAlign = 16;
     static constexpr int kTileTargetBytes = 27648;
+    static constexpr int kPairCost = 49;  // of a pass in units of two rows, against 40 in units of four
     static constexpr int kMaxCols = 16384;
     // x staging: 16 words per lane slot, slot = 4 * block-column + g
     static constexpr int kXWords = 16;

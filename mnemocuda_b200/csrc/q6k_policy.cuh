@@ -53,6 +53,7 @@ struct Q6 {
     static constexpr bool kGroup4Tail = false;  // per-element tail, reference src/kernels.cu:474
     static constexpr int kBaseAlign = 2;
     static constexpr int kTileTargetBytes = 30720;
+    static constexpr int kPairCost = 47;  // of a pass in units of two rows, against 40 in units of four
     static constexpr int kMaxCols = 16384;
     // x staging: 16 words per lane slot; slot = 4 * block-column + 2 * half + jj; word = 4g + i
     static constexpr int kXWords = 16;

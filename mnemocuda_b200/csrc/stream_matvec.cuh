@@ -911,11 +911,11 @@ inline bool prepare(Params &P, const char *where, int grid_cap, int force_ru, La
     const int n_x = (P.mode == kMoeDown) ? P.n_slots : 1;
 
     // RU: what the longest range costs. A pass of a unit of four rows hides the most latency; on its own it takes 1.45 times, in
-    // units of two 1.17 times as long (measured over 2048 to 50000 rows of 1536 to 8192 columns, Q4_K, Q5_K, Q6_K: counting
+    // units of two 1.17 times as long (Q4_K, whose rows take less arithmetic to hide: 1.22; measured over 2048 to 50000 rows of 1536 to 8192 columns, Q4_K, Q5_K, Q6_K: counting
     // passes alone chose single rows for most tall matrices and took up to 1.6 times as long there, 57.3 us against 36.6 for
     // 50000 x 4096 Q6_K). Units of four need three of them per warp: with fewer the ring has too few tiles to overlap.
     int ru = 1, best = 1 << 30;
-    constexpr int kPassCost[3] = {58, 47, 40};
+    constexpr int kPassCost[3] = {58, F::kPairCost, 40};
     for (int cand = 1, i = 0; cand <= 4; cand *= 2, i++) {
         const int rows = mult * per_cta;
         const int units = (rows + sweep1 * cand - 1) / (sweep1 * cand), cost = units * cand * kPassCost[i];
