@@ -324,16 +324,18 @@ static __device__ long long g_trace[kSMs * 2][48];  // one copy per translation 
 // Four values -> two int8 levels, v ~= sc * (a + b / 254), inv = 1 / sc. Adding 1.5 * 2^23 rounds to the nearest integer and
 // leaves it in the low byte: FMAs and byte permutes instead of the round and convert instructions, which run at a sixteenth of
 // their rate (a 4096-column vector was staged in 2.2 us, three quarters of it conversions). |v| <= 127 sc, so |a| <= 127; the
-// remainder is at most sc / 2, so |b| <= 127.
+// remainder is at most sc / 2, so |b| <= 127. Products and sums are rounded one by one, so the levels are those of
+// rint(v * inv) and rint(r * inv * 254): a product fused into the rounding addition moves a level where v * inv lies within
+// its last bit of a half.
 __device__ __forceinline__ void split_levels(const float (&v)[4], float sc, float inv, uint32_t &p1, uint32_t &p2)
 {
     constexpr float kRound = 12582912.0f;
     uint32_t a[4], b[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-        const float t = fmaf(v[i], inv, kRound);
+        const float t = __fadd_rn(__fmul_rn(v[i], inv), kRound);
         a[i] = __float_as_uint(t);
-        b[i] = __float_as_uint(fmaf(fmaf(-(t - kRound), sc, v[i]) * inv, 254.0f, kRound));
+        b[i] = __float_as_uint(__fadd_rn(__fmul_rn(__fmul_rn(fmaf(-(t - kRound), sc, v[i]), inv), 254.0f), kRound));
     }
     p1 = __byte_perm(__byte_perm(a[0], a[1], 0x0040), __byte_perm(a[2], a[3], 0x0040), 0x5410);
     p2 = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);

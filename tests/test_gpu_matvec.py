@@ -355,3 +355,40 @@ def test_qkv_in_one_launch(K, q_rows, kv_rows, cols, with_norm):
                                    (v, (wv, oracle.matvec_q6k, kv_rows))):
             _, y64, ad = fn(w, xn, rows, cols, full=True)
             assert_close_matvec(host(got), y64, ad, f"qkv {rows}x{cols} rep {rep}")
+
+
+def _levels(v, amax, fused):
+    """The two int8 levels of a group's columns (one integer per column, q1 * 254 + q2) in fp32 arithmetic; `fused`: a product
+    that is not rounded before it is rounded to an integer."""
+    f = np.float32
+    sc, inv = f(amax * f(1 / 127)), f(f(127) / amax)
+    product = lambda a, b: a.astype(np.float64) * np.float64(b) if fused else (a * f(b)).astype(np.float64)
+    a = np.rint(product(v, inv))
+    r = (v.astype(np.float64) - a * np.float64(sc)).astype(f)
+    return (a * 254 + np.rint(product((r * inv).astype(f), 254.0))).astype(np.int64)
+
+
+def test_activation_levels_are_rounded_products(K):
+    """The levels are rint(v * inv) and rint(r * inv * 254) of products rounded to fp32: what a fused product would round the other
+    way is chosen here. A matrix with a one in each column gives them back, to the bit."""
+    rng, f = np.random.default_rng(5), np.float32
+    w = np.zeros((256, synth.Q4K_BLOCK), np.uint8)
+    w[:, :2] = np.frombuffer(np.float16(1).tobytes(), np.uint8)
+    w[:, [4, 5, 6, 7, 12, 13, 14, 15]] = 1  # every scale 1, every minimum 0
+    for c in range(256):
+        w[c, 16 + (c >> 6) * 32 + (c & 31)] = 16 if c & 32 else 1
+    for _ in range(4):
+        x, want = np.empty(256, f), np.empty(256, f)
+        for g in range(8):
+            amax = f(rng.uniform(0.5, 200))
+            inv = f(f(127) / amax)
+            n = 400000
+            v = ((rng.integers(-126, 127, n) + (rng.integers(-126, 126, n) + 0.5) / 254) / np.float64(inv)).astype(f)
+            v = v[_levels(v, amax, True) != _levels(v, amax, False)][:31]
+            assert len(v) == 31
+            x[32 * g:32 * g + 32] = np.concatenate([[amax], v])
+            k = f(f(amax * f(1 / 127)) * (f(1 / (254 * 16)) if g & 1 else f(1 / 254)))
+            want[32 * g:32 * g + 32] = k * f(_levels(x[32 * g:32 * g + 32], amax, False) * (16 if g & 1 else 1))
+        y = torch.empty(256, device="cuda")
+        K.cuda_matvec_q4k(dev(w.reshape(-1)), dev(x), y, 256, 256)
+        assert np.array_equal(host(y), want)
