@@ -1204,6 +1204,19 @@ static bool fused_layout(FusedParams &P, int &smem_bytes)
     return false;
 }
 
+// Whether moe_fused() takes a routed block of this shape on the current device (weights and vectors aligned).
+bool moe_fused_covers(int H, int EFF, int k, bool down_q6)
+{
+    FusedParams P{};
+    P.H = H;
+    P.EFF = EFF;
+    P.n_slots = k;
+    P.grid = device_sms();
+    int smem_bytes = 0;
+    if (H > 4 * 3 * stream::kQuantThreads || !fused_plan(P, smem_bytes)) return false;
+    return down_q6 ? fused_layout<Q6>(P, smem_bytes) : fused_layout<Q4>(P, smem_bytes);
+}
+
 void moe_fused_init()
 {
     fused_attr<Q6, false>();

@@ -18,20 +18,31 @@
 //   * the input vector of an operation is split by every CTA into two int8 levels as it arrives;
 //   * a CTA's rows of the hidden vector stay in its shared memory: it updates them in both halves of every layer.
 //
-// The top-k a CTA does for itself by counting: the rank of an expert is how many logits are larger. Only where equal logits
-// straddle the boundary does the reference's replace-the-minimum walk decide, and is then run.
+// Every sum is taken in the order of the kernels that do the same layer by layer (decode.cu: run_layer), so both give the same
+// bits. A rounding of another order is no error, but deep models with close router logits magnify it to another expert: 48 layers of
+// synthetic 30B weights ended in another token for two seeds of eleven. Kept are the groups of blocks and their trees in a row's sum,
+// the thread mapping behind the norms and the router logits, the order of attention chunks, and the reference's expert slots.
 //
-// The code of a layer is run once per layer: what counts is its size (270 KB with a copy of every step per operation, 106 KB as
+// The top-k a CTA does for itself by counting: the rank of an expert is how many logits are larger; how many of those came before
+// it in the reference's replace-the-minimum walk tells whether that accepted it, from which its slot follows. Only where equal
+// logits meet is the walk itself run.
+//
+// The code of a layer is run once per layer: what counts is its size (270 KB with a copy of every step per operation, 134 KB as
 // one loop over the operations) and that nothing lives in local memory, which the weight stream and 227 KB of shared memory
-// leave no L1 for. Hence eight warps with 255 registers (sixteen with 128 spilled 2 KB a thread: 2870 us instead of 1930 per token
-// below), several rows per warp in flight instead, thread_id() and cta_id() read anew by every step, and the launch's
+// leave no L1 for. Hence eight warps with 255 registers (sixteen with 128 spilled 2 KB a thread and took half as long again),
+// several rows per warp in flight instead, thread_id() and cta_id() read anew by every step, and the launch's
 // parameters, divisions already done, in shared memory.
 //
-// Measured, per token: 30B shape at position 4095 (48 layers) 3240 -> 1643 us, 8 layers of the 235B shape at 8191 925 -> 629; a
-// layer is 33 / 65 us. What bounds it: seven exchanges between all SMs (a value written is with its readers 1 us later, and they
-// wait for the slowest CTA: 20 of the 33 us), then instruction issue of the products (Q6_K down: 9 us at the 235B shape,
-// where gate / up runs at the copy rate). Tried and slower: two K / V tiles in flight per warp, the selection by repeated warp
-// maxima (150 cycles a round), the next round of a wide vector requested ahead (all three: registers), units of two rows.
+// Measured, per token: 30B shape at position 4095 (48 layers) 1769 us, 8 layers of the 235B shape at 8191 669 us (layer by layer
+// 3276 / 931); a layer is 35 / 67.5 us. Where a layer's time goes, by clock stamps of warp 0, mean over CTAs and layers, 30B / 235B:
+//   waits for the operation's input (its slowest writer, and 1 us from a store to its readers)   7.8 / 13.6 us
+//   norm, router logit, split into levels                                                        4.3 /  6.0
+//   selection, with the exchange of the logits                                                   2.0 /  1.9
+//   query heads, attention partials                                                              4.4 /  7.8
+//   rows: Q, K, V | O | gate, up | down                                        2.5, 1.6, 5.0, 3.0 / 5.5, 3.7, 13.6, 9.7
+// (gate / up is at the copy rate at the 235B shape.) Tried and slower: two K / V tiles in flight per warp, the selection by
+// repeated warp maxima (150 cycles a round), the next round of a wide vector requested ahead (all three: registers), units of two
+// rows, the partials' merge with the chunk maxima taken by four warps.
 //
 // Every wait is bounded: a cell or a copy that does not come raises the abort flag of the CTA and the device error word, and
 // the CTA leaves after its copies in flight.
@@ -45,6 +56,7 @@
 
 namespace mb200 {
 int pdl_enabled();
+bool moe_fused_covers(int H, int EFF, int k, bool down_q6);
 
 namespace persist {
 namespace {
@@ -52,10 +64,12 @@ namespace {
 constexpr int kWarps = 8, kWork = kWarps * 32;
 constexpr int kStages = 5;         // ring stages per warp at most
 constexpr int kPitch = 132;        // floats between heads of a warp's attention result
-constexpr int kKvPitch = 272;      // bytes between K / V rows in shared memory
+constexpr int kKPitch = 320, kVPitch = 272;  // bytes between K / V rows in shared memory: free of bank conflicts as each is read
+constexpr int kVOff = 16 * kKPitch;          // of the V rows behind the K rows
 constexpr int kMaxDownRows = 64;   // rows of the hidden vector per CTA
 constexpr int kMaxK = kWarps;    // a warp per slot, or several
 constexpr int kMaxExperts = 256;   // two threads per expert
+constexpr int kMaxChunks = 160;    // of the attention's positions
 constexpr uint32_t kPolls = 1u << 19;  // a fraction of a second
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -78,15 +92,26 @@ __device__ __forceinline__ int cta_id()
 
 struct Misc {
     uint64_t bars[kWarps][kStages];
-    uint64_t row_bar;
-    unsigned long long launch;
-    float red[2][kWarps];
+    uint64_t row_bar, ranked;
+    uint32_t tag;                           // of the launch's first layer
+    int pos, row_pend;                      // row_pend: parity of the router row on its way, or -1
+    alignas(16) float red[3][12];          // partial sums of the norm and of the router logit (see stage_vec)
     float am[kWarps][16], al[kWarps][16];  // attention: running maximum / sum per warp and head
     float hid[kMaxDownRows];               // the CTA's rows of the hidden vector: it writes them in both of a layer's halves
-    float part[kMaxK][kMaxDownRows];
-    alignas(16) uint32_t key[kMaxExperts]; // ordered logits
-    int top_id[kMaxK + 1];
+    union {
+        float part[kMaxK][kMaxDownRows];   // the down projection's rows, by rank of the expert
+        struct {                           // before them: experts in the walk's order; the keys it accepts, and their order
+            alignas(16) uint32_t acc_key[kMaxExperts + 4];
+            uint8_t eid[kMaxExperts], by_rank[kMaxExperts];
+            float red32[32];
+        };
+    };
+    alignas(16) uint32_t key[kMaxExperts]; // ordered logits, in the order of the reference's walk
+    uint32_t accepted[kMaxExperts / 16];   // a bit per candidate
+    int top_id[kMaxK + 1], top_pos[kMaxK + 1];  // by rank: expert, place in the walk
     uint32_t top_key[kMaxK + 1];
+    int walked, slot_pos[kMaxK];           // the walk itself was run; candidate per output slot
+    int order[kMaxK];                      // by output slot: rank
     float swt[kMaxK];
     float rope[128], norm[2][128];         // cosines and sines of the position; this layer's q and k norm weights
     int abort_flag;
@@ -186,25 +211,16 @@ __device__ __forceinline__ void stage_quad(int xc, const float4 t, int c0, int l
 {
     const float v[4] = {t.x, t.y, t.z, t.w};
     float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
-    float sum = (v[0] + v[1]) + (v[2] + v[3]);
+    float sum = __fadd_rn(__fadd_rn(v[0], v[1]), __fadd_rn(v[2], v[3]));
 #pragma unroll
     for (int o = 1; o <= 4; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));  // 8 lanes = 32 columns
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     const float sc = amax * (1.0f / 127.0f);
-    const float inv = amax > 0.0f ? __fdividef(127.0f, amax) : 0.0f, inv2 = inv * 254.0f;
-    // adding 1.5 * 2^23 rounds to the nearest integer and leaves it in the low bits: no conversions, which run at an eighth of
-    // the FMA rate
-    constexpr float kRound = 12582912.0f;
-    uint32_t a[4], b[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float ai = fmaf(v[i], inv, kRound);
-        a[i] = __float_as_uint(ai);
-        b[i] = __float_as_uint(fmaf(fmaf(-(ai - kRound), sc, v[i]), inv2, kRound));  // |remainder| <= sc / 2: at most 127
-    }
-    const uint32_t p1 = __byte_perm(__byte_perm(a[0], a[1], 0x0040), __byte_perm(a[2], a[3], 0x0040), 0x5410);
-    const uint32_t p2 = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+    // (the division never of 0: that takes its slow path, and whole blocks of activations are 0)
+    const float inv = 127.0f / (amax > 0.0f ? amax : 1.0f);
+    uint32_t p1, p2;
+    stream::split_levels(v, sc, amax > 0.0f ? inv : 0.0f, p1, p2);
     const int at = chunk_at(c0 >> 4) * 16 + (c0 & 12);
     *reinterpret_cast<uint32_t *>(smem + kX + at) = p1;
     *reinterpret_cast<uint32_t *>(smem + kX + xc + at) = p2;
@@ -242,30 +258,110 @@ __device__ __forceinline__ void load_x(Q6::XRegs &r, int xc, int col, int sub)
     }
 }
 
+// A row is summed in the order of the streaming matvec: groups of blocks (four lanes a block) as a tree, lanes far apart first, then
+// the groups one after the other. Pass by pass: 2^lv blocks side by side, groups of 2^lt of them (one, or several where the groups are
+// small), a reduction per pass. Where a row is an even number of groups of eight (`paired`: lv 3, lt 2), a lane takes in two passes two
+// blocks that the tree adds first and adds them itself, with two groups side by side in the warp: a reduction per two passes. A
+// row's sum is in the lanes l with (l & result_lanes()) == 0, for the pass's row result_row().
+struct Passes {
+    int col, step;  // first block of the lane; of a pass
+    bool paired;
+    __device__ __forceinline__ Passes(int lv, int lt, int q)
+    {
+        paired = lv == 3 && lt == 2;
+        col = paired ? (q & 3) + (q >> 2) * 8 : q & ((1 << lv) - 1);
+        step = 1 << lv;
+    }
+    __device__ __forceinline__ int at(int c) const { return col + (paired ? (c >> 1) * 16 + (c & 1) * 4 : c * step); }
+    __device__ __forceinline__ bool reduces(int c) const { return !paired || (c & 1); }
+};
+template <int RU>
+__device__ __forceinline__ int result_lanes(int lv, int lt)
+{
+    return (((4 << lv) - 1) & ~((4 << lt) - 1)) | ((4 << lt) / RU - 1);
+}
+template <int RU>
+__device__ __forceinline__ int result_row(int lt, int lane)
+{
+    return (lane & ((4 << lt) - 1)) >> (lt + (RU == 4 ? 0 : 1));
+}
+template <int RU>
+__device__ __forceinline__ float tree_sum(const float (&a)[RU], int lt, int lane)
+{
+    int off = 2 << lt;
+    float v;
+    bool hi = (lane & off) != 0;
+    if (RU == 4) {
+        float k0 = hi ? a[2] : a[0], k1 = hi ? a[3] : a[1];
+        k0 += __shfl_xor_sync(0xffffffffu, hi ? a[0] : a[2], off);
+        k1 += __shfl_xor_sync(0xffffffffu, hi ? a[1] : a[3], off);
+        off >>= 1;
+        hi = (lane & off) != 0;
+        v = hi ? k1 : k0;
+        v += __shfl_xor_sync(0xffffffffu, hi ? k0 : k1, off);
+    } else {
+        v = hi ? a[1] : a[0];
+        v += __shfl_xor_sync(0xffffffffu, hi ? a[0] : a[1], off);
+    }
+#pragma unroll
+    for (int o = 16 / RU; o > 2; o >>= 1)
+        if (o < off) v += __shfl_xor_sync(0xffffffffu, v, o);
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1) {
+        const float t = v + __shfl_xor_sync(0xffffffffu, v, o);
+        v = o < off ? t : v;
+    }
+    return v;
+}
+__device__ __forceinline__ float add_groups(float sum, float s, int lv, int lt, int lane)
+{
+    if (lt == lv) return sum + s;
+    const int first = (lane & ~((4 << lv) - 1)) | (lane & ((4 << lt) - 1)), end = 1 << (lv - lt);
+#pragma unroll 1
+    for (int j = 0; j < end; j += 4) {
+        float t[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) t[i] = __shfl_sync(0xffffffffu, s, first + ((j + i) * 4 << lt));
+#pragma unroll
+        for (int i = 0; i < 4; i++) sum = j + i < end ? sum + t[i] : sum;
+    }
+    return sum;
+}
+
+// Products that are not fused into what follows
+__device__ __forceinline__ float4 times(const float4 a, const float4 b)
+{
+    return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
+}
+
 // Stages K columns (every thread of the CTA calls it; K a multiple of 256): src holds floats, or cells if tag != 0. norm_w:
-// RMS-normalised with it. logit_cell: the row of shared memory at off_row times the (normalised) vector goes there with
-// the tag, before the splitting starts. With either of them K <= 16 kWork: the whole vector in registers. Returns whether the CTA
-// has given up.
-__device__ __forceinline__ bool stage_vec(const void *src, uint32_t tag, int K, const float *norm_w, float eps, uint2 *logit_cell)
+// RMS-normalised with it (K <= 16 kWork: the whole vector in registers). logit_cell (with norm_w): the row of shared memory at
+// off_row times the normalised vector goes there with the tag, before the splitting starts. Returns whether the CTA has given up.
+//
+// The sums are added in the order of the kernels that do the same layer by layer, so that both give the same bits (a rounding of
+// another order grows: where a router has two logits as close, another expert). Two orders exist. `fold`: the norm inside the
+// matvec and the one-launch expert block, twelve warps of which thread t has the quads t, t + 384, ... and the logit takes the
+// scale afterwards; here thread t does the work of threads t and, below 128, t + 256, from shared memory. Otherwise: a norm kernel
+// of 1024 threads (column c in thread c mod 1024) and a router of 128 (quad q in thread q mod 128) on its result.
+__device__ __forceinline__ bool stage_vec(const void *src, uint32_t tag, int K, const float *norm_w, float eps, uint2 *logit_cell, bool fold)
 {
     Misc &M = misc();
     const int tid = thread_id(), lane = tid & 31, warp = tid >> 5;
-    const bool whole = norm_w || logit_cell;
-    const int xc = head().xc;
+    const int xc = head().xc, nq = K >> 2;
 #pragma unroll 1
-    for (int base = tid * 4; base < K || whole; base += kWork * 16) {
+    for (int q0 = tid; q0 < nq || norm_w; q0 += kWork * 4) {
         float4 v[4], g[4];
         if (norm_w) {
 #pragma unroll
             for (int u = 0; u < 4; u++)
-                g[u] = base + u * kWork * 4 < K ? __ldg(reinterpret_cast<const float4 *>(norm_w + base + u * kWork * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                g[u] = q0 + u * kWork < nq ? __ldg(reinterpret_cast<const float4 *>(norm_w) + q0 + u * kWork) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         if (tag) {
             uint32_t todo = 0;
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                todo |= (base + u * kWork * 4 < K ? 1u : 0u) << u;
+                todo |= (q0 + u * kWork < nq ? 1u : 0u) << u;
             }
 #pragma unroll 1
             for (uint32_t i = 0; todo; i++) {  // what has not come is asked for again
@@ -274,7 +370,7 @@ __device__ __forceinline__ bool stage_vec(const void *src, uint32_t tag, int K, 
                 for (int u = 0; u < 4; u++) {
                     a[u] = b[u] = make_uint4(0, 0, 0, 0);
                     if (todo >> u & 1) {
-                        const uint2 *p = static_cast<const uint2 *>(src) + base + u * kWork * 4;
+                        const uint2 *p = static_cast<const uint2 *>(src) + 4 * (q0 + u * kWork);
                         a[u] = ld_cells2(p);
                         b[u] = ld_cells2(p + 2);
                     }
@@ -292,56 +388,99 @@ __device__ __forceinline__ bool stage_vec(const void *src, uint32_t tag, int K, 
         } else {
 #pragma unroll
             for (int u = 0; u < 4; u++)
-                v[u] = base + u * kWork * 4 < K ? __ldcg(reinterpret_cast<const float4 *>(static_cast<const float *>(src) + base + u * kWork * 4))
-                                                : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[u] = q0 + u * kWork < nq ? __ldcg(static_cast<const float4 *>(src) + q0 + u * kWork) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        if (whole) {
-            float ss = 0.0f, dot = 0.0f;
-            if (norm_w) {
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    ss = fmaf(v[u].x, v[u].x, fmaf(v[u].y, v[u].y, fmaf(v[u].z, v[u].z, fmaf(v[u].w, v[u].w, ss))));
-                    v[u].x *= g[u].x; v[u].y *= g[u].y; v[u].z *= g[u].z; v[u].w *= g[u].w;
-                }
-            }
-            if (logit_cell) {
+        if (norm_w) {
+            const float4 *row = reinterpret_cast<const float4 *>(smem + head().off_row);
+            // (idle until gate / up is requested; before the first projections, where it is not, the row is)
+            float4 *raw = reinterpret_cast<float4 *>(smem + (logit_cell || !fold ? head().off_ring : head().off_row)), *weighted = raw + nq;
+            if (fold) {
 #pragma unroll
                 for (int u = 0; u < 4; u++)
-                    if (base + u * kWork * 4 < K) {
-                        const float4 r = *reinterpret_cast<const float4 *>(smem + head().off_row + (base + u * kWork * 4) * 4);
-                        dot = fmaf(v[u].x, r.x, fmaf(v[u].y, r.y, fmaf(v[u].z, r.z, fmaf(v[u].w, r.w, dot))));
+                    if (q0 + u * kWork < nq) {
+                        raw[q0 + u * kWork] = v[u];
+                        if (logit_cell) weighted[q0 + u * kWork] = times(v[u], g[u]);
                     }
-            }
+                cta_sync();
+                float s[4] = {0.f, 0.f, 0.f, 0.f}, d[2] = {0.f, 0.f};  // s: the sum behind the scale; 2, 3: behind the logit's
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                ss += __shfl_xor_sync(0xffffffffu, ss, o);
-                dot += __shfl_xor_sync(0xffffffffu, dot, o);
-            }
-            if (lane == 0) {
-                M.red[0][warp] = ss;
-                M.red[1][warp] = dot;
+                for (int u = 0; u < 3; u++) {
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        const int q = tid + kWork * k + 384 * u;
+                        if (q >= nq || (k && warp >= 4)) break;
+                        const float4 x = raw[q];
+                        s[k] = fmaf(x.x, x.x, s[k]); s[k] = fmaf(x.y, x.y, s[k]); s[k] = fmaf(x.z, x.z, s[k]); s[k] = fmaf(x.w, x.w, s[k]);
+                        if (logit_cell) {
+                            const float4 r = row[q], h = weighted[q];
+                            s[2 + k] = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, s[2 + k]))));
+                            d[k] = fmaf(r.x, h.x, d[k]); d[k] = fmaf(r.y, h.y, d[k]); d[k] = fmaf(r.z, h.z, d[k]); d[k] = fmaf(r.w, h.w, d[k]);
+                        }
+                    }
+                }
+                const float all = tree_sum<4>(s, 3, lane), dots = tree_sum<2>(d, 3, lane);
+                const int k4 = result_row<4>(3, lane), k2 = result_row<2>(3, lane);
+                if ((lane & result_lanes<4>(3, 3)) == 0 && (!(k4 & 1) || warp < 4)) M.red[k4 >> 1][warp + 8 * (k4 & 1)] = all;
+                if ((lane & result_lanes<2>(3, 3)) == 0 && (!k2 || warp < 4)) M.red[2][warp + 8 * k2] = dots;
+            } else {
+                float s[4] = {0.f, 0.f, 0.f, 0.f};  // of four threads of the norm kernel
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    s[0] = fmaf(v[u].x, v[u].x, s[0]);
+                    s[1] = fmaf(v[u].y, v[u].y, s[1]);
+                    s[2] = fmaf(v[u].z, v[u].z, s[2]);
+                    s[3] = fmaf(v[u].w, v[u].w, s[3]);
+                }
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+                    for (int e = 0; e < 4; e++) s[e] += __shfl_xor_sync(0xffffffffu, s[e], o);
+                if ((lane & 7) == 0) M.red32[tid >> 3] = (s[0] + s[2]) + (s[1] + s[3]);
             }
             cta_sync();
             float t = 0.0f;
+            if (fold) {  // lanes 30 and 31 of the last warp: the logit and the sum its scale takes
+                const float *red = M.red[warp == kWarps - 1 && lane >= 30 ? 32 - lane : 0];
 #pragma unroll
-            for (int w = 0; w < kWarps; w++) t += M.red[0][w];  // fixed order: the same scale on every thread and CTA
-            const float scale = norm_w ? 1.0f / sqrtf(t / static_cast<float>(K) + eps) : 1.0f;
-            if (logit_cell && tid == 0) {
-                float d = 0.0f;
-#pragma unroll
-                for (int w = 0; w < kWarps; w++) d += M.red[1][w];
-                st_cell(logit_cell, d * scale, tag);
+                for (int w = 0; w < 12; w++) t += red[w];
+            } else {
+                t = warp_sum(M.red32[lane]);
+            }
+            float scale = 1.0f / sqrtf(t / static_cast<float>(K) + eps);
+            if (fold) {
+                t = __shfl_sync(0xffffffffu, t, 30);
+                if (logit_cell && tid == kWork - 1) st_cell(logit_cell, t * scale, tag);
+                scale = __shfl_sync(0xffffffffu, scale, 0);
             }
 #pragma unroll
-            for (int u = 0; u < 4; u++) { v[u].x *= scale; v[u].y *= scale; v[u].z *= scale; v[u].w *= scale; }
+            for (int u = 0; u < 4; u++) v[u] = times(times(v[u], make_float4(scale, scale, scale, scale)), g[u]);
+            if (logit_cell && !fold) {
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (q0 + u * kWork < nq) raw[q0 + u * kWork] = v[u];
+                cta_sync();
+                if (tid < 128) {
+                    float d = 0.0f;
+#pragma unroll 2
+                    for (int q = tid; q < nq; q += 128) {
+                        const float4 r = row[q], x = raw[q];
+                        d = fmaf(r.x, x.x, d); d = fmaf(r.y, x.y, d); d = fmaf(r.z, x.z, d); d = fmaf(r.w, x.w, d);
+                    }
+                    d = warp_sum(d);
+                    if (lane == 0) M.red[0][warp] = d;
+                    asm volatile("bar.sync 2, 128;" ::: "memory");
+                    if (tid == 0) st_cell(logit_cell, (M.red[0][0] + M.red[0][1]) + (M.red[0][2] + M.red[0][3]), tag);
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // ring or row were written as plain memory
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-            const int c0 = base + u * kWork * 4;
-            if (c0 - lane * 4 >= K) break;  // warp-uniform: a warp covers 128 columns
-            stage_quad(xc, v[u], c0, lane);
+            const int q = q0 + u * kWork;
+            if (q - lane >= nq) break;  // warp-uniform: a warp covers 128 columns
+            stage_quad(xc, v[u], 4 * q, lane);
         }
-        if (whole) break;
+        if (norm_w) break;
     }
     return cta_aborted();
 }
@@ -381,15 +520,16 @@ __device__ __forceinline__ uint32_t prefetch(const uint8_t *w, int r0, int n, ui
 // Those rows (first units requested by prefetch() with the same arguments) times the staged vector from super-block xcol on:
 // dst[row] = value (with keep: added to keep[row], which takes the sum), as a cell if tag != 0. Returns the ring's parities.
 template <class F, int RU>
-__device__ __forceinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, int r0, int n, void *dst, uint32_t tag, float *keep, int xcol,
-                                        int stages, uint32_t parity)
+__device__ __forceinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, int lt, int r0, int n, void *dst, uint32_t tag, float *keep,
+                                        int xcol, int stages, uint32_t parity)
 {
     uint8_t *buf = ring();
     uint64_t *bars = ring_bars();
     const int xc = head().xc;
     const int lane = thread_id() & 31, q = lane >> 2, sub = lane & 3;
-    const int v = 1 << lv, rpp = 8 >> lv, cq = q & (v - 1), rq = q >> lv, W = 4 << lv;
-    const int groups = (bpr + v - 1) >> lv, ur = RU * rpp;
+    const int rpp = 8 >> lv, rq = q >> lv, one = result_lanes<RU>(lv, lt);
+    const int groups = (bpr + (1 << lv) - 1) >> lv, ur = RU * rpp;
+    const Passes P(lv, lt, q);
     const uint32_t row_bytes = bpr * F::kBlockBytes, sb = stage_bytes_of(ur * row_bytes);
     typename F::XRegs xr;
     int s = 0;
@@ -399,13 +539,13 @@ __device__ __forceinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, in
         uint32_t skew = 0;
         if (F::kBlockBytes % 16) skew = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(w) + (size_t)(r0 + r) * row_bytes) & 15u;
         const uint8_t *base = buf + s * sb + skew + rq * row_bytes;
-        float acc[RU];
+        float sum = 0.0f, acc[RU];
 #pragma unroll
         for (int i = 0; i < RU; i++) acc[i] = 0.0f;
 #pragma unroll 1
         for (int c = 0; c < groups; c++) {
-            const int col = (c << lv) + cq;
-            const bool in = col < bpr;  // a ragged last group
+            const int col = P.at(c);
+            const bool in = col < bpr;  // a ragged last pass
             const int at = in ? col : 0;
             if (groups > 1 || r == 0) load_x(xr, xc, xcol + at, sub);
 #pragma unroll
@@ -414,14 +554,17 @@ __device__ __forceinline__ uint32_t matvec(const uint8_t *w, int bpr, int lv, in
                 const float d = F::block_dot(base + (i * rpp) * row_bytes + at * F::kBlockBytes, sub, xr);
                 acc[i] += in ? d : 0.0f;
             }
+            if (P.reduces(c)) {
+                sum = add_groups(sum, tree_sum<RU>(acc, lt, lane), lv, lt, lane);
+#pragma unroll
+                for (int i = 0; i < RU; i++) acc[i] = 0.0f;
+            }
         }
         __syncwarp();
         const int nr = r + stages * ur;
         if (lane == 0 && nr < n) issue_unit(w, r0 + nr, min(ur, n - nr), row_bytes, buf + s * sb, &bars[s]);
-        int which;
-        const float sum = stream::packed_sum<RU, false>(acc, W, lane, which);
-        const int row = r + which * rpp + rq;
-        if ((lane & (W / RU - 1)) == 0 && row < n) {
+        const int row = r + result_row<RU>(lt, lane) * rpp + rq;
+        if ((lane & one) == 0 && row < n) {
             float o = sum;
             if (keep) keep[r0 + row] = o += keep[r0 + row];
             if (tag)
@@ -451,15 +594,10 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint4 &a, uint32_t
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b0), "r"(b1));
 }
-template <bool TRANS>
-__device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t (&r)[4])
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t addr, uint32_t (&r)[4])
 {
-    if (TRANS)
-        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-    else
-        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 __device__ __forceinline__ uint32_t pack2(float a, float b)
 {
@@ -473,13 +611,13 @@ __device__ __forceinline__ float4 norm_rope(float4 v, int which, bool normed, fl
     const Misc &M = misc();
     const int lane = thread_id() & 31;
     const float *w = M.norm[which];
-    const float ss = warp_sum(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
+    const float ss = warp_sum(fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x))));
     if (normed) {
         const float f = 1.0f / sqrtf(ss * (1.0f / 128.0f) + eps);
-        v.x *= f * w[lane];
-        v.y *= f * w[lane + 32];
-        v.z *= f * w[lane + 64];
-        v.w *= f * w[lane + 96];
+        v.x = v.x * f * w[lane];
+        v.y = v.y * f * w[lane + 32];
+        v.z = v.z * f * w[lane + 64];
+        v.w = v.w * f * w[lane + 96];
     }
     const float c0 = M.rope[lane], c1 = M.rope[lane + 32], s0 = M.rope[64 + lane], s1 = M.rope[96 + lane];
     return make_float4(v.x * c0 - v.z * s0, v.y * c1 - v.w * s1, v.x * s0 + v.z * c0, v.y * s1 + v.w * c1);
@@ -488,13 +626,13 @@ __device__ __forceinline__ float4 norm_rope(float4 v, int which, bool normed, fl
 // K / V rows of a tile of 16 positions, a row per lane
 __device__ __forceinline__ void load_kv(const __half *kv_k, const __half *kv_v, int tile, int pos, int n_kv, int kvh)
 {
-    const int lane = thread_id() & 31;
+    const int lane = thread_id() & 31, r = lane & 15;
     uint8_t *buf = ring();
     uint64_t *bar = ring_bars();
     if (lane == 0) mbar_expect_tx(bar, 32 * 256);
     __syncwarp();
-    const int p = min(tile * 16 + (lane & 15), pos);
-    bulk_g2s(buf + lane * kKvPitch, (lane < 16 ? kv_k : kv_v) + ((size_t)p * n_kv + kvh) * 128, 256, bar);
+    bulk_g2s(buf + (lane < 16 ? r * kKPitch : kVOff + r * kVPitch), (lane < 16 ? kv_k : kv_v) + ((size_t)min(tile * 16 + r, pos) * n_kv + kvh) * 128,
+             256, bar);
 }
 
 // This warp's tiles (tile, tile + kWarps, ... < t1; the first has been requested into the ring) for the 16 query heads whose
@@ -513,9 +651,8 @@ __device__ __forceinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_
 #pragma unroll
     for (int u = 0; u < 16; u++) O[u][0] = O[u][1] = O[u][2] = O[u][3] = 0.0f;
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;
-    const uint32_t kbase = smem_u32(buf), vbase = kbase + 16 * kKvPitch;
-    const uint32_t ka = kbase + (lane & 7) * kKvPitch + (lane >> 3) * 16;
-    const uint32_t va = vbase + ((lane & 7) + ((lane >> 3) & 1) * 8) * kKvPitch + (lane >> 4) * 16;
+    const uint8_t *ka = buf + g * kKPitch + t * 16;
+    const uint32_t va = smem_u32(buf) + kVOff + ((lane & 7) + ((lane >> 3) & 1) * 8) * kVPitch + (lane >> 4) * 16;
 #pragma unroll 1
     for (;;) {
         ring_wait(bars, 0, parity);
@@ -527,13 +664,13 @@ __device__ __forceinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_
             const float4 kr = norm_rope(make_float4(kv[0], kv[1], kv[2], kv[3]), 1, k_normed, eps);
             const float kn[4] = {kr.x, kr.y, kr.z, kr.w};
             const size_t row = ((size_t)pos * n_kv + kvh) * 128;
-            uint8_t *kd = buf + (pos & 15) * kKvPitch;
+            uint8_t *kd = buf + (pos & 15) * kKPitch, *vd = buf + kVOff + (pos & 15) * kVPitch;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const int d = lane + 32 * i;
                 const __half hk = __float2half_rn(kn[i]), hv = __float2half_rn(vv[i]);
                 *reinterpret_cast<__half *>(kd + 2 * d) = hk;
-                *reinterpret_cast<__half *>(kd + 16 * kKvPitch + 2 * d) = hv;
+                *reinterpret_cast<__half *>(vd + 2 * d) = hv;
                 if (store) {
                     kv_k[row + d] = hk;
                     kv_v[row + d] = hv;
@@ -541,25 +678,25 @@ __device__ __forceinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_
             }
             __syncwarp();
         }
-        float S[2][4], T[2][4];  // hi and lo halves of Q: independent chains
+        float S[2][4];
 #pragma unroll
         for (int n = 0; n < 2; n++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) S[n][e] = T[n][e] = 0.0f;
+            for (int e = 0; e < 4; e++) S[n][e] = 0.0f;
 #pragma unroll 1
-        for (int jj = 0; jj < 4; jj++) {
+        for (int jj = 0; jj < 4; jj++) {  // 32 dims, eight of a lane: two steps
             const uint8_t *f = smem + kX + (2 * jj * 32 + lane) * 16;
             const uint4 h0 = *reinterpret_cast<const uint4 *>(f), h1 = *reinterpret_cast<const uint4 *>(f + 512);
             const uint4 lo0 = *reinterpret_cast<const uint4 *>(f + 4096), lo1 = *reinterpret_cast<const uint4 *>(f + 4096 + 512);
-#pragma unroll
-            for (int n = 0; n < 2; n++) {
-                uint32_t b[4];
-                ldmatrix4<false>(ka + n * 8 * kKvPitch + jj * 64, b);
-                mma16816(S[n], h0, b[0], b[1]);
-                mma16816(T[n], lo0, b[0], b[1]);
-                mma16816(S[n], h1, b[2], b[3]);
-                mma16816(T[n], lo1, b[2], b[3]);
-            }
+            const uint4 b0 = *reinterpret_cast<const uint4 *>(ka + jj * 64), b1 = *reinterpret_cast<const uint4 *>(ka + 8 * kKPitch + jj * 64);
+            mma16816(S[0], h0, b0.x, b0.y);
+            mma16816(S[1], h0, b1.x, b1.y);
+            mma16816(S[0], lo0, b0.x, b0.y);
+            mma16816(S[1], lo0, b1.x, b1.y);
+            mma16816(S[0], h1, b0.z, b0.w);
+            mma16816(S[1], h1, b1.z, b1.w);
+            mma16816(S[0], lo1, b0.z, b0.w);
+            mma16816(S[1], lo1, b1.z, b1.w);
         }
         float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
@@ -567,8 +704,8 @@ __device__ __forceinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_
 #pragma unroll
             for (int e = 0; e < 2; e++) {
                 const bool in = tile * 16 + n * 8 + 2 * t + e <= pos;
-                S[n][e] = in ? S[n][e] + T[n][e] : -INFINITY;
-                S[n][2 + e] = in ? S[n][2 + e] + T[n][2 + e] : -INFINITY;
+                S[n][e] = in ? S[n][e] : -INFINITY;
+                S[n][2 + e] = in ? S[n][2 + e] : -INFINITY;
                 mx0 = fmaxf(mx0, S[n][e]);
                 mx1 = fmaxf(mx1, S[n][2 + e]);
             }
@@ -603,7 +740,7 @@ __device__ __forceinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_
 #pragma unroll
         for (int u = 0; u < 16; u += 2) {
             uint32_t b[4];
-            ldmatrix4<true>(va + u * 16, b);
+            ldmatrix4_trans(va + u * 16, b);
             mma16816(O[u], pa, b[0], b[1]);
             mma16816(O[u + 1], pa, b[2], b[3]);
         }
@@ -648,8 +785,8 @@ __device__ __forceinline__ void q_fragments(const uint2 *c_q, uint32_t tag, int 
         }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-            const int d = lane + 32 * i, kk = d & 15;
-            const int at = ((d >> 4) * 32 + (h & 7) * 4 + ((kk & 7) >> 1)) * 16 + ((h >> 3) + 2 * (kk >> 3)) * 4 + (kk & 1) * 2;
+            const int e = lane & 7;  // of the eight dims 32 i + 8 t .. + 7: the lower four in step 2 i, the others in the next
+            const int at = ((2 * i + (e >> 2)) * 32 + (h & 7) * 4 + (lane >> 3)) * 16 + ((h >> 3) + (e & 2)) * 4 + (e & 1) * 2;
             const float s = v[i] * sc;
             const __half hi = __float2half_rn(s);
             *reinterpret_cast<__half *>(smem + kX + at) = hi;
@@ -684,62 +821,94 @@ __device__ __forceinline__ void attn_partial(int nw, int nh, uint2 *c_part, uint
     }
 }
 
-// Merges the nc chunks' partials of one head (hq of head block b): the CTA's warps over the chunks; cells of the result.
+// Merges the nc chunks' partials of one head (hq of head block b), cells of the result. Warp 0 has the chunks' maxima and sums, the
+// others bring the partials into shared memory (the ring is idle); then a thread per dim adds them up in chunk order.
 __device__ __forceinline__ void merge_head(int b, int hq, int nc, int chunks, const uint2 *c_part, const uint2 *c_ml, uint2 *dst, uint32_t tag)
 {
-    Misc &M = misc();
     const int tid = thread_id(), lane = tid & 31, warp = tid >> 5;
-    float m = -INFINITY, s = 0.0f;
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 1
-    for (int c0 = warp; c0 < nc; c0 += 5 * kWarps) {
-        uint4 ms[5], o0[5], o1[5];
+    float *fm = reinterpret_cast<float *>(smem + kX), *fl = fm + kMaxChunks, *part = reinterpret_cast<float *>(smem + head().off_ring);
+    if (warp == 0) {
+        constexpr int kPer = kMaxChunks / 32;
+        float m[kPer], l[kPer], mt = -INFINITY, lt = 0.0f;
 #pragma unroll 1
         for (uint32_t i = 0;; i++) {
             bool ok = true;
 #pragma unroll
-            for (int u = 0; u < 5; u++) {
-                const size_t slot = ((size_t)b * chunks + min(c0 + u * kWarps, nc - 1)) * 16 + hq;
-                ms[u] = ld_cells2(c_ml + slot * 2);
-                o0[u] = ld_cells2(c_part + slot * 128 + 4 * lane);
-                o1[u] = ld_cells2(c_part + slot * 128 + 4 * lane + 2);
-                ok = ok && ms[u].y == tag && ms[u].w == tag && o0[u].y == tag && o0[u].w == tag && o1[u].y == tag && o1[u].w == tag;
+            for (int u = 0; u < kPer; u++) {
+                m[u] = -INFINITY;
+                l[u] = 0.0f;
+                if (lane + 32 * u < nc) {
+                    const uint4 v = ld_cells2(c_ml + (((size_t)b * chunks + lane + 32 * u) * 16 + hq) * 2);
+                    m[u] = __uint_as_float(v.x);
+                    l[u] = __uint_as_float(v.z);
+                    ok = ok && v.y == tag && v.w == tag;
+                }
             }
             if (ok || *gave_up()) break;
             if (i == kPolls) *gave_up() = 1;
         }
         __syncwarp();
 #pragma unroll
-        for (int u = 0; u < 5; u++) {
-            if (c0 + u * kWarps >= nc) break;
-            const float mu = __uint_as_float(ms[u].x), mn = fmaxf(m, mu), fo = exp2f(m - mn), fn = exp2f(mu - mn);
-            s = s * fo + __uint_as_float(ms[u].z) * fn;
-            a.x = a.x * fo + __uint_as_float(o0[u].x) * fn;
-            a.y = a.y * fo + __uint_as_float(o0[u].z) * fn;
-            a.z = a.z * fo + __uint_as_float(o1[u].x) * fn;
-            a.w = a.w * fo + __uint_as_float(o1[u].z) * fn;
-            m = mn;
+        for (int u = 0; u < kPer; u++) mt = fmaxf(mt, m[u]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, o));
+#pragma unroll
+        for (int u = 0; u < kPer; u++) {
+            if (32 * u >= nc) break;
+            const float f = exp2f(m[u] - mt);  // 0 beyond the last chunk
+            fm[lane + 32 * u] = f;
+            lt = fmaf(l[u], f, lt);            // chunk c in lane c mod 16
+            lt = fmaf(__shfl_down_sync(0xffffffffu, l[u], 16), __shfl_down_sync(0xffffffffu, f, 16), lt);
         }
-    }
-    float *buf = reinterpret_cast<float *>(smem + kX);  // [kWarps][128]
-    *reinterpret_cast<float4 *>(buf + warp * 128 + 4 * lane) = a;
-    if (lane == 0) {
-        M.red[0][warp] = m;
-        M.red[1][warp] = s;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) lt += __shfl_xor_sync(0xffffffffu, lt, o);
+        if (lane == 0) *fl = lt > 0.0f ? 1.0f / lt : 0.0f;
+    } else {
+#pragma unroll 1
+        for (int c0 = warp - 1; c0 < nc; c0 += 6 * (kWarps - 1)) {
+            uint4 o0[6], o1[6];
+#pragma unroll 1
+            for (uint32_t i = 0;; i++) {
+                bool ok = true;
+#pragma unroll
+                for (int u = 0; u < 6; u++) {
+                    const uint2 *p = c_part + (((size_t)b * chunks + min(c0 + u * (kWarps - 1), nc - 1)) * 16 + hq) * 128 + 4 * lane;
+                    o0[u] = ld_cells2(p);
+                    o1[u] = ld_cells2(p + 2);
+                    ok = ok && o0[u].y == tag && o0[u].w == tag && o1[u].y == tag && o1[u].w == tag;
+                }
+                if (ok || *gave_up()) break;
+                if (i == kPolls) *gave_up() = 1;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 6; u++) {
+                const int c = c0 + u * (kWarps - 1);
+                if (c >= nc) break;
+                *reinterpret_cast<uint4 *>(part + c * 128 + 4 * lane) = make_uint4(o0[u].x, o0[u].z, o1[u].x, o1[u].z);
+            }
+        }
     }
     cta_sync();
     if (tid < 128) {
-        float mt = -INFINITY, st = 0.0f, o = 0.0f;
+        float o = 0.0f;
+        float p[8];
 #pragma unroll
-        for (int w = 0; w < kWarps; w++) mt = fmaxf(mt, M.red[0][w]);
+        for (int u = 0; u < 8; u++) p[u] = u < nc ? part[u * 128 + tid] : 0.0f;
+#pragma unroll 1
+        for (int c = 0; c < nc; c += 8) {  // (the weights beyond the last chunk are 0)
+            const float4 f0 = *reinterpret_cast<const float4 *>(fm + c), f1 = *reinterpret_cast<const float4 *>(fm + c + 4);
+            const float f[8] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w};
 #pragma unroll
-        for (int w = 0; w < kWarps; w++) {
-            const float f = exp2f(M.red[0][w] - mt);  // 0 for a warp without a chunk
-            st = fmaf(M.red[1][w], f, st);
-            o = fmaf(buf[w * 128 + tid], f, o);
+            for (int u = 0; u < 8; u++) {
+                const float x = p[u];
+                p[u] = c + 8 + u < nc ? part[(c + 8 + u) * 128 + tid] : 0.0f;
+                o = fmaf(x, f[u], o);
+            }
         }
-        st_cell(dst + tid, o / st, tag);
+        st_cell(dst + tid, o * *fl, tag);
     }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the ring was written and read as plain memory
     cta_sync();
 }
 
@@ -751,117 +920,199 @@ __device__ __forceinline__ uint32_t ordered(float v)
 }
 __device__ __forceinline__ float unordered(uint32_t k) { return __uint_as_float(k ^ ((k >> 31) ? 0x80000000u : 0xFFFFFFFFu)); }
 
-// One thread: the reference's walk (n <= 32 k: nothing is dropped before the merge) over the logits in (e % 32, e / 32) order,
-// replacing the first minimum when strictly greater.
+// One thread: the reference's walk over the logits in (e % 32, e / 32) order (n <= 32 k: nothing is dropped before the merge),
+// replacing the first minimum when strictly greater. M.slot_pos: candidate of each slot.
 __device__ __noinline__ void walk(int n, int k)
 {
     Misc &M = misc();
 #pragma unroll 1
-    for (int i = 0; i < k; i++) {
-        M.top_id[i] = 0;
-        M.top_key[i] = 0;
-    }
+    for (int i = 0; i < k; i++) M.slot_pos[i] = -1;
 #pragma unroll 1
-    for (int l = 0; l < 32; l++)
+    for (int p = 0; p < n; p++) {
+        int at = 0;
+        uint32_t least = 0xFFFFFFFFu;
 #pragma unroll 1
-        for (int e = l; e < n; e += 32) {
-            int at = 0;
-#pragma unroll 1
-            for (int i = 1; i < k; i++)
-                if (M.top_key[i] < M.top_key[at]) at = i;
-            if (M.key[e] > M.top_key[at]) {
-                M.top_key[at] = M.key[e];
-                M.top_id[at] = e;
+        for (int i = 0; i < k; i++) {
+            const uint32_t v = M.slot_pos[i] < 0 ? 0 : M.key[M.slot_pos[i]];
+            if (v < least) {
+                least = v;
+                at = i;
             }
         }
+        if (M.key[p] > least) M.slot_pos[at] = p;
+    }
 }
 
-// The k largest of n logits (every thread of the CTA calls it): lane i < k of every warp returns the i-th expert, M.top_key
-// keeps their logits. -1: the CTA has given up.
-__device__ __forceinline__ int select_experts(const uint2 *cells, uint32_t tag, int n, int k)
+// The k largest of n logits (every thread of the CTA calls it): M.top_id, the largest first, and what select_weights() needs. False:
+// the CTA has given up.
+__device__ __forceinline__ bool select_experts(const uint2 *cells, uint32_t tag, int n, int k)
 {
     Misc &M = misc();
-    const int tid = thread_id(), lane = tid & 31;
+    const int tid = thread_id(), lane = tid & 31, warp = tid >> 5;
     static_assert(kWork >= kMaxExperts, "a thread per logit");
-    if (tid < kMaxExperts) M.key[tid] = tid < n ? ordered(wait_value(cells + tid, tag)) : 0;
-    if (cta_aborted()) return -1;
+    if (tid < kMaxExperts) {
+        if (tid < n) {
+            const int l = tid & 31, p = l * (n >> 5) + min(l, n & 31) + (tid >> 5);  // its place in the walk
+            M.eid[p] = static_cast<uint8_t>(tid);
+            M.key[p] = ordered(wait_value(cells + tid, tag));
+        } else {
+            M.key[tid] = 0;
+        }
+    }
+    if (tid == 0) M.walked = 0;
+    if (cta_aborted()) return false;
     {
         const int half = ((n + 7) >> 3) * 4, lo = (tid & 1) ? half : 0, hi = lo + half;  // keys beyond n are 0
 #pragma unroll 1
-        for (int e = tid >> 1; e - (lane >> 1) < n; e += kWork / 2) {  // warp-uniform; two threads per expert
-            const uint32_t me = M.key[e];
-            int rank = 0;
-#pragma unroll 4
-            for (int i = lo; i < hi; i += 4) {  // an equal one before it counts as larger (a key is never the largest integer)
+        for (int p = tid >> 1, it = 0; p - (lane >> 1) < n; p += kWork / 2, it++) {  // warp-uniform; two threads per candidate
+            const uint32_t me = M.key[p];
+            uint32_t count = 0;  // of larger ones (an equal one before it counts: a key is never the largest integer); high half: before it
+#pragma unroll 2
+            for (int i = lo; i < hi; i += 4) {
                 const uint4 o = *reinterpret_cast<const uint4 *>(&M.key[i]);
-                rank += (o.x + (i < e) > me) + (o.y + (i + 1 < e) > me) + (o.z + (i + 2 < e) > me) + (o.w + (i + 3 < e) > me);
+                const uint32_t c0 = i < p, c1 = i + 1 < p, c2 = i + 2 < p, c3 = i + 3 < p;
+                count += (o.x + c0 > me ? (c0 << 16) + 1 : 0) + (o.y + c1 > me ? (c1 << 16) + 1 : 0) + (o.z + c2 > me ? (c2 << 16) + 1 : 0) +
+                         (o.w + c3 > me ? (c3 << 16) + 1 : 0);
             }
-            rank += __shfl_xor_sync(0xffffffffu, rank, 1);
-            if (rank <= k && e < n && !(tid & 1)) {
-                M.top_id[rank] = e;
+            count += __shfl_xor_sync(0xffffffffu, count, 1);
+            const int rank = count & 0xFFFF;
+            const bool mine = p < n && !(tid & 1);
+            if (mine && rank <= k) {
+                M.top_id[rank] = M.eid[p];
+                M.top_pos[rank] = p;
                 M.top_key[rank] = me;
             }
+            // the walk accepts what fewer than k before it are as large as
+            const bool accept = mine && static_cast<int>(count >> 16) < k;
+            const uint32_t bits = __ballot_sync(0xffffffffu, accept);
+            if (lane == 0) M.accepted[it * kWarps + warp] = bits;
+            if (!(tid & 1)) M.acc_key[p] = accept ? me : 0xFFFFFFFFu;  // (larger than any key)
         }
     }
     cta_sync();
     if (n > k && M.top_key[k - 1] == M.top_key[k]) {  // the same for the whole CTA
         cta_sync();
-        if (tid == 0) walk(n, k);
+        if (tid == 0) {
+            walk(n, k);
+            for (int i = 0; i < k; i++) {
+                M.top_id[i] = M.eid[M.slot_pos[i]];
+                M.top_pos[i] = M.slot_pos[i];
+                M.top_key[i] = M.key[M.slot_pos[i]];
+            }
+            M.walked = 1;
+        }
         cta_sync();
     }
-    return M.top_id[lane < k ? lane : 0];
+    return true;
 }
-// One warp, later (the requests for the experts do not need them): the weights of the selected, to M.swt.
-__device__ __forceinline__ void select_weights(int k)
+// The reference's output slots of the selected (M.order) and their weights (M.swt): of the accepted candidates the i-th takes slot i,
+// a later one that of the candidate it replaces, the one of rank i - k from below. Not needed before the down projection, hence in
+// two parts. First, by all warps while their first weights are on the way: the ranks among the accepted.
+__device__ __forceinline__ void rank_accepted(int n)
+{
+    Misc &M = misc();
+    const int tid = thread_id(), lane = tid & 31;
+    if (M.walked != 1) {
+        const int half = ((n + 7) >> 3) * 4, lo = (tid & 1) ? half : 0, hi = lo + half;
+#pragma unroll 1
+        for (int p = tid >> 1; p - (lane >> 1) < n; p += kWork / 2) {
+            const uint32_t me = M.acc_key[p];
+            uint32_t count = 0;  // smaller ones; high half: equal ones
+#pragma unroll 1
+            for (int i = lo; i < hi; i += 4) {
+                const uint4 o = *reinterpret_cast<const uint4 *>(&M.acc_key[i]);
+                count += (o.x < me) + (o.y < me) + (o.z < me) + (o.w < me);
+                count += ((o.x == me) + (o.y == me) + (o.z == me) + (o.w == me)) << 16;
+            }
+            count += __shfl_xor_sync(0xffffffffu, count, 1);
+            if (!(tid & 1) && me != 0xFFFFFFFFu) {
+                int t = __popc(M.accepted[p >> 4] & ((1u << (2 * (p & 15))) - 1u));
+#pragma unroll 1
+                for (int w = 0; w < p >> 4; w++) t += __popc(M.accepted[w]);
+                M.by_rank[count & 0xFFFF] = static_cast<uint8_t>(t);
+                if (count >> 17) M.walked = 2;  // equal ones among them: the walk itself
+            }
+        }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&M.ranked);
+}
+// Then, by one warp.
+__device__ __forceinline__ void select_weights(int n, int k, uint32_t parity)
 {
     Misc &M = misc();
     const int lane = thread_id() & 31;
-    const float v = lane < k ? unordered(M.top_key[lane]) : -INFINITY;
+    wait_copy(&M.ranked, parity);
+    const int walked = *const_cast<volatile int *>(&M.walked);
+    if (walked == 0) {
+        const int m = __reduce_add_sync(0xffffffffu, lane * 16 < n ? __popc(M.accepted[lane]) : 0);
+        if (lane < k) {  // the i-th largest: where its chain of replacements began (each of them came before what replaced it)
+            int t = M.by_rank[max(m - 1 - lane, 0)];
+#pragma unroll 1
+            for (int i = 0; i < n && t >= k; i++) t = M.by_rank[t - k];
+            M.order[t < k ? t : 0] = lane;  // (t >= k: only if the CTA has given up)
+        }
+    } else if (walked == 1) {
+        if (lane < k) M.order[lane] = lane;
+    } else {
+        if (lane == 0) walk(n, k);
+        __syncwarp();
+        if (lane < k) {
+#pragma unroll 1
+            for (int i = 0; i < k; i++)
+                if (M.top_pos[i] == M.slot_pos[lane]) M.order[lane] = i;
+        }
+    }
+    __syncwarp();
+    const float v = lane < k ? unordered(M.top_key[M.order[lane]]) : -INFINITY;
     float mx = v;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int o = kMaxK / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     const float e = lane < k ? expf(v - mx) : 0.0f;
-    const float sum = warp_sum(e);
+    float sum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kMaxK; i++) sum += __shfl_sync(0xffffffffu, e, i);  // (0 beyond the k-th)
     if (lane < k) M.swt[lane] = e / sum;
 }
 
 // ---- gate / up: items [i0, i0 + n), item i = a pass of gate rows and the same up rows of the i / ipe-th routed expert. Two items
 // a stage: their four products hide one another's latency, and one reduction serves them (a warp has 3 to 11 items). ----
 // Every lane calls it: lane 2 j + h requests half h (gate, up) of item i + j of the stage, j < 2.
-__device__ __forceinline__ void issue_items(const uint8_t *experts, size_t estride, uint32_t up_off, int id, int i, int end, int ipe, uint32_t magic,
+__device__ __forceinline__ void issue_items(const uint8_t *experts, size_t estride, uint32_t up_off, int i, int end, int ipe, uint32_t magic,
                                             uint32_t half, bool mine, int j, int h, uint8_t *dst, uint64_t *bar)
 {
     const int item = i + j, slot = __umulhi(item, magic);
-    const int ex = __shfl_sync(0xffffffffu, id, slot & 31);
     const bool in = mine && item < end;
     if (in && j == 0 && h == 0) mbar_expect_tx(bar, (i + 1 < end ? 4 : 2) * half);
     __syncwarp();
-    if (in) bulk_g2s(dst + (2 * j + h) * half, experts + (size_t)ex * estride + (item - slot * ipe) * half + (h ? up_off : 0), half, bar);
+    if (in) bulk_g2s(dst + (2 * j + h) * half, experts + (size_t)misc().top_id[slot] * estride + (item - slot * ipe) * half + (h ? up_off : 0), half, bar);
 }
-// id: lane i holds the i-th routed expert. Writes SwiGLU's result as cells act[slot * EFF + row].
-__device__ __forceinline__ uint32_t gate_up(const uint8_t *experts, size_t estride, uint32_t up_off, int id, int i0, int n, int ipe, uint32_t magic,
-                                            int bpr, int lv, int EFF, uint2 *act, uint32_t tag, int stages, uint32_t parity)
+// Writes SwiGLU's result as cells act[slot * EFF + row].
+__device__ __forceinline__ uint32_t gate_up(const uint8_t *experts, size_t estride, uint32_t up_off, int i0, int n, int ipe, uint32_t magic,
+                                            int bpr, int lv, int lt, int EFF, uint2 *act, uint32_t tag, int stages, uint32_t parity)
 {
     uint8_t *buf = ring();
     uint64_t *bars = ring_bars();
     const int xc = head().xc;
     const int lane = thread_id() & 31, q = lane >> 2, sub = lane & 3;
-    const int v = 1 << lv, rpp = 8 >> lv, cq = q & (v - 1), rq = q >> lv, W = 4 << lv;
-    const int groups = (bpr + v - 1) >> lv, end = i0 + n;
+    const int rpp = 8 >> lv, rq = q >> lv, one = result_lanes<4>(lv, lt);
+    const int groups = (bpr + (1 << lv) - 1) >> lv, end = i0 + n;
+    const Passes P(lv, lt, q);
     const uint32_t row_bytes = bpr * kQ4KBlock, half = rpp * row_bytes, sb = 4 * half;
     const int ij = (lane >> 1) & 1, ih = lane & 1, is = lane >> 2;  // of a request: item, half, stage
-    issue_items(experts, estride, up_off, id, i0 + 2 * is, end, ipe, magic, half, is < stages, ij, ih, buf + is * sb, &bars[is < stages ? is : 0]);
+    issue_items(experts, estride, up_off, i0 + 2 * is, end, ipe, magic, half, is < stages, ij, ih, buf + is * sb, &bars[is < stages ? is : 0]);
+    rank_accepted(head().n_experts);
     Q4::XRegs xr;
     int s = 0;
 #pragma unroll 1
     for (int i = i0; i < end; i += 2) {
         ring_wait(bars, s, parity);
         const uint8_t *base = buf + s * sb + rq * row_bytes;
-        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // gate, up of the two items
+        float sum = 0.0f, acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // gate, up of the two items
 #pragma unroll 1
         for (int c = 0; c < groups; c++) {
-            const int col = (c << lv) + cq;
-            const bool in = col < bpr;  // a ragged last group
+            const int col = P.at(c);
+            const bool in = col < bpr;  // a ragged last pass
             const int at = in ? col : 0;
             if (groups > 1 || i == i0) load_x(xr, xc, at, sub);
 #pragma unroll
@@ -870,14 +1121,17 @@ __device__ __forceinline__ uint32_t gate_up(const uint8_t *experts, size_t estri
                 const float d = Q4::block_dot(base + u * half + at * kQ4KBlock, sub, xr);
                 acc[u] += in ? d : 0.0f;
             }
+            if (P.reduces(c)) {
+                sum = add_groups(sum, tree_sum<4>(acc, lt, lane), lv, lt, lane);
+#pragma unroll
+                for (int u = 0; u < 4; u++) acc[u] = 0.0f;
+            }
         }
         __syncwarp();
-        issue_items(experts, estride, up_off, id, i + 2 * stages, end, ipe, magic, half, lane < 4, ij, ih, buf + s * sb, &bars[s]);
-        int which;
-        const float g = stream::packed_sum<4, false>(acc, W, lane, which);
-        const float u = __shfl_xor_sync(0xffffffffu, g, W >> 2);  // which ^ 1: a quarter of the row's lanes away
-        const int item = i + (which >> 1);
-        if ((lane & (W / 4 - 1)) == 0 && !(which & 1) && item < end) {
+        issue_items(experts, estride, up_off, i + 2 * stages, end, ipe, magic, half, lane < 4, ij, ih, buf + s * sb, &bars[s]);
+        const float g = sum, u = __shfl_xor_sync(0xffffffffu, g, 1 << lt);  // which ^ 1: a quarter of a group's lanes away
+        const int which = result_row<4>(lt, lane), item = i + (which >> 1);
+        if ((lane & one) == 0 && !(which & 1) && item < end) {
             const int slot = __umulhi(item, magic);
             st_cell(act + slot * EFF + (item - slot * ipe) * rpp + rq, g / (1.0f + expf(-g)) * u, tag);
         }
@@ -898,7 +1152,9 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
     if (tid < kWarps * kStages) mbar_init(&M.bars[0][0] + tid, 1);
     if (tid == kWork - 1) {
         mbar_init(&M.row_bar, 1);
+        mbar_init(&M.ranked, kWarps);
         M.abort_flag = 0;
+        M.row_pend = -1;
     }
     __syncthreads();
     // What a warp does in every layer, in shared memory: it is looked up once per operation
@@ -923,23 +1179,20 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
     }
     mbar_fence_init();
     __syncthreads();
-    const bool has_row = cta < P.n_experts;
+    auto has_row = [&] { return cta_id() < P.n_experts; };
     auto request_row = [&](int l) {
         mbar_expect_tx(&M.row_bar, P.H * 4);
         bulk_g2s(smem + P.off_row, params.L[l].router + (size_t)cta_id() * P.H, P.H * 4, &M.row_bar);
     };
-    int row_pend = has_row ? 0 : -1;  // parity of the router row on its way
-    if (has_row && tid == 0) request_row(0);
 
-    uint32_t parity = 0, pend = 0, tag = 0;  // pend: stages in flight while the CTA may still give up
-    int pos = 0, id = 0;                     // id: lane i holds the i-th routed expert
-    bool ok = true;
+    uint32_t parity = 0, pend = 0;  // pend: stages in flight while the CTA may still give up
     // One pass of the loop: an operation (there is one copy of every step's code), preceded by the request for its weights. The
     // pass before the first only requests.
 #pragma unroll 1
-    for (int it = -1, l = 0, op = kDown;; it++) {
-        const int tid = thread_id(), lane = tid & 31, warp = tid >> 5, cta = cta_id();
-        if (it >= 0) {
+    for (int l = -1, op = kDown;;) {
+        const int tid = thread_id(), warp = tid >> 5, cta = cta_id();
+        const uint32_t tag = M.tag + l;
+        if (l >= 0) {
             const Layer &L = params.L[l];
             // ---- the input vector ----
             {
@@ -956,35 +1209,32 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                 } else if (op == kO) {
                     src = P.c_attn;
                     K = P.QD;
+                    if (tid == 0 && has_row()) {
+                        M.row_pend = l & 1;
+                        request_row(l);
+                    }
                 } else if (op == kExperts) {  // the router logit of this CTA's expert on the way
                     src = P.c_h1;
                     norm_w = L.ffn_norm;
                     K = P.H;
-                    logit = has_row ? P.c_logit + cta : nullptr;
-                    if (has_row) wait_copy(&M.row_bar, l & 1);
-                    row_pend = -1;
+                    logit = has_row() ? P.c_logit + cta : nullptr;
+                    if (has_row()) wait_copy(&M.row_bar, l & 1);
+                    if (tid == 0) M.row_pend = -1;
                 }
                 // the norm weights of the heads: on their way while the vector is waited for
                 const float *hw = tid < 128 ? L.q_norm : L.k_norm;
                 float hn = 0.0f;
                 if (op == kQKV && tid < 256 && hw) hn = __ldg(hw + (tid & 127));
-                ok = !stage_vec(src, t, K, norm_w, P.eps, logit);
-                if (!ok) break;
+                if (stage_vec(src, t, K, norm_w, P.eps, logit, op == kQKV || L.fold)) break;
                 if (op == kQKV && tid < 256) M.norm[tid >> 7][tid & 127] = hn;
             }
             // ---- its rows ----
             if (op == kExperts) {
-                if (has_row && l + 1 < P.n_layers) {
-                    row_pend = (l + 1) & 1;
-                    if (tid == 0) request_row(l + 1);
-                }
-                id = select_experts(P.c_logit, tag, P.n_experts, P.k);
-                ok = id >= 0;
-                if (!ok) break;
+                if (!select_experts(P.c_logit, tag, P.n_experts, P.k)) break;
                 const int2 own = M.own[warp][kExperts];
-                parity = gate_up(L.experts, L.estride, L.up_off, id, own.x, own.y, P.ipe, P.ipe_magic, P.mH.bpr, P.mH.lv, P.EFF, P.c_act, tag,
+                parity = gate_up(L.experts, L.estride, L.up_off, own.x, own.y, P.ipe, P.ipe_magic, P.mH.bpr, P.mH.lv, P.mH.lt, P.EFF, P.c_act, tag,
                                  P.stages[5], parity);
-                if (warp == kWarps - 1) select_weights(P.k);
+                if (warp == kWarps - 1) select_weights(P.n_experts, P.k, l & 1);
             } else {
                 const int2 own = M.own[warp][op];
                 const int qm = M.own_qm[warp], slot = M.own_slot[warp];
@@ -994,7 +1244,7 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                 const int R0 = M.R0;
                 uint32_t t = tag;
                 bool q6 = qm == 2 && L.v_q6;
-                int bpr = P.mH.bpr, lv = P.mH.lv, xcol = 0, kind = q6 ? 1 : 0;
+                int bpr = P.mH.bpr, lv = P.mH.lv, lt = P.mH.lt, xcol = 0, kind = q6 ? 1 : 0;
                 if (op == kO) {
                     w = L.wo;
                     dst = P.c_h1;
@@ -1002,21 +1252,23 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                     q6 = false;
                     bpr = P.mQ.bpr;
                     lv = P.mQ.lv;
+                    lt = P.mQ.lt;
                     kind = 2;
                 } else if (op == kDown) {
-                    w = L.experts + (size_t)__shfl_sync(0xffffffffu, id, slot & 31) * L.estride + L.down_off;
+                    w = L.experts + (size_t)M.top_id[slot < P.k ? slot : 0] * L.estride + L.down_off;
                     dst = M.part[slot < P.k ? slot : 0] - R0;
                     t = 0;
                     q6 = L.down_q6;
                     bpr = P.mE.bpr;
                     lv = P.mE.lv;
+                    lt = P.mE.lt;
                     kind = q6 ? 4 : 3;
                     xcol = slot * bpr;
                 }
                 if (q6)
-                    parity = matvec<Q6, 2>(w, bpr, lv, own.x, own.y, dst, t, keep, xcol, P.stages[kind], parity);
+                    parity = matvec<Q6, 2>(w, bpr, lv, lt, own.x, own.y, dst, t, keep, xcol, P.stages[kind], parity);
                 else
-                    parity = matvec<Q4, 4>(w, bpr, lv, own.x, own.y, dst, t, keep, xcol, P.stages[kind], parity);
+                    parity = matvec<Q4, 4>(w, bpr, lv, lt, own.x, own.y, dst, t, keep, xcol, P.stages[kind], parity);
                 pend = 0;
             }
             // ---- attention of this CTA's positions ----
@@ -1025,16 +1277,15 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                 if (base < tile1) {
                     const int kvh = M.kvh, qb = M.qb;
                     if (tile0 < tile1) {
-                        load_kv(L.kv_k, L.kv_v, tile0, pos, P.n_kv, kvh);
+                        load_kv(L.kv_k, L.kv_v, tile0, M.pos, P.n_kv, kvh);
                         pend = 1;
                     }
                     cta_sync();  // the staged vector has been read
                     const int nh = min(16, P.gqa - qb * 16);
                     q_fragments(P.c_q + (kvh * P.gqa + qb * 16) * 128, tag, nh, L.q_norm != nullptr, P.eps, P.scale * kLog2e);
-                    ok = !cta_aborted();
-                    if (!ok) break;
+                    if (cta_aborted()) break;
                     if (tile0 < tile1)
-                        parity = attn_tiles(tile0, tile1, pos, P.n_kv, kvh, L.kv_k, L.kv_v, qb == 0, P.c_k, P.c_v, tag,
+                        parity = attn_tiles(tile0, tile1, M.pos, P.n_kv, kvh, L.kv_k, L.kv_v, qb == 0, P.c_k, P.c_v, tag,
                                             L.k_norm != nullptr, P.eps, parity);
                     pend = 0;
                     cta_sync();
@@ -1048,7 +1299,7 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
             }
         }
         // ---- the next operation's weights; gate / up requests its own: they depend on the routing ----
-        const int next = (op + 1) & 3, ln = l + (op == kDown && it >= 0 ? 1 : 0);
+        const int next = (op + 1) & 3, ln = l + (op == kDown ? 1 : 0);
         if (ln < P.n_layers && next != kExperts) {
             const Layer &L = params.L[ln];
             const int2 own = M.own[warp][next];
@@ -1063,7 +1314,7 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                 lv = P.mQ.lv;
                 kind = 2;
             } else if (next == kDown) {
-                w = L.experts + (size_t)__shfl_sync(0xffffffffu, id, M.own_slot[warp] & 31) * L.estride + L.down_off;
+                w = L.experts + (size_t)M.top_id[M.own_slot[warp] < P.k ? M.own_slot[warp] : 0] * L.estride + L.down_off;
                 q6 = L.down_q6;
                 bpr = P.mE.bpr;
                 lv = P.mE.lv;
@@ -1071,7 +1322,7 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
             }
             pend = prefetch(w, own.x, own.y, bpr * (q6 ? kQ6KBlock : kQ4KBlock), (q6 ? 4 : 5) - lv, P.stages[kind]);
         }
-        if (it < 0) {
+        if (l < 0) {
             if (P.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
             if (tid == 0) {
                 // arrivals of the launches before this one (nobody of this launch arrives before every CTA has read it: the last
@@ -1083,12 +1334,9 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                 const long long r = static_cast<long long>(c - n * grid);
                 if (r < 0) n--;
                 if (r >= grid) n++;
-                M.launch = n;
-            }
-            __syncthreads();
-            tag = static_cast<uint32_t>(M.launch) * 128u + 1u;
-            pos = __ldcg(P.pos);
-            if (tid == 0) {
+                M.tag = static_cast<uint32_t>(n) * 128u + 1u;
+                const int pos = __ldcg(P.pos);
+                M.pos = pos;
                 const int tpc = ((pos >> 4) + P.chunks) / P.chunks, ab = cta / P.chunks, ac = cta - ab * P.chunks;  // tiles per chunk; ours
                 M.nc = ((pos >> 4) + tpc) / tpc;
                 M.kvh = ab / P.qblocks;
@@ -1103,12 +1351,13 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
             const int R0 = M.R0, rows = M.rows;
             if (tid < rows) M.hid[tid] = __ldcg(P.hidden + R0 + tid);
             if (tid < 128) M.rope[tid] = __ldcg(tid < 64 ? P.cos_t + tid : P.sin_t + tid - 64);
+            __syncthreads();
         } else if (op == kDown) {
             const int R0 = M.R0, rows = M.rows;
             if (tid < rows) {
                 float y = 0.0f;
 #pragma unroll 4
-                for (int i = 0; i < P.k; i++) y = fmaf(M.swt[i], M.part[i][tid], y);
+                for (int i = 0; i < P.k; i++) y = fmaf(M.swt[i], M.part[M.order[i]][tid], y);  // in the order of the slots
                 y += M.hid[tid];
                 M.hid[tid] = y;
                 if (ln < P.n_layers)
@@ -1117,29 +1366,33 @@ __global__ void __launch_bounds__(kWork, 1) persist_kernel(const __grid_constant
                     P.hidden[R0 + tid] = y;
             }
             if (ln == P.n_layers) break;
-            tag++;
         }
         op = next;
         l = ln;
     }
     if (P.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (!ok) {  // given up: leave after the copies in flight
+    if (cta_aborted()) {  // leave after the copies in flight
+        const int tid = thread_id();
         if (tid == 0) atomicExch(P.err, MB200_ERR_TIMEOUT);
 #pragma unroll 1
         for (int s = 0; s < kStages; s++)
-            if (pend >> s & 1) mbar_wait(&M.bars[warp][s], (parity >> s) & 1);
-        if (row_pend >= 0) mbar_wait(&M.row_bar, row_pend);
+            if (pend >> s & 1) mbar_wait(&M.bars[tid >> 5][s], (parity >> s) & 1);
+        if (tid == 0 && M.row_pend >= 0) mbar_wait(&M.row_bar, M.row_pend);
     }
     __syncthreads();
-    if (tid == 0) asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(P.ctr) : "memory");
+    if (thread_id() == 0) asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(P.ctr) : "memory");
 }
 
 Split split(int w0, int nw, int passes) { return Split{w0, nw, passes / nw, passes % nw}; }
+// 2^lt: the streaming matvec's column groups (stream::prepare): the largest power of two that divides the blocks of a row, and
+// eight (the last group ragged) where that makes more groups than it has warps.
 Map map_of(int cols)
 {
-    Map m{cols / 256, 0};
-    while (m.lv < 3 && !(m.bpr >> m.lv & 1)) m.lv++;
-    if (m.lv < 2 && m.bpr >= 8) m.lv = 3;  // a ragged last group costs less than single blocks side by side
+    Map m{cols / 256, 0, 0};
+    while (m.lt < 3 && !(m.bpr >> m.lt & 1)) m.lt++;
+    if (m.bpr >> m.lt > stream::kConsumers) m.lt = 3;
+    m.lv = m.lt < 2 && m.bpr >= 8 ? 3 : m.lt;  // a ragged last pass costs less than single blocks side by side
+    if (m.lt == 3 && m.bpr % 16 == 0) m.lt = 2;  // paired: half of a group is added in the lanes
     return m;
 }
 int stage_rows(const Map &m, bool q6) { return (q6 ? 2 : 4) << (3 - m.lv); }
@@ -1203,6 +1456,7 @@ bool plan(Params &P)
     auto up = [](int v) { return (v + 127) & ~127; };
     P.off_row = up(kX + 2 * P.xc + P.xc / 8 + P.xc / 4);
     P.off_ring = up(P.off_row + P.H * 4);
+    for (int l = 0; l < P.n_layers; l++) P.L[l].fold = moe_fused_covers(P.H, P.EFF, P.k, P.L[l].down_q6 != 0);
     P.ring_bytes = ((kSmemBytes - P.off_ring) / kWarps) & ~127;
     bool v6 = false, d4 = false, d6 = false;
     for (int l = 0; l < P.n_layers; l++) {
@@ -1217,7 +1471,7 @@ bool plan(Params &P)
         P.stages[i] = P.ring_bytes / bytes[i] < kStages ? P.ring_bytes / bytes[i] : kStages;
         if (used[i] && P.stages[i] < 1) return false;
     }
-    return 32 * kKvPitch <= P.ring_bytes && 16 * kPitch * 4 <= P.ring_bytes;
+    return kVOff + 16 * kVPitch <= P.ring_bytes && 16 * kPitch * 4 <= P.ring_bytes && P.chunks <= kMaxChunks && P.chunks * 512 <= kWarps * P.ring_bytes;
 }
 
 int launch(Params &P, cudaStream_t stream)

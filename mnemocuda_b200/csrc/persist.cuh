@@ -17,6 +17,7 @@ struct Layer {
     size_t estride;
     uint32_t up_off, down_off;  // inside an expert's blob (the gate rows come first)
     int v_q6, down_q6;
+    int fold;  // the layer's expert block alone would be one launch with the norm inside: whose order of sums stage_vec follows
 };
 
 // `passes` work items over warps [w0, w0 + nw): warp i takes per items, the first rem warps one more.
@@ -25,9 +26,9 @@ struct Split {
 };
 
 // Lane map of a matrix with `bpr` super-blocks per row: a pass of a warp is v = 2^lv blocks of 8 / v rows; ceil(bpr / v) passes
-// cover the columns, the last one ragged where v does not divide bpr.
+// cover the columns, the last one ragged where v does not divide bpr. A row is summed in groups of 2^lt blocks.
 struct Map {
-    int bpr, lv;
+    int bpr, lv, lt;
 };
 
 struct Head {

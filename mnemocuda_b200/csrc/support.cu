@@ -343,11 +343,11 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
         const bool more = tile + kAttnWarps < n_tiles;
         if (more) load(tile + kAttnWarps, nxt);
 
-        float Sx[2][4], Sl[2][4];  // four independent chains (two position halves x hi / lo), added at the end
+        float Sx[2][4];  // two independent chains (the position halves)
 #pragma unroll
         for (int nt = 0; nt < 2; nt++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) Sx[nt][e] = Sl[nt][e] = 0.0f;
+            for (int e = 0; e < 4; e++) Sx[nt][e] = 0.0f;
 #pragma unroll
         for (int j = 0; j < 8; j++) {
             const uint4 ah = afrag[j * 32 + lane], al = afrag[(8 + j) * 32 + lane];
@@ -356,13 +356,9 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
                 const uint4 kk = cur.k[nt][j >> 1];
                 const uint32_t b0 = (j & 1) ? kk.z : kk.x, b1 = (j & 1) ? kk.w : kk.y;
                 mma16816(Sx[nt], ah.x, ah.y, ah.z, ah.w, b0, b1);
-                mma16816(Sl[nt], al.x, al.y, al.z, al.w, b0, b1);
+                mma16816(Sx[nt], al.x, al.y, al.z, al.w, b0, b1);
             }
         }
-#pragma unroll
-        for (int nt = 0; nt < 2; nt++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) Sx[nt][e] += Sl[nt][e];
         // mask positions beyond the chunk, running max / sum in the log2 domain
         float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
