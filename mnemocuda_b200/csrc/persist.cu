@@ -623,16 +623,17 @@ __device__ __forceinline__ float4 norm_rope(float4 v, int which, bool normed, fl
     return make_float4(v.x * c0 - v.z * s0, v.y * c1 - v.w * s1, v.x * s0 + v.z * c0, v.y * s1 + v.w * c1);
 }
 
-// K / V rows of a tile of 16 positions, a row per lane
+// K / V rows of a tile of 16 positions, a row per lane; only rows before `pos`: the cache has nothing yet at the others
 __device__ __forceinline__ void load_kv(const __half *kv_k, const __half *kv_v, int tile, int pos, int n_kv, int kvh)
 {
-    const int lane = thread_id() & 31, r = lane & 15;
+    const int lane = thread_id() & 31, r = lane & 15, rows = min(16, pos - tile * 16);
     uint8_t *buf = ring();
     uint64_t *bar = ring_bars();
-    if (lane == 0) mbar_expect_tx(bar, 32 * 256);
+    if (lane == 0) mbar_expect_tx(bar, 2 * rows * 256);
     __syncwarp();
-    bulk_g2s(buf + (lane < 16 ? r * kKPitch : kVOff + r * kVPitch), (lane < 16 ? kv_k : kv_v) + ((size_t)min(tile * 16 + r, pos) * n_kv + kvh) * 128,
-             256, bar);
+    if (r < rows)
+        bulk_g2s(buf + (lane < 16 ? r * kKPitch : kVOff + r * kVPitch), (lane < 16 ? kv_k : kv_v) + ((size_t)(tile * 16 + r) * n_kv + kvh) * 128,
+                 256, bar);
 }
 
 // This warp's tiles (tile, tile + kWarps, ... < t1; the first has been requested into the ring) for the 16 query heads whose
@@ -665,6 +666,9 @@ __device__ __forceinline__ uint32_t attn_tiles(int tile, int t1, int pos, int n_
             const float kn[4] = {kr.x, kr.y, kr.z, kr.w};
             const size_t row = ((size_t)pos * n_kv + kvh) * 128;
             uint8_t *kd = buf + (pos & 15) * kKPitch, *vd = buf + kVOff + (pos & 15) * kVPitch;
+            // the rows behind it: their scores are masked, but a probability of 0 times what the ring held might be NaN
+            for (int i = ((pos & 15) + 1) * 16 + lane; i < 256; i += 32)
+                *reinterpret_cast<uint4 *>(buf + kVOff + (i >> 4) * kVPitch + (i & 15) * 16) = make_uint4(0, 0, 0, 0);
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const int d = lane + 32 * i;

@@ -130,3 +130,28 @@ def test_one_launch_is_layer_by_layer_to_the_bit(case):
     assert torch.equal(model.hidden, want[-1]) and torch.equal(model.logits, want_logits) and int(model.token.item()) == want_token
     assert all(torch.equal(a, b) for a, b in zip(rows(), want_rows))
     assert K.mb200_device_error() == 0
+
+
+@pytest.mark.parametrize("pos", [0, 5, 16, 23, 30, 47])
+def test_unwritten_cache_rows_do_not_matter(pos):
+    """The cache holds NaN from the position on, where nothing has been stored yet, in both forms of a layer (32 query heads on a KV
+    head: two blocks of them read the row that one stores)."""
+    from mnemocuda_b200 import kernels as K
+    from mnemocuda_b200.decode import DecodeConfig, ResidentModel
+    K.mb200_init()
+    cfg = DecodeConfig(n_layers=2, hidden=2048, n_heads=32, n_kv_heads=1, head_dim=128, n_experts=16, top_k=4, moe_inter=512, vocab=512,
+                       ctx_len=64)
+    model = ResidentModel(cfg, "cuda", seed=3, kv_prefill=pos, norm_weights="random")
+    got = {}
+    for fill in (0.0, float("nan")):
+        for form in (model.layer, lambda l: layer_by_layer(model, l)):
+            for T in model.layers:
+                T["kv_k"][pos:], T["kv_v"][pos:] = fill, fill
+            model.set_state(9, pos)
+            model.begin()
+            for l in range(cfg.n_layers):
+                form(l)
+            got[fill, form] = model.hidden.clone()
+            assert torch.isfinite(model.hidden).all()
+    want = list(got.values())[0]
+    assert all(torch.equal(h, want) for h in got.values())
