@@ -59,7 +59,9 @@ struct SplitQ4 {
     uint32_t s1, c1, rs, cr;
     __device__ __forceinline__ void set(float s, float b)
     {
-        const float M = round_magic<10>(fmaf(16.0f, fabsf(s), fabsf(b)));  // 16 |s| + |b| < 2^11 u
+        // 16 |s1| + |b1| <= 2^11 u, so that it is an fp16 number too: 16 |s| + |b| stays 1/128 below, which is more than the 8.5 u
+        // that rounding may add
+        const float M = round_magic<10>(fmaf(16.0f, fabsf(s), fabsf(b)) * 1.0078125f);
         const float s1f = (s + M) - M, b1f = (b + M) - M, rsf = s - s1f;
         s1 = dup_half(s1f);
         rs = dup_half(rsf);

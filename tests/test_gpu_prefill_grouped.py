@@ -41,3 +41,33 @@ def test_token_counts_at_tile_edges(K, counts, H, EFF, down):
                                  np.zeros(H, np.float32)).astype(np.float64)
         assert np.linalg.norm(got[t] - want) <= 3e-4 * np.linalg.norm(want), (t, e)
     assert K.mb200_device_error() == 0
+
+
+@pytest.mark.parametrize("d,scale,dmin,m", [(0.0005245209, 19, 0.0014314651, 63), (0.0025806427, 1, 0.004219055, 5),
+                                            (0.00076055527, 57, 0.0061187744, 50)])
+def test_q4k_scales_that_round_up_to_the_next_power_of_two(K, d, scale, dmin, m):
+    """16 s + b of these sub-blocks lies just below a power of two and, rounded to the unit of the exact half of the split, just above it.
+    Gate and up of such sub-blocks only, against fp64; the bound is twelve times what fp32 accumulation over K leaves (1e-5) and a tenth
+    of what a weight off by one unit everywhere would (1e-3)."""
+    H, EFF, M = 512, 256, 24
+    rng = np.random.default_rng(6)
+    blocks = rng.integers(0, 256, (2 * EFF * H // 256, synth.Q4K_BLOCK)).astype(np.uint8)
+    blocks[:, :4] = np.array([d, dmin], np.float16).view(np.uint8)
+    blocks[:, 4:8] = scale | (scale >> 4 << 6)
+    blocks[:, 8:12] = m | (m >> 4 << 6)
+    blocks[:, 12:16] = (scale & 15) | ((m & 15) << 4)
+    g, u, dn = synth.expert_sizes(H, EFF, 14)
+    expert = np.concatenate([blocks.reshape(-1), synth.q6k_matrix(7, H, EFF).reshape(-1)])
+    x = rng.standard_normal((M, H)).astype(np.float16)
+    n = K.mb200_moe_prefill_workspace_bytes(M, 1, H, EFF, 1)
+    ws = torch.empty(n + 256, dtype=torch.uint8, device="cuda")
+    ws = ws[-ws.data_ptr() % 256:]
+    y = torch.empty(M, H, device="cuda")
+    K.mb200_moe_prefill(dev(expert), g + u + dn, g, u, 14, 1, 1, H, EFF, dev(x), dev(np.zeros((M, 1), np.int32)),
+                        dev(np.ones((M, 1), np.float32)), None, y, M, 0, ws)
+    w = oracle.dequant_q4k(blocks.reshape(-1), 2 * EFF, H).astype(np.float64)
+    gate, up = x.astype(np.float64) @ w[:EFF].T, x.astype(np.float64) @ w[EFF:].T
+    want = (gate / (1 + np.exp(-gate)) * up) @ oracle.dequant_q6k(expert[g + u:], H, EFF).astype(np.float64).T
+    err = np.linalg.norm(host(y) - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert err.max() <= 1.2e-4, err.max()
+    assert K.mb200_device_error() == 0
