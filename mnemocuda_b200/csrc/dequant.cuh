@@ -1,12 +1,16 @@
 // Weights -> pairs of fp16 (hi, lo) for the tensor cores, in packed fp16 arithmetic.
 //
-// A weight of a sub-block is w = s * n - b with n a small integer and s = d * scale, b = dmin * min of the sub-block
-// (Q6_K: w = s * (q - 32)). With a unit u, a power of two chosen per sub-block so that no |w| of it exceeds 2048 u,
-// s1 = s and b1 = b rounded to multiples of u make hi = s1 * n - b1 an integer multiple of u of at most 11 bits: one
-// HFMA2 computes it EXACTLY for two weights. lo = (s - s1) * n - (b - b1), the rest, is at most about 8 u and is rounded
-// to fp16 once: hi + lo is w to 2^-18 of the sub-block's largest weight or better. Two instructions per two weights
-// for both halves, where converting an fp32 weight, converting back, subtracting and converting the remainder took
-// ten (the producers of the grouped GEMM were issue-bound on exactly that).
+// A Q4_K weight is w = s * n - b with n a small integer and s = d * scale, b = dmin * min of the sub-block. With a unit u, a
+// power of two chosen per sub-block so that no |w| of it exceeds 2048 u, s1 = s and b1 = b rounded to multiples of u make
+// hi = s1 * n - b1 an integer multiple of u of at most 11 bits: one HFMA2 computes it EXACTLY for two weights.
+// lo = (s - s1) * n - (b - b1), the rest, is at most 8 u and is rounded to fp16 once. A Q6_K weight is w = s * (q - 32), s of 18
+// bits: with s = s1 + s2 in fp16 halves, hi is the rounded product with s1, and lo what that rounding left (one HFMA2, exact) plus
+// the product with s2, rounded once. Converting an fp32 weight, converting back, subtracting and converting the remainder took ten
+// instructions per two weights (the producers of the grouped GEMM were issue-bound on exactly that); these are three and four.
+// Error of hi + lo, root mean square over the weights of synthetic blocks: Q4_K 7e-7, Q6_K 2e-8 of the weights' (a second half
+// rounded from fp32: 1e-8 and 0). Results against fp64, six shapes from 1024 x 256 to 4096 x 1536, are as far off as with that,
+// 0.6 to 2.3e-5: fp32 accumulation decides. (A Q4_K lo from operands 16 + n, one instruction less, has 1.3e-6, a Q6_K lo from a
+// rounded s alike; results at 1024 x 256 were then 10 % further off. The exact ones cost 3 % of the time.)
 //
 // What is left is getting n out of the packed bits, on the integer pipe, which has half the FMA pipe's rate. A nibble shifted
 // to bits 6..9 of a 16-bit half and OR-ed with 0x4C00 is 16 + n: one shift and one LOP3 for two weights, no byte permute and
@@ -66,7 +70,7 @@ struct SplitQ4 {
         s1 = dup_half(s1f);
         rs = dup_half(rsf);
         c1 = dup_half(fmaf(-16.0f, s1f, -b1f));
-        cr = dup_half(fmaf(-16.0f, rsf, b1f - b));
+        cr = dup_half(b1f - b);
     }
 };
 // 32 weights whose nibbles are the low (HIGH = false) or high nibbles of 8 words, two per register in k_order
@@ -78,9 +82,9 @@ __device__ __forceinline__ void split_q4(const uint32_t (&w)[8], const SplitQ4 &
         const uint32_t v0 = ((HIGH ? w[i] << 2 : w[i] << 6) & 0x03C003C0u) | 0x4C004C00u;
         const uint32_t v1 = ((HIGH ? w[i] >> 6 : w[i] >> 2) & 0x03C003C0u) | 0x4C004C00u;
         hi[2 * i] = hfma2(v0, f.s1, f.c1);
-        lo[2 * i] = hfma2(v0, f.rs, f.cr);
+        lo[2 * i] = hfma2(hadd2(v0, 0xCC00CC00u), f.rs, f.cr);  // - 16
         hi[2 * i + 1] = hfma2(v1, f.s1, f.c1);
-        lo[2 * i + 1] = hfma2(v1, f.rs, f.cr);
+        lo[2 * i + 1] = hfma2(hadd2(v1, 0xCC00CC00u), f.rs, f.cr);
     }
 }
 
@@ -88,10 +92,8 @@ struct SplitQ6 {
     uint32_t s1, rs;
     __device__ __forceinline__ void set(float s)
     {
-        const float M = round_magic<5>(fabsf(s));  // |s (q - 32)| <= 2^11 u
-        const float s1f = (s + M) - M;
-        s1 = dup_half(s1f);
-        rs = dup_half(s - s1f);
+        s1 = dup_half(s);
+        rs = dup_half(s - __half2float(__ushort_as_half(static_cast<unsigned short>(s1))));  // exact: s has 18 bits
     }
 };
 // 32 weights q - 32: q = the nibble of `l` at bit 4 (LHI = false: at bit 0) | two bits of `h` at bit HB, << 4, of each byte.
@@ -106,9 +108,9 @@ __device__ __forceinline__ void split_q6(const uint32_t *l, const uint32_t *h, c
         const uint32_t q0 = ((LHI ? l[i] : l[i] << 4) & 0x00F000F0u) | h0, q1 = ((LHI ? l[i] >> 8 : l[i] >> 4) & 0x00F000F0u) | h1;
         const uint32_t v0 = hadd2(q0, 0xD600D600u), v1 = hadd2(q1, 0xD600D600u);  // - 96
         hi[2 * i] = hmul2(v0, f[i >> 2].s1);
-        lo[2 * i] = hmul2(v0, f[i >> 2].rs);
+        lo[2 * i] = hfma2(v0, f[i >> 2].rs, hfma2(v0, f[i >> 2].s1, hi[2 * i] ^ 0x80008000u));
         hi[2 * i + 1] = hmul2(v1, f[i >> 2].s1);
-        lo[2 * i + 1] = hmul2(v1, f[i >> 2].rs);
+        lo[2 * i + 1] = hfma2(v1, f[i >> 2].rs, hfma2(v1, f[i >> 2].s1, hi[2 * i + 1] ^ 0x80008000u));
     }
 }
 

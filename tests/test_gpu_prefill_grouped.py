@@ -71,3 +71,35 @@ def test_q4k_scales_that_round_up_to_the_next_power_of_two(K, d, scale, dmin, m)
     err = np.linalg.norm(host(y) - want, axis=1) / np.linalg.norm(want, axis=1)
     assert err.max() <= 1.2e-4, err.max()
     assert K.mb200_device_error() == 0
+
+
+def test_q6k_weights_keep_22_bits(K):
+    """One column of each expert's down projection at a time: a token's input picks it by way of a gate / up row of its own. Each
+    result is a weight times a known activation, off by the weight's two halves (4.4e-7), the activation's (2.4e-7) and fp32 rounding."""
+    H, EFF, NE = 256, 256, 6
+    g, u, d = synth.expert_sizes(H, EFF, 14)
+    rng = np.random.default_rng(8)
+    experts, want = [], []
+    for e in range(NE):
+        gate_up = np.zeros((2 * EFF, H // 256, synth.Q4K_BLOCK), np.uint8)
+        col = int(rng.integers(0, EFF))
+        for row in (col, EFF + col):  # 3 / 16 in column 0, nothing elsewhere
+            gate_up[row, 0, :2] = np.array([1 / 16], np.float16).view(np.uint8)
+            gate_up[row, 0, 4] = 1
+            gate_up[row, 0, 16] = 3
+        down = synth.q6k_matrix(900 + e, H, EFF).reshape(H, -1)
+        down[:, 192:208] = rng.integers(0, 256, (H, 16))  # scales of all eight bits
+        experts.append(np.concatenate([gate_up.reshape(-1), down.reshape(-1)]))
+        a = 3.0 * 3.0 / (1 + np.exp(-3.0))
+        want.append(a * oracle.dequant_q6k(down.reshape(-1), H, EFF).astype(np.float64)[:, col])
+    x = np.zeros((NE, H), np.float16)
+    x[:, 0] = 16
+    n = K.mb200_moe_prefill_workspace_bytes(NE, 1, H, EFF, NE)
+    ws = torch.empty(n + 256, dtype=torch.uint8, device="cuda")
+    ws = ws[-ws.data_ptr() % 256:]
+    y = torch.empty(NE, H, device="cuda")
+    K.mb200_moe_prefill(dev(np.concatenate(experts)), g + u + d, g, u, 14, NE, 1, H, EFF, dev(x), dev(np.arange(NE, dtype=np.int32).reshape(NE, 1)),
+                        dev(np.ones((NE, 1), np.float32)), None, y, NE, 0, ws)
+    got, want = host(y).astype(np.float64), np.array(want)
+    assert np.all(np.abs(got - want) <= 1e-6 * np.abs(want))
+    assert K.mb200_device_error() == 0
