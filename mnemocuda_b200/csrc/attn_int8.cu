@@ -7,7 +7,8 @@
 // of instruction issue (half of it byte -> fp16), 3.4 us for launch, Q and the warps' merge, 2.7 for the cluster's and
 // 2.6 for the last CTA's.
 //   * int8 values become fp16 exactly (0x6400 | (v + 128) is 1152 + v); q and the probabilities are carried as
-//     hi + lo fp16 pairs (22 bits), accumulation is fp32, so nothing is rounded beyond fp32 arithmetic's own size.
+//     hi + lo fp16 pairs (22 bits), accumulation is fp32, so nothing is rounded beyond fp32 arithmetic's own size. A head's q
+//     is brought into fp16's range by a power of two of its own, which its scores take back.
 //   * The K scale multiplies the score. The V scale is folded into the probability: the accumulators hold
 //     sum p * (vs / vmax) * v with vmax the largest V scale the warp has met, so the fp16 pair never leaves its range
 //     whatever the scales are; vmax multiplies back at the end.
@@ -93,6 +94,7 @@ attn_int8_kernel(const float *q, const int8_t *__restrict__ kv_k, const int8_t *
     float *lsm = msm + kWarps * 16;                               // [8][16] sums
     float *cml = lsm + kWarps * 16;                               // [2][16] the CTA's max and sum
     __shared__ int is_last;
+    __shared__ float head_scale[16];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int qb = (gqa + 15) / 16;
@@ -126,21 +128,30 @@ attn_int8_kernel(const float *q, const int8_t *__restrict__ kv_k, const int8_t *
     Tile cur, nxt;
     if (warp < n_tiles) load(warp, cur);
 
-    {   // Q fragments, hi + lo of q * scale * log2 e: warp j builds step j
-        const int d0 = 32 * t + 4 * warp;
+    // Q fragments, hi + lo of q * scale * log2 e times a power of two that brings the head's largest to 2^12: a warp per head, lane
+    // (t, j) has the four dims 32 t + 4 j .. + 3 of step j. The scores take the power back (head_scale).
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const int h = warp + kWarps * i;
         const float sc = scale * kLog2e;
-        float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
-        if (g < nh) r0 = __ldcg(reinterpret_cast<const float4 *>(q + (size_t)(h0 + g) * kHD + d0));
-        if (g + 8 < nh) r1 = __ldcg(reinterpret_cast<const float4 *>(q + (size_t)(h0 + g + 8) * kHD + d0));
-        uint4 ah, al;
-        split2(r0.x * sc, r0.y * sc, ah.x, al.x);
-        split2(r1.x * sc, r1.y * sc, ah.y, al.y);
-        split2(r0.z * sc, r0.w * sc, ah.z, al.z);
-        split2(r1.z * sc, r1.w * sc, ah.w, al.w);
-        afrag[warp * 32 + lane] = ah;
-        afrag[(8 + warp) * 32 + lane] = al;
+        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (h < nh) r = __ldcg(reinterpret_cast<const float4 *>(q + (size_t)(h0 + h) * kHD) + lane);
+        r.x *= sc; r.y *= sc; r.z *= sc; r.w *= sc;
+        const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(fabsf(r.x), fabsf(r.y)), fmaxf(fabsf(r.z), fabsf(r.w)))));
+        const uint32_t e = min(max(top >> 23, 13u), 253u);  // its exponent; the power and its inverse stay normal
+        const float up = __uint_as_float((266u - e) << 23);
+        uint32_t hi[2], lo[2];
+        split2(r.x * up, r.y * up, hi[0], lo[0]);
+        split2(r.z * up, r.w * up, hi[1], lo[1]);
+        uint32_t *f = reinterpret_cast<uint32_t *>(afrag + (lane & 7) * 32 + warp * 4 + (lane >> 3)) + i;
+        f[0] = hi[0];  // rows g, g + 8 of k 2t, 2t + 1; of k 2t + 8, 2t + 9
+        f[2] = hi[1];
+        f[8 * 32 * 4] = lo[0];
+        f[8 * 32 * 4 + 2] = lo[1];
+        if (lane == 0) head_scale[h] = __uint_as_float((e - 12u) << 23);
     }
     __syncthreads();
+    const float f0 = head_scale[g], f1 = head_scale[g + 8];
 
     float O[16][4];
 #pragma unroll
@@ -176,8 +187,8 @@ attn_int8_kernel(const float *q, const int8_t *__restrict__ kv_k, const int8_t *
                 const float ks = __shfl_sync(0xffffffffu, cur.sc, i);
                 vs[nt * 2 + e] = __shfl_sync(0xffffffffu, cur.sc, 16 + i);
                 const bool in = base + i < p_end;
-                S[nt][e] = in ? (S[nt][e] + Sl[nt][e]) * ks : -INFINITY;
-                S[nt][2 + e] = in ? (S[nt][2 + e] + Sl[nt][2 + e]) * ks : -INFINITY;
+                S[nt][e] = in ? (S[nt][e] + Sl[nt][e]) * (ks * f0) : -INFINITY;
+                S[nt][2 + e] = in ? (S[nt][2 + e] + Sl[nt][2 + e]) * (ks * f1) : -INFINITY;
                 mx0 = fmaxf(mx0, S[nt][e]);
                 mx1 = fmaxf(mx1, S[nt][2 + e]);
                 vt = fmaxf(vt, fabsf(vs[nt * 2 + e]));

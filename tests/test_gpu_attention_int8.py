@@ -40,6 +40,25 @@ def test_int8_attention_edges(K, nh, nkv, S, spread):
         assert rel.max() <= 2e-5, rel.max()
 
 
+@pytest.mark.parametrize("nh,nkv,S", [(4, 4, 33), (16, 2, 129), (40, 2, 300)])
+def test_int8_attention_query_range(K, nh, nkv, S):
+    """Heads whose q lies ten decades apart, with scores of order one by way of the K scales: q itself does not fit fp16."""
+    rng = np.random.default_rng(S)
+    k8 = rng.integers(-127, 128, (S, nkv, 128), dtype=np.int8)
+    v8 = rng.integers(-127, 128, (S, nkv, 128), dtype=np.int8)
+    vs = ((0.5 + rng.random((S, nkv))) / 127).astype(np.float32)
+    for size in (1e-9, 1.0, 1e7, 1e12):
+        ks = ((0.5 + rng.random((S, nkv))) / 127 / size).astype(np.float32)
+        q = synth.normal_f32(4200 + S, nh * 128).reshape(nh, 128) * np.float32(size)
+        q[1::3] *= np.float32(1e-5)
+        want = oracle.attention_int8kv(q.reshape(-1), k8, v8, ks, vs, nh, 128, nkv, S, nh // nkv, 128 ** -0.5).reshape(nh, 128).astype(np.float64)
+        out = torch.empty(nh * 128, device="cuda")
+        K.cuda_attention_int8kv(dev(q.reshape(-1)), dev(k8), dev(v8), dev(ks), dev(vs), out, nh, 128, nkv, S, nh // nkv, 128 ** -0.5)
+        got = host(out).reshape(nh, 128).astype(np.float64)
+        rel = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
+        assert rel.max() <= 2e-5, (size, rel.max())
+
+
 @pytest.mark.parametrize("V", [7, 256, 2049, 262144, 300001])
 def test_sample_top_p_sizes(K, V):
     logits = (synth.normal_f32(4200 + V, V) * 2.0).astype(np.float32)
