@@ -6,6 +6,7 @@ import fails with an error that says how to build it.
 from __future__ import annotations
 
 import ctypes as C
+import importlib
 import os
 import re
 
@@ -138,15 +139,20 @@ def lib() -> C.CDLL:
 
 
 class _NotBuilt:
-    """Stands in for the binding in a tree that has not been built: importing works, calling says what is missing."""
+    """Stands in for the binding in a tree that has not been built: importing works, calling says what is missing, and once the
+    tree has been built it calls the binding."""
 
     def __getattr__(self, name):
-        raise ImportError(f"{NATIVE_PATH} is missing: build it with `python -m mnemocuda_b200.build`. "
-                          "There is no CPU or PyTorch fallback for these kernels.")
+        binding = native()
+        if isinstance(binding, _NotBuilt):
+            raise ImportError(f"{NATIVE_PATH} is missing: build it with `python -m mnemocuda_b200.build`. "
+                              "There is no CPU or PyTorch fallback for these kernels.")
+        return getattr(binding, name)
 
 
 def native():
     if not (os.path.exists(NATIVE_PATH) and os.path.exists(LIB_PATH)):
         return _NotBuilt()
+    importlib.invalidate_caches()  # the file may be newer than what the import system has seen of this folder
     from . import _native
     return _native

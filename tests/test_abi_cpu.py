@@ -41,6 +41,34 @@ def test_host_mirror_rejects_cpu_tensors():
         kernels.cuda_matvec_q4k(torch.zeros(144, dtype=torch.uint8), torch.zeros(256), torch.zeros(1), 1, 256, stream=0)
 
 
+def test_kernels_imported_before_the_build_work_after_it(tmp_path):
+    """A process that imports the package, builds it and calls it."""
+    import shutil
+    import subprocess
+    import sys
+    build.build()
+    pkg = tmp_path / "mnemocuda_b200"
+    shutil.copytree(_lib._HERE, pkg, ignore=shutil.ignore_patterns("*.so", "_obj", "__pycache__", "csrc"))
+    code = f"""
+import shutil, torch
+from mnemocuda_b200 import kernels
+call = lambda: kernels.cuda_matvec_q4k(torch.zeros(144, dtype=torch.uint8), torch.zeros(256), torch.zeros(1), 1, 256, stream=0)
+try:
+    call()
+    raise SystemExit("called without a library")
+except ImportError:
+    pass
+for lib in ({_lib.LIB_PATH!r}, {_lib.NATIVE_PATH!r}):
+    shutil.copy(lib, {str(pkg)!r})
+try:
+    call()
+except ValueError:  # the binding's own check: not a device tensor
+    print("bound")
+"""
+    run = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, timeout=300)
+    assert run.stdout.strip() == "bound", run.stdout + run.stderr
+
+
 def test_synth_distributions_and_sizes():
     b = synth.q4k_blocks(1, 4000)
     assert b.shape == (4000, 144)
