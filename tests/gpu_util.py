@@ -31,3 +31,15 @@ def assert_close_matvec(got: np.ndarray, want64: np.ndarray, abs_dot: np.ndarray
         worst = np.max(np.abs(got - want64) / bound)
         assert worst <= 1.0, f"{what}: per-row error {worst:.3e} x the 1e-3*sum|w x| bound"
     return err / denom if denom > 0 else 0.0
+
+
+def layer_by_layer(model, l):
+    """A layer by the kernels of their own that sharded models, and shapes outside the one-launch kernel, run."""
+    import ctypes as C
+    from mnemocuda_b200 import _lib
+    from mnemocuda_b200 import kernels as K
+    lib, d, ws, st = _lib.lib(), C.byref(model.desc), model.workspace.data_ptr(), K._stream(None)
+    attn = torch.empty(model.cfg.q_dim, device="cuda")
+    K._check(lib.mb200_decode_layer_attn(d, l, ws, model.pos.data_ptr(), attn.data_ptr(), st), "attention")
+    K._check(lib.mb200_decode_layer_oproj(d, l, ws, attn.data_ptr(), model.hidden.data_ptr(), st), "O projection")
+    K._check(lib.mb200_decode_layer_moe(d, l, ws, 1, model.hidden.data_ptr(), st), "experts")

@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from oracle import oracle
+from tests.gpu_util import layer_by_layer
 
 pytestmark = pytest.mark.gpu
 
@@ -49,10 +50,10 @@ def oracle_token(model, Ls, kv, token, pos):
 
 
 SHAPES = {
-    # fused MoE kernel not applicable (hidden 512): router kernel + the two routed stream kernels
+    # layer by layer: the one-launch expert block does not apply (hidden 512), router kernel + the two routed stream kernels
     "tiny": dict(n_layers=3, hidden=512, n_heads=4, n_kv_heads=2, head_dim=128, n_experts=8, top_k=2, moe_inter=256,
                  vocab=1000, ctx_len=48),
-    # one-launch MoE block applies (hidden 2048, intermediate 512); 4 query heads per KV head
+    # layer by layer: the one-launch expert block applies (hidden 2048, intermediate 512); 4 query heads per KV head
     "mid": dict(n_layers=2, hidden=2048, n_heads=16, n_kv_heads=4, head_dim=128, n_experts=16, top_k=4, moe_inter=512,
                 vocab=2048, ctx_len=64),
 }
@@ -145,10 +146,8 @@ def test_greedy_tokens_match_oracle_and_graph_replay(K, pdl):
 
 
 def test_launch_overlap_does_not_change_the_tokens(K):
-    """Programmatic dependent launch lets each kernel of the chain become resident before its producer has
-    finished; the tokens must be those of plain launches. Buffers are reused from layer to layer with different
-    contents, so a kernel that read a producer's output through a non-coherent or stale cached path would show
-    here (the 30B expert shape takes the router kernel + two routed stream kernels, the 235B one the fused kernel)."""
+    """Programmatic dependent launch lets each kernel of a token become resident before its producer has
+    finished; the tokens must be those of plain launches (embedding, the one-launch layers, lm_head, sampling)."""
     from mnemocuda_b200.decode import DecodeConfig, ResidentModel
     for cfg in (DecodeConfig.qwen3_30b(ctx_len=512, n_layers=6), DecodeConfig.qwen3_235b(ctx_len=512, n_layers=3)):
         cfg.vocab = 8192
@@ -172,6 +171,51 @@ def test_launch_overlap_does_not_change_the_tokens(K):
         assert runs[True][0] == runs[False][0] == runs[True][1], (cfg.name, runs)
         del model
         torch.cuda.empty_cache()
+
+
+def test_launch_overlap_layer_by_layer(K):
+    """The same for the layers as kernels of their own, as sharded models run them. Buffers are reused from layer to layer with
+    different contents, so a kernel that read a producer's output through a non-coherent or stale cached path would show here (the
+    30B expert shape takes the router kernel + two routed stream kernels, the 235B one the one-launch expert block)."""
+    from mnemocuda_b200.decode import DecodeConfig, ResidentModel
+    for cfg in (DecodeConfig.qwen3_30b(ctx_len=512, n_layers=6), DecodeConfig.qwen3_235b(ctx_len=512, n_layers=3)):
+        cfg.vocab = 8192
+        model = ResidentModel(cfg, "cuda", seed=13, kv_prefill=cfg.ctx_len - 8)
+        runs = []
+        for mode in (False, True, True):
+            prev = K.mb200_set_pdl(mode)
+            try:
+                model.set_state(3, cfg.ctx_len - 8)
+                hidden = []
+                for _ in range(6):
+                    model.begin()
+                    for l in range(cfg.n_layers):
+                        layer_by_layer(model, l)
+                    hidden.append(model.hidden.clone())
+                    model.finish()
+                runs.append(torch.stack(hidden))
+            finally:
+                K.mb200_set_pdl(prev)
+        assert torch.equal(runs[0], runs[1]) and torch.equal(runs[0], runs[2]), cfg.name
+        del model
+        torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("shape", ["tiny", "mid"])
+def test_layer_by_layer_matches_oracle(K, shape, pdl):
+    from mnemocuda_b200.decode import DecodeConfig, ResidentModel
+    cfg = DecodeConfig(**SHAPES[shape])
+    pos = cfg.ctx_len - 5
+    model = ResidentModel(cfg, "cuda", seed=7, kv_prefill=pos, norm_weights="random")
+    kv = [[T[n].cpu().numpy().view(np.uint16).copy() for n in ("kv_k", "kv_v")] for T in model.layers]
+    model.set_state(17, pos)
+    model.begin()
+    for l in range(cfg.n_layers):
+        h = model.hidden.cpu().numpy()  # teacher forcing
+        want, _ = oracle.decode_layer(h, host_layer(model, l), cfg_dict(cfg), pos, kv[l][0], kv[l][1])
+        layer_by_layer(model, l)
+        got = model.hidden.cpu().numpy().astype(np.float64)
+        assert np.linalg.norm(got - want) <= 1e-3 * np.linalg.norm(want), l
 
 
 def test_one_layer_at_the_235b_shape(K, pdl):

@@ -6,6 +6,7 @@ import torch
 
 from oracle import oracle
 from test_gpu_decode import cfg_dict, host_layer
+from tests.gpu_util import layer_by_layer
 
 pytestmark = pytest.mark.gpu
 
@@ -50,18 +51,6 @@ def test_layers_in_one_launch_match_oracle(case):
             b = w.view(np.float16).reshape(cfg.ctx_len, -1)[pos].astype(np.float64)
             assert np.linalg.norm(a - b) <= 4e-3 * np.linalg.norm(b)
     assert K.mb200_device_error() == 0
-
-
-def layer_by_layer(model, l):
-    """A layer by the kernels of their own that sharded models, and shapes outside the one-launch kernel, run."""
-    import ctypes as C
-    from mnemocuda_b200 import _lib
-    from mnemocuda_b200 import kernels as K
-    lib, d, ws, st = _lib.lib(), C.byref(model.desc), model.workspace.data_ptr(), K._stream(None)
-    attn = torch.empty(model.cfg.q_dim, device="cuda")
-    K._check(lib.mb200_decode_layer_attn(d, l, ws, model.pos.data_ptr(), attn.data_ptr(), st), "attention")
-    K._check(lib.mb200_decode_layer_oproj(d, l, ws, attn.data_ptr(), model.hidden.data_ptr(), st), "O projection")
-    K._check(lib.mb200_decode_layer_moe(d, l, ws, 1, model.hidden.data_ptr(), st), "experts")
 
 
 def kernels_of(call):
