@@ -45,6 +45,12 @@ __device__ __forceinline__ uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c)
                               *reinterpret_cast<const __half2 *>(&c));
     return *reinterpret_cast<const uint32_t *>(&r);
 }
+__device__ __forceinline__ uint32_t hfms2(uint32_t a, uint32_t b, uint32_t c)  // a b - c
+{
+    const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b),
+                              __hneg2(*reinterpret_cast<const __half2 *>(&c)));
+    return *reinterpret_cast<const uint32_t *>(&r);
+}
 // 1.5 * 2^23 * u with u = 2^(exponent of t - DROP): adding and subtracting it rounds to a multiple of u
 template <int DROP>
 __device__ __forceinline__ float round_magic(float t)
@@ -108,9 +114,9 @@ __device__ __forceinline__ void split_q6(const uint32_t *l, const uint32_t *h, c
         const uint32_t q0 = ((LHI ? l[i] : l[i] << 4) & 0x00F000F0u) | h0, q1 = ((LHI ? l[i] >> 8 : l[i] >> 4) & 0x00F000F0u) | h1;
         const uint32_t v0 = hadd2(q0, 0xD600D600u), v1 = hadd2(q1, 0xD600D600u);  // - 96
         hi[2 * i] = hmul2(v0, f[i >> 2].s1);
-        lo[2 * i] = hfma2(v0, f[i >> 2].rs, hfma2(v0, f[i >> 2].s1, hi[2 * i] ^ 0x80008000u));
+        lo[2 * i] = hfma2(v0, f[i >> 2].rs, hfms2(v0, f[i >> 2].s1, hi[2 * i]));
         hi[2 * i + 1] = hmul2(v1, f[i >> 2].s1);
-        lo[2 * i + 1] = hfma2(v1, f[i >> 2].rs, hfma2(v1, f[i >> 2].s1, hi[2 * i + 1] ^ 0x80008000u));
+        lo[2 * i + 1] = hfma2(v1, f[i >> 2].rs, hfms2(v1, f[i >> 2].s1, hi[2 * i + 1]));
     }
 }
 
