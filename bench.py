@@ -46,7 +46,7 @@ sys.path.insert(0, ROOT)
 
 METRIC = "Q4K/Q6K matvec HBM GB/s"
 UNIT = "GB/s"
-WORKLOAD = ("configs[1]: MoE expert block, batch 1, Qwen3-235B shape -- router fp32 128x4096 + top-8 of 128 "
+WORKLOAD = ("MoE expert block, batch 1, Qwen3-235B shape -- router fp32 128x4096 + top-8 of 128 "
             "experts, Q4_K gate/up 2x(1536x4096)+SwiGLU, Q6_K down 4096x1536, weighted sum + residual")
 
 # DRAM traffic per launch (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of the kernel at

@@ -2,10 +2,9 @@
 //
 // Grid (KV head x block of 16 query heads, chunk of positions); every K / V byte is read once for all query heads of
 // the block. The cache is 128 + 4 bytes per row, so the kernel is HBM-bound once the arithmetic is on
-// mma.sync.m16n8k16: 64 heads / 4 KV heads / 32768 positions take 21.6 us against 136 with fp32 FMAs and a five-step warp
-// reduction per position and head (5.3 us at the copy rate). What is left: about 1.4 us per sixteen positions and warp
-// of instruction issue (half of it byte -> fp16), 3.4 us for launch, Q and the warps' merge, 2.7 for the cluster's and
-// 2.6 for the last CTA's.
+// mma.sync.m16n8k16: 64 heads / 4 KV heads / 32768 positions take 21 us (5.3 us at the copy rate; 136 with fp32 FMAs and a
+// five-step warp reduction per position and head). What is left is latency: a CTA has eight warps, 20 % of the issue slots are
+// used, and the merges of the warps, the cluster and the last CTA come one after the other behind barriers and a ticket.
 //   * int8 values become fp16 exactly (0x6400 | (v + 128) is 1152 + v); q and the probabilities are carried as
 //     hi + lo fp16 pairs (22 bits), accumulation is fp32, so nothing is rounded beyond fp32 arithmetic's own size. A head's q
 //     is brought into fp16's range by a power of two of its own, which its scores take back.

@@ -1,7 +1,6 @@
 // _native: the Python side of the kernel ABI without ctypes. A call of a few microseconds on the GPU cost 8-9 us on the host
 // (tensor checks in Python, torch.cuda.current_stream(), ctypes' argument conversion); here the checks, the pointers and the
-// current stream are read through the C API and the library is called directly (a 512 x 2048 matvec in a loop: 8.5 us a call
-// before, 3.8 now).
+// current stream are read through the C API and the library is called directly (a 512 x 2048 matvec in a loop: 3.8 us a call).
 //
 // Every function of the table takes its arguments by position, the stream (None = torch's current one) last. What a parameter
 // accepts is one letter: P a tensor, F a float32 tensor, H a float16 tensor, I an int32 tensor, N a tensor or None, V a

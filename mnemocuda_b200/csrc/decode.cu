@@ -8,9 +8,10 @@
 //     the position, so ONE captured CUDA graph is replayed token after token with no node
 //     patched (the reference patches three kernel nodes per layer per token,
 //     src/forward.c:636-662).
-// Per layer: RMSNorm -> Q,K (one launch) and V matvecs -> q/k norm + RoPE + KV store (one
-// launch) -> attention -> O projection + residual -> RMSNorm -> MoE block (one launch where
-// the fused kernel covers the shape) -- 8 launches against the reference's ~45.
+// All layers are one launch where the shape and the weight types allow it (persist.cu). Otherwise, and for a model sharded over
+// devices, a layer is five to eight launches against the reference's ~45: Q, K, V on RMSNorm(hidden) (one to three) -> q/k norm +
+// RoPE + KV store -> attention -> O projection + residual -> MoE block (one where the fused kernel covers the shape, else norm,
+// router, gate / up, down). Both forms give the same bits.
 // The library allocates nothing: every buffer is inside the caller's workspace.
 #include <cstdio>
 #include <cstring>

@@ -19,9 +19,9 @@
 // dequantises its own rows and loads half of the activations, which makes the MMAs the bound (496 cycles per chunk of the 512
 // they take at N = 256; 780 with the activation tile loaded by every CTA).
 //
-// Measured (start of this form -> with it): Q4_K 512 x 8192 x 4096 41.0 -> 35.0 us (clock-throttled in a loop: 21 us of cycles at
-// 1.92 GHz), 2048 x 8192 x 4096 154 -> 135, 200 x 4096 x 4096 32.8 -> 12.8, 16 x 4096 x 4096 32.9 -> 8.4 (host-bound);
-// Q6_K 512 x 8192 x 4096 73.9 -> 42.8, 130 x 7795 x 5120 80.2 -> 37.1, 33 x 2022 x 2560 35.1 -> 12.4.
+// Measured: Q4_K 512 x 8192 x 4096 35 us (clock-throttled in a loop: 21 us of cycles at 1.92 GHz), 2048 x 8192 x 4096 135,
+// 200 x 4096 x 4096 12.8, 16 x 4096 x 4096 8.4 (host-bound); Q6_K 512 x 8192 x 4096 42.8, 130 x 7795 x 5120 37.1,
+// 33 x 2022 x 2560 12.4. (Weights through shared memory, one tile size and no K split: 1.2 to 4 times as long.)
 #include <cooperative_groups.h>
 
 #include <cstdio>

@@ -11,7 +11,7 @@ def host(t: torch.Tensor) -> np.ndarray:
     return t.detach().cpu().numpy()
 
 
-# north_star tolerance: each output within 1e-3 relative L2 of the fp32 reference.
+# Each output within 1e-3 relative L2 of the fp32 reference.
 REL_L2_TOL = 1e-3
 
 
