@@ -16,8 +16,8 @@
 // ones -- every weight then dequantised more than once, on SMs that would otherwise idle -- where there are not, and for still
 // smaller shapes the CTAs of a cluster share the K range of a tile and add their accumulators through distributed shared
 // memory, in rank order (deterministic). At the large end two CTAs share a tile of 256 rows x 256 tokens (cta_group::2): each
-// dequantises its own rows and loads half of the activations, which makes the MMAs the bound (496 cycles per chunk of the 512
-// they take at N = 256; 780 with the activation tile loaded by every CTA).
+// dequantises its own rows and loads half of the activations, which makes the MMAs the bound (512 x 8192 x 4096: the tensor pipe
+// is busy 66 % of the launch's cycles, ramp and epilogue included).
 //
 // Measured: Q4_K 512 x 8192 x 4096 35 us (clock-throttled in a loop: 21 us of cycles at 1.92 GHz), 2048 x 8192 x 4096 135,
 // 200 x 4096 x 4096 12.8, 16 x 4096 x 4096 8.4 (host-bound); Q6_K 512 x 8192 x 4096 42.8, 130 x 7795 x 5120 37.1,
