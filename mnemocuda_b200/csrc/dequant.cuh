@@ -1,21 +1,18 @@
-// Weights -> pairs of fp16 (hi, lo) for the tensor cores, in packed fp16 arithmetic.
+// Weights -> small integers in fp16 for the tensor cores, in packed fp16 arithmetic.
 //
-// A Q4_K weight is w = s * n - b with n a small integer and s = d * scale, b = dmin * min of the sub-block. With a unit u, a
-// power of two chosen per sub-block so that no |w| of it exceeds 2048 u, s1 = s and b1 = b rounded to multiples of u make
-// hi = s1 * n - b1 an integer multiple of u of at most 11 bits: one HFMA2 computes it EXACTLY for two weights.
-// lo = (s - s1) * n - (b - b1), the rest, is at most 8 u and is rounded to fp16 once. A Q6_K weight is w = s * (q - 32), s of 18
-// bits: with s = s1 + s2 in fp16 halves, hi is the rounded product with s1, and lo what that rounding left (one HFMA2, exact) plus
-// the product with s2, rounded once. Converting an fp32 weight, converting back, subtracting and converting the remainder took ten
-// instructions per two weights (the producers of the grouped GEMM were issue-bound on exactly that); these are three and four.
-// Error of hi + lo, root mean square over the weights of synthetic blocks: Q4_K 7e-7, Q6_K 2e-8 of the weights' (a second half
-// rounded from fp32: 1e-8 and 0). Results against fp64, six shapes from 1024 x 256 to 4096 x 1536, are as far off as with that,
-// 0.6 to 2.3e-5: fp32 accumulation decides. (A Q4_K lo from operands 16 + n, one instruction less, has 1.3e-6, a Q6_K lo from a
-// rounded s alike; results at 1024 x 256 were then 10 % further off. The exact ones cost 3 % of the time.)
+// A Q4_K weight is d * (scale * n) - dmin * min, a Q6_K weight d * (scale * (q - 32)): apart from d and dmin, which belong to a whole
+// super-block of a row, integers. scale * n is at most 945 and exact in fp16; scale * (q - 32) has 12 bits and a sign and is hi, the
+// rounded product, plus lo, what that left (-1, 0 or 1). The grouped GEMM multiplies these and applies d and dmin to its sums, so
+// no weight is ever rounded.
 //
-// What is left is getting n out of the packed bits, on the integer pipe, which has half the FMA pipe's rate. A nibble shifted
-// to bits 6..9 of a 16-bit half and OR-ed with 0x4C00 is 16 + n: one shift and one LOP3 for two weights, no byte permute and
-// no subtraction, because the 16 goes into the addend exactly (16 s1 + b1 is a multiple of u below 2^11 u as well). The two
-// weights are then bytes 0 and 2 (1 and 3) of a word: inside every four columns the order is 0, 2, 1, 3, and the
+// A field of at most 10 bits, masked out of a 16-bit half, IS an fp16 number: a subnormal, n * 2^-24, or 2^4 times that for a field
+// that starts at bit 4. So a nibble needs one AND -- the low ones of bytes 0, 2, the high ones of bytes 0, 2, both again after one
+// shift by 8 for bytes 1, 3 -- and one HMUL2 by 16 * scale or scale gives scale * n * 2^-20: nine instructions for eight weights, where
+// fp16 halves of the scaled weight took twenty (its unit per sub-block, operands 16 + n, two FMAs, a subtraction). The two bits of a
+// Q6_K weight are shifted beside its nibble and OR-ed in (11 integer instructions for eight weights, on the pipe that has half the
+// FMA pipe's rate), 32 is subtracted, and a product and an FMA give hi and lo.
+//
+// The two weights of a register are bytes 0 and 2 (1 and 3) of a word: inside every four columns the order is 0, 2, 1, 3, and the
 // activations are laid out the same way (k_order).
 #pragma once
 #include <cuda_fp16.h>
@@ -24,11 +21,6 @@
 
 namespace mb200 {
 
-__device__ __forceinline__ uint32_t dup_half(float v)
-{
-    const __half2 h = __float2half2_rn(v);
-    return *reinterpret_cast<const uint32_t *>(&h);
-}
 __device__ __forceinline__ uint32_t hadd2(uint32_t a, uint32_t b)
 {
     const __half2 r = __hadd2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
@@ -51,72 +43,32 @@ __device__ __forceinline__ uint32_t hfms2(uint32_t a, uint32_t b, uint32_t c)  /
                               __hneg2(*reinterpret_cast<const __half2 *>(&c)));
     return *reinterpret_cast<const uint32_t *>(&r);
 }
-// 1.5 * 2^23 * u with u = 2^(exponent of t - DROP): adding and subtracting it rounds to a multiple of u
-template <int DROP>
-__device__ __forceinline__ float round_magic(float t)
-{
-    return __uint_as_float((__float_as_uint(t) & 0x7F800000u) + (static_cast<uint32_t>(23 - DROP) << 23) + 0x00400000u);
-}
-
 // Position of column k in the operand layout: columns 1 and 2 of every four change places.
 __host__ __device__ constexpr int k_order(int k) { return (k & ~3) | ((k & 1) << 1) | ((k >> 1) & 1); }
 
-// d * v for an integer v of at most 23 bits: v in the mantissa of 2^23, one FMA (c = -2^23 d) instead of a conversion
-__device__ __forceinline__ float mul_small(float d, float c, uint32_t v) { return fmaf(d, __uint_as_float(0x4B000000u | v), c); }
+constexpr float kIntScale = 1048576.0f;  // 2^20: what an operand of the integer forms has to be multiplied by
 
-// One Q4_K sub-block's scale and min as the packed factors of hi and lo for operands 16 + n.
-struct SplitQ4 {
-    uint32_t s1, c1, rs, cr;
-    __device__ __forceinline__ void set(float s, float b)
+// The two scales of a 64-column group (sc2: two bytes, the low nibbles' first) as factors of their masked nibbles.
+struct ScaleQ4 {
+    uint32_t lo, hi;
+    __device__ __forceinline__ explicit ScaleQ4(uint32_t sc2)
     {
-        // 16 |s1| + |b1| <= 2^11 u, so that it is an fp16 number too: 16 |s| + |b| stays 1/128 below, which is more than the 8.5 u
-        // that rounding may add
-        const float M = round_magic<10>(fmaf(16.0f, fabsf(s), fabsf(b)) * 1.0078125f);
-        const float s1f = (s + M) - M, b1f = (b + M) - M, rsf = s - s1f;
-        s1 = dup_half(s1f);
-        rs = dup_half(rsf);
-        c1 = dup_half(fmaf(-16.0f, s1f, -b1f));
-        cr = dup_half(b1f - b);
+        const uint32_t s = hmul2(__byte_perm(sc2, 0u, 0x4140), 0x74007400u);  // sc 2^-24 -> 2^-10
+        const uint32_t t = hmul2(s, 0x64007400u);                             // 2^4 sc (low nibbles), sc
+        lo = __byte_perm(t, 0u, 0x1010);
+        hi = __byte_perm(t, 0u, 0x3232);
     }
 };
-// 32 weights whose nibbles are the low (HIGH = false) or high nibbles of 8 words, two per register in k_order
-template <bool HIGH>
-__device__ __forceinline__ void split_q4(const uint32_t (&w)[8], const SplitQ4 &f, uint32_t (&hi)[16], uint32_t (&lo)[16])
+// 32 + 32 weights scale * n * 2^-20, of the low and of the high nibbles of 8 words, two per register in k_order
+__device__ __forceinline__ void int_q4(const uint32_t (&w)[8], const ScaleQ4 &f, uint32_t (&lo)[16], uint32_t (&hi)[16])
 {
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        const uint32_t v0 = ((HIGH ? w[i] << 2 : w[i] << 6) & 0x03C003C0u) | 0x4C004C00u;
-        const uint32_t v1 = ((HIGH ? w[i] >> 6 : w[i] >> 2) & 0x03C003C0u) | 0x4C004C00u;
-        hi[2 * i] = hfma2(v0, f.s1, f.c1);
-        lo[2 * i] = hfma2(hadd2(v0, 0xCC00CC00u), f.rs, f.cr);  // - 16
-        hi[2 * i + 1] = hfma2(v1, f.s1, f.c1);
-        lo[2 * i + 1] = hfma2(hadd2(v1, 0xCC00CC00u), f.rs, f.cr);
-    }
-}
-
-struct SplitQ6 {
-    uint32_t s1, rs;
-    __device__ __forceinline__ void set(float s)
-    {
-        s1 = dup_half(s);
-        rs = dup_half(s - __half2float(__ushort_as_half(static_cast<unsigned short>(s1))));  // exact: s has 18 bits
-    }
-};
-// 32 weights q - 32: q = the nibble of `l` at bit 4 (LHI = false: at bit 0) | two bits of `h` at bit HB, << 4, of each byte.
-// q goes to bits 4..9 of a half: 64 + q. The first 16 weights have scale f[0], the others f[1].
-template <bool LHI, int HB>
-__device__ __forceinline__ void split_q6(const uint32_t *l, const uint32_t *h, const SplitQ6 (&f)[2], uint32_t (&hi)[16],
-                                         uint32_t (&lo)[16])
-{
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const uint32_t h0 = ((h[i] << (8 - HB)) & 0x03000300u) | 0x54005400u, h1 = ((h[i] >> HB) & 0x03000300u) | 0x54005400u;
-        const uint32_t q0 = ((LHI ? l[i] : l[i] << 4) & 0x00F000F0u) | h0, q1 = ((LHI ? l[i] >> 8 : l[i] >> 4) & 0x00F000F0u) | h1;
-        const uint32_t v0 = hadd2(q0, 0xD600D600u), v1 = hadd2(q1, 0xD600D600u);  // - 96
-        hi[2 * i] = hmul2(v0, f[i >> 2].s1);
-        lo[2 * i] = hfma2(v0, f[i >> 2].rs, hfms2(v0, f[i >> 2].s1, hi[2 * i]));
-        hi[2 * i + 1] = hmul2(v1, f[i >> 2].s1);
-        lo[2 * i + 1] = hfma2(v1, f[i >> 2].rs, hfms2(v1, f[i >> 2].s1, hi[2 * i + 1]));
+        const uint32_t v = w[i] >> 8;
+        lo[2 * i] = hmul2(w[i] & 0x000F000Fu, f.lo);
+        lo[2 * i + 1] = hmul2(v & 0x000F000Fu, f.lo);
+        hi[2 * i] = hmul2(w[i] & 0x00F000F0u, f.hi);
+        hi[2 * i + 1] = hmul2(v & 0x00F000F0u, f.hi);
     }
 }
 
@@ -165,5 +117,61 @@ struct RawQ6 {  // half a block: 128 weights
         d = __half2float(__ushort_as_half(static_cast<unsigned short>(skew ? wp[52] >> 16 : wp[52])));
     }
 };
+// A quarter of a block, from a slot of shared memory in which the block begins `skew` bytes (even, below 16) from the start: 32 bytes
+// of ql and the qh bytes of the same half. Quarter u covers columns 128 (u / 2) + 32 (u % 2) + {0..31},
+// from the low nibbles, and 64 more, from the high ones.
+constexpr int kQ6Slot = 240;  // 15 x 16 bytes: an odd number, so that the rows of a warp spread over all banks
+struct QuarterQ6 {
+    uint32_t ql[8], qh[8], sc[2];  // sc: the two scales of the low nibbles (bytes 0, 1), of the high ones
+    float d;
+    // HALF: the block may begin two bytes into the word at `row` (half = 2), where the words have to be shifted
+    template <bool HALF>
+    __device__ __forceinline__ void load(const uint8_t *row, int half, int u)
+    {
+        const uint32_t *wp = reinterpret_cast<const uint32_t *>(row);
+        const uint32_t sel = half ? 0x5432u : 0x3210u;
+        auto words = [&](const uint32_t *p, uint32_t (&v)[8]) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = p[i];
+            if (HALF) {
+                const uint32_t last = p[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) v[i] = __byte_perm(v[i], i < 7 ? v[i + 1] : last, sel);
+            }
+        };
+        words(wp + 8 * u, ql);
+        words(wp + 32 + 8 * (u >> 1), qh);
+        const uint32_t a = wp[48 + 2 * (u >> 1)], b = wp[49 + 2 * (u >> 1)], c = HALF ? wp[50 + 2 * (u >> 1)] : 0u;
+        const uint32_t sel2 = sel >> (u & 1 ? 8 : 0);  // bytes 2, 3 for the odd quarters
+        sc[0] = __byte_perm(a, b, sel2);
+        sc[1] = __byte_perm(b, c, sel2);
+        d = __half2float(__ushort_as_half(static_cast<unsigned short>(half ? wp[52] >> 16 : wp[52])));
+    }
+};
+// 16 + 16 weights of a quarter, from words 4 `part` .. + 3: scale * (q - 32) * 2^-20, eight registers of hi halves and eight of lo ones, of
+// the low nibbles (`low`) and the high ones (`high`)
+__device__ __forceinline__ void int_q6(const QuarterQ6 &raw, int part, int odd, uint32_t (&low)[16], uint32_t (&high)[16])
+{
+    // int8 + 128 in the low bits of 1024; minus 1152; the low nibbles' times 2^4, which the high ones carry
+    auto scale = [&](uint32_t sc) { return hadd2(__byte_perm(sc ^ 0x8080u, 0x64646464u, part ? 0x4141 : 0x4040), 0xE480E480u); };
+    const uint32_t fl = hmul2(scale(raw.sc[0]), 0x4C004C00u), fh = scale(raw.sc[1]);
+    const int left = 4 - 2 * odd, right = 4 + 2 * odd;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t w0 = raw.ql[4 * part + i], w1 = w0 >> 8, h0 = raw.qh[4 * part + i] << left, h1 = raw.qh[4 * part + i] >> right;
+        const uint32_t a0 = hadd2((w0 & 0x000F000Fu) | (h0 & 0x00300030u), 0x80208020u);
+        const uint32_t a1 = hadd2((w1 & 0x000F000Fu) | (h1 & 0x00300030u), 0x80208020u);
+        const uint32_t b0 = hadd2((w0 & 0x00F000F0u) | (h0 & 0x03000300u), 0x82008200u);
+        const uint32_t b1 = hadd2((w1 & 0x00F000F0u) | (h1 & 0x03000300u), 0x82008200u);
+        low[2 * i] = hmul2(a0, fl);
+        low[2 * i + 1] = hmul2(a1, fl);
+        high[2 * i] = hmul2(b0, fh);
+        high[2 * i + 1] = hmul2(b1, fh);
+        low[8 + 2 * i] = hfms2(a0, fl, low[2 * i]);
+        low[8 + 2 * i + 1] = hfms2(a1, fl, low[2 * i + 1]);
+        high[8 + 2 * i] = hfms2(b0, fh, high[2 * i]);
+        high[8 + 2 * i + 1] = hfms2(b1, fh, high[2 * i + 1]);
+    }
+}
 
 }  // namespace mb200

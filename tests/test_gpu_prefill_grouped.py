@@ -103,3 +103,31 @@ def test_q6k_weights_keep_22_bits(K):
     got, want = host(y).astype(np.float64), np.array(want)
     assert np.all(np.abs(got - want) <= 1e-6 * np.abs(want))
     assert K.mb200_device_error() == 0
+
+
+@pytest.mark.parametrize("counts,H,EFF,down", [((5, 33), 1280, 512, 14), ((40, 0, 64), 256, 1024, 14), ((65, 32), 512, 2048, 14),
+                                               ((1, 96), 2304, 1280, 12), ((31, 66), 256, 256, 12)])
+def test_rows_per_group_and_sums_of_activations(K, counts, H, EFF, down):
+    """Q6_K down rows taken 8, 4, 2 and 1 at a time (EFF / 256 odd, 2, 4, 8), activation sums of one, one over four and nine super-blocks
+    a row, both accumulators of a tile full, nearly empty and unused; against fp64. Weights are exact here and activations pairs of
+    halves (2^-22), so what is left is fp32 accumulation, 1.5e-6; weights rounded to fp16 once would be off by 2.4e-4."""
+    NE, M = len(counts), sum(counts)
+    g, u, d = synth.expert_sizes(H, EFF, down)
+    experts = [synth.expert_blob(1900 + e, H, EFF, down) for e in range(NE)]
+    x = synth.normal_f16(1901, M * H).reshape(M, H)
+    ids = np.random.default_rng(1902).permutation(np.repeat(np.arange(NE), counts)).astype(np.int32).reshape(M, 1)
+    n = K.mb200_moe_prefill_workspace_bytes(M, 1, H, EFF, NE)
+    ws = torch.empty(n + 256, dtype=torch.uint8, device="cuda")
+    ws = ws[-ws.data_ptr() % 256:]
+    y = torch.full((M, H), float("nan"), device="cuda")
+    K.mb200_moe_prefill(dev(np.concatenate(experts)), g + u + d, g, u, down, NE, 1, H, EFF, dev(x), dev(ids), dev(np.ones((M, 1), np.float32)), None,
+                        y, M, 0, ws)
+    got = host(y).astype(np.float64)
+    for e in range(NE):
+        t = ids[:, 0] == e
+        w = oracle.dequant_q4k(experts[e][:g + u], 2 * EFF, H).astype(np.float64)
+        w2 = (oracle.dequant_q6k if down == 14 else oracle.dequant_q4k)(experts[e][g + u:g + u + d], H, EFF).astype(np.float64)
+        gate, up = x[t].astype(np.float64) @ w[:EFF].T, x[t].astype(np.float64) @ w[EFF:].T
+        want = (gate / (1 + np.exp(-gate)) * up) @ w2.T
+        assert np.all(np.linalg.norm(got[t] - want, axis=1) <= 2e-5 * np.linalg.norm(want, axis=1)), e
+    assert K.mb200_device_error() == 0
