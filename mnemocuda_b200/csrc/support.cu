@@ -16,6 +16,8 @@
 // fp32 accumulation), the position chunks are combined flash-decoding style: every CTA
 // leaves (max, sum, weighted V) in a workspace and the last CTA of a KV head to finish
 // (device-wide ticket) merges them.
+#include <cooperative_groups.h>
+
 #include <cstdio>
 
 #include "common.cuh"
@@ -748,219 +750,304 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ l
 // ------------------------------------------------- temperature + top-p ----
 // The reference samples in one 256-thread block (src/kernels.cu:2073-2174): p_i = exp((l_i - max) / T), every
 // thread keeps the eight largest p of its residue class i mod 256, thread 0 picks the 2048 candidates largest
-// first until their sum reaches top_p * sum(p), draws once from xoroshiro128+ and walks the nucleus. Here:
-// the maximum comes from the argmax scan above; 32 CTAs scan eight residue classes each (so that a warp's loads
-// are whole 32-byte sectors), merge the classes' candidates, and the last CTA to finish (ticket) sorts the 2048
-// candidates and walks them with the reference's arithmetic (float sums in descending order). Among equal
-// probabilities the smaller token id is preferred; the sum of all p is added in another order than the
-// reference's, so a cut that falls within rounding of top_p * sum can come out one candidate apart.
+// first until their sum reaches top_p * sum(p), draws once from xoroshiro128+ and walks the nucleus. Here one cluster
+// of eight CTAs does all of it, each for 32 residue classes, and the first sorts and walks the candidates with the reference's
+// arithmetic (float sums in descending order). Among equal probabilities the smaller token id is preferred; the sum of all p
+// is added in another order than the reference's, so a cut that falls within rounding of top_p * sum can come out one candidate
+// apart.
 //
-// All latency (600 KB of logits): what counts is the length of the dependent chain. A candidate is one 64-bit key
-// {bits of p, ~id}, ordered as the preference is (p >= 0). The sort starts from the classes' sorted runs of eight and
-// keeps them in registers: strides below 8 inside a thread, below 256 by shuffles, and only six steps through shared
-// memory. The walk's three float sums over the nucleus are prefixes of one and the same sequence, so ONE serial chain
-// of additions leaves all of them and the two searches run on all threads. 28 us per token at 151936 with the argmax scan
-// (with the sort in shared memory and its 66 barriers, three serial walks by one thread and scan loads one at a time 60-72).
-constexpr int kSampleClasses = 256, kSampleKeep = 8, kSampleCands = kSampleClasses * kSampleKeep;
-constexpr int kSampleCtas = kSampleClasses / 8;
+// All latency (600 KB of logits): what counts is the length of the dependent chain, and where eight SMs meet. A thread keeps its
+// logits in registers across the search for the maximum, which the CTAs exchange through distributed shared memory instead of a
+// launch of its own. A candidate is one 64-bit key {bits of p, ~id}, ordered as the preference is (p >= 0). The eighth largest of a
+// class's 32 thread maxima bounds its eighth largest key from below, so eight threads at most have anything to offer, a dozen keys
+// mostly, and a warp ranks them. Warps sort 32 candidates each; a key's place among a CTA's 256, then among all, is the number of
+// larger keys in the other sorted lists, by binary search. The walk's three float sums over the nucleus are prefixes of one and the
+// same sequence, so ONE serial chain of additions leaves all of them and the two searches run on all threads.
+// 13.6 us per token at 151936 (28.9 with the maximum in a launch ahead, 32 CTAs that picked by rounds of a warp-wide maximum, a ticket
+// and a last CTA that sorted). By clock stamps: logits 1 us, maximum 1.3, probabilities 1.7, picking 3.2, sorting 256 2.1, places 1.6,
+// the chain 2.2 (640 additions); three cluster barriers are 2 of it.
+constexpr int kSampleKeep = 8, kSampleCands = 256 * kSampleKeep;
+constexpr int kSampleCtas = 8, kSampleClasses = 256 / kSampleCtas;  // classes of a CTA: one per lane
 constexpr int kSampleThreads = 1024;
-constexpr int kSampleSmem = kSampleThreads * kSampleKeep * 8 + kSampleCands * 8;
-__device__ float g_sample_pair[2];
-__device__ __align__(16) unsigned long long g_sample_key[kSampleCands];
-__device__ float g_sample_sum[kSampleCtas];
-__device__ int g_sample_ticket;
+constexpr int kSampleHeld = 20;  // logits a thread keeps (163840 in all); further ones are read again
+constexpr int kSampleOffer = kSampleKeep * kSampleHeld;             // keys offered per class at most: eight threads' all
+static_assert(kSampleClasses == 32 && kSampleHeld % 4 == 0, "lanes are classes; partial sums go by fours");
 
-__device__ __forceinline__ unsigned long long cand_key(float p, int id)  // 0 = no candidate
+struct SampleShared {
+    alignas(16) unsigned long long lists[kSampleCtas][256];  // sorted candidates of every CTA, in every CTA
+    int place[kSampleCtas][256];                 // the first CTA's: where they go
+    unsigned long long sorted[kSampleCands];     // the first CTA's: all of them
+    float csum[32], cmax[kSampleCtas];           // the first CTA's / every CTA's: written by all
+    float smax[32], ssum[4][32];
+    unsigned long long bound[kSampleClasses];
+    int offered[kSampleClasses];
+    alignas(16) unsigned long long mine[256];    // this CTA's candidates, eight per class
+    int larger[4][256];
+    int len, nucleus, pick;
+    union {
+        struct {
+            alignas(16) unsigned long long tmax[kSampleClasses][34];  // [class][warp]
+            unsigned long long offer[kSampleClasses][kSampleOffer];
+            float part[128][33];                                      // partial sums: [jj][class]
+        };
+        struct {  // the walk
+            alignas(16) float p[kSampleCands];
+            alignas(16) float cum[kSampleCands];
+        };
+    };
+};
+
+__device__ __forceinline__ unsigned long long cand_key(float p, int id)  // never 0, which is no candidate
 {
-    return id < 0 ? 0ull : (static_cast<unsigned long long>(__float_as_uint(p)) << 32) | (~static_cast<unsigned>(id));
+    return (static_cast<unsigned long long>(__float_as_uint(p)) << 32) | (~static_cast<unsigned>(id));
 }
-__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k)
+// How many of a descending list's LEN keys are larger than `key`
+template <int LEN>
+__device__ __forceinline__ int larger_in(const unsigned long long *list, unsigned long long key)
 {
-    const unsigned hi = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(k >> 32));
-    const unsigned lo = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(k >> 32) == hi ? static_cast<unsigned>(k) : 0u);
-    return (static_cast<unsigned long long>(hi) << 32) | lo;
-}
-__device__ __forceinline__ void sample_barrier() { asm volatile("bar.sync 1, 256;" ::: "memory"); }  // the sort's threads
-// Descending bitonic sort of 2048 keys, eight consecutive ones per thread (256 threads). On entry every thread's
-// eight are sorted: descending in even threads, ascending in odd ones. xch: 2048 keys of shared memory.
-__device__ __forceinline__ void sort_keys(unsigned long long (&v)[kSampleKeep], unsigned long long *xch, int tid)
-{
-#pragma unroll 1
-    for (int size = 16; size <= kSampleCands; size <<= 1) {
-        const bool desc = ((tid * kSampleKeep) & size) == 0;
-#pragma unroll 1
-        for (int d = size >> 4; d > 0; d >>= 1) {  // stride 8 d: the same position of thread tid ^ d
-            const bool keep_max = ((tid & d) == 0) == desc;
-            if (d >= 32) {
+    int before = 0;
 #pragma unroll
-                for (int q = 0; q < kSampleKeep; q++) xch[q * 256 + tid] = v[q];
-                sample_barrier();
-            }
-#pragma unroll
-            for (int q = 0; q < kSampleKeep; q++) {
-                const unsigned long long o = d >= 32 ? xch[q * 256 + (tid ^ d)] : __shfl_xor_sync(0xffffffffu, v[q], d);
-                if ((o > v[q]) == keep_max) v[q] = o;
-            }
-            if (d >= 32) sample_barrier();
-        }
-#pragma unroll
-        for (int s = 4; s > 0; s >>= 1)
-#pragma unroll
-            for (int q = 0; q < kSampleKeep; q++)
-                if ((q & s) == 0 && (v[q + s] > v[q]) == desc) {
-                    const unsigned long long o = v[q];
-                    v[q] = v[q + s];
-                    v[q + s] = o;
-                }
-    }
+    for (int step = LEN / 2; step > 0; step >>= 1)
+        if (list[before + step - 1] > key) before += step;
+    return before + (list[before] > key);  // the steps add up to LEN - 1: one comparison is left
 }
 
-__global__ void __launch_bounds__(kSampleThreads) sample_top_p_kernel(const float *__restrict__ logits, int n, float temperature,
-                                                                      float top_p, unsigned long long seed, int *result)
+__global__ void __cluster_dims__(kSampleCtas, 1, 1) __launch_bounds__(kSampleThreads)
+sample_top_p_kernel(const float *__restrict__ logits, int n, float temperature, float top_p, unsigned long long seed, int *result)
 {
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) uint8_t sample_smem[];
+    SampleShared &S = *reinterpret_cast<SampleShared *>(sample_smem);
+    cg::cluster_group cluster = cg::this_cluster();
     pdl_enter();
-    extern __shared__ __align__(16) unsigned long long keys[];  // [1024 x 8] candidates of the scan, later the sort's
-    float *sp = reinterpret_cast<float *>(keys + kSampleThreads * kSampleKeep), *cum = sp + kSampleCands;
-    __shared__ float ssum[32];
-    __shared__ int is_last, s_len, s_nucleus, s_pick;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const float mx = __ldcg(&g_sample_pair[0]);
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = static_cast<int>(blockIdx.x);
     const float inv_t = 1.0f / temperature;
-    // ---- scan: thread (jj = tid / 8, k = tid % 8) takes i = 256 (jj + 128 m) + 8 blockIdx.x + k; its first eight are its
-    // list as they come (that is all of them up to 262144 logits), later ones replace the list's smallest ----
-    const int k = tid & 7, jj = tid >> 3;
-    constexpr int kStep = 256 * (kSampleThreads / 8);
-    float vp[kSampleKeep], lg[kSampleKeep];
-    int vi[kSampleKeep];
-    const int first = 256 * jj + 8 * blockIdx.x + k;
-#pragma unroll
-    for (int q = 0; q < kSampleKeep; q++) lg[q] = first + q * kStep < n ? __ldcg(logits + first + q * kStep) : 0.0f;
-    float sum = 0.0f;
-#pragma unroll
-    for (int q = 0; q < kSampleKeep; q++) {
-        const int i = first + q * kStep;
-        const bool in = i < n;
-        vp[q] = in ? expf((lg[q] - mx) * inv_t) : -1.0f;
-        vi[q] = in ? i : -1;
-        if (in) sum += vp[q];
+    if (tid < kSampleClasses) {
+        S.bound[tid] = 0;
+        S.offered[tid] = 0;
     }
-    for (int i = first + kSampleKeep * kStep; i < n; i += kStep) {
-        const float p = expf((__ldcg(logits + i) - mx) * inv_t);
-        sum += p;
-        int mi = 0;
 #pragma unroll
-        for (int q = 1; q < kSampleKeep; q++)
-            if (vp[q] < vp[mi]) mi = q;
-#pragma unroll
-        for (int q = 0; q < kSampleKeep; q++)
-            if (q == mi && p > vp[q]) {
-                vp[q] = p;
-                vi[q] = i;
-            }
+    for (int u = 0; u < 2; u++) {  // empty places
+        S.lists[0][tid + 1024 * u] = 0;
+        S.sorted[tid + 1024 * u] = 0;
     }
-    // lists to shared memory, class-major: class k holds 128 threads x 8 = 1024 candidates, 256 for each of four warps
+    // thread (warp, lane): the elements i = base + 8192 q, q < count, of class i mod 256 = 32 rank + lane
+    constexpr int kStep = 256 * 32;
+    const int base = 256 * warp + kSampleClasses * rank + lane;
+    const int count = base < n ? (n - base + kStep - 1) / kStep : 0;
+    float p[kSampleHeld];
 #pragma unroll
-    for (int q = 0; q < kSampleKeep; q++) keys[(k * kSampleKeep + q) * 128 + jj] = cand_key(vp[q], vi[q]);
-    sum = warp_sum(sum);
-    if (lane == 0) ssum[warp] = sum;
+    for (int q = 0; q < kSampleHeld; q++) p[q] = q < count ? __ldcg(logits + base + q * kStep) : -INFINITY;
+    float mx = -1e30f;
+#pragma unroll
+    for (int q = 0; q < kSampleHeld; q++) mx = fmaxf(mx, p[q]);
+    for (int q = kSampleHeld; q < count; q++) mx = fmaxf(mx, __ldcg(logits + base + q * kStep));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) S.smax[warp] = mx;
     __syncthreads();
-    // ---- warp (class c, quarter): the eight best of its 256, by rounds of a warp-wide maximum; then one warp per class
-    // the eight best of the four quarters' ----
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    if (warp == 0) {
+        mx = S.smax[lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        if (lane < kSampleCtas) *cluster.map_shared_rank(&S.cmax[rank], lane) = mx;
+    }
+    cluster.sync();
+    mx = S.cmax[0];
+#pragma unroll
+    for (int c = 1; c < kSampleCtas; c++) mx = fmaxf(mx, S.cmax[c]);
+
+    // ---- probabilities, their partial sums (of the elements with q mod 4 = j, ascending) and the largest key ----
+    auto prob = [&](float l) { return expf((l - mx) * inv_t); };
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    unsigned top = 0;  // bits of the largest probability (none is negative) and the first element that has it
+    int top_at = -1;
+    auto consider = [&](float v, int i) {
+        if (__float_as_uint(v) > top || top_at < 0) {
+            top = __float_as_uint(v);
+            top_at = i;
+        }
+    };
+#pragma unroll
+    for (int q = 0; q < kSampleHeld; q++) {
+        p[q] = prob(p[q]);  // 0 past the end
+        s[q & 3] += p[q];
+        if (q < count) consider(p[q], base + q * kStep);
+    }
+    for (int q0 = kSampleHeld; q0 < count; q0 += 4)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (q0 + j < count) {
+                const float v = prob(__ldcg(logits + base + (q0 + j) * kStep));
+                s[j] += v;
+                consider(v, base + (q0 + j) * kStep);
+            }
+    const unsigned long long best = top_at < 0 ? 0 : cand_key(__uint_as_float(top), top_at);
+    S.tmax[lane][warp] = best;
+#pragma unroll
+    for (int j = 0; j < 4; j++) S.part[warp + 32 * j][lane] = s[j];
+    __syncthreads();
+    // ---- warp w: the eighth largest of the 32 thread maxima of class w; and four of the sums' groups of 32 ----
     {
-        const int c = warp >> 2, quarter = warp & 3;
-        unsigned long long v[kSampleKeep], mine = 0;
+        const unsigned long long key = S.tmax[warp][lane];
+        int larger = 0;
 #pragma unroll
-        for (int q = 0; q < kSampleKeep; q++) v[q] = keys[(c * kSampleKeep + q) * 128 + quarter * 32 + lane];
-#pragma unroll 1
-        for (int round = 0; round < kSampleKeep; round++) {
-            unsigned long long best = v[0];
-#pragma unroll
-            for (int q = 1; q < kSampleKeep; q++) best = v[q] > best ? v[q] : best;
-            best = warp_max_key(best);
-            if (lane == round) mine = best;
-#pragma unroll
-            for (int q = 0; q < kSampleKeep; q++)
-                if (v[q] == best) v[q] = 0;  // keys are unique: the winner's owner retires it
+        for (int j = 0; j < 32; j += 2) {
+            const ulonglong2 o = *reinterpret_cast<const ulonglong2 *>(&S.tmax[warp][j]);
+            larger += (o.x > key) + (o.y > key);
         }
-        __syncthreads();
-        if (lane < kSampleKeep) keys[warp * kSampleKeep + lane] = mine;
-        __syncthreads();
-        if (warp < 8) {
-            unsigned long long key = keys[warp * 32 + lane];
-            mine = 0;
+        if (larger == kSampleKeep - 1) S.bound[warp] = key;  // keys are unique, but for empty ones: 0, as the bound is without this
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int g = (4 * warp + u) & 31, b = warp >> 3;
+            const float v = warp_sum(S.part[4 * g + (lane >> 3)][8 * b + (lane & 7)]);
+            if (lane == 0) S.ssum[b][g] = v;
+        }
+    }
+    __syncthreads();
+    // ---- every thread offers its keys from that bound on; where a thread has read more than it holds, its eight largest of them ----
+    {
+        const unsigned long long bound = S.bound[lane];
+        const unsigned bound_hi = static_cast<unsigned>(bound >> 32);
+        auto offer = [&](unsigned long long key) { S.offer[lane][atomicAdd(&S.offered[lane], 1)] = key; };
+        if (count <= kSampleHeld) {
+#pragma unroll
+            for (int q = 0; q < kSampleHeld; q++)
+                if (q < count && __float_as_uint(p[q]) >= bound_hi) {
+                    const unsigned long long key = cand_key(p[q], base + q * kStep);
+                    if (key >= bound) offer(key);
+                }
+        } else {
+            unsigned long long key = best;
 #pragma unroll 1
-            for (int round = 0; round < kSampleKeep; round++) {
-                const unsigned long long best = warp_max_key(key);
-                if (lane == round) mine = best;
-                if (key == best) key = 0;
+            for (int r = 0; r < kSampleKeep && key != 0 && key >= bound; r++) {
+                offer(key);
+                unsigned long long next = 0;
+#pragma unroll 1
+                for (int q = 0; q < count; q++) {
+                    const unsigned long long k = cand_key(prob(__ldcg(logits + base + q * kStep)), base + q * kStep);
+                    if (k < key) next = max(next, k);
+                }
+                key = next;
             }
-            if (lane < kSampleKeep) g_sample_key[(8 * blockIdx.x + warp) * kSampleKeep + lane] = mine;
-        }
-        if (warp == 8) {
-            const float s = warp_sum(ssum[lane]);
-            if (lane == 0) g_sample_sum[blockIdx.x] = s;
         }
     }
     __syncthreads();
-    if (tid == 0) {  // one fence for the CTA: the barrier orders the other threads' stores before it
-        __threadfence();
-        is_last = (atomicAdd(&g_sample_ticket, 1) == static_cast<int>(gridDim.x) - 1);
-        __threadfence();
+    // ---- warp w: the eight best keys of class w ----
+    {
+        const int m = S.offered[warp];
+        const unsigned long long *offers = S.offer[warp];
+        if (lane < kSampleKeep && lane >= m) S.mine[warp * kSampleKeep + lane] = 0;
+        for (int i = lane; i < m; i += 32) {
+            const unsigned long long key = offers[i];
+            int larger = 0;
+            for (int j = 0; j < m; j++) larger += offers[j] > key;
+            if (larger < kSampleKeep) S.mine[warp * kSampleKeep + larger] = key;
+        }
+        if (warp < 4) {
+            const float v = warp_sum(S.ssum[warp][lane]);
+            if (lane == 0) *cluster.map_shared_rank(&S.csum[4 * rank + warp], 0) = v;
+        }
     }
     __syncthreads();
-    if (!is_last || tid >= 256) return;
-    // ---- last CTA, 256 threads: sort the candidates (probability descending, token id ascending), walk them ----
-    unsigned long long v[kSampleKeep];
+    // ---- the CTA's 256 in order, to all CTAs: eight warps sort 32 each; then thread (i, quarter) looks into two of the eight lists ----
+    const int i = tid & 255, quarter = tid >> 8;
+    if (tid < 256) {
+        unsigned long long key = S.mine[tid];
 #pragma unroll
-    for (int q = 0; q < kSampleKeep; q++) v[q] = __ldcg(&g_sample_key[tid * kSampleKeep + ((tid & 1) ? kSampleKeep - 1 - q : q)]);
-    if (tid < kSampleCtas) ssum[tid] = __ldcg(&g_sample_sum[tid]);
-    sort_keys(v, keys, tid);
+        for (int size = 2; size <= 32; size <<= 1)
 #pragma unroll
-    for (int q = 0; q < kSampleKeep; q++) sp[tid * kSampleKeep + q] = __uint_as_float(static_cast<unsigned>(v[q] >> 32));
+            for (int d = size >> 1; d > 0; d >>= 1) {
+                const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, d);
+                const bool keep_max = ((lane & d) == 0) == ((lane & size) == 0);  // size 32: the whole warp descending
+                if ((o > key) == keep_max) key = o;
+            }
+        S.mine[tid] = key;
+    }
+    __syncthreads();
+    {
+        const unsigned long long key = S.mine[i];
+        const int larger = larger_in<32>(S.mine + 64 * quarter, key) + larger_in<32>(S.mine + 64 * quarter + 32, key);
+        S.larger[quarter][i] = larger;
+        __syncthreads();
+        const int place = S.larger[0][i] + S.larger[1][i] + S.larger[2][i] + S.larger[3][i];
+        if (key != 0) S.lists[rank][place] = key;
+        __syncthreads();  // remote stores of neighbouring lanes to neighbouring places: scattered ones took three times as long
+        const int c = tid >> 7, j = 2 * (tid & 127);
+        if (c != rank)
+            *reinterpret_cast<ulonglong2 *>(cluster.map_shared_rank(&S.lists[rank][j], c)) = *reinterpret_cast<const ulonglong2 *>(&S.lists[rank][j]);
+    }
+    cluster.sync();
+    // ---- the place of this CTA's keys among all: thread (i, quarter) looks into two lists ----
+    {
+        const unsigned long long key = S.lists[rank][i];
+        S.larger[quarter][i] = larger_in<256>(S.lists[2 * quarter], key) + larger_in<256>(S.lists[2 * quarter + 1], key);
+        __syncthreads();
+        if (tid < 256) *cluster.map_shared_rank(&S.place[rank][i], 0) = S.larger[0][i] + S.larger[1][i] + S.larger[2][i] + S.larger[3][i];
+    }
+    cluster.sync();
+    if (rank != 0) return;
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const unsigned long long key = S.lists[0][tid + 1024 * u];
+        if (key != 0) S.sorted[S.place[0][tid + 1024 * u]] = key;
+    }
+    __syncthreads();
+    // ---- the first CTA: the walk ----
+    const unsigned long long *keys = S.sorted;
+#pragma unroll
+    for (int u = 0; u < 2; u++) S.p[tid + 1024 * u] = __uint_as_float(static_cast<unsigned>(keys[tid + 1024 * u] >> 32));
     if (tid == 0) {
-        s_nucleus = kSampleCands;
-        s_pick = kSampleCands;
+        S.nucleus = kSampleCands;
+        S.pick = kSampleCands;
     }
-    sample_barrier();
+    __syncthreads();
     float total = 0.0f;
-    for (int c = 0; c < static_cast<int>(gridDim.x); c++) total += ssum[c];
+#pragma unroll
+    for (int c = 0; c < 32; c++) total += S.csum[c];
     const float mass = top_p * total;
     if (tid == 0) {  // the running sums, in order, as far as anyone will look
         float acc = 0.0f;
         int c = 0;
-        float4 x[4];
+        float4 x[4], y[4];
+        auto fetch = [&](float4 (&v)[4], int at) {
 #pragma unroll
-        for (int u = 0; u < 4; u++) x[u] = *reinterpret_cast<const float4 *>(sp + 4 * u);
-        while (c < kSampleCands && acc < mass && x[0].x > 0.0f) {
-            float4 y[4];  // the next sixteen are fetched while these are added
-            const int nx = min(c + 16, kSampleCands - 16);
-#pragma unroll
-            for (int u = 0; u < 4; u++) y[u] = *reinterpret_cast<const float4 *>(sp + nx + 4 * u);
+            for (int u = 0; u < 4; u++) v[u] = *reinterpret_cast<const float4 *>(S.p + min(at, kSampleCands - 16) + 4 * u);
+        };
+        auto add = [&](float4 (&v)[4]) {
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                x[u].x = acc += x[u].x;
-                x[u].y = acc += x[u].y;
-                x[u].z = acc += x[u].z;
-                x[u].w = acc += x[u].w;
-                *reinterpret_cast<float4 *>(cum + c + 4 * u) = x[u];
-                x[u] = y[u];
+                v[u].x = acc += v[u].x;
+                v[u].y = acc += v[u].y;
+                v[u].z = acc += v[u].z;
+                v[u].w = acc += v[u].w;
+                *reinterpret_cast<float4 *>(S.cum + c + 4 * u) = v[u];
             }
             c += 16;
+        };
+        fetch(x, 0);
+        while (c < kSampleCands && acc < mass && x[0].x > 0.0f) {  // each sixteen are fetched while the ones before are added
+            fetch(y, c + 16);
+            add(x);
+            fetch(x, c + 16);
+            add(y);
         }
-        s_len = c;
+        S.len = c;
     }
-    sample_barrier();
-    const int len = s_len;
+    __syncthreads();
+    const int len = S.len;
     // the nucleus ends after the first candidate that reaches the mass, or before the first of probability zero
-    for (int c = tid; c < len; c += 256) {
-        if (sp[c] <= 0.0f)
-            atomicMin(&s_nucleus, c);
-        else if (cum[c] >= mass)
-            atomicMin(&s_nucleus, c + 1);
+    for (int c = tid; c < len; c += kSampleThreads) {
+        if (S.p[c] <= 0.0f)
+            atomicMin(&S.nucleus, c);
+        else if (S.cum[c] >= mass)
+            atomicMin(&S.nucleus, c + 1);
     }
-    if (tid == 0) atomicMin(&s_nucleus, len);  // everything before len was walked, nothing after it counts
-    sample_barrier();
-    const int nucleus = s_nucleus;
+    if (tid == 0) atomicMin(&S.nucleus, len);  // everything before len was walked, nothing after it counts
+    __syncthreads();
+    const int nucleus = S.nucleus;
     unsigned long long rs0 = seed, rs1 = seed ^ 0xDEADBEEFCAFEBABEULL;
 #pragma unroll
     for (int w = 0; w < 4; w++) {  // three warm-up rounds and the draw
@@ -969,18 +1056,17 @@ __global__ void __launch_bounds__(kSampleThreads) sample_top_p_kernel(const floa
         rs1 = t ^ rs1 ^ (t >> 17) ^ (rs1 >> 26);
     }
     const float r = static_cast<float>((rs0 + rs1) >> 11) * (1.0f / 9007199254740992.0f);
-    const float target = nucleus > 0 ? r * cum[nucleus - 1] : 0.0f;
-    for (int c = tid; c < nucleus; c += 256)
-        if (cum[c] >= target) {
-            atomicMin(&s_pick, c);
+    const float target = nucleus > 0 ? r * S.cum[nucleus - 1] : 0.0f;
+    for (int c = tid; c < nucleus; c += kSampleThreads)
+        if (S.cum[c] >= target) {
+            atomicMin(&S.pick, c);
             break;
         }
-    sample_barrier();
-    const int pick = s_pick < nucleus ? s_pick : 0;
-#pragma unroll
-    for (int q = 0; q < kSampleKeep; q++)
-        if (tid * kSampleKeep + q == pick) *result = v[q] ? static_cast<int>(~static_cast<unsigned>(v[q])) : -1;
-    if (tid == 0) g_sample_ticket = 0;
+    __syncthreads();
+    if (tid == 0) {
+        const unsigned long long key = keys[S.pick < nucleus ? S.pick : 0];
+        *result = key ? static_cast<int>(~static_cast<unsigned>(key)) : -1;
+    }
 }
 
 // The best of the shards' (value, index) pairs, by the same order as above; writes the token and advances the position.
@@ -1050,27 +1136,13 @@ bool attn_attr()
 
 }  // namespace
 
-// Device address of the sampling kernels' (max, index) pair, looked up once per device (cuda_kernels_init does it,
-// so that no symbol is resolved inside a stream capture).
-float *sample_pair_addr()
-{
-    static float *addr[kMaxDevices] = {};
-    const int dev = current_device();
-    if (!addr[dev]) {
-        void *p = nullptr;
-        if (cudaGetSymbolAddress(&p, g_sample_pair) != cudaSuccess) return nullptr;
-        addr[dev] = static_cast<float *>(p);
-    }
-    return addr[dev];
-}
-
 // The sampling kernel's shared-memory opt-in, once per device.
 void sample_attr()
 {
     static bool done[kMaxDevices] = {false};
     const int dev = current_device();
     if (done[dev]) return;
-    cudaFuncSetAttribute(sample_top_p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSampleSmem);
+    cudaFuncSetAttribute(sample_top_p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SampleShared));
     done[dev] = true;
 }
 
@@ -1079,7 +1151,6 @@ void support_init()
     attn_attr();
     sample_attr();
     (void)static_attn();
-    (void)sample_pair_addr();
 }
 
 int attn_chunks_for(int n_kv_heads, int gqa, int max_slots)
@@ -1302,14 +1373,8 @@ void cuda_sample_token(const float *logits, int vocab_size, float temperature, f
 {
     if (vocab_size <= 0) return;
     if (temperature > 0.0f) {
-        float *pair = sample_pair_addr();
-        if (!pair) {
-            set_status(MB200_ERR_LAUNCH, "cuda_sample_token");
-            return;
-        }
-        launch_argmax_pair(logits, vocab_size, 0, pair, stream);  // the maximum, for exp(l - max)
         sample_attr();
-        launch_k(sample_top_p_kernel, dim3(kSampleCtas), dim3(kSampleThreads), kSampleSmem, stream, logits, vocab_size, temperature, top_p,
+        launch_k(sample_top_p_kernel, dim3(kSampleCtas), dim3(kSampleThreads), sizeof(SampleShared), stream, logits, vocab_size, temperature, top_p,
                  rng_state, d_result);
         MB200_CHECK_LAUNCH("cuda_sample_token");
         return;

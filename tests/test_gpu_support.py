@@ -213,6 +213,30 @@ def test_sample_token_top_p_degenerate_and_repeat(K):
     assert int(res.item()) == 777
 
 
+@pytest.mark.parametrize("V", [1, 255, 257, 8193, 163840, 163841, 270001])
+def test_sample_token_top_p_sizes(K, V):
+    """One element, a class short of one, the step between rows of the cluster's warps, and what the threads hold and what they read again
+    (163840 | 163841). Against the oracle (by the rule above: one state may disagree); and equal logits, where the candidates are the
+    smallest ids in order, their sums whole numbers and the token follows from the draw alone."""
+    logits = (synth.normal_f32(98, V) * 3).astype(np.float32)
+    d_l, res = dev(logits), torch.full((1,), -1, dtype=torch.int32, device="cuda")
+    seeds = [int(s) for s in np.random.default_rng(99).integers(1, 2 ** 63, 12)]
+    miss = 0
+    for seed in seeds:
+        K.cuda_sample_token(d_l, V, 0.9, 0.9, seed, res)
+        miss += int(res.item()) != oracle.sample_top_p(logits, 0.9, 0.9, seed)
+    assert miss <= 1, miss
+    flat, n, mask = torch.zeros(V, device="cuda"), min(V, 2048), 2 ** 64 - 1
+    for seed in seeds:
+        s0, s1 = seed, seed ^ 0xDEADBEEFCAFEBABE
+        for _ in range(4):
+            t = (s0 ^ (s0 << 23)) & mask
+            s0, s1 = s1, t ^ s1 ^ (t >> 17) ^ (s1 >> 26)
+        r = np.float32(((s0 + s1) & mask) >> 11) * np.float32(1 / 9007199254740992)
+        K.cuda_sample_token(flat, V, 1.0, 1.0, seed, res)
+        assert int(res.item()) == max(0, int(np.ceil(r * np.float32(n))) - 1)
+
+
 def test_kernel_pointer_exports(K):
     from mnemocuda_b200 import _lib
     lib = _lib.lib()
