@@ -2,9 +2,10 @@
 //
 // Grid (KV head x block of 16 query heads, chunk of positions); every K / V byte is read once for all query heads of
 // the block. The cache is 128 + 4 bytes per row, so the kernel is HBM-bound once the arithmetic is on
-// mma.sync.m16n8k16: 64 heads / 4 KV heads / 32768 positions take 21 us (5.3 us at the copy rate; 136 with fp32 FMAs and a
-// five-step warp reduction per position and head). What is left is latency: a CTA has eight warps, 20 % of the issue slots are
-// used, and the merges of the warps, the cluster and the last CTA come one after the other behind barriers and a ticket.
+// mma.sync.m16n8k16: 64 heads / 4 KV heads / 32768 positions take 16.1 us (5.3 us at the copy rate; 21.4 with eight warps that held a
+// tile ahead in registers, 136 with fp32 FMAs and a five-step warp reduction per position and head), 32 / 8 heads 18.8 (29.4). By clock
+// stamps, 64 / 4 at 32768: 3 us until q is in fragments (while the first tiles stream), 7.2 the tiles (the MMAs alone are 5), then one
+// after the other the merges of the warps (1.1), the cluster (0.5) and, behind a ticket (1.3), the last CTA (1.2).
 //   * int8 values become fp16 exactly (0x6400 | (v + 128) is 1152 + v); q and the probabilities are carried as
 //     hi + lo fp16 pairs (22 bits), accumulation is fp32, so nothing is rounded beyond fp32 arithmetic's own size. A head's q
 //     is brought into fp16's range by a power of two of its own, which its scores take back.
@@ -26,11 +27,15 @@ int pdl_enabled();
 namespace {
 namespace cg = cooperative_groups;
 
-constexpr int kWarps = 8, kThreads = kWarps * 32;
+constexpr int kWarps = 12, kThreads = kWarps * 32;
+constexpr int kStages = 2;    // tiles on their way per warp
 constexpr int kHD = 128;      // head dimension
 constexpr int kTile = 16;     // positions per warp step
+constexpr int kRow = 144;     // bytes between K / V rows of a stage: 16-byte reads of eight lanes hit all banks
+constexpr int kStageBytes = 2 * kTile * kRow + 2 * kTile * 4;  // K rows, V rows, K scales, V scales
 constexpr int kPitch = 132;   // floats between heads in the shared-memory results (4 x 33: conflict-free stores)
 constexpr int kMaxGroups = 64;   // (KV head, query-head block) pairs per launch
+constexpr int kBatch = 20;     // partials a merging thread has on their way
 constexpr int kMaxSlots = 256;   // (group, cluster) pairs per launch
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -44,7 +49,7 @@ __device__ Work g_work;
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1)
 {
-    asm volatile(
+    asm(
         "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
@@ -79,19 +84,22 @@ __device__ __forceinline__ uint32_t to_half2(uint32_t w, uint32_t sel)
 // Fragments (g = lane / 4, t = lane % 4):
 //  Q K^T:  the 16 k of step j are dims 32 t + 4 j + {0,1 | 2,3}: a thread's share of a K row is 32 contiguous bytes
 //  P V:    k = position in the tile, column g of output tile u = dim 16 g + u: 16 contiguous bytes of four V rows
-template <int CL>
+// PACK: at most eight query heads per KV head; rows g are their q and probabilities' hi halves, rows g + 8 the lo ones, one MMA for both.
+template <int CL, bool PACK>
 __global__ void __launch_bounds__(kThreads, 1)
 attn_int8_kernel(const float *q, const int8_t *__restrict__ kv_k, const int8_t *__restrict__ kv_v, const float *k_scales,
                  const float *v_scales, float *out, int n_kv_heads, int gqa, int seq_len, float scale, int tiles_per_chunk)
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    constexpr int HB = PACK ? 8 : 16, kMergers = HB * 16;  // heads of a CTA; threads that merge, sixteen per head
     extern __shared__ __align__(16) uint8_t smem_raw[];
     uint4 *afrag = reinterpret_cast<uint4 *>(smem_raw);           // [2 hi/lo][8 steps][32 lanes]
-    float *osm = reinterpret_cast<float *>(smem_raw + 8192);      // [8 warps][16 heads][kPitch]; later the CTA's partial in [0]
-    float *msm = osm + kWarps * 16 * kPitch;                      // [8][16] running maxima (log2 domain)
-    float *lsm = msm + kWarps * 16;                               // [8][16] sums
+    float *msm = reinterpret_cast<float *>(smem_raw + 8192);      // [warps][16] running maxima (log2 domain)
+    float *lsm = msm + kWarps * 16;                               // [warps][16] sums
     float *cml = lsm + kWarps * 16;                               // [2][16] the CTA's max and sum
+    uint8_t *rings = reinterpret_cast<uint8_t *>(cml + 32);       // [warps][stages]
+    float *osm = reinterpret_cast<float *>(rings);                // then [warps][16 heads][kPitch]; last the CTA's partial in [0]
     __shared__ int is_last;
     __shared__ float head_scale[16];
 
@@ -102,39 +110,47 @@ attn_int8_kernel(const float *q, const int8_t *__restrict__ kv_k, const int8_t *
     const int p_begin = min(seq_len, static_cast<int>(blockIdx.y) * tiles_per_chunk * kTile);
     const int p_end = min(seq_len, p_begin + tiles_per_chunk * kTile);
     const size_t row_stride = (size_t)n_kv_heads * kHD;
-    const int8_t *kbase = kv_k + (size_t)kvh * kHD + 32 * t;
-    const int8_t *vbase = kv_v + (size_t)kvh * kHD + 16 * g;
-    const float *sbase = (lane < 16 ? k_scales : v_scales) + kvh;  // lanes 0-15: K scales of the tile, 16-31: V scales
-
-    struct Tile {
-        uint4 k[2][2], v[4];
-        float sc;
-    };
     const int n_tiles = (p_end - p_begin + kTile - 1) / kTile, last = max(p_end - 1, 0);
-    auto load = [&](int tile, Tile &x) {
-        const int base = p_begin + tile * kTile;
+    // A warp's tiles go through a ring of its own, requested two tiles ahead (one tile ahead in registers, every step waited for
+    // memory): lane copies 16 bytes of rows lane / 8 + 4 i, and the K scale (lanes 0-15) or V scale of row lane % 16.
+    uint8_t *ring = rings + warp * kStages * kStageBytes;
+    const int8_t *ksrc = kv_k + (size_t)kvh * kHD + 16 * (lane & 7), *vsrc = kv_v + (size_t)kvh * kHD + 16 * (lane & 7);
+    const float *ssrc = (lane < 16 ? k_scales : v_scales) + kvh;
+    const uint32_t dst = smem_u32(ring) + (lane >> 3) * kRow + 16 * (lane & 7), sdst = smem_u32(ring) + 2 * kTile * kRow + 4 * lane;
+    auto request = [&](int tile, int stage) {
+        if (tile < n_tiles) {
+            const int base = p_begin + tile * kTile;
 #pragma unroll
-        for (int nt = 0; nt < 2; nt++) {
-            const uint4 *src = reinterpret_cast<const uint4 *>(kbase + (size_t)min(base + nt * 8 + g, last) * row_stride);
-            x.k[nt][0] = __ldcg(src);
-            x.k[nt][1] = __ldcg(src + 1);
+            for (int i = 0; i < 4; i++) {
+                const size_t row = (size_t)min(base + (lane >> 3) + 4 * i, last) * row_stride;
+                const uint32_t to = dst + stage * kStageBytes + 4 * i * kRow;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(ksrc + row) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + kTile * kRow), "l"(vsrc + row) : "memory");
+            }
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sdst + stage * kStageBytes),
+                         "l"(ssrc + (size_t)min(base + (lane & 15), last) * n_kv_heads)
+                         : "memory");
         }
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-            x.v[r] = __ldcg(reinterpret_cast<const uint4 *>(vbase + (size_t)min(base + 2 * t + (r & 1) + (r >> 1) * 8, last) * row_stride));
-        x.sc = __ldcg(sbase + (size_t)min(base + (lane & 15), last) * n_kv_heads);
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    Tile cur, nxt;
-    if (warp < n_tiles) load(warp, cur);
+    // q comes before the tiles: behind 150 KB of them it took 4 us.
+    constexpr int kQ = (HB + kWarps - 1) / kWarps;
+    float4 qr[kQ];
+#pragma unroll
+    for (int i = 0; i < kQ; i++) {
+        const int h = warp + kWarps * i;
+        qr[i] = h < nh ? __ldcg(reinterpret_cast<const float4 *>(q + (size_t)(h0 + h) * kHD) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    request(warp, 0);
 
     // Q fragments, hi + lo of q * scale * log2 e times a power of two that brings the head's largest to 2^12: a warp per head, lane
     // (t, j) has the four dims 32 t + 4 j .. + 3 of step j. The scores take the power back (head_scale).
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
+    for (int i = 0; i < kQ; i++) {
         const int h = warp + kWarps * i;
+        if (h >= HB) break;
         const float sc = scale * kLog2e;
-        float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (h < nh) r = __ldcg(reinterpret_cast<const float4 *>(q + (size_t)(h0 + h) * kHD) + lane);
+        float4 r = qr[i];
         r.x *= sc; r.y *= sc; r.z *= sc; r.w *= sc;
         const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fmaxf(fabsf(r.x), fabsf(r.y)), fmaxf(fabsf(r.z), fabsf(r.w)))));
         const uint32_t e = min(max(top >> 23, 13u), 253u);  // its exponent; the power and its inverse stay normal
@@ -142,23 +158,39 @@ attn_int8_kernel(const float *q, const int8_t *__restrict__ kv_k, const int8_t *
         uint32_t hi[2], lo[2];
         split2(r.x * up, r.y * up, hi[0], lo[0]);
         split2(r.z * up, r.w * up, hi[1], lo[1]);
-        uint32_t *f = reinterpret_cast<uint32_t *>(afrag + (lane & 7) * 32 + warp * 4 + (lane >> 3)) + i;
-        f[0] = hi[0];  // rows g, g + 8 of k 2t, 2t + 1; of k 2t + 8, 2t + 9
+        // rows g, g + 8 of k 2t, 2t + 1; of k 2t + 8, 2t + 9
+        uint32_t *f = reinterpret_cast<uint32_t *>(afrag + (lane & 7) * 32 + (h & 7) * 4 + (lane >> 3)) + (h >> 3);
+        uint32_t *fl = f + (PACK ? 1 : 8 * 32 * 4);
+        f[0] = hi[0];
         f[2] = hi[1];
-        f[8 * 32 * 4] = lo[0];
-        f[8 * 32 * 4 + 2] = lo[1];
+        fl[0] = lo[0];
+        fl[2] = lo[1];
         if (lane == 0) head_scale[h] = __uint_as_float((e - 12u) << 23);
     }
     __syncthreads();
-    const float f0 = head_scale[g], f1 = head_scale[g + 8];
+    // Requests beyond what the memory system takes hold up the warp that makes them: only the first tile's come before the fragments.
+#pragma unroll
+    for (int i = 1; i < kStages; i++) request(warp + kWarps * i, i);
+    const float f0 = head_scale[g], f1 = PACK ? 0.0f : head_scale[g + 8];
 
     float O[16][4];
 #pragma unroll
     for (int u = 0; u < 16; u++) O[u][0] = O[u][1] = O[u][2] = O[u][3] = 0.0f;
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f, vmax = 0.0f;
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f, vmax = 0.0f, vinv = 0.0f;
+    int stage = 0;
     for (int tile = warp; tile < n_tiles; tile += kWarps) {
         const int base = p_begin + tile * kTile;
-        if (tile + kWarps < n_tiles) load(tile + kWarps, nxt);
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
+        __syncwarp();
+        const uint8_t *st = ring + stage * kStageBytes;
+        const uint8_t *krow = st + g * kRow + 32 * t, *vrow = st + kTile * kRow + 2 * t * kRow + 16 * g;
+        const float2 *scales = reinterpret_cast<const float2 *>(st + 2 * kTile * kRow) + t;  // of positions 2t, 2t + 1; four apart: 8 further
+        const float2 ks[2] = {scales[0], scales[4]}, vs2[2] = {scales[8], scales[12]};
+        uint4 kq[2][2];
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) kq[nt][i] = *reinterpret_cast<const uint4 *>(krow + nt * 8 * kRow + 16 * i);
         // four independent accumulator chains (two position halves x hi / lo), added at the end
         float S[2][4], Sl[2][4];
 #pragma unroll
@@ -167,87 +199,108 @@ attn_int8_kernel(const float *q, const int8_t *__restrict__ kv_k, const int8_t *
             for (int e = 0; e < 4; e++) S[nt][e] = Sl[nt][e] = 0.0f;
 #pragma unroll
         for (int j = 0; j < 8; j++) {
-            const uint4 ah = afrag[j * 32 + lane], al = afrag[(8 + j) * 32 + lane];
+            const uint4 ah = afrag[j * 32 + lane], al = PACK ? ah : afrag[(8 + j) * 32 + lane];
 #pragma unroll
             for (int nt = 0; nt < 2; nt++) {
-                const uint4 kk = cur.k[nt][j >> 2];
+                const uint4 kk = kq[nt][j >> 2];
                 const uint32_t u = ((j & 3) == 0 ? kk.x : (j & 3) == 1 ? kk.y : (j & 3) == 2 ? kk.z : kk.w) ^ 0x80808080u;
                 const uint32_t b0 = to_half2(u, 0x4140), b1 = to_half2(u, 0x4342);
-                mma16816(S[nt], ah.x, ah.y, ah.z, ah.w, b0, b1);
-                mma16816(Sl[nt], al.x, al.y, al.z, al.w, b0, b1);
+                mma16816(PACK && (j & 1) ? Sl[nt] : S[nt], ah.x, ah.y, ah.z, ah.w, b0, b1);
+                if (!PACK) mma16816(Sl[nt], al.x, al.y, al.z, al.w, b0, b1);
             }
         }
-        float mx0 = -INFINITY, mx1 = -INFINITY, vs[4], vt = 0.0f;
+        float mx0 = -INFINITY, mx1 = -INFINITY, vt = 0.0f;
+        const float vs[4] = {vs2[0].x, vs2[0].y, vs2[1].x, vs2[1].y};
 #pragma unroll
         for (int nt = 0; nt < 2; nt++) {
 #pragma unroll
             for (int e = 0; e < 2; e++) {
-                const int i = nt * 8 + 2 * t + e;
-                const float ks = __shfl_sync(0xffffffffu, cur.sc, i);
-                vs[nt * 2 + e] = __shfl_sync(0xffffffffu, cur.sc, 16 + i);
-                const bool in = base + i < p_end;
-                S[nt][e] = in ? (S[nt][e] + Sl[nt][e]) * (ks * f0) : -INFINITY;
-                S[nt][2 + e] = in ? (S[nt][2 + e] + Sl[nt][2 + e]) * (ks * f1) : -INFINITY;
+                const float k = e ? ks[nt].y : ks[nt].x;
+                const bool in = base + nt * 8 + 2 * t + e < p_end;
+                if (PACK) {
+                    S[nt][e] = in ? ((S[nt][e] + Sl[nt][e]) + (S[nt][2 + e] + Sl[nt][2 + e])) * (k * f0) : -INFINITY;
+                } else {
+                    S[nt][e] = in ? (S[nt][e] + Sl[nt][e]) * (k * f0) : -INFINITY;
+                    S[nt][2 + e] = in ? (S[nt][2 + e] + Sl[nt][2 + e]) * (k * f1) : -INFINITY;
+                    mx1 = fmaxf(mx1, S[nt][2 + e]);
+                }
                 mx0 = fmaxf(mx0, S[nt][e]);
-                mx1 = fmaxf(mx1, S[nt][2 + e]);
                 vt = fmaxf(vt, fabsf(vs[nt * 2 + e]));
             }
         }
 #pragma unroll
         for (int o = 1; o <= 2; o <<= 1) {
             mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, o));
-            mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
+            if (!PACK) mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, o));
             vt = fmaxf(vt, __shfl_xor_sync(0xffffffffu, vt, o));
         }
-        const float n0 = fmaxf(m0, mx0), n1 = fmaxf(m1, mx1), nv = fmaxf(vmax, vt);
-        const float r0 = exp2_fast(m0 - n0), r1 = exp2_fast(m1 - n1);  // 2^-inf = 0 on the first tile
-        const float vinv = nv > 0.0f ? 1.0f / nv : 0.0f;
-        const float rv = vmax * vinv;
-        m0 = n0;
-        m1 = n1;
-        vmax = nv;
-        l0 *= r0;
-        l1 *= r1;
-        const float o0 = r0 * rv, o1 = r1 * rv;
-        if (__any_sync(0xffffffffu, o0 != 1.0f || o1 != 1.0f)) {  // the running maxima settle after a few tiles
+        // What the accumulators are relative to, a head's maximum and the largest V scale, follows only when it falls behind by more
+        // than 2^8 and 2^4: products stay below 2^12, inside fp16's range, and most tiles need not touch the 64 accumulators.
+        const bool up0 = mx0 > m0 + 8.0f, up1 = !PACK && mx1 > m1 + 8.0f, upv = vt > 16.0f * vmax;
+        if (__any_sync(0xffffffffu, up0 || up1 || upv)) {
+            const float n0 = up0 ? mx0 : m0, n1 = up1 ? mx1 : m1, nv = upv ? vt : vmax;
+            const float r0 = n0 == m0 ? 1.0f : exp2_fast(m0 - n0), r1 = n1 == m1 ? 1.0f : exp2_fast(m1 - n1);  // 2^-inf = 0 on the first tile
+            vinv = nv > 0.0f ? 1.0f / nv : 0.0f;
+            const float rv = nv == vmax ? 1.0f : vmax * vinv, o0 = r0 * rv, o1 = r1 * rv;
+            m0 = n0;
+            m1 = n1;
+            vmax = nv;
+            l0 *= r0;
+            l1 *= r1;
 #pragma unroll
             for (int u = 0; u < 16; u++) {
                 O[u][0] *= o0;
                 O[u][1] *= o0;
-                O[u][2] *= o1;
-                O[u][3] *= o1;
+                O[u][2] *= PACK ? o0 : o1;
+                O[u][3] *= PACK ? o0 : o1;
             }
         }
-        uint32_t ph[4], pl[4];
+        uint32_t ph[4], pl[4];  // rows g: positions 8 nt + 2t, 2t + 1 in 2 nt; rows g + 8 in 2 nt + 1
 #pragma unroll
         for (int nt = 0; nt < 2; nt++) {
-            const float p0 = exp2_fast(S[nt][0] - n0), p1 = exp2_fast(S[nt][1] - n0);
-            const float p2 = exp2_fast(S[nt][2] - n1), p3 = exp2_fast(S[nt][3] - n1);
-            l0 += p0 + p1;
-            l1 += p2 + p3;
             const float va = vs[nt * 2] * vinv, vb = vs[nt * 2 + 1] * vinv;
-            split2(p0 * va, p1 * vb, ph[nt * 2], pl[nt * 2]);          // row g,     positions 8 nt + 2t, 2t + 1
-            split2(p2 * va, p3 * vb, ph[nt * 2 + 1], pl[nt * 2 + 1]);  // row g + 8
+            const float p0 = exp2_fast(S[nt][0] - m0), p1 = exp2_fast(S[nt][1] - m0);
+            l0 += p0 + p1;
+            if (PACK) {
+                split2(p0 * va, p1 * vb, ph[nt * 2], ph[nt * 2 + 1]);
+            } else {
+                const float p2 = exp2_fast(S[nt][2] - m1), p3 = exp2_fast(S[nt][3] - m1);
+                l1 += p2 + p3;
+                split2(p0 * va, p1 * vb, ph[nt * 2], pl[nt * 2]);
+                split2(p2 * va, p3 * vb, ph[nt * 2 + 1], pl[nt * 2 + 1]);
+            }
         }
-        const uint32_t vw[4][4] = {{cur.v[0].x, cur.v[0].y, cur.v[0].z, cur.v[0].w}, {cur.v[1].x, cur.v[1].y, cur.v[1].z, cur.v[1].w},
-                                   {cur.v[2].x, cur.v[2].y, cur.v[2].z, cur.v[2].w}, {cur.v[3].x, cur.v[3].y, cur.v[3].z, cur.v[3].w}};
+        uint32_t vw[4][4];  // rows 2t, 2t + 1, 2t + 8, 2t + 9
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(vrow + ((r & 1) + (r >> 1) * 8) * kRow);
+            vw[r][0] = v.x; vw[r][1] = v.y; vw[r][2] = v.z; vw[r][3] = v.w;
+        }
 #pragma unroll
         for (int w = 0; w < 4; w++) {
             // bytes of rows 2t and 2t + 1 (and of 2t + 8, 2t + 9) interleaved: one dim's pair side by side
-            const uint32_t a = vw[0][w] ^ 0x80808080u, b = vw[1][w] ^ 0x80808080u;
+            const uint32_t a = vw[0][w] ^ 0x80808080u, a2 = vw[1][w] ^ 0x80808080u;
             const uint32_t c = vw[2][w] ^ 0x80808080u, d = vw[3][w] ^ 0x80808080u;
-            const uint32_t ab[2] = {__byte_perm(a, b, 0x5140), __byte_perm(a, b, 0x7362)};
+            const uint32_t ab[2] = {__byte_perm(a, a2, 0x5140), __byte_perm(a, a2, 0x7362)};
             const uint32_t cd[2] = {__byte_perm(c, d, 0x5140), __byte_perm(c, d, 0x7362)};
+            uint32_t b[8];
 #pragma unroll
             for (int i = 0; i < 4; i++) {
                 const uint32_t sel = (i & 1) ? 0x4342 : 0x4140;
-                const uint32_t b0 = to_half2(ab[i >> 1], sel), b1 = to_half2(cd[i >> 1], sel);
-                mma16816(O[4 * w + i], ph[0], ph[1], ph[2], ph[3], b0, b1);
-                mma16816(O[4 * w + i], pl[0], pl[1], pl[2], pl[3], b0, b1);
+                b[2 * i] = to_half2(ab[i >> 1], sel);
+                b[2 * i + 1] = to_half2(cd[i >> 1], sel);
+                mma16816(O[4 * w + i], ph[0], ph[1], ph[2], ph[3], b[2 * i], b[2 * i + 1]);
             }
+            if (!PACK)
+#pragma unroll
+                for (int i = 0; i < 4; i++) mma16816(O[4 * w + i], pl[0], pl[1], pl[2], pl[3], b[2 * i], b[2 * i + 1]);
         }
-        cur = nxt;
+        __syncwarp();  // all lanes have read the stage
+        request(tile + kWarps * kStages, stage);
+        if (++stage == kStages) stage = 0;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // the rings become the warps' results
     // ---- the warps' shares to shared memory ----
 #pragma unroll
     for (int o = 1; o <= 2; o <<= 1) {
@@ -256,122 +309,158 @@ attn_int8_kernel(const float *q, const int8_t *__restrict__ kv_k, const int8_t *
     }
     if (t == 0) {
         msm[warp * 16 + g] = m0;
-        msm[warp * 16 + g + 8] = m1;
         lsm[warp * 16 + g] = l0;
-        lsm[warp * 16 + g + 8] = l1;
+        if (!PACK) {
+            msm[warp * 16 + g + 8] = m1;
+            lsm[warp * 16 + g + 8] = l1;
+        }
     }
     {
         float *ow = osm + warp * 16 * kPitch;  // dim d of a head sits at (d / 32) * 33 + d % 32
 #pragma unroll
         for (int u = 0; u < 16; u++) {
-            ow[g * kPitch + 33 * t + u] = O[u][0] * vmax;        // dim 16 (2t) + u
-            ow[g * kPitch + 33 * t + 16 + u] = O[u][1] * vmax;   // dim 16 (2t + 1) + u
-            ow[(g + 8) * kPitch + 33 * t + u] = O[u][2] * vmax;
-            ow[(g + 8) * kPitch + 33 * t + 16 + u] = O[u][3] * vmax;
+            const float a = PACK ? O[u][0] + O[u][2] : O[u][0], b = PACK ? O[u][1] + O[u][3] : O[u][1];
+            ow[g * kPitch + 33 * t + u] = a * vmax;        // dim 16 (2t) + u
+            ow[g * kPitch + 33 * t + 16 + u] = b * vmax;   // dim 16 (2t + 1) + u
+            if (!PACK) {
+                ow[(g + 8) * kPitch + 33 * t + u] = O[u][2] * vmax;
+                ow[(g + 8) * kPitch + 33 * t + 16 + u] = O[u][3] * vmax;
+            }
         }
     }
     __syncthreads();
     // ---- the CTA's partial: thread -> head tid / 16, dims 8 (tid % 16) .. + 7 ----
-    const int head = tid >> 4, d0 = (tid & 15) * 8;
+    const int head = (tid & (kMergers - 1)) >> 4, d0 = (tid & 15) * 8;
+    const bool merges = tid < kMergers;
     const int at = (d0 >> 5) * 33 + (d0 & 31);
     float M = -INFINITY, L = 0.0f, acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (merges) {
 #pragma unroll
-    for (int w = 0; w < kWarps; w++) M = fmaxf(M, msm[w * 16 + head]);
+        for (int w = 0; w < kWarps; w++) M = fmaxf(M, msm[w * 16 + head]);
 #pragma unroll
-    for (int w = 0; w < kWarps; w++) {
-        const float mw = msm[w * 16 + head];
-        const float f = (mw == -INFINITY) ? 0.0f : exp2_fast(mw - M);
-        L = fmaf(lsm[w * 16 + head], f, L);
-        const float *ow = osm + (w * 16 + head) * kPitch + at;
+        for (int w = 0; w < kWarps; w++) {
+            const float mw = msm[w * 16 + head];
+            const float f = (mw == -INFINITY) ? 0.0f : exp2_fast(mw - M);
+            L = fmaf(lsm[w * 16 + head], f, L);
+            const float *ow = osm + (w * 16 + head) * kPitch + at;
 #pragma unroll
-        for (int i = 0; i < 8; i++) acc[i] = fmaf(ow[i], f, acc[i]);
+            for (int i = 0; i < 8; i++) acc[i] = fmaf(ow[i], f, acc[i]);
+        }
     }
-    auto store_out = [&](float *dst, const float (&v)[8], float f) {
-        *reinterpret_cast<float4 *>(dst) = make_float4(v[0] * f, v[1] * f, v[2] * f, v[3] * f);
-        *reinterpret_cast<float4 *>(dst + 4) = make_float4(v[4] * f, v[5] * f, v[6] * f, v[7] * f);
+    auto store_out = [&](float *to, const float (&v)[8], float f) {
+        *reinterpret_cast<float4 *>(to) = make_float4(v[0] * f, v[1] * f, v[2] * f, v[3] * f);
+        *reinterpret_cast<float4 *>(to + 4) = make_float4(v[4] * f, v[5] * f, v[6] * f, v[7] * f);
     };
-    int rank = 0;
-    bool mine = true;  // this thread's (head, dims) belong to this CTA's share of the merge
-    if (CL > 1) {
-        // post the partial (each thread overwrites only what it alone has read), then merge heads [8 rank, 8 rank + 8)
-        cg::cluster_group cl = cg::this_cluster();
-        rank = static_cast<int>(cl.block_rank());
-#pragma unroll
-        for (int i = 0; i < 8; i++) osm[head * kPitch + at + i] = acc[i];
+    if (CL == 1) {
+        if (merges && head < nh) store_out(out + (size_t)(h0 + head) * kHD + d0, acc, L > 0.0f ? 1.0f / L : 0.0f);
+        return;
+    }
+    // post the partial, then merge half of the heads each
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = static_cast<int>(cl.block_rank());
+    float *post = reinterpret_cast<float *>(afrag);  // [heads][128], 8 KB: the fragments have been read
+    if (merges) {
+        store_out(post + head * kHD + d0, acc, 1.0f);
         if ((tid & 15) == 0) {
             cml[head] = M;
             cml[16 + head] = L;
         }
-        cl.sync();
-        mine = (head >> 3) == rank;
-        if (mine) {
-            const float *po = cl.map_shared_rank(osm, rank ^ 1), *pm = cl.map_shared_rank(cml, rank ^ 1);
-            const float Mo = pm[head], Lo = pm[16 + head], Mt = fmaxf(M, Mo);
-            const float fa = (M == -INFINITY) ? 0.0f : exp2_fast(M - Mt), fb = (Mo == -INFINITY) ? 0.0f : exp2_fast(Mo - Mt);
-            L = L * fa + Lo * fb;
-            M = Mt;
-#pragma unroll
-            for (int i = 0; i < 8; i++) acc[i] = acc[i] * fa + po[head * kPitch + at + i] * fb;
-        }
-        cl.sync();  // the partner has read this CTA's shared memory
     }
+    cl.sync();
     const int S = gridDim.y / CL;  // partials per head block
+    const size_t slot = (size_t)blockIdx.x * S + blockIdx.y / CL;
+    if (merges && head / (HB / 2) == rank) {
+        const float *po = cl.map_shared_rank(post, rank ^ 1) + head * kHD + d0, *pm = cl.map_shared_rank(cml, rank ^ 1);
+        const float4 pa = *reinterpret_cast<const float4 *>(po), pb = *reinterpret_cast<const float4 *>(po + 4);
+        const float other[8] = {pa.x, pa.y, pa.z, pa.w, pb.x, pb.y, pb.z, pb.w};
+        const float Mo = pm[head], Lo = pm[16 + head], Mt = fmaxf(M, Mo);
+        const float fa = (M == -INFINITY) ? 0.0f : exp2_fast(M - Mt), fb = (Mo == -INFINITY) ? 0.0f : exp2_fast(Mo - Mt);
+        L = L * fa + Lo * fb;
+        M = Mt;
+#pragma unroll
+        for (int i = 0; i < 8; i++) acc[i] = acc[i] * fa + other[i] * fb;
+        if (S == 1) {
+            if (head < nh) store_out(out + (size_t)(h0 + head) * kHD + d0, acc, L > 0.0f ? 1.0f / L : 0.0f);
+        } else {
+            store_out(g_work.part + (slot * 16 + head) * kHD + d0, acc, 1.0f);
+            if ((tid & 15) == 0) {
+                g_work.ml[(slot * 2 + 0) * 16 + head] = M;
+                g_work.ml[(slot * 2 + 1) * 16 + head] = L;
+            }
+        }
+    }
+    // This CTA has read the partner's shared memory; it leaves when the partner has read its own.
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    auto partner_done = [] { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); };
     if (S == 1) {
-        if (mine && head < nh) store_out(out + (size_t)(h0 + head) * kHD + d0, acc, L > 0.0f ? 1.0f / L : 0.0f);
+        partner_done();
         return;
     }
-    const size_t slot = (size_t)blockIdx.x * S + blockIdx.y / CL;
-    if (mine) {
-        store_out(g_work.part + (slot * 16 + head) * kHD + d0, acc, 1.0f);
-        if ((tid & 15) == 0) {
-            g_work.ml[(slot * 2 + 0) * 16 + head] = M;
-            g_work.ml[(slot * 2 + 1) * 16 + head] = L;
-        }
+    __syncthreads();
+    if (tid == 0) {  // one release for the CTA: the barrier orders the other threads' stores before it
+        int ticket;
+        asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(ticket) : "l"(&g_work.tickets[blockIdx.x * 2 + rank]) : "memory");
+        is_last = ticket == S - 1;
     }
     __syncthreads();
-    if (tid == 0) {  // one fence for the CTA: the barrier orders the other threads' stores before it
-        __threadfence();
-        is_last = atomicAdd(&g_work.tickets[blockIdx.x * 2 + rank], 1) == S - 1;
-        __threadfence();
+    if (!is_last) {
+        partner_done();
+        return;
     }
-    __syncthreads();
-    if (!is_last) return;
-    if (mine && head < nh) {
+    // ---- the last CTA of this half of the heads: a warp per head, four dims per thread, kBatch partials' loads in flight ----
+    const int mh = HB / 2 * rank + warp;
+    if (warp < HB / 2 && mh < nh) {
         const size_t s0 = (size_t)blockIdx.x * S;
-        float Mt = -INFINITY;
-        for (int c0 = 0; c0 < S; c0 += 8) {  // eight partials' loads in flight at a time
-            float mv[8];
+        const float *part = g_work.part + (s0 * 16 + mh) * kHD + 4 * lane;
+        auto fetch = [&](float4 (&v)[kBatch], int c0) {
 #pragma unroll
-            for (int u = 0; u < 8; u++) mv[u] = __ldcg(g_work.ml + ((s0 + min(c0 + u, S - 1)) * 2) * 16 + head);
+            for (int u = 0; u < kBatch; u++)
+                v[u] = c0 + u < S ? __ldcg(reinterpret_cast<const float4 *>(part + (size_t)(c0 + u) * 16 * kHD)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        float4 v[kBatch];
+        fetch(v, 0);
+        float *weight = osm + warp * kPitch;  // of the partials (the results have been merged)
+        float m[kMaxSlots / 64], l[kMaxSlots / 64], Mt = -INFINITY, Lt = 0.0f;
 #pragma unroll
-            for (int u = 0; u < 8; u++) Mt = fmaxf(Mt, mv[u]);
+        for (int i = 0; i < kMaxSlots / 64; i++) {
+            const int c = lane + 32 * i;
+            m[i] = c < S ? __ldcg(g_work.ml + ((s0 + c) * 2) * 16 + mh) : -INFINITY;
+            l[i] = c < S ? __ldcg(g_work.ml + ((s0 + c) * 2 + 1) * 16 + mh) : 0.0f;
+            Mt = fmaxf(Mt, m[i]);
         }
-        float Lt = 0.0f, o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int c0 = 0; c0 < S; c0 += 8) {
-            float mv[8], lv[8];
-            float4 a[8], b[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const size_t sl = s0 + min(c0 + u, S - 1);
-                mv[u] = __ldcg(g_work.ml + (sl * 2) * 16 + head);
-                lv[u] = __ldcg(g_work.ml + (sl * 2 + 1) * 16 + head);
-                a[u] = __ldcg(reinterpret_cast<const float4 *>(g_work.part + (sl * 16 + head) * kHD + d0));
-                b[u] = __ldcg(reinterpret_cast<const float4 *>(g_work.part + (sl * 16 + head) * kHD + d0 + 4));
-            }
+        for (int o = 16; o > 0; o >>= 1) Mt = fmaxf(Mt, __shfl_xor_sync(0xffffffffu, Mt, o));
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const float f = (c0 + u >= S || mv[u] == -INFINITY) ? 0.0f : exp2_fast(mv[u] - Mt);
-                Lt = fmaf(lv[u], f, Lt);
-                o[0] = fmaf(a[u].x, f, o[0]); o[1] = fmaf(a[u].y, f, o[1]); o[2] = fmaf(a[u].z, f, o[2]); o[3] = fmaf(a[u].w, f, o[3]);
-                o[4] = fmaf(b[u].x, f, o[4]); o[5] = fmaf(b[u].y, f, o[5]); o[6] = fmaf(b[u].z, f, o[6]); o[7] = fmaf(b[u].w, f, o[7]);
+        for (int i = 0; i < kMaxSlots / 64; i++) {
+            const int c = lane + 32 * i;
+            const float f = m[i] == -INFINITY ? 0.0f : exp2_fast(m[i] - Mt);
+            if (c < S) weight[c] = f;
+            Lt = fmaf(l[i], f, Lt);
+        }
+        Lt = warp_sum(Lt);
+        __syncwarp();
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int c0 = 0; c0 < S; c0 += kBatch) {
+            if (c0) fetch(v, c0);
+#pragma unroll
+            for (int u = 0; u < kBatch; u++) {
+                const float f = c0 + u < S ? weight[c0 + u] : 0.0f;
+                o.x = fmaf(v[u].x, f, o.x);
+                o.y = fmaf(v[u].y, f, o.y);
+                o.z = fmaf(v[u].z, f, o.z);
+                o.w = fmaf(v[u].w, f, o.w);
             }
         }
-        store_out(out + (size_t)(h0 + head) * kHD + d0, o, Lt > 0.0f ? 1.0f / Lt : 0.0f);
+        const float inv = Lt > 0.0f ? 1.0f / Lt : 0.0f;
+        *reinterpret_cast<float4 *>(out + (size_t)(h0 + mh) * kHD + 4 * lane) = make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv);
     }
     if (tid == 0) g_work.tickets[blockIdx.x * 2 + rank] = 0;  // ready for the next launch
+    partner_done();
 }
 
-constexpr int kSmem = 8192 + (kWarps * 16 * kPitch + 2 * kWarps * 16 + 32) * 4;
+constexpr int kRingBytes = kWarps * kStages * kStageBytes, kResultBytes = kWarps * 16 * kPitch * 4;
+constexpr int kSmem = 8192 + (2 * kWarps * 16 + 32) * 4 + (kRingBytes > kResultBytes ? kRingBytes : kResultBytes);
+static_assert(kSmem <= 227 * 1024, "shared memory budget");
 
 template <int CL>
 void launch(const float *q, const int8_t *k, const int8_t *v, const float *ks, const float *vs, float *out, int groups, int chunks,
@@ -392,7 +481,7 @@ void launch(const float *q, const int8_t *k, const int8_t *v, const float *ks, c
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    cudaLaunchKernelEx(&cfg, attn_int8_kernel<CL>, q, k, v, ks, vs, out, n_kv_heads, gqa, seq_len, scale, (tiles + chunks - 1) / chunks);
+    cudaLaunchKernelEx(&cfg, gqa <= 8 ? attn_int8_kernel<CL, true> : attn_int8_kernel<CL, false>, q, k, v, ks, vs, out, n_kv_heads, gqa, seq_len, scale, (tiles + chunks - 1) / chunks);
 }
 
 }  // namespace
@@ -402,8 +491,8 @@ void attn_int8_init()
     static bool done[kMaxDevices] = {false};
     const int dev = current_device();
     if (done[dev]) return;
-    cudaFuncSetAttribute(attn_int8_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    cudaFuncSetAttribute(attn_int8_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    for (auto kernel : {attn_int8_kernel<1, false>, attn_int8_kernel<1, true>, attn_int8_kernel<2, false>, attn_int8_kernel<2, true>})
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     done[dev] = true;
 }
 

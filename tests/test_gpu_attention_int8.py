@@ -59,6 +59,32 @@ def test_int8_attention_query_range(K, nh, nkv, S):
         assert rel.max() <= 2e-5, (size, rel.max())
 
 
+@pytest.mark.parametrize("gqa", [1, 8, 9, 16])
+@pytest.mark.parametrize("ramp", [1, -1, 0])
+def test_int8_attention_moving_maxima(K, gqa, ramp):
+    """Scores and V scales that rise, fall or jump along the positions, past the 2^8 and 2^4 by which the kernel lets its maxima fall behind
+    (heads in one and in two halves of an MMA's rows). Scores reach 28, so their fp32 rounding moves a probability by 2e-6. A probability
+    times its V scale is a pair of halves relative to the largest V scale a warp has met, good to 2^-25 of that: where the order is
+    random every warp meets the largest, and what counts has the smallest, so it spans 2^6 there (2^-19 of the result). The bound is
+    that of the other cases."""
+    S, nkv = 12 * 16 * 5 + 3, 2
+    rng = np.random.default_rng(gqa + 7)
+    at = np.arange(S) / S if ramp > 0 else 1 - np.arange(S) / S if ramp < 0 else rng.random(S)
+    k8 = np.broadcast_to(rng.integers(-127, 128, (1, nkv, 128), dtype=np.int8), (S, nkv, 128)).copy()
+    v8 = rng.integers(-127, 128, (S, nkv, 128), dtype=np.int8)
+    q = synth.normal_f32(4300, nkv * gqa * 128).reshape(nkv, gqa, 128)
+    dots = np.einsum("hgd,hd->hg", q.astype(np.float64), k8[0].astype(np.float64))
+    q = (q / (dots[..., None] * 128 ** -0.5)).astype(np.float32)  # every head's score is the K scale
+    ks = np.repeat((28 * at).astype(np.float32)[:, None], nkv, 1)
+    vs = np.repeat((2.0 ** ((-20 if ramp else -6) * at)).astype(np.float32)[:, None] / 127, nkv, 1)
+    want = oracle.attention_int8kv(q.reshape(-1), k8, v8, ks, vs, nkv * gqa, 128, nkv, S, gqa, 128 ** -0.5).reshape(-1, 128).astype(np.float64)
+    out = torch.full((nkv * gqa * 128,), float("nan"), device="cuda")
+    K.cuda_attention_int8kv(dev(q.reshape(-1)), dev(k8), dev(v8), dev(ks), dev(vs), out, nkv * gqa, 128, nkv, S, gqa, 128 ** -0.5)
+    got = host(out).reshape(-1, 128).astype(np.float64)
+    rel = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert rel.max() <= 2e-5, rel.max()
+
+
 @pytest.mark.parametrize("V", [7, 256, 2049, 262144, 300001])
 def test_sample_top_p_sizes(K, V):
     logits = (synth.normal_f32(4200 + V, V) * 2.0).astype(np.float32)
