@@ -227,6 +227,8 @@ constexpr int kAttnThreads = 256;
 constexpr int kAttnWarps = kAttnThreads / 32;
 constexpr int kHD = 128;      // head dimension of the tensor-core kernel
 constexpr int kTile = 16;     // positions per warp step
+constexpr int kAttnStages = 2;             // tiles on their way per warp
+constexpr int kStageBytes = 2 * kTile * 256;  // K rows, V rows
 constexpr int kOPitch = 132;  // floats between heads in the warps' shared-memory results (4 x 33, see the stores)
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -269,9 +271,10 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
     P.seq_len = seq_len_arg; P.pos_ptr = pos_ptr; P.scale = scale; P.part = part; P.ml = ml; P.tickets = tickets;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     uint4 *afrag = reinterpret_cast<uint4 *>(smem_raw);                         // [2 hi/lo][8 steps][32 lanes]
-    float *osm = reinterpret_cast<float *>(smem_raw + 8192);                    // [8 warps][16 heads][kOPitch]
-    float *msm = osm + kAttnWarps * 16 * kOPitch;                               // [8][16]
+    float *msm = reinterpret_cast<float *>(smem_raw + 8192);                    // [8][16]
     float *lsm = msm + kAttnWarps * 16;                                         // [8][16]
+    uint8_t *rings = reinterpret_cast<uint8_t *>(lsm + kAttnWarps * 16);        // [8 warps][stages]
+    float *osm = reinterpret_cast<float *>(rings);                              // then [8 warps][16 heads][kOPitch]
     __shared__ int is_last;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
@@ -283,46 +286,47 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
     const int seq_len = P.pos_ptr ? __ldcg(P.pos_ptr) + 1 : P.seq_len;
     const int tiles_total = (seq_len + kTile - 1) / kTile;
     const int tpc = (tiles_total + S - 1) / S;
+    const int SN = tpc > 0 ? (tiles_total + tpc - 1) / tpc : 1;  // chunks that hold positions; the others have nothing to add to a merge
+    if (chunk >= SN) return;
     const int p_begin = min(seq_len, chunk * tpc * kTile), p_end = min(seq_len, (chunk + 1) * tpc * kTile);
     const size_t row_stride = (size_t)P.n_kv_heads * kHD;  // halves between consecutive positions
-    const __half *kbase = P.kv_k + (size_t)kvh * kHD;
-    const __half *vbase = P.kv_v + (size_t)kvh * kHD;
 
+    // q comes before the tiles: behind all of them it would take as long as they do.
+    const int j = warp, d0q = (j >> 1) * 32 + t * 8 + (j & 1) * 4;
+    float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0;
+    if (g < nh) q0 = __ldcg(reinterpret_cast<const float4 *>(P.q + (size_t)(h0 + g) * kHD + d0q));
+    if (g + 8 < nh) q1 = __ldcg(reinterpret_cast<const float4 *>(P.q + (size_t)(h0 + g + 8) * kHD + d0q));
+
+    // A warp's tiles go through a ring of its own in shared memory, requested two ahead (with one ahead in registers a step waited for
+    // memory: 32 / 8 heads at 32768 positions 34.2 instead of 29.4 us, 64 / 8 at 8192 15.6 instead of 13.0; three ahead leave the merge too
+    // little L1 for the partial results, 3 us more). Lane copies 16-byte unit lane % 16 of rows lane / 16 + 2 i; a row's units are permuted (xor) so that the 16-byte reads
+    // below meet in no bank: K by the row's parity, V by which pair of rows it belongs to.
     const int n_tiles = (p_end - p_begin + kTile - 1) / kTile;
     const int last_row = max(p_end - 1, 0);
-    struct Tile {
-        uint4 k[2][4], v[4][2];
-    };
-    auto load = [&](int tile, Tile &x) {
-        const int base = p_begin + tile * kTile;
+    uint8_t *ring = rings + warp * kAttnStages * kStageBytes;
+    const int unit = lane & 15, row0 = lane >> 4;
+    const __half *ksrc = P.kv_k + (size_t)kvh * kHD + 8 * unit, *vsrc = P.kv_v + (size_t)kvh * kHD + 8 * unit;
+    const uint32_t dst = smem_u32(ring) + 256 * row0;
+    auto v_swizzle = [](int pair) { return (pair & 1) | ((pair & 2) << 1); };
+    auto request = [&](int tile, int stage) {
+        if (tile < n_tiles) {
 #pragma unroll
-        for (int nt = 0; nt < 2; nt++) {
-            const uint4 *src = reinterpret_cast<const uint4 *>(kbase + (size_t)min(base + nt * 8 + g, last_row) * row_stride) + t;
-#pragma unroll
-            for (int i = 0; i < 4; i++) x.k[nt][i] = __ldcg(src + i * 4);  // bytes 64 i + 16 t of the row
+            for (int i = 0; i < 8; i++) {
+                const size_t row = (size_t)min(p_begin + tile * kTile + row0 + 2 * i, last_row) * row_stride;
+                const uint32_t to = dst + stage * kStageBytes + 512 * i;
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16 * (unit ^ (4 * row0))), "l"(ksrc + row) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 256 * kTile + 16 * (unit ^ v_swizzle(i & 3))), "l"(vsrc + row)
+                             : "memory");
+            }
         }
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int p = min(base + 2 * t + (r & 1) + (r >> 1) * 8, last_row);
-            const uint4 *src = reinterpret_cast<const uint4 *>(vbase + (size_t)p * row_stride) + g * 2;
-            x.v[r][0] = __ldcg(src);
-            x.v[r][1] = __ldcg(src + 1);
-        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    // K and V of a warp's next tile are in flight during the whole of the current one (with V requested at the start of its
-    // own tile a step waited for it: 39 instead of 34 us for 32 / 8 heads at 32768 positions, 14.5 instead of 13.9 for
-    // 64 / 4 at 8192).
-    Tile cur, nxt;
-    if (warp < n_tiles) load(warp, cur);
+    request(warp, 0);
 
     // ---- Q fragments (hi + lo halves of q * scale * log2 e) into shared memory: warp j builds step j ----
     {
-        const int j = warp, d0 = (j >> 1) * 32 + t * 8 + (j & 1) * 4;
         const float sc = P.scale * kLog2e;
-        float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
-        if (g < nh) r0 = __ldcg(reinterpret_cast<const float4 *>(P.q + (size_t)(h0 + g) * kHD + d0));
-        if (g + 8 < nh) r1 = __ldcg(reinterpret_cast<const float4 *>(P.q + (size_t)(h0 + g + 8) * kHD + d0));
-        const float v[8] = {r0.x * sc, r0.y * sc, r0.z * sc, r0.w * sc, r1.x * sc, r1.y * sc, r1.z * sc, r1.w * sc};
+        const float v[8] = {q0.x * sc, q0.y * sc, q0.z * sc, q0.w * sc, q1.x * sc, q1.y * sc, q1.z * sc, q1.w * sc};
         float hi[8], lo[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
@@ -335,16 +339,31 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
             make_uint4(pack_half2(lo[0], lo[1]), pack_half2(lo[4], lo[5]), pack_half2(lo[2], lo[3]), pack_half2(lo[6], lo[7]));
     }
     __syncthreads();
+    // Requests beyond what the memory system takes hold up the warp that makes them: only the first tile's come before the fragments.
+#pragma unroll
+    for (int i = 1; i < kAttnStages; i++) request(warp + kAttnWarps * i, i);
 
     float O[16][4];
 #pragma unroll
     for (int u = 0; u < 16; u++) O[u][0] = O[u][1] = O[u][2] = O[u][3] = 0.0f;
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;  // rows g and g + 8 (l: this thread's share)
 
+    int stage = 0;
     for (int tile = warp; tile < n_tiles; tile += kAttnWarps) {
         const int base = p_begin + tile * kTile;
-        const bool more = tile + kAttnWarps < n_tiles;
-        if (more) load(tile + kAttnWarps, nxt);
+        asm volatile("cp.async.wait_group %0;" ::"n"(kAttnStages - 1) : "memory");
+        __syncwarp();
+        const uint8_t *st = ring + stage * kStageBytes;
+        uint4 kq[2][4], vq[4][2];  // bytes 64 i + 16 t of K rows g, g + 8; 32 g of V rows 2t, 2t + 1, 2t + 8, 2t + 9
+#pragma unroll
+        for (int nt = 0; nt < 2; nt++)
+#pragma unroll
+            for (int i = 0; i < 4; i++) kq[nt][i] = *reinterpret_cast<const uint4 *>(st + (nt * 8 + g) * 256 + 16 * ((4 * i + t) ^ (4 * (g & 1))));
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                vq[r][h] = *reinterpret_cast<const uint4 *>(st + (kTile + 2 * t + (r & 1) + (r >> 1) * 8) * 256 + 16 * ((2 * g + h) ^ v_swizzle(t)));
 
         float Sx[2][4];  // two independent chains (the position halves)
 #pragma unroll
@@ -356,7 +375,7 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
             const uint4 ah = afrag[j * 32 + lane], al = afrag[(8 + j) * 32 + lane];
 #pragma unroll
             for (int nt = 0; nt < 2; nt++) {
-                const uint4 kk = cur.k[nt][j >> 1];
+                const uint4 kk = kq[nt][j >> 1];
                 const uint32_t b0 = (j & 1) ? kk.z : kk.x, b1 = (j & 1) ? kk.w : kk.y;
                 mma16816(Sx[nt], ah.x, ah.y, ah.z, ah.w, b0, b1);
                 mma16816(Sx[nt], al.x, al.y, al.z, al.w, b0, b1);
@@ -413,7 +432,7 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
         for (int r = 0; r < 4; r++)
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                vw[r][4 * h] = cur.v[r][h].x; vw[r][4 * h + 1] = cur.v[r][h].y; vw[r][4 * h + 2] = cur.v[r][h].z; vw[r][4 * h + 3] = cur.v[r][h].w;
+                vw[r][4 * h] = vq[r][h].x; vw[r][4 * h + 1] = vq[r][h].y; vw[r][4 * h + 2] = vq[r][h].z; vw[r][4 * h + 3] = vq[r][h].w;
             }
 #pragma unroll
         for (int u = 0; u < 16; u++) {
@@ -422,8 +441,12 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
             const uint32_t b1 = __byte_perm(vw[2][u >> 1], vw[3][u >> 1], sel);
             mma16816(O[u], pa[0], pa[1], pa[2], pa[3], b0, b1);
         }
-        cur = nxt;
+        __syncwarp();  // all lanes have read the stage
+        request(tile + kAttnWarps * kAttnStages, stage);
+        if (++stage == kAttnStages) stage = 0;
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();  // the rings become the warps' results
     // ---- this warp's share to shared memory ----
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
     l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
@@ -474,11 +497,10 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
         }
     }
     __syncthreads();
-    if (tid == 0) {  // one fence for the CTA: the barrier orders the other threads' stores before it
-        __threadfence();
-        const int ticket = atomicAdd(P.tickets + blockIdx.x, 1);
-        is_last = (ticket == S - 1);
-        __threadfence();
+    if (tid == 0) {  // one release for the CTA: the barrier orders the other threads' stores before it
+        int ticket;
+        asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(ticket) : "l"(P.tickets + blockIdx.x) : "memory");
+        is_last = (ticket == SN - 1);
     }
     __syncthreads();
     if (!is_last) return;
@@ -491,15 +513,15 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
     if (head < nh) {
         const int sub = tid & 15;
         const unsigned half_mask = 0xFFFFu << (tid & 16);
-        float *fsm = osm;  // [S][16] weights of the chunks (the warps' results above have been consumed)
-        constexpr int kMaxPer = 10;  // chunks per lane: S <= 160
+        float *fsm = osm;  // [SN][16] weights of the chunks (the warps' results above have been consumed)
+        constexpr int kMaxPer = 10;  // chunks per lane: SN <= 160
         float mc[kMaxPer], lc[kMaxPer];
 #pragma unroll
         for (int i = 0; i < kMaxPer; i++) {
             const int c = sub + 16 * i;
-            const size_t sl = (size_t)blockIdx.x * S + (c < S ? c : 0);
-            mc[i] = c < S ? __ldcg(P.ml + (sl * 2 + 0) * 16 + head) : -INFINITY;
-            lc[i] = c < S ? __ldcg(P.ml + (sl * 2 + 1) * 16 + head) : 0.0f;
+            const size_t sl = (size_t)blockIdx.x * S + (c < SN ? c : 0);
+            mc[i] = c < SN ? __ldcg(P.ml + (sl * 2 + 0) * 16 + head) : -INFINITY;
+            lc[i] = c < SN ? __ldcg(P.ml + (sl * 2 + 1) * 16 + head) : 0.0f;
         }
         float Mt = -INFINITY;
 #pragma unroll
@@ -512,18 +534,18 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
             const int c = sub + 16 * i;
             const float f = (mc[i] == -INFINITY) ? 0.0f : exp2f(mc[i] - Mt);
             Lt = fmaf(lc[i], f, Lt);
-            if (c < S) fsm[c * 16 + head] = f;
+            if (c < SN) fsm[c * 16 + head] = f;
         }
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) Lt += __shfl_xor_sync(half_mask, Lt, o);
         __syncwarp(half_mask);
         float o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int c0 = 0; c0 < S; c0 += 16) {
+        for (int c0 = 0; c0 < SN; c0 += 16) {
             float4 a[16], b[16];
 #pragma unroll
             for (int u = 0; u < 16; u++) {
                 a[u] = b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (c0 + u < S) {
+                if (c0 + u < SN) {
                     const size_t sl = (size_t)blockIdx.x * S + c0 + u;
                     a[u] = __ldcg(reinterpret_cast<const float4 *>(P.part + (sl * 16 + head) * kHD + d0));
                     b[u] = __ldcg(reinterpret_cast<const float4 *>(P.part + (sl * 16 + head) * kHD + d0 + 4));
@@ -531,7 +553,7 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
             }
 #pragma unroll
             for (int u = 0; u < 16; u++) {
-                const float f = (c0 + u < S) ? fsm[(c0 + u) * 16 + head] : 0.0f;  // in chunk order
+                const float f = (c0 + u < SN) ? fsm[(c0 + u) * 16 + head] : 0.0f;  // in chunk order
                 o[0] = fmaf(a[u].x, f, o[0]); o[1] = fmaf(a[u].y, f, o[1]); o[2] = fmaf(a[u].z, f, o[2]); o[3] = fmaf(a[u].w, f, o[3]);
                 o[4] = fmaf(b[u].x, f, o[4]); o[5] = fmaf(b[u].y, f, o[5]); o[6] = fmaf(b[u].z, f, o[6]); o[7] = fmaf(b[u].w, f, o[7]);
             }
@@ -544,7 +566,9 @@ attn_decode_kernel(const float *__restrict__ q, const __half *__restrict__ kv_k,
     if (tid == 0) P.tickets[blockIdx.x] = 0;  // ready for the next launch
 }
 
-constexpr int kAttnSmem = 8192 + (kAttnWarps * 16 * kOPitch + 2 * kAttnWarps * 16) * 4;
+constexpr int kAttnRings = kAttnWarps * kAttnStages * kStageBytes, kAttnResults = kAttnWarps * 16 * kOPitch * 4;
+constexpr int kAttnSmem = 8192 + 2 * kAttnWarps * 16 * 4 + (kAttnRings > kAttnResults ? kAttnRings : kAttnResults);
+static_assert(kAttnSmem <= 227 * 1024, "shared memory budget");
 
 // Any head dimension (<= 1024): one CTA per query head, online softmax per warp over a
 // strided share of the positions, warps merged through shared memory. Correct, not fast.
