@@ -90,57 +90,44 @@ __device__ __forceinline__ void copy_q6k_row(uint32_t dst_lane, const uint8_t *b
     cp_async4(dst_lane, a);
     if (lane < 53 - 32) cp_async4(dst_lane + 128, a + 128);
 }
+// N words of a row that may begin two bytes into the first (HALF, half = 2)
+template <bool HALF, int N>
+__device__ __forceinline__ void q6k_words(const uint32_t *p, int half, uint32_t (&v)[N])
+{
+#pragma unroll
+    for (int i = 0; i < N; i++) v[i] = p[i];
+    if (HALF) {
+        const uint32_t last = p[N], sel = half ? 0x5432u : 0x3210u;
+#pragma unroll
+        for (int i = 0; i < N; i++) v[i] = __byte_perm(v[i], i < N - 1 ? v[i + 1] : last, sel);
+    }
+}
 struct RawQ6 {  // half a block: 128 weights
     uint32_t ql[16], qh[8], sc[2];
     float d;
-    __device__ __forceinline__ void load(const uint8_t *row, uint32_t skew, int half)
+    template <bool HALF>
+    __device__ __forceinline__ void load(const uint8_t *row, int half, int h)
     {
-        const uint32_t sel = skew ? 0x5432u : 0x3210u;
         const uint32_t *wp = reinterpret_cast<const uint32_t *>(row);
-        uint32_t prev = wp[16 * half];
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const uint32_t nx = wp[16 * half + i + 1];
-            ql[i] = __byte_perm(prev, nx, sel);
-            prev = nx;
-        }
-        prev = wp[32 + 8 * half];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const uint32_t nx = wp[32 + 8 * half + i + 1];
-            qh[i] = __byte_perm(prev, nx, sel);
-            prev = nx;
-        }
-        const uint32_t a = wp[48 + 2 * half], b = wp[49 + 2 * half], c = wp[50 + 2 * half];
-        sc[0] = __byte_perm(a, b, sel);
-        sc[1] = __byte_perm(b, c, sel);
-        d = __half2float(__ushort_as_half(static_cast<unsigned short>(skew ? wp[52] >> 16 : wp[52])));
+        q6k_words<HALF>(wp + 16 * h, half, ql);
+        q6k_words<HALF>(wp + 32 + 8 * h, half, qh);
+        q6k_words<HALF>(wp + 48 + 2 * h, half, sc);
+        d = __half2float(__ushort_as_half(static_cast<unsigned short>(half ? wp[52] >> 16 : wp[52])));
     }
 };
 // A quarter of a block, from a slot of shared memory in which the block begins `skew` bytes (even, below 16) from the start: 32 bytes
 // of ql and the qh bytes of the same half. Quarter u covers columns 128 (u / 2) + 32 (u % 2) + {0..31},
 // from the low nibbles, and 64 more, from the high ones.
-constexpr int kQ6Slot = 240;  // 15 x 16 bytes: an odd number, so that the rows of a warp spread over all banks
 struct QuarterQ6 {
     uint32_t ql[8], qh[8], sc[2];  // sc: the two scales of the low nibbles (bytes 0, 1), of the high ones
     float d;
-    // HALF: the block may begin two bytes into the word at `row` (half = 2), where the words have to be shifted
     template <bool HALF>
     __device__ __forceinline__ void load(const uint8_t *row, int half, int u)
     {
         const uint32_t *wp = reinterpret_cast<const uint32_t *>(row);
         const uint32_t sel = half ? 0x5432u : 0x3210u;
-        auto words = [&](const uint32_t *p, uint32_t (&v)[8]) {
-#pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = p[i];
-            if (HALF) {
-                const uint32_t last = p[8];
-#pragma unroll
-                for (int i = 0; i < 8; i++) v[i] = __byte_perm(v[i], i < 7 ? v[i + 1] : last, sel);
-            }
-        };
-        words(wp + 8 * u, ql);
-        words(wp + 32 + 8 * (u >> 1), qh);
+        q6k_words<HALF>(wp + 8 * u, half, ql);
+        q6k_words<HALF>(wp + 32 + 8 * (u >> 1), half, qh);
         const uint32_t a = wp[48 + 2 * (u >> 1)], b = wp[49 + 2 * (u >> 1)], c = HALF ? wp[50 + 2 * (u >> 1)] : 0u;
         const uint32_t sel2 = sel >> (u & 1 ? 8 : 0);  // bytes 2, 3 for the odd quarters
         sc[0] = __byte_perm(a, b, sel2);
@@ -171,6 +158,79 @@ __device__ __forceinline__ void int_q6(const QuarterQ6 &raw, int part, int odd, 
         low[8 + 2 * i + 1] = hfms2(a1, fl, low[2 * i + 1]);
         high[8 + 2 * i] = hfms2(b0, fh, high[2 * i]);
         high[8 + 2 * i + 1] = hfms2(b1, fh, high[2 * i + 1]);
+    }
+}
+
+// ---- weights rounded to fp16 once (the dense GEMM, whose accumulators run through all of K) ----
+// scale * n and scale * q - 32 scale are exact in fp32 out of one FMA whose factors are fp16 (Blackwell's mixed-precision FMA runs at the
+// rate of the fp32 one), d and the min follow in fp32, then one rounding. The masked fields are fp16 numbers as they are (above), so a
+// weight costs the integer pipe 1.1 instructions instead of the 1.9 of bytes permuted into fp32 mantissas; that pipe has half the
+// rate (Q4_K 512 x 512 x 8192 in tiles of 128: 30.2 instead of 33.4 us).
+
+// a * b + c, a and b the low or high halves of their registers
+template <bool AH, bool BH>
+__device__ __forceinline__ float mixed_fma(uint32_t a, uint32_t b, float c)
+{
+    float r;
+    const unsigned short x = static_cast<unsigned short>(AH ? a >> 16 : a), y = static_cast<unsigned short>(BH ? b >> 16 : b);
+    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(r) : "h"(x), "h"(y), "f"(c));
+    return r;
+}
+// (a, b) * (f, f) + (c, c)
+__device__ __forceinline__ void fma_pair(float &a, float &b, float f, float c)
+{
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %2};\n\tmov.b64 z, {%3, %3};\n\t"
+        "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "+f"(a), "+f"(b)
+        : "f"(f), "f"(c));
+}
+__device__ __forceinline__ uint32_t pack_halves(float lo, float hi)
+{
+    const __half2 h = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+// two bytes of up to 10 bits each as fp16 numbers
+__device__ __forceinline__ uint32_t small_half2(uint32_t two_bytes)
+{
+    return hadd2(__byte_perm(two_bytes, 0x64646464u, 0x4140), 0xE400E400u);  // 1024 + v - 1024
+}
+// 32 weights d * sc * n + c (sc in the low half), n the low or high nibbles of 8 words, in column order
+template <bool HIGH>
+__device__ __forceinline__ void round_q4(const uint32_t (&w)[8], uint32_t sc, float d, float c, uint32_t (&o)[16])
+{
+    constexpr uint32_t mask = HIGH ? 0x00F000F0u : 0x000F000Fu;
+    const float f = d * (HIGH ? 1048576.0f : 16777216.0f);  // a masked nibble is n 2^-20 or n 2^-24
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t even = w[i] & mask, odd = (w[i] >> 8) & mask;
+        float v[4] = {mixed_fma<false, false>(even, sc, 0.0f), mixed_fma<false, false>(odd, sc, 0.0f),
+                      mixed_fma<true, false>(even, sc, 0.0f), mixed_fma<true, false>(odd, sc, 0.0f)};
+        fma_pair(v[0], v[1], f, c);
+        fma_pair(v[2], v[3], f, c);
+        o[2 * i] = pack_halves(v[0], v[1]);
+        o[2 * i + 1] = pack_halves(v[2], v[3]);
+    }
+}
+// 32 weights d * sc * (q - 32) of half a block, thirty-two-group 2 c + h. Here a byte permuted into the mantissa of 2.0f (v = 2 + q / 64) and
+// one FMA per weight, s (q - 32) = 64 s v - 160 s, take less: the exact integers above have 12 bits, a second multiplication, and do not
+// share their shifts between the nibbles as the grouped GEMM's do (Q6_K 512 x 512 x 8192: 34.3 instead of 30.5 us in tiles of 64).
+__device__ __forceinline__ void round_q6(const RawQ6 &raw, int c, int h, uint32_t (&o)[16])
+{
+    float a[2], b[2];
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const float s = raw.d * static_cast<float>(static_cast<int8_t>(raw.sc[c] >> (16 * h + 8 * i)));
+        a[i] = 64.0f * s;
+        b[i] = -160.0f * s;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t l = c ? raw.ql[8 * h + i] >> 4 : raw.ql[8 * h + i];
+        const uint32_t hb = c == 0 ? (h == 0 ? raw.qh[i] << 4 : raw.qh[i] << 2) : (h == 0 ? raw.qh[i] : raw.qh[i] >> 2);
+        const uint32_t n = (l & 0x0F0F0F0Fu) | (hb & 0x30303030u);
+        const float s = a[i >> 2], m = b[i >> 2];
+        o[2 * i] = pack_halves(fmaf(s, __uint_as_float(__byte_perm(n, 0x40000000u, 0x7044)), m), fmaf(s, __uint_as_float(__byte_perm(n, 0x40000000u, 0x7144)), m));
+        o[2 * i + 1] = pack_halves(fmaf(s, __uint_as_float(__byte_perm(n, 0x40000000u, 0x7244)), m), fmaf(s, __uint_as_float(__byte_perm(n, 0x40000000u, 0x7344)), m));
     }
 }
 

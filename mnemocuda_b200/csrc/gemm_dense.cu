@@ -4,24 +4,24 @@
 // (The reference's "tensor-core GEMM", src/gemm_q4k.cu:201-266, is an int8 mma.sync experiment at batch 1.)
 //
 // The weight rows are the UMMA M dimension (128 per CTA, one TMEM lane each), the tokens the N dimension (BT per CTA), K goes in
-// chunks of 64. Per CTA: a warp that loads activations (TMA, 128-byte swizzle), a warp that issues the MMAs, one or two that
-// bring raw super-blocks into a shared-memory ring (Q4_K: TMA, rows of 144-byte blocks make a tensor map; Q6_K: 4-byte
-// cp.async walking along the rows, as 210-byte blocks fit no tensor map), and 16 warps that dequantise a row per thread and
-// store the fp16 operand straight into TMEM. A stage of the ring is a chunk: 32 TMEM columns of weights and BT x 128 bytes of
-// activations behind one pair of barriers.
+// chunks of 64. Per CTA: a warp that loads activations (TMA, 128-byte swizzle), a warp that issues the MMAs, one that brings raw
+// super-blocks into a shared-memory ring (TMA: rows of 144-byte Q4_K blocks make a tensor map, of 210-byte Q6_K blocks 1 to 8 rows
+// together do; a Q6_K tensor off its 16 bytes, or with rows left over, by two warps of 4-byte cp.async), and 16 warps that
+// dequantise a row per thread and store the fp16 operand straight into TMEM. A stage of the ring is a chunk: 32 TMEM columns of weights
+// and BT x 128 bytes of activations behind one pair of barriers.
 //
-// What bounds a tile is one of: the dequant warps (about 300 cycles per chunk and SM whatever BT is), the activation tile's
-// way from L2 (BT x 128 bytes per chunk at 42 bytes per cycle and SM), a fixed 6000 cycles of launch, ramp and epilogue. So BT
-// and the number of K splits are chosen per shape (plan()): wide tiles where there are enough of them to fill the SMs, narrow
+// What bounds a tile is one of: the dequant warps (370 to 480 cycles per chunk and SM at up to 128 tokens), the activation tile's
+// way from L2 and the MMAs (590 at 256), and a start and an end of 2 to 7 us, the longer the wider the tile and the fuller the GPU.
+// So BT and the number of K splits are chosen per shape (plan()): wide tiles where there are enough of them to fill the SMs, narrow
 // ones -- every weight then dequantised more than once, on SMs that would otherwise idle -- where there are not, and for still
 // smaller shapes the CTAs of a cluster share the K range of a tile and add their accumulators through distributed shared
-// memory, in rank order (deterministic). At the large end two CTAs share a tile of 256 rows x 256 tokens (cta_group::2): each
-// dequantises its own rows and loads half of the activations, which makes the MMAs the bound (512 x 8192 x 4096: the tensor pipe
-// is busy 66 % of the launch's cycles, ramp and epilogue included).
+// memory, in rank order (deterministic). At the large end two CTAs may share a tile of 256 rows x 256 tokens (cta_group::2): each
+// dequantises its own rows and loads half of the activations.
 //
-// Measured: Q4_K 512 x 8192 x 4096 35 us (clock-throttled in a loop: 21 us of cycles at 1.92 GHz), 2048 x 8192 x 4096 135,
-// 200 x 4096 x 4096 12.8, 16 x 4096 x 4096 8.4 (host-bound); Q6_K 512 x 8192 x 4096 42.8, 130 x 7795 x 5120 37.1,
-// 33 x 2022 x 2560 12.4. (Weights through shared memory, one tile size and no K split: 1.2 to 4 times as long.)
+// Measured (in brackets: shapes placed by the cycles of the SMs alone, Q6_K by cp.async, loaders in one-thread branches, byte permutes for
+// Q4_K): Q4_K 512 x 8192 x 4096 28.2 us in a burst (28.9), 33.6 under the power cap in a loop (34.2); 2048 x 8192 x 4096 110 (113),
+// 197 x 4096 x 4096 11.7 (12.8), 197 x 2048 x 2048 7.1 (16.0), 512 x 512 x 8192 10.6 (17.3), 8 x 2048 x 2048 3.5 (7.8); Q6_K 512 x 8192 x 4096
+// 29.7 (35.9), 197 x 8192 x 4096 18.4 (30.9), 197 x 4096 x 1536 7.4 (11.0), 8 x 8192 x 4096 12.5 (16.9).
 #include <cooperative_groups.h>
 
 #include <cstdio>
@@ -57,6 +57,7 @@ struct Params {
     const uint8_t *w;
     float *out;
     int M, N, bpr;
+    int group;  // Q6_K: rows a tensor map takes together (encode_q6k_groups), 0: by cp.async
     int pdl;
     int *err;
 };
@@ -67,7 +68,7 @@ struct Cfg {
     static constexpr int kXRows = PAIR ? BT / 2 : BT;
     static constexpr int kStages = BT == 256 ? (PAIR ? 8 : 5) : BT == 128 ? 8 : 14;  // what TMEM (BT + 32 columns each) and shared memory hold
     static constexpr int kXBytes = kXRows * 128;
-    static constexpr int kWBytes = QT == 4 ? kRows * kQ4KBlock : kRows * kQ6Pitch;
+    static constexpr int kWBytes = QT == 4 ? kRows * kQ4KBlock : kRows * kQ6Slot;
     static constexpr int kWStages = QT == 6 && BT == 256 && !PAIR ? 2 : 3;
     static constexpr int kOffW = kStages * kXBytes;
     static constexpr int kOffBar = kOffW + kWStages * kWBytes;
@@ -75,32 +76,45 @@ struct Cfg {
     static_assert(kSmem <= 227 * 1024 && BT + 32 * kStages <= 512, "shared memory / tensor memory budget");
 };
 
-// See the grouped GEMM: a wait that runs out raises the abort flag, after which no wait of the CTA waits any more.
-__device__ __noinline__ void wait_slow(uint64_t *bar, uint32_t parity, volatile int *abort_flag)
+// The S partial tiles [token][128 rows] of a cluster, in rank order: rank `split` takes every S-th token, a warp a token, a lane four
+// rows, up to eight 16-byte loads in flight (with one of four bytes at a time Q6_K 8 x 2048 x 2048 took 10.6 instead of 8.5 us).
+template <int S, int BT>
+__device__ __forceinline__ void add_splits(cg::cluster_group cl, uint8_t *smem, const Params &P, int split, int n0, int t0, int w, int lane)
 {
-    for (uint32_t i = 0; i < kWaitBudget; i++)
-        if (*abort_flag || mbar_try_wait(bar, parity)) return;
-    *abort_flag = 1;
-}
-__device__ __forceinline__ void wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag)
-{
-    if (!mbar_try_wait(bar, parity)) wait_slow(bar, parity, abort_flag);
-}
-
-// 32 weights -> 16 registers of fp16 pairs. A small integer in byte 2 of 2.0f (0x40000000) is v = 2 + n / 64: an int -> float
-// conversion for one byte permute; w = s n - b = (64 s) v - (128 s + b) in fp32, rounded to fp16 once.
-__device__ __forceinline__ void pack_f16(const uint32_t (&n)[8], const float (&a)[2], const float (&b)[2], uint32_t (&o)[16])
-{
+    constexpr int U = 8 / S, kStep = S * 4 * kGroups;
+    const float4 *peer[S];
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const float s = a[i >> 2], c = b[i >> 2];
-        const float w0 = fmaf(s, __uint_as_float(__byte_perm(n[i], 0x40000000u, 0x7044)), c);
-        const float w1 = fmaf(s, __uint_as_float(__byte_perm(n[i], 0x40000000u, 0x7144)), c);
-        const float w2 = fmaf(s, __uint_as_float(__byte_perm(n[i], 0x40000000u, 0x7244)), c);
-        const float w3 = fmaf(s, __uint_as_float(__byte_perm(n[i], 0x40000000u, 0x7344)), c);
-        const __half2 p0 = __floats2half2_rn(w0, w1), p1 = __floats2half2_rn(w2, w3);
-        o[2 * i] = *reinterpret_cast<const uint32_t *>(&p0);
-        o[2 * i + 1] = *reinterpret_cast<const uint32_t *>(&p1);
+    for (int p = 0; p < S; p++) peer[p] = cl.map_shared_rank(reinterpret_cast<const float4 *>(smem), p) + lane;
+    const int tokens = min(BT, P.M - t0), n = n0 + 4 * lane;
+    const bool vec = n + 3 < P.N && (P.N & 3) == 0 && (reinterpret_cast<uintptr_t>(P.out) & 15) == 0;
+    for (int t = split + S * w; t < tokens; t += U * kStep) {
+        float4 v[U][S];
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int p = 0; p < S; p++)
+                if (t + u * kStep < tokens) v[u][p] = peer[p][(t + u * kStep) * (kRows / 4)];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (t + u * kStep >= tokens) break;
+            float4 a = v[u][0];
+#pragma unroll
+            for (int p = 1; p < S; p++) {
+                a.x += v[u][p].x;
+                a.y += v[u][p].y;
+                a.z += v[u][p].z;
+                a.w += v[u][p].w;
+            }
+            float *o = P.out + (size_t)(t0 + t + u * kStep) * P.N + n;
+            if (vec) {
+                *reinterpret_cast<float4 *>(o) = a;
+            } else {
+                if (n < P.N) o[0] = a.x;
+                if (n + 1 < P.N) o[1] = a.y;
+                if (n + 2 < P.N) o[2] = a.z;
+                if (n + 3 < P.N) o[3] = a.w;
+            }
+        }
     }
 }
 
@@ -117,7 +131,7 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
     uint64_t *wfull = empty + S, *wempty = wfull + WS, *acc_full = wempty + WS, *pfull = acc_full + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(pfull + S);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = static_cast<int>(warp_uniform(tid >> 5));
     const int n0 = blockIdx.x * kRows, t0 = blockIdx.y * BT;
     const int split = blockIdx.z, splits = gridDim.z;
     const int b0 = P.bpr * split / splits, nb = P.bpr * (split + 1) / splits - b0;  // this CTA's super-blocks
@@ -133,7 +147,7 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
             mbar_init(&pfull[s], 1);     // PAIR: the other CTA's stage is full
         }
         for (int s = 0; s < WS; s++) {
-            mbar_init(&wfull[s], QT == 4 ? 1 : 64);  // TMA: the expect_tx arrival; cp.async: every thread of the two warps
+            mbar_init(&wfull[s], QT == 4 || P.group ? 1 : 64);  // TMA: the expect_tx arrival; cp.async: every thread of the two warps
             mbar_init(&wempty[s], 8);                // the two groups that share a super-block
         }
         mbar_init(acc_full, 1);
@@ -146,38 +160,44 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
     tc_fence_after();
     const int rank = PAIR ? static_cast<int>(blockIdx.x & 1) : 0;
     if (P.pdl) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = warp_uniform(*tmem_slot), leader = elect_lane();
 
+    // Loaders and issuer run converged through their loops, one lane's copies and MMAs take effect (tcgen.cuh).
     if (warp == 0) {
-        if (lane == 0) {  // ---- activations ----
-            if (P.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");  // X may come from the kernel upstream
-            int s = 0, ph = 1;
-            for (int j = 0; j < units; j += kGroups) {
-                const int G = min(kGroups, units - j);
-                for (int cgi = 0; cgi < 2 * G; cgi++) {
-                    wait(&empty[s], ph, abort_flag);  // passes at once while the stage has not been used
-                    const int k = 256 * b0 + (cgi < G ? 128 * (j + cgi) : 128 * (j + cgi - G) + 64);
+        // ---- activations ----
+        if (P.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");  // X may come from the kernel upstream
+        int s = 0;
+        uint32_t ph = 1;
+        for (int j = 0; j < units; j += kGroups) {
+            const int G = min(kGroups, units - j);
+            for (int cgi = 0; cgi < 2 * G; cgi++) {
+                wait(&empty[s], ph, abort_flag);  // passes at once while the stage has not been used
+                __syncwarp();
+                const int k = 256 * b0 + (cgi < G ? 128 * (j + cgi) : 128 * (j + cgi - G) + 64);
+                if (leader) {
                     mbar_expect_tx(&full[s], C::kXBytes);
                     tma_load_2d(smem + s * C::kXBytes, &xmap, k, t0 + rank * C::kXRows, &full[s]);
-                    if (++s == S) {
-                        s = 0;
-                        ph ^= 1;
-                    }
+                }
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1;
                 }
             }
         }
     } else if (warp == 1) {
-        // ---- MMA issuer: the warp runs converged, one lane's instructions take effect (tcgen.cuh) ----
-        const uint32_t leader = elect_lane(), tm = warp_uniform(tmem), x0 = warp_uniform(smem_u32(smem));
+        // ---- MMA issuer ----
         constexpr uint32_t idesc = umma_idesc_f16(PAIR ? 2 * kRows : kRows, BT);
-        int s = 0, ph = 0;
+        const uint32_t full0 = warp_uniform(smem_u32(full)), desc0 = desc_lo(warp_uniform(smem_u32(smem)));
+        const uint32_t to_empty = 8 * S, to_pfull = 8 * static_cast<uint32_t>(pfull - full);
+        int s = 0;
+        uint32_t ph = 0;
         for (int kb = 0; kb < 2 * units; kb++) {
-            wait(&full[s], ph, abort_flag);
-            if (PAIR && rank == 0) wait(&pfull[s], ph, abort_flag);
+            const uint32_t bar = full0 + 8 * s;
+            wait(bar, ph, abort_flag);
+            if (PAIR && rank == 0) wait(bar + to_pfull, ph, abort_flag);
             tc_fence_after();
             __syncwarp();
-            const uint64_t db = smem_desc_sw128(x0 + s * C::kXBytes);
-            const uint32_t a = tm + BT + 32 * s;
+            const uint32_t db = desc0 + s * (C::kXBytes / 16), a = tmem + BT + 32 * s;
             if (leader) {
                 if (PAIR && rank == 1) {  // tell the first CTA, which issues for both
                     tc_fence_before();
@@ -186,14 +206,14 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
 #pragma unroll
                     for (int kk = 0; kk < 4; kk++) {  // 16 fp16 of K = 8 operand columns = 2 descriptor units
                         if (PAIR)
-                            umma2_f16_ta(tm, a + 8 * kk, db + 2 * kk, idesc, (kb | kk) != 0);
+                            umma2_f16_ta(tmem, a + 8 * kk, desc64(db + 2 * kk), idesc, (kb | kk) != 0);
                         else
-                            umma_f16_ta(tm, a + 8 * kk, db + 2 * kk, idesc, (kb | kk) != 0);
+                            umma_f16_ta(tmem, a + 8 * kk, desc64(db + 2 * kk), idesc, (kb | kk) != 0);
                     }
                     if (PAIR)
                         umma2_commit(&empty[s]);
                     else
-                        umma_commit(&empty[s]);
+                        umma_commit(bar + to_empty);
                 }
             }
             __syncwarp();
@@ -211,14 +231,24 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
         __syncwarp();
     } else if (warp < C::kDq0) {
         // ---- raw weights: 128 rows x one super-block per stage; they never depend on the kernel upstream ----
-        if (QT == 6 || lane == 0) {
-            int s = 0, ph = 1;
+        if (warp == 2 || !P.group) {
+            int s = 0;
+            uint32_t ph = 1;
             for (int b = 0; b < nb; b++) {
                 wait(&wempty[s], ph, abort_flag);
+                __syncwarp();
                 uint8_t *dst = smem + C::kOffW + s * C::kWBytes;
-                if (QT == 4) {
-                    mbar_expect_tx(&wfull[s], C::kWBytes);
-                    tma_load_2d(dst, &wmap, (b0 + b) * kQ4KBlock, n0, &wfull[s]);  // rows past N arrive as zeros
+                if (QT == 4 || P.group) {
+                    if (leader) {
+                        mbar_expect_tx(&wfull[s], C::kWBytes);
+                        if (QT == 4) {
+                            tma_load_2d(dst, &wmap, (b0 + b) * kQ4KBlock, n0, &wfull[s]);  // rows past N arrive as zeros
+                        } else {
+                            for (int j = 0; j < P.group; j++)
+                                tma_load_2d(dst + (j * kRows / P.group) * kQ6Slot, &wmap, ((j * P.bpr + b0 + b) * kQ6KBlock) & ~15, n0 / P.group,
+                                            &wfull[s]);
+                        }
+                    }
                 } else {
                     const int r0 = (warp - 2) * 64, rows = min(64, P.N - n0 - r0);  // rows past N are not stored in the end
                     const uint8_t *blk = P.w + ((size_t)(n0 + r0) * P.bpr + b0 + b) * kQ6KBlock;
@@ -236,7 +266,7 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
                     ph ^= 1;
                 }
             }
-            if (QT == 6) asm volatile("cp.async.wait_all;" ::: "memory");
+            if (QT == 6 && !P.group) asm volatile("cp.async.wait_all;" ::: "memory");
         }
     } else {
         // ---- dequant: thread = row r of the tile; group g ----
@@ -255,8 +285,16 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[it % S]);
         };
-        uint32_t row_addr = 0;  // Q6_K: low bits of the row's address
-        if (QT == 6) row_addr = static_cast<uint32_t>(reinterpret_cast<uintptr_t>(P.w)) + ((uint32_t)(n0 + r) * (uint32_t)P.bpr + b0) * kQ6KBlock;
+        // Q6_K: where the row's blocks lie in a stage, and the bytes (mod 16) by which they are off
+        const uint8_t *row = nullptr;
+        uint32_t row_addr = 0;
+        if (QT == 6) {
+            const int rg = P.group ? r & (P.group - 1) : 0;
+            row = smem + C::kOffW + (P.group ? (rg * (kRows / P.group) + r / P.group) * kQ6Slot : r * kQ6Pitch);
+            row_addr = P.group ? (uint32_t)(rg * P.bpr + b0) * kQ6KBlock
+                               : (static_cast<uint32_t>(reinterpret_cast<uintptr_t>(P.w)) + ((uint32_t)(n0 + r) * (uint32_t)P.bpr + b0) * kQ6KBlock) & 3u;
+        }
+        const uint32_t off_mask = P.group ? 15u : 3u;
         for (int j = 0; j < units; j += kGroups) {
             const int G = min(kGroups, units - j), u = j + g;
             if (g >= G) break;
@@ -264,7 +302,7 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
             wait(&wfull[ws], (sb / WS) & 1, abort_flag);
             __syncwarp();
             const uint8_t *blk = smem + C::kOffW + ws * C::kWBytes;
-            uint32_t o[16], n8[8];
+            uint32_t o[16];
             if (QT == 4) {
                 blk += r * kQ4KBlock;
                 const uint4 hdr = *reinterpret_cast<const uint4 *>(blk);
@@ -273,30 +311,27 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
                 for (int i = 0; i < 4; i++) qv[i] = *reinterpret_cast<const uint4 *>(blk + 16 + 64 * half + 16 * i);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&wempty[ws]);
-                const float2 dd = __half22float2(*reinterpret_cast<const __half2 *>(&hdr.x));
+                const float d = __half2float(__ushort_as_half(static_cast<unsigned short>(hdr.x)));
 #pragma unroll
                 for (int c = 0; c < 2; c++) {
                     const int it = 2 * j + c * G + g;
                     uint32_t sc2, m2, ta = 0;
                     q4k_scale_pair(hdr.y, hdr.z, hdr.w, 2 * half + c, sc2, m2);
+                    const uint32_t sc = small_half2(sc2), m = small_half2(m2), minus_dmin = (hdr.x >> 16) ^ 0x8000u;
                     const uint32_t wq[8] = {qv[2 * c].x, qv[2 * c].y, qv[2 * c].z, qv[2 * c].w,
                                             qv[2 * c + 1].x, qv[2 * c + 1].y, qv[2 * c + 1].z, qv[2 * c + 1].w};
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        const float a = 64.0f * (dd.x * static_cast<float>(h ? sc2 >> 8 : sc2 & 0xFFu));
-                        const float b = -(2.0f * a + dd.y * static_cast<float>(h ? m2 >> 8 : m2 & 0xFFu));
-#pragma unroll
-                        for (int i = 0; i < 8; i++) n8[i] = (h ? wq[i] >> 4 : wq[i]) & 0x0F0F0F0Fu;
-                        const float av[2] = {a, a}, bv[2] = {b, b};
-                        pack_f16(n8, av, bv, o);
-                        if (h == 0) ta = stage_free(it);
-                        tmem_st16(ta + 16 * h, o);
-                    }
+                    round_q4<false>(wq, sc, d, mixed_fma<false, false>(m, minus_dmin, 0.0f), o);
+                    ta = stage_free(it);
+                    tmem_st16(ta, o);
+                    round_q4<true>(wq, sc >> 16, d, mixed_fma<true, false>(m, minus_dmin, 0.0f), o);
+                    tmem_st16(ta + 16, o);
                     publish(it);
                 }
             } else {
+                const uint32_t off = (row_addr + sb * kQ6KBlock) & off_mask;
+                const uint8_t *words = row + ws * C::kWBytes + (off & 12u);
                 RawQ6 raw;
-                raw.load(blk + r * kQ6Pitch, (row_addr + sb * kQ6KBlock) & 2u, half);
+                if (__any_sync(0xffffffffu, off & 2u)) raw.load<true>(words, off & 2u, half); else raw.load<false>(words, 0, half);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&wempty[ws]);
 #pragma unroll
@@ -305,20 +340,7 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
                     uint32_t ta = 0;
 #pragma unroll
                     for (int h = 0; h < 2; h++) {  // thirty-two-group 2 c + h of the half, two scales
-                        float av[2], bv[2];
-#pragma unroll
-                        for (int i = 0; i < 2; i++) {
-                            const float s = raw.d * static_cast<float>(static_cast<int8_t>(raw.sc[c] >> (16 * h + 8 * i)));
-                            av[i] = 64.0f * s;
-                            bv[i] = -160.0f * s;
-                        }
-#pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            const uint32_t l = c ? raw.ql[8 * h + i] >> 4 : raw.ql[8 * h + i];
-                            const uint32_t hb = c == 0 ? (h == 0 ? raw.qh[i] << 4 : raw.qh[i] << 2) : (h == 0 ? raw.qh[i] : raw.qh[i] >> 2);
-                            n8[i] = (l & 0x0F0F0F0Fu) | (hb & 0x30303030u);
-                        }
-                        pack_f16(n8, av, bv, o);
+                        round_q6(raw, c, h, o);
                         if (h == 0) ta = stage_free(it);
                         tmem_st16(ta + 16 * h, o);
                     }
@@ -354,20 +376,13 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
         cg::cluster_group cl = cg::this_cluster();
         cl.sync();
         if (warp >= C::kDq0) {
-            const int i = tid - C::kDq0 * 32, r = i & 127;
-            const float *red = reinterpret_cast<const float *>(smem);
-            const float *peer[kMaxSplit];
-#pragma unroll
-            for (int p = 0; p < kMaxSplit; p++) peer[p] = cl.map_shared_rank(red, p < splits ? p : 0);
-            const int tokens = min(BT, P.M - t0);
-            for (int t = split + splits * (i >> 7); t < tokens; t += splits * 4) {
-                float v[kMaxSplit];
-#pragma unroll
-                for (int p = 0; p < kMaxSplit; p++) v[p] = p < splits ? peer[p][t * kRows + r] : 0.0f;
-                float acc = v[0];
-#pragma unroll
-                for (int p = 1; p < kMaxSplit; p++) acc += v[p];
-                if (n0 + r < P.N) P.out[(size_t)(t0 + t) * P.N + n0 + r] = acc;
+            switch (splits) {
+                case 2: add_splits<2, BT>(cl, smem, P, split, n0, t0, warp - C::kDq0, lane); break;
+                case 3: add_splits<3, BT>(cl, smem, P, split, n0, t0, warp - C::kDq0, lane); break;
+                case 4: add_splits<4, BT>(cl, smem, P, split, n0, t0, warp - C::kDq0, lane); break;
+                case 5: add_splits<5, BT>(cl, smem, P, split, n0, t0, warp - C::kDq0, lane); break;
+                case 6: add_splits<6, BT>(cl, smem, P, split, n0, t0, warp - C::kDq0, lane); break;
+                default: add_splits<8, BT>(cl, smem, P, split, n0, t0, warp - C::kDq0, lane);
             }
         }
         cl.sync();  // nobody leaves while its shared memory is being read
@@ -379,32 +394,6 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
     if (tid == 0 && *abort_flag) atomicExch(P.err, MB200_ERR_TIMEOUT);
 }
 
-struct Plan {
-    int bt, splits;
-    bool pair;
-};
-// The cheapest form by the cost model of the file's head, in SM cycles: whole waves of tiles, a tile being 6000 cycles plus its
-// chunks, and 2500 for adding up splits. Ties go to the wider tile.
-Plan plan(int M, int N, int K)
-{
-    const int sms = device_sms(), bpr = K / 256, row_tiles = (N + kRows - 1) / kRows;
-    Plan best{256, 1, false};
-    long best_cost = -1;
-    auto offer = [&](int bt, int s, bool pair, int per) {
-        const long tiles = (long)(pair ? row_tiles + (row_tiles & 1) : row_tiles) * ((M + bt - 1) / bt) * s;
-        if (s > 1 && tiles > sms) return;
-        const long cost = (tiles + sms - 1) / sms * (6000 + 4L * ((bpr + s - 1) / s) * per + (s > 1 ? 2500 : 0));
-        if (best_cost < 0 || cost < best_cost) {
-            best_cost = cost;
-            best = {bt, s, pair};
-        }
-    };
-    offer(256, 1, true, 530);
-    for (int bt = 256; bt >= 64; bt /= 2)
-        for (int s = 1; s <= kMaxSplit && s <= bpr; s *= 2) offer(bt, s, false, 3 * bt > 300 ? 3 * bt : 300);
-    return best;
-}
-
 template <int QT, int BT, bool PAIR>
 void attr()
 {
@@ -412,6 +401,67 @@ void attr()
     if (done[current_device()]) return;
     cudaFuncSetAttribute(gemm_dense_kernel<QT, BT, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<QT, BT, PAIR>::kSmem);
     done[current_device()] = true;
+}
+
+// CTAs that run at a time when clusters of `s` have to find room in one GPC each: 148, 148, 135, 132, 130, 132, -, 120 for one CTA per SM.
+int clustered_ctas(int s)
+{
+    static int known[kMaxDevices][kMaxSplit + 1] = {};
+    int &n = known[current_device()][s];
+    if (n == 0) {
+        attr<4, 64, false>();
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kMaxSplit, 1, s);
+        cfg.blockDim = dim3(Cfg<4, 64, false>::kThreads);
+        cfg.dynamicSmemBytes = Cfg<4, 64, false>::kSmem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = s;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, gemm_dense_kernel<4, 64, false>, &cfg) != cudaSuccess) cudaGetLastError();
+        n = clusters > 0 ? clusters * s : device_sms() / s * s;
+    }
+    return n;
+}
+
+struct Plan {
+    int bt, splits;
+    bool pair;
+};
+// The cheapest form by a cost model in ns, fitted to 21 shapes x all forms of either type (1.5 % above the best form on average, 17 % at
+// most; by SM cycles and 148 CTAs for whatever clusters it was up to 2.2 times the best: 128 CTAs in clusters of eight are two waves).
+// A wave costs its longest tile -- super-blocks by token tile -- plus a start and an end that grow with the tile and with how much
+// of the GPU is started; adding up splits comes on top.
+Plan plan(int qt, int M, int N, int K)
+{
+    static const struct {
+        int sb, fixed, fill;
+    } kCost[2][4] = {{{740, 0, 3500}, {780, 1800, 3200}, {1190, 3600, 3600}, {1180, 3600, 3600}},    // Q4_K: 64, 128, 256 tokens, a pair
+                     {{810, 0, 4400}, {960, 800, 4600}, {1210, 3100, 5200}, {1200, 3100, 5200}}};  // Q6_K
+    const int sms = device_sms(), bpr = K / 256, row_tiles = (N + kRows - 1) / kRows;
+    Plan best{256, 1, true};
+    long best_cost = -1;
+    auto offer = [&](int form, int s) {
+        const bool pair = form == 3;
+        const int bt = pair ? 256 : 64 << form, rows = pair ? row_tiles + (row_tiles & 1) : row_tiles;
+        const long tiles = (long)rows * ((M + bt - 1) / bt) * s, room = clustered_ctas(pair ? 2 : s);
+        if (s > 1 && tiles > room) return;
+        const auto &c = kCost[qt == 6][form];
+        const long cost = (tiles + room - 1) / room * ((long)(bpr + s - 1) / s * c.sb + c.fixed + c.fill * (tiles < sms ? tiles : sms) / sms) +
+                          (s > 1 ? 1250 + 50 * s : 0);
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best = {bt, s, pair};
+        }
+    };
+    offer(3, 1);
+    for (int form = 2; form >= 0; form--)
+        for (int s : {1, 2, 3, 4, 5, 6, 8})
+            if (s <= bpr) offer(form, s);
+    return best;
 }
 
 template <int QT, int BT, bool PAIR>
@@ -448,13 +498,17 @@ int launch_gemm(const void *w, const void *x_f16, float *out, int M, int N, int 
         return MB200_ERR_UNSUPPORTED;
     }
     if ((reinterpret_cast<uintptr_t>(x_f16) & 15) || (reinterpret_cast<uintptr_t>(w) & (QT == 4 ? 15 : 1))) return MB200_ERR_ARG;
-    Params P{static_cast<const uint8_t *>(w), out, M, N, K / 256, pdl_enabled(), device_error_word()};
+    Params P{static_cast<const uint8_t *>(w), out, M, N, K / 256, 0, pdl_enabled(), device_error_word()};
     CUtensorMap wmap = {};
-    if (QT == 4 && !encode_q4k_rows(&wmap, w, P.bpr, N, 1, 0, kRows)) {
+    if (QT == 6 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {
+        P.group = q6k_group(P.bpr);
+        if (N % P.group) P.group = 0;
+    }
+    if ((QT == 4 && !encode_q4k_rows(&wmap, w, P.bpr, N, 1, 0, kRows)) || (P.group && !encode_q6k_groups(&wmap, w, P.bpr, P.group, N, 1, 0, kRows))) {
         fprintf(stderr, "[mnemo_b200] %s: a tensor map could not be encoded\n", where);
         return MB200_ERR_ARG;
     }
-    const Plan p = plan(M, N, K);
+    const Plan p = plan(QT, M, N, K);
     if (p.pair) return launch<QT, 256, true>(P, wmap, x_f16, K, 1, stream);
     if (p.bt == 64) return launch<QT, 64, false>(P, wmap, x_f16, K, p.splits, stream);
     if (p.bt == 128) return launch<QT, 128, false>(P, wmap, x_f16, K, p.splits, stream);
@@ -474,6 +528,7 @@ void gemm_init()
     attr<6, 256, false>();
     attr<6, 256, true>();
     (void)encode_tiled();
+    for (int s : {1, 2, 3, 4, 5, 6, 8}) (void)clustered_ctas(s);
 }
 
 }  // namespace mb200

@@ -215,6 +215,32 @@ __device__ __forceinline__ uint64_t desc64(uint32_t lo)
 }
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) { return desc64(desc_lo(saddr)); }
 
+// Waits inside the GEMMs. A wait that runs out raises the CTA's abort flag and from then on every wait of the CTA returns at
+// once: the roles run through their loops on whatever the buffers hold (all addresses stay in bounds) and the kernel reports
+// the timeout. Nothing is checked on the fast path; a check per step (a shared-memory load and a vote) cost the issuing warp
+// 100 of its 400 cycles per chunk. (try_wait with a time limit sleeps in between: 10 % slower.)
+// Asking costs issue slots that the dequantising warps need: PATIENT waits (the loaders', which run stages ahead) pause in between.
+template <bool PATIENT = false>
+__device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, volatile int *abort_flag)
+{
+    for (uint32_t i = 0; i < kWaitBudget; i++) {
+#pragma unroll 1
+        for (int j = 0; j < 64; j++) {
+            if (mbar_try_wait(bar, parity)) return;
+            if (PATIENT) __nanosleep(100);
+        }
+        if (*abort_flag) return;
+    }
+    *abort_flag = 1;
+}
+template <bool PATIENT = false>
+__device__ __forceinline__ void wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag)
+{
+    wait<PATIENT>(smem_u32(bar), parity, abort_flag);
+}
+
+constexpr int kQ6Slot = 240;  // bytes of a Q6_K block in a stage: 15 x 16, an odd number, so that the rows of a warp spread over all banks
+
 // ---- host: tensor maps ----
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -244,6 +270,21 @@ inline bool encode_q4k_rows(CUtensorMap *map, const void *w, int bpr, size_t row
     const cuuint64_t dims[3] = {static_cast<cuuint64_t>(bpr) * kQ4KBlock, rows, static_cast<cuuint64_t>(mats)};
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(bpr) * kQ4KBlock, mat_stride};
     const cuuint32_t box[3] = {kQ4KBlock, static_cast<cuuint32_t>(box_rows), 1}, estr[3] = {1, 1, 1};
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, mat_stride ? 3 : 2, const_cast<void *>(w), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Q6_K: rows of 210-byte blocks have no stride a tensor map can take, but 1, 2, 4 or 8 rows together are a multiple of 16 bytes. Row j of
+// every such group is a box of its own, from the last multiple of 16 before its block: all of the box's rows are off by the same bytes.
+inline int q6k_group(int bpr) { return bpr % 8 == 0 ? 1 : bpr % 4 == 0 ? 2 : bpr % 2 == 0 ? 4 : 8; }
+inline bool encode_q6k_groups(CUtensorMap *map, const void *w, int bpr, int group, int rows, int mats, size_t mat_stride, int box_rows)
+{
+    EncodeTiledFn enc = encode_tiled();
+    if (!enc) return false;
+    const cuuint64_t bytes = static_cast<cuuint64_t>(bpr) * kQ6KBlock * group;
+    const cuuint64_t dims[3] = {bytes, static_cast<cuuint64_t>(rows / group), static_cast<cuuint64_t>(mats)}, strides[2] = {bytes, mat_stride};
+    const cuuint32_t box[3] = {kQ6Slot, static_cast<cuuint32_t>(box_rows / group), 1}, estr[3] = {1, 1, 1};
     return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, mat_stride ? 3 : 2, const_cast<void *>(w), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;

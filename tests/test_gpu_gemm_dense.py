@@ -44,3 +44,25 @@ def test_every_form(K, kind, M, N, Kd):
         assert rel.max() <= 1e-3, (pdl, rel.max())
     assert bool((guard[M * N:] == 7.0).all())
     assert K.mb200_device_error() == 0
+
+
+@pytest.mark.parametrize("kind,M,N,Kd", [("q6k", 1, 104, 256), ("q6k", 3, 100, 256), ("q6k", 17, 132, 512), ("q6k", 17, 130, 512),
+                                         ("q6k", 33, 258, 1024), ("q6k", 65, 701, 2048), ("q6k", 16, 104, 768), ("q6k", 33, 104, 1280),
+                                         ("q6k", 64, 104, 1536), ("q6k", 200, 1000, 1536), ("q4k", 16, 100, 768), ("q4k", 33, 100, 1280),
+                                         ("q4k", 64, 100, 1536), ("q4k", 130, 1500, 1536)])
+def test_rows_in_groups_and_splits(K, kind, M, N, Kd):
+    """Q6_K on 16-byte addresses, where 8, 4, 2 or 1 rows at a time make a tensor map (K / 256 odd, 2, 4, 8), and with rows left over
+    of that, which go the other way; K shared by 3, 5 and 6 CTAs. The bound is the one above (weights rounded to fp16 once: 2.8e-4)."""
+    gen, ref, call = ((synth.q4k_matrix, oracle.gemm_q4k_f16, K.mb200_gemm_q4k_f16) if kind == "q4k" else
+                      (synth.q6k_matrix, oracle.gemm_q6k_f16, K.mb200_gemm_q6k_f16))
+    w = gen(2800 + N, N, Kd)
+    x = synth.normal_f16(2801 + M, M * Kd).reshape(M, Kd)
+    want = ref(w, x, M, N, Kd).astype(np.float64)
+    guard = torch.full((M * N + 64,), 7.0, device="cuda")
+    out = guard[:M * N].view(M, N)
+    out.fill_(float("nan"))
+    call(dev(w), dev(x), out, M, N, Kd)
+    rel = np.linalg.norm(host(out).astype(np.float64) - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert rel.max() <= 1e-3, rel.max()
+    assert bool((guard[M * N:] == 7.0).all())
+    assert K.mb200_device_error() == 0
