@@ -22,8 +22,27 @@ using stream::Params;
 
 }  // namespace
 
-void q4k_init() { stream::init_attrs<Q4>(); }
+void q4k_mma_init();
+bool matvec_q4k_mma(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream, const char *where);
+
+void q4k_init()
+{
+    stream::init_attrs<Q4>();
+    q4k_mma_init();
+}
 int pdl_enabled() { return stream::pdl_mode(); }
+
+// The streaming form for every width: its sums have the order of the one-launch decode step's, which the layer-by-layer step repeats.
+void q4k_matvec(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream)
+{
+    Params P{};
+    P.seg[0] = {static_cast<const uint8_t *>(weights), y, n_rows, 0};
+    P.nseg = 1;
+    P.x = x;
+    P.n_cols = n_cols;
+    P.mode = stream::kStore;
+    stream::launch<Q4>(P, stream, "cuda_matvec_q4k");
+}
 
 // Two Q4_K tensors of different heights that share x, one launch (the decode path's Q and K projections;
 // the reference's three-tensor form, cuda_matvec_q4k_qkv, needs V to be Q4_K too, which Q4_K_M files are not).
@@ -97,13 +116,8 @@ extern "C" {
 void cuda_matvec_q4k(const void *weights, const float *x, float *y, int n_rows, int n_cols,
                      cudaStream_t stream)
 {
-    Params P{};
-    P.seg[0] = {static_cast<const uint8_t *>(weights), y, n_rows, 0};
-    P.nseg = 1;
-    P.x = x;
-    P.n_cols = n_cols;
-    P.mode = stream::kStore;
-    stream::launch<Q4>(P, stream, "cuda_matvec_q4k");
+    if (!matvec_q4k_mma(weights, x, y, n_rows, n_cols, stream, "cuda_matvec_q4k"))
+        q4k_matvec(weights, x, y, n_rows, n_cols, stream);
 }
 
 void cuda_matvec_q4k_add(const void *weights, const float *x, const float *residual, float *y,

@@ -1,0 +1,380 @@
+// Q4_K matvec y = W x on the integer tensor path (mma.sync m16n8k32, u8 x s8 -> s32), for rows of whole super-blocks up to
+// 4096 columns; the streaming kernel (stream_matvec.cuh) has the rest.
+//
+// Arithmetic as there (q4k_policy.cuh): x is split once per CTA into two int8 levels per 32 columns, the dot products of the
+// nibbles with both levels are exact integers, and they are scaled in fp32. What differs is who multiplies. An MMA takes 16
+// rows x 32 bytes of nibbles; its eight result columns are four sub-blocks x two levels: B holds a sub-block's levels in its
+// two columns, at the k of its nibbles, and zeros elsewhere, so four MMAs into the same accumulators leave each lane both
+// levels of one sub-block of two rows, which is what it then scales. 16 rows of a super-block take 8 MMAs and 150 other
+// instructions, the streaming kernel's dp4a two times 205; the launch's fixed work is smaller too.
+//
+// What bounds it: in a chain of launches, the way from one y to the next x: of 6.1 us at 8192 x 4096, 0.65 from the end of the
+// grid to the next one's wait, 1.3 for x and its levels, 0.5 a stage of 14 rows (a warp's own chain of loads, MMAs and scaling),
+// 0.35 for the last sums; the weights arrive meanwhile. So a CTA whose weights fit takes at most half of an SM (113 KB of
+// shared memory, 112 registers a thread): under programmatic dependent launch the next launch's CTA starts beside it and
+// has its weights in shared memory when y is done. Chains of 16 launches against the streaming kernel: 8192 x 4096 8.1 -> 6.1 us,
+// 4096 x 4096 6.4 -> 4.1, 6144 x 2048 5.1 -> 3.7, 512 x 2048 3.7 -> 2.7, 50000 x 4096 26.5 -> 20.0 (5.7 TB/s);
+// no size of 1 to 50000 rows was slower, with or without dependent launches, and the error against 64 bits is the same.
+// Beyond 4096 columns a warp's levels no longer stay in its registers: 1000 x 16384 took 8.7 us and more against 8.4.
+//
+// Stages: whole rows, one bulk copy each (a copy per row costs the requesting warp 60 ns a row); a warp takes 16 rows of one
+// or two super-block columns, the last warp requests the stages and adds the columns' sums in ascending order.
+#include "q4k_policy.cuh"
+#include "tcgen.cuh"
+
+namespace mb200 {
+namespace {
+
+constexpr int kWarps = 8, kMvThreads = (kWarps + 1) * 32, kXThreads = kWarps * 32;
+constexpr int kXCols = 128 / kWarps;  // columns of x a thread splits: 4096 in a round
+constexpr int kMvStages = 6;
+constexpr int kMvMaxCols = 2 * kWarps * 256;
+constexpr int kHalfSm = 113 * 1024, kWholeSm = 226 * 1024;  // half: (228 KB - 2 x 1 KB) / 2
+constexpr int kHalfTiles = 3;        // a CTA with more stages than these takes the whole SM
+// x comes in behind whatever weights its SM has asked for before: 97 KB of them cost it 0.7 us. So of a ring in the whole SM
+// no more than kAheadBytes are requested before x is here, and the next launch starts when it is (4096 x 4096: 5.1 us with the
+// next launch at once, 4.4 so), unless the launch is so small that starting the next one is what takes its time
+// (512 x 2048, 4.6 KB a CTA: 2.67 at once, 3.04 with x; 2048 x 1536, 12 KB: 2.68, 2.76; 4096 x 2304, 36 KB: 4.04, 3.99).
+constexpr int kAheadBytes = 80 * 1024, kEarlyBytes = 20 * 1024;
+
+struct MvArgs {
+    const uint8_t *w;
+    const float *x;
+    float *y;
+    int per, rem;  // rows / CTAs, rows % CTAs
+    int bpr;       // super-blocks of a row
+    int cols;      // warps side by side on a row: warp column c takes super-blocks c and c + cols
+    int rows;      // rows of a stage, at most 16 per warp of a column
+    int stages;
+    int ahead;     // stages requested before x is here
+    int early;     // 1: the next launch may start at once
+    int odd;       // 1: lanes of odd rows start with the other half of a super-block
+    int pdl;
+    // shared memory: mbarriers, levels of x, scale per sub-block, sums of sub-blocks, sums of a stage [stage][column][row], stages
+    int s1, sum, part, stage0, stage_bytes, total;
+    int *err;
+};
+constexpr int kZero = 2 * kMvStages * 8, kX = kZero + 32;  // 16 zero bytes; the levels of x
+constexpr int kXBlock = 8 * 64 + 4 * 64;                    // of a super-block: [sub-block][level][32], and those of even sub-blocks negated
+
+__device__ __forceinline__ void imma(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1)
+{
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// A lane's share of one row: sub-blocks t and t + 4, with the integers of both levels.
+struct XLane {
+    float k0, k1, sx0, sx1;  // scale / 254 (an odd sub-block's nibbles count sixteen times: / 16) and sum of x
+};
+__device__ __forceinline__ float scaled(float sc0, float m0, float sc1, float m1, uint32_t dd, int a0, int b0, int a1, int b1, const XLane &x)
+{
+    const float2 d = __half22float2(*reinterpret_cast<const __half2 *>(&dd));
+    float p = sc0 * (x.k0 * static_cast<float>(a0 * 254 + b0));
+    p = fmaf(sc1, x.k1 * static_cast<float>(a1 * 254 + b1), p);
+    return fmaf(d.x, p, -d.y * fmaf(m1, x.sx1, m0 * x.sx0));
+}
+__device__ __forceinline__ float byte_float(uint32_t v, int i)  // 2^23 + byte, less 2^23
+{
+    return __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440 + i)) - 8388608.0f;
+}
+
+// kXCols columns of x from c0 on -> two int8 levels, v ~= sc * (a + b / 254), where XFrag reads them
+__device__ __forceinline__ void split_x(const float (&v)[kXCols], int c0, bool valid, int lane, uint8_t *smem, const MvArgs &P)
+{
+    constexpr int kLanes = 32 / kXCols;  // of a sub-block
+    float amax = fabsf(v[0]), sum = v[0];
+#pragma unroll
+    for (int i = 1; i < kXCols; i++) {
+        amax = fmaxf(amax, fabsf(v[i]));
+        sum += v[i];
+    }
+#pragma unroll
+    for (int i = 1; i < kLanes; i *= 2) {
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, i));
+        sum += __shfl_xor_sync(0xffffffffu, sum, i);
+    }
+    const float sc = amax * (1.0f / 127.0f), inv = amax > 0.0f ? 127.0f / amax : 0.0f;
+    uint32_t p1[kXCols / 4], p2[kXCols / 4];
+#pragma unroll
+    for (int i = 0; i < kXCols / 4; i++) {
+        const float q[4] = {v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]};
+        stream::split_levels(q, sc, inv, p1[i], p2[i]);
+    }
+    if (!valid) return;
+    const int chunk = c0 >> 5;
+    uint8_t *to = smem + kX + (chunk >> 3) * kXBlock + (c0 & 31);
+#pragma unroll
+    for (int i = 0; i < kXCols / 8; i++) {
+        *reinterpret_cast<uint2 *>(to + (chunk & 7) * 64 + 8 * i) = make_uint2(p1[2 * i], p1[2 * i + 1]);
+        *reinterpret_cast<uint2 *>(to + (chunk & 7) * 64 + 32 + 8 * i) = make_uint2(p2[2 * i], p2[2 * i + 1]);
+        if (!(chunk & 1)) {
+            *reinterpret_cast<uint2 *>(to + 512 + (chunk & 6) * 32 + 8 * i) = make_uint2(__vneg4(p1[2 * i]), __vneg4(p1[2 * i + 1]));
+            *reinterpret_cast<uint2 *>(to + 512 + (chunk & 6) * 32 + 32 + 8 * i) = make_uint2(__vneg4(p2[2 * i]), __vneg4(p2[2 * i + 1]));
+        }
+    }
+    if (lane % kLanes == 0) {
+        reinterpret_cast<float *>(smem + P.s1)[chunk] = sc * ((chunk & 1) ? 1.0f / (254.0f * 16.0f) : 1.0f / 254.0f);
+        reinterpret_cast<float *>(smem + P.sum)[chunk] = sum;
+    }
+}
+
+// A lane's levels of one super-block: [half][8 bytes of the lane's 16][word]. The lane's k belong to sub-blocks j (low
+// nibbles) and j + 1 (high nibbles); only the columns of these sub-blocks' levels hold them.
+// low nibbles . x = bytes . x + high nibbles . (-x): one mask a word of weights.
+struct XFrag {
+    uint4 bytes[2], high[2];
+    XLane l;
+    __device__ __forceinline__ void load(const uint8_t *smem, const MvArgs &P, int sb, int g, int t)
+    {
+        const int j = 2 * (t >> 1), at = kX + sb * kXBlock + (g & 1) * 32 + (t & 1) * 16;
+        const bool is_lo = (g >> 1) == j, is_hi = (g >> 1) == j + 1;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            bytes[h] = *reinterpret_cast<const uint4 *>(smem + (is_lo ? at + (4 * h + j) * 64 : kZero));
+            high[h] = *reinterpret_cast<const uint4 *>(smem + (is_lo ? at + 512 + (4 * h + j) * 32 : is_hi ? at + (4 * h + j) * 64 + 64 : kZero));
+        }
+        const float *s1 = reinterpret_cast<const float *>(smem + P.s1) + sb * 8 + t, *xs = reinterpret_cast<const float *>(smem + P.sum) + sb * 8 + t;
+        l = {s1[0], s1[4], xs[0], xs[4]};
+    }
+};
+
+// The lane's part of 16 rows of one super-block: of rows g and g + 8.
+__device__ __forceinline__ void dot16(const uint8_t *pa, const uint8_t *pb, int t, bool turned, const XFrag &x, float &va, float &vb)
+{
+    // 64 bytes of a row over its four lanes; with rows a multiple of 128 bytes apart, the odd ones the other 64 first
+    const int o = 16 + 16 * t + (turned ? 64 : 0), o1 = 16 + 16 * t + (turned ? 0 : 64);
+    const uint4 a0 = *reinterpret_cast<const uint4 *>(pa + o), b0 = *reinterpret_cast<const uint4 *>(pb + o);
+    const uint4 a1 = *reinterpret_cast<const uint4 *>(pa + o1), b1 = *reinterpret_cast<const uint4 *>(pb + o1);
+    const uint4 ha = *reinterpret_cast<const uint4 *>(pa), hb = *reinterpret_cast<const uint4 *>(pb);
+    int c[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    constexpr uint32_t kHi = 0xF0F0F0F0u;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const uint4 u = (h == 0) != turned ? a0 : a1, v = (h == 0) != turned ? b0 : b1;
+        imma(c[h], u.x, v.x, u.y, v.y, x.bytes[h].x, x.bytes[h].y);
+        imma(c[h], u.x & kHi, v.x & kHi, u.y & kHi, v.y & kHi, x.high[h].x, x.high[h].y);
+        imma(c[h], u.z, v.z, u.w, v.w, x.bytes[h].z, x.bytes[h].w);
+        imma(c[h], u.z & kHi, v.z & kHi, u.w & kHi, v.w & kHi, x.high[h].z, x.high[h].w);
+    }
+    // scales and mins of sub-blocks t and t + 4 of both rows side by side: [scale, min] of row g, [scale, min] of row g + 8
+    const uint32_t q = __byte_perm(__byte_perm(ha.y, ha.z, 0x40 + 0x11 * t), __byte_perm(hb.y, hb.z, 0x40 + 0x11 * t), 0x5410);
+    const uint32_t w = __byte_perm(ha.w, hb.w, 0x4400 + 0x1111 * t);
+    const uint32_t s0 = q & 0x3F3F3F3Fu, s1 = ((q >> 2) & 0x30303030u) | (__byte_perm(w, w >> 4, 0x7250) & 0x0F0F0F0Fu);
+    va = scaled(byte_float(s0, 0), byte_float(s0, 1), byte_float(s1, 0), byte_float(s1, 1), ha.x, c[0][0], c[0][1], c[1][0], c[1][1], x.l);
+    vb = scaled(byte_float(s0, 2), byte_float(s0, 3), byte_float(s1, 2), byte_float(s1, 3), hb.x, c[0][2], c[0][3], c[1][2], c[1][3], x.l);
+}
+
+// NB: super-blocks a warp takes side by side (1 where a row has no more than the warps)
+template <int NB>
+__global__ void __launch_bounds__(kMvThreads, 2) matvec_q4k_mma_kernel(const __grid_constant__ MvArgs P)
+{
+    extern __shared__ __align__(128) uint8_t smem[];
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + kMvStages;
+    float *part = reinterpret_cast<float *>(smem + P.part);
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    const int cta = blockIdx.x;
+    const int first = cta * P.per + min(cta, P.rem), n_rows = P.per + (cta < P.rem ? 1 : 0);
+    const int S = P.stages, pitch = P.bpr * kQ4KBlock;
+
+    if (warp == kWarps) {
+        // ---- requests the stages, adds up their sums ----
+        const uint32_t row_bytes = P.bpr * kQ4KBlock;
+        const uint8_t *w = P.w + (size_t)first * row_bytes;
+        const bool leader = elect_lane();
+        int req = 0;  // rows requested
+        auto request = [&](int slot) {
+            const int rows = min(P.rows, n_rows - req);
+            if (leader) {
+                mbar_expect_tx(&full[slot], rows * row_bytes);
+                bulk_g2s(smem + P.stage0 + slot * P.stage_bytes, w + (size_t)req * row_bytes, rows * row_bytes, &full[slot]);
+            }
+            req += rows;
+        };
+        if (lane == 0) {
+            *reinterpret_cast<uint4 *>(smem + kZero) = make_uint4(0u, 0u, 0u, 0u);
+            for (int s = 0; s < S; s++) {
+                mbar_init(&full[s], 1);
+                mbar_init(&empty[s], kWarps);
+            }
+            mbar_fence_init();
+        }
+        if (P.pdl && P.early) stream::grid_dep_launch();
+        for (int s = 0; s < P.ahead && req < n_rows; s++) request(s);
+        __syncthreads();
+        for (int s = P.ahead; s < S && req < n_rows; s++) request(s);
+        if (P.pdl) stream::grid_dep_wait();  // y may still be in use by the upstream kernel
+        int slot = 0, phase = 0;
+        for (int row = 0; row < n_rows; row += P.rows) {
+            const int rows = min(P.rows, n_rows - row);
+            if (!mbar_wait(&empty[slot], phase)) {  // (a warp whose wait ran out has left: this one runs out too)
+                if (lane == 0) atomicExch(P.err, MB200_ERR_TIMEOUT);
+                return;
+            }
+            const float *pt = part + slot * P.cols * P.rows;
+            float *y = P.y + first + row;
+            for (int r = lane; r < rows; r += 32) {
+                float v = 0.0f;
+#pragma unroll 4
+                for (int c = 0; c < P.cols; c++) v += pt[c * P.rows + r];
+                y[r] = v;
+            }
+            __syncwarp();
+            if (req < n_rows) request(slot);
+            if (++slot == S) {
+                slot = 0;
+                phase ^= 1;
+            }
+        }
+        return;
+    }
+
+    // ---- the levels of x ----
+    if (P.pdl) {
+        // x may be cold; asked for here, it waits in the L2 for the upstream kernel's end
+        for (int c = threadIdx.x * 32; c < P.bpr * 256; c += kXThreads * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(P.x + c));
+        stream::grid_dep_wait();  // x is produced by the upstream kernel
+    }
+    {
+        const int K = P.bpr * 256;
+        const bool vec_ok = (reinterpret_cast<uintptr_t>(P.x) & 15) == 0;
+        bool told = !P.pdl || P.early || static_cast<int>(threadIdx.x) * kXCols >= K;
+        for (int c0 = threadIdx.x * kXCols; c0 - lane * kXCols < K; c0 += kXThreads * kXCols) {
+            float v[kXCols];
+#pragma unroll
+            for (int i = 0; i < kXCols; i += 4) {
+                float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (c0 < K) {
+                    if (vec_ok)
+                        q = __ldcg(reinterpret_cast<const float4 *>(P.x + c0 + i));
+                    else
+                        q = make_float4(__ldcg(P.x + c0 + i), __ldcg(P.x + c0 + i + 1), __ldcg(P.x + c0 + i + 2), __ldcg(P.x + c0 + i + 3));
+                }
+                v[i] = q.x, v[i + 1] = q.y, v[i + 2] = q.z, v[i + 3] = q.w;
+            }
+            if (!told && __float_as_uint(v[0]) != 0x7fc12345u) {  // (reads x: not before it has arrived)
+                told = true;
+                stream::grid_dep_launch();
+            }
+            split_x(v, c0, c0 < K, lane, smem, P);
+        }
+    }
+    __syncthreads();
+
+    // ---- products ----
+    const int g = lane >> 2, t = lane & 3;
+    int col = warp, tile = 0;  // the warp's column and its first row of a stage
+    while (col >= P.cols) {
+        col -= P.cols;
+        tile += 16;
+    }
+    const bool turned = P.odd & g & 1;
+    XFrag x[NB];
+    int at[NB];  // the warp's super-blocks in a row; a row's last ones may not go round
+#pragma unroll
+    for (int n = 0; n < NB; n++) {
+        const int sb = min(col + n * P.cols, P.bpr - 1);
+        x[n].load(smem, P, sb, g, t);
+        at[n] = sb * kQ4KBlock;
+    }
+    const bool both = col + (NB - 1) * P.cols < P.bpr;
+    int slot = 0, phase = 0;
+    for (int row = 0; row < n_rows; row += P.rows) {
+        const int left = min(P.rows, n_rows - row) - tile;  // rows from the warp's first on
+        if (!mbar_wait(&full[slot], phase)) return;
+        if (left > 0) {
+            const uint8_t *st = smem + P.stage0 + slot * P.stage_bytes + tile * pitch;
+            const uint8_t *ra = st + min(g, left - 1) * pitch, *rb = st + min(g + 8, left - 1) * pitch;
+            float va[NB], vb[NB];
+#pragma unroll
+            for (int n = 0; n < NB; n++) dot16(ra + at[n], rb + at[n], t, turned, x[n], va[n], vb[n]);
+            if (NB == 2 && both) {
+                va[0] += va[NB - 1];
+                vb[0] += vb[NB - 1];
+            }
+            // sub-blocks of a row over four lanes: even lanes go on with row g, odd lanes with row g + 8
+            float v = ((t & 1) ? vb[0] : va[0]) + __shfl_xor_sync(0xffffffffu, (t & 1) ? va[0] : vb[0], 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            const int r = tile + g + 8 * t;
+            if (t < 2 && r < P.rows) part[(slot * P.cols + col) * P.rows + r] = v;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[slot]);
+        if (++slot == S) {
+            slot = 0;
+            phase ^= 1;
+        }
+    }
+}
+
+// The shared memory of `stages` stages of `rows` rows
+int fit(MvArgs &P, int rows, int stages)
+{
+    P.rows = rows;
+    P.stages = stages;
+    P.s1 = kX + P.bpr * kXBlock;
+    P.sum = P.s1 + P.bpr * 32;
+    P.part = P.sum + P.bpr * 32;
+    P.stage0 = (P.part + stages * P.cols * rows * 4 + 127) & ~127;
+    P.stage_bytes = rows * P.bpr * kQ4KBlock;
+    P.total = P.stage0 + stages * P.stage_bytes;
+    return P.total;
+}
+
+}  // namespace
+
+void q4k_mma_init()
+{
+    static bool done[kMaxDevices] = {false};
+    const int dev = current_device();
+    if (done[dev]) return;
+    cudaFuncSetAttribute(matvec_q4k_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+    cudaFuncSetAttribute(matvec_q4k_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+    done[dev] = true;
+}
+
+bool matvec_q4k_mma(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream, const char *where)
+{
+    if (n_rows < 1 || n_cols < 256 || n_cols % 256 || n_cols > kMvMaxCols /* a warp's levels stay in registers */ || (reinterpret_cast<uintptr_t>(weights) & 15)) return false;
+    q4k_mma_init();
+    MvArgs P{};
+    P.w = static_cast<const uint8_t *>(weights);
+    P.x = x;
+    P.y = y;
+    P.bpr = n_cols / 256;
+    const int nb = P.bpr <= kWarps ? 1 : 2;
+    P.cols = (P.bpr + nb - 1) / nb;
+    P.odd = P.bpr % 8 == 0;
+    const int sms = device_sms(), grid = n_rows < sms ? n_rows : sms;
+    P.per = n_rows / grid;
+    P.rem = n_rows % grid;
+    // As few stages of the same size as fit: all of them in half an SM, or a ring in the whole of it. (8192 x 4096, 56 rows a
+    // CTA: 7.0 us with three of four stages in half an SM, where the fourth comes behind the next launch's; 6.1 in the whole.)
+    const int rows = P.per + (P.rem ? 1 : 0), most = kWarps / P.cols * 16, tiles = (rows + most - 1) / most;
+    if (tiles > kHalfTiles || fit(P, (rows + tiles - 1) / tiles, tiles) > kHalfSm) {
+        int s = kMvStages;
+        while (fit(P, most, s) > kWholeSm) s--;
+        for (int n = tiles; fit(P, (rows + n - 1) / n, n < s ? n : s) > kWholeSm;) n++;
+    }
+    P.ahead = P.total <= kHalfSm ? P.stages : kAheadBytes / P.stage_bytes;
+    P.early = rows * P.bpr * kQ4KBlock <= kEarlyBytes;
+    P.pdl = stream::pdl_mode();
+    P.err = device_error_word();
+
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kMvThreads);
+    cfg.dynamicSmemBytes = P.total;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = P.pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, nb == 1 ? matvec_q4k_mma_kernel<1> : matvec_q4k_mma_kernel<2>, P);
+    MB200_CHECK_LAUNCH(where);
+    return true;
+}
+
+}  // namespace mb200

@@ -392,3 +392,36 @@ def test_activation_levels_are_rounded_products(K):
         y = torch.empty(256, device="cuda")
         K.cuda_matvec_q4k(dev(w.reshape(-1)), dev(x), y, 256, 256)
         assert np.array_equal(host(y), want)
+
+
+@pytest.mark.parametrize("pdl", [False, True])
+@pytest.mark.parametrize("rows,cols", [
+    (1, 256), (147, 256), (149, 256), (2, 1792),             # one row a CTA or fewer, one super-block, seven
+    (148 * 16, 2048), (148 * 16 + 1, 2048), (5 * 148, 4096),  # a whole tile of 16 rows, one more row
+    (4800, 1024), (3000, 768), (148 * 48 + 5, 2304),          # several tiles a stage, idle warps, an odd number of super-blocks
+    (148 * 42, 4096), (148 * 43, 4096), (148 * 14 * 6 + 3, 4096),  # the last that fits half an SM, the first ring, slots reused
+    (148 * 200, 512), (20000, 3840),
+])
+def test_matvec_q4k_on_the_tensor_path(K, rows, cols, pdl):
+    """Whole super-blocks up to 4096 columns against fp64 and against the streaming kernel (which the form with a residual
+    takes). Both forms split x alike, add exact integers and round a few fp32 terms per super-block: their distance is at most
+    twice the error that the tolerance against fp64 allows either."""
+    w, x = synth.q4k_matrix(11 + rows, min(rows, 4000), cols), synth.normal_f32(12 + cols, cols + 1)
+    w = np.tile(w.reshape(-1), -(-rows // 4000))[: rows * cols // 256 * 144] if rows > 4000 else w
+    wd, xd = dev(w), dev(x)
+    y, ys = torch.full((rows + 1,), 5.0, device="cuda"), torch.empty(rows, device="cuda")
+    before = K.mb200_set_pdl(pdl)
+    try:
+        for shift in (0, 1):  # x on a 16-byte boundary and off it
+            K.cuda_matvec_q4k(wd, xd[shift:], y, rows, cols)
+            K.cuda_matvec_q4k(wd, xd[shift:], y, rows, cols)  # beside the launch before it
+            K.cuda_matvec_q4k_add(wd, xd[shift:], torch.zeros(rows, device="cuda"), ys, rows, cols)
+            some = np.unique(np.r_[0:min(rows, 200), max(rows - 200, 0):rows])
+            blocks = np.asarray(w).reshape(rows, -1)[some].reshape(-1)
+            _, y64, ad = oracle.matvec_q4k(blocks, x[shift: shift + cols], len(some), cols, full=True)
+            assert_close_matvec(host(y)[some], y64, ad, f"q4k {rows}x{cols}")
+            a, b = host(y)[:rows].astype(np.float64), host(ys).astype(np.float64)
+            assert np.linalg.norm(a - b) <= 2e-3 * np.linalg.norm(b) and float(y[rows]) == 5.0
+            assert np.abs(a - b).max() <= 1e-4 * np.abs(b).max()  # two levels: 1.6e-5 of a group's largest |x|, each form
+    finally:
+        K.mb200_set_pdl(before)
