@@ -1,5 +1,5 @@
 // Q4_K matvec y = W x on the integer tensor path (mma.sync m16n8k32, u8 x s8 -> s32), for rows of whole super-blocks up to
-// 4096 columns; the streaming kernel (stream_matvec.cuh) has the rest.
+// 8192 columns; the streaming kernel (stream_matvec.cuh) has the rest.
 //
 // Arithmetic as there (q4k_policy.cuh): x is split once per CTA into two int8 levels per 32 columns, the dot products of the
 // nibbles with both levels are exact integers, and they are scaled in fp32. What differs is who multiplies. An MMA takes 16
@@ -15,10 +15,12 @@
 // has its weights in shared memory when y is done. Chains of 16 launches against the streaming kernel: 8192 x 4096 8.1 -> 6.1 us,
 // 4096 x 4096 6.4 -> 4.1, 6144 x 2048 5.1 -> 3.7, 512 x 2048 3.7 -> 2.7, 50000 x 4096 26.5 -> 20.0 (5.7 TB/s);
 // no size of 1 to 50000 rows was slower, with or without dependent launches, and the error against 64 bits is the same.
-// Beyond 4096 columns a warp's levels no longer stay in its registers: 1000 x 16384 took 8.7 us and more against 8.4.
+// Up to 4096 columns a warp keeps the levels of its one or two super-blocks in registers with two CTAs on an SM; with three
+// or four, up to 8192, a CTA needs the SM's registers for itself: 4096 x 8192 9.3 -> 6.8 us, 2000 x 6144 5.9 -> 5.1. With six
+// (4096 x 12288: 12.3 us against 12.0) and with levels read again for each stage (1000 x 16384: 8.7 against 8.4) it is no faster.
 //
 // Stages: whole rows, one bulk copy each (a copy per row costs the requesting warp 60 ns a row); a warp takes 16 rows of one
-// or two super-block columns, the last warp requests the stages and adds the columns' sums in ascending order.
+// to four super-block columns, the last warp requests the stages and adds the columns' sums in ascending order.
 #include "q4k_policy.cuh"
 #include "tcgen.cuh"
 
@@ -28,7 +30,7 @@ namespace {
 constexpr int kWarps = 8, kMvThreads = (kWarps + 1) * 32, kXThreads = kWarps * 32;
 constexpr int kXCols = 128 / kWarps;  // columns of x a thread splits: 4096 in a round
 constexpr int kMvStages = 6;
-constexpr int kMvMaxCols = 2 * kWarps * 256;
+constexpr int kMvMaxCols = 4 * kWarps * 256;
 constexpr int kHalfSm = 113 * 1024, kWholeSm = 226 * 1024;  // half: (228 KB - 2 x 1 KB) / 2
 constexpr int kHalfTiles = 3;        // a CTA with more stages than these takes the whole SM
 // x comes in behind whatever weights its SM has asked for before: 97 KB of them cost it 0.7 us. So of a ring in the whole SM
@@ -43,7 +45,7 @@ struct MvArgs {
     float *y;
     int per, rem;  // rows / CTAs, rows % CTAs
     int bpr;       // super-blocks of a row
-    int cols;      // warps side by side on a row: warp column c takes super-blocks c and c + cols
+    int cols;      // warps side by side on a row: warp column c takes super-blocks c, c + cols, ...
     int rows;      // rows of a stage, at most 16 per warp of a column
     int stages;
     int ahead;     // stages requested before x is here
@@ -166,9 +168,9 @@ __device__ __forceinline__ void dot16(const uint8_t *pa, const uint8_t *pb, int 
     vb = scaled(byte_float(s0, 2), byte_float(s0, 3), byte_float(s1, 2), byte_float(s1, 3), hb.x, c[0][2], c[0][3], c[1][2], c[1][3], x.l);
 }
 
-// NB: super-blocks a warp takes side by side (1 where a row has no more than the warps)
+// NB: super-blocks a warp takes side by side
 template <int NB>
-__global__ void __launch_bounds__(kMvThreads, 2) matvec_q4k_mma_kernel(const __grid_constant__ MvArgs P)
+__global__ void __launch_bounds__(kMvThreads, NB <= 2 ? 2 : 1) matvec_q4k_mma_kernel(const __grid_constant__ MvArgs P)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + kMvStages;
@@ -270,6 +272,7 @@ __global__ void __launch_bounds__(kMvThreads, 2) matvec_q4k_mma_kernel(const __g
         tile += 16;
     }
     const bool turned = P.odd & g & 1;
+    const bool all = col + (NB - 1) * P.cols < P.bpr;
     XFrag x[NB];
     int at[NB];  // the warp's super-blocks in a row; a row's last ones may not go round
 #pragma unroll
@@ -278,7 +281,6 @@ __global__ void __launch_bounds__(kMvThreads, 2) matvec_q4k_mma_kernel(const __g
         x[n].load(smem, P, sb, g, t);
         at[n] = sb * kQ4KBlock;
     }
-    const bool both = col + (NB - 1) * P.cols < P.bpr;
     int slot = 0, phase = 0;
     for (int row = 0; row < n_rows; row += P.rows) {
         const int left = min(P.rows, n_rows - row) - tile;  // rows from the warp's first on
@@ -289,10 +291,12 @@ __global__ void __launch_bounds__(kMvThreads, 2) matvec_q4k_mma_kernel(const __g
             float va[NB], vb[NB];
 #pragma unroll
             for (int n = 0; n < NB; n++) dot16(ra + at[n], rb + at[n], t, turned, x[n], va[n], vb[n]);
-            if (NB == 2 && both) {
-                va[0] += va[NB - 1];
-                vb[0] += vb[NB - 1];
-            }
+#pragma unroll
+            for (int n = 1; n < NB; n++)
+                if (n + 1 < NB || all) {
+                    va[0] += va[n];
+                    vb[0] += vb[n];
+                }
             // sub-blocks of a row over four lanes: even lanes go on with row g, odd lanes with row g + 8
             float v = ((t & 1) ? vb[0] : va[0]) + __shfl_xor_sync(0xffffffffu, (t & 1) ? va[0] : vb[0], 1);
             v += __shfl_xor_sync(0xffffffffu, v, 2);
@@ -331,19 +335,24 @@ void q4k_mma_init()
     if (done[dev]) return;
     cudaFuncSetAttribute(matvec_q4k_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
     cudaFuncSetAttribute(matvec_q4k_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+    cudaFuncSetAttribute(matvec_q4k_mma_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+    cudaFuncSetAttribute(matvec_q4k_mma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
     done[dev] = true;
 }
 
 bool matvec_q4k_mma(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream, const char *where)
 {
-    if (n_rows < 1 || n_cols < 256 || n_cols % 256 || n_cols > kMvMaxCols /* a warp's levels stay in registers */ || (reinterpret_cast<uintptr_t>(weights) & 15)) return false;
+    if (n_rows < 1 || n_cols < 256 || n_cols % 256 || n_cols > kMvMaxCols || (reinterpret_cast<uintptr_t>(weights) & 15)) return false;
+    // Of wide rows a few per CTA are no better here, with a CTA to an SM: 100 x 4352 4.3 us against 4.0, 500 x 6144 4.8 against
+    // 4.6, but 1025 x 5120 4.4 against 5.0.
+    if (n_cols > 2 * kWarps * 256 && n_rows < 4 * device_sms()) return false;
     q4k_mma_init();
     MvArgs P{};
     P.w = static_cast<const uint8_t *>(weights);
     P.x = x;
     P.y = y;
     P.bpr = n_cols / 256;
-    const int nb = P.bpr <= kWarps ? 1 : 2;
+    const int nb = P.bpr <= kWarps ? 1 : P.bpr <= 2 * kWarps ? 2 : P.bpr <= 3 * kWarps ? 3 : 4;
     P.cols = (P.bpr + nb - 1) / nb;
     P.odd = P.bpr % 8 == 0;
     const int sms = device_sms(), grid = n_rows < sms ? n_rows : sms;
@@ -352,12 +361,12 @@ bool matvec_q4k_mma(const void *weights, const float *x, float *y, int n_rows, i
     // As few stages of the same size as fit: all of them in half an SM, or a ring in the whole of it. (8192 x 4096, 56 rows a
     // CTA: 7.0 us with three of four stages in half an SM, where the fourth comes behind the next launch's; 6.1 in the whole.)
     const int rows = P.per + (P.rem ? 1 : 0), most = kWarps / P.cols * 16, tiles = (rows + most - 1) / most;
-    if (tiles > kHalfTiles || fit(P, (rows + tiles - 1) / tiles, tiles) > kHalfSm) {
+    if (nb > 2 || tiles > kHalfTiles || fit(P, (rows + tiles - 1) / tiles, tiles) > kHalfSm) {
         int s = kMvStages;
-        while (fit(P, most, s) > kWholeSm) s--;
+        while (s > 3 && fit(P, most, s) > kWholeSm) s--;
         for (int n = tiles; fit(P, (rows + n - 1) / n, n < s ? n : s) > kWholeSm;) n++;
     }
-    P.ahead = P.total <= kHalfSm ? P.stages : kAheadBytes / P.stage_bytes;
+    P.ahead = P.total <= kHalfSm ? P.stages : P.stage_bytes > kAheadBytes ? 1 : kAheadBytes / P.stage_bytes;
     P.early = rows * P.bpr * kQ4KBlock <= kEarlyBytes;
     P.pdl = stream::pdl_mode();
     P.err = device_error_word();
@@ -372,7 +381,7 @@ bool matvec_q4k_mma(const void *weights, const float *x, float *y, int n_rows, i
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = P.pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, nb == 1 ? matvec_q4k_mma_kernel<1> : matvec_q4k_mma_kernel<2>, P);
+    cudaLaunchKernelEx(&cfg, nb == 1 ? matvec_q4k_mma_kernel<1> : nb == 2 ? matvec_q4k_mma_kernel<2> : nb == 3 ? matvec_q4k_mma_kernel<3> : matvec_q4k_mma_kernel<4>, P);
     MB200_CHECK_LAUNCH(where);
     return true;
 }

@@ -401,9 +401,10 @@ def test_activation_levels_are_rounded_products(K):
     (4800, 1024), (3000, 768), (148 * 48 + 5, 2304),          # several tiles a stage, idle warps, an odd number of super-blocks
     (148 * 42, 4096), (148 * 43, 4096), (148 * 14 * 6 + 3, 4096),  # the last that fits half an SM, the first ring, slots reused
     (148 * 200, 512), (20000, 3840),
+    (592, 4352), (700, 6144), (148 * 30 + 1, 6400), (5000, 8192),  # three and four super-blocks a warp
 ])
 def test_matvec_q4k_on_the_tensor_path(K, rows, cols, pdl):
-    """Whole super-blocks up to 4096 columns against fp64 and against the streaming kernel (which the form with a residual
+    """Whole super-blocks up to 8192 columns against fp64 and against the streaming kernel (which the form with a residual
     takes). Both forms split x alike, add exact integers and round a few fp32 terms per super-block: their distance is at most
     twice the error that the tolerance against fp64 allows either."""
     w, x = synth.q4k_matrix(11 + rows, min(rows, 4000), cols), synth.normal_f32(12 + cols, cols + 1)
