@@ -26,6 +26,7 @@ void qkv_q4k_q6k(const void *wq, float *q, int q_rows, const void *wk, float *k,
 void q4k_matvec2(const void *wa, float *ya, int rows_a, const void *wb, float *yb, int rows_b, const float *x,
                  int n_cols, cudaStream_t stream, const char *where, const float *norm_w, float norm_eps);
 void q4k_matvec(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream);
+void q5k_matvec(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream);
 int moe_fused_mode();
 
 namespace {
@@ -104,7 +105,7 @@ int matvec(const void *w, int type, const float *x, float *y, int rows, int cols
         case 14: cuda_matvec_q6k(w, x, y, rows, cols, s); return MB200_OK;
         case 8: cuda_matvec_q8_0(w, x, y, rows, cols, s); return MB200_OK;
         case 11: cuda_matvec_q3k(w, x, y, rows, cols, s); return MB200_OK;
-        case 13: cuda_matvec_q5k(w, x, y, rows, cols, s); return MB200_OK;
+        case 13: q5k_matvec(w, x, y, rows, cols, s); return MB200_OK;
         default: return MB200_ERR_UNSUPPORTED;
     }
 }

@@ -1,4 +1,4 @@
-// Q4_K matvec y = W x on the integer tensor path (mma.sync m16n8k32, u8 x s8 -> s32), for rows of whole super-blocks up to
+// Q4_K and Q5_K matvecs y = W x on the integer tensor path (mma.sync m16n8k32, u8 x s8 -> s32), for rows of whole super-blocks up to
 // 8192 columns; the streaming kernel (stream_matvec.cuh) has the rest.
 //
 // Arithmetic as there (q4k_policy.cuh): x is split once per CTA into two int8 levels per 32 columns, the dot products of the
@@ -18,6 +18,8 @@
 // Up to 4096 columns a warp keeps the levels of its one or two super-blocks in registers with two CTAs on an SM; with three
 // or four, up to 8192, a CTA needs the SM's registers for itself: 4096 x 8192 9.3 -> 6.8 us, 2000 x 6144 5.9 -> 5.1. With six
 // (4096 x 12288: 12.3 us against 12.0) and with levels read again for each stage (1000 x 16384: 8.7 against 8.4) it is no faster.
+// Q5_K, with 160 instructions more a unit to put the fifth bits in their places: 8192 x 4096 10.1 -> 8.3 us, 512 x 2048 3.8 -> 2.8,
+// 5461 x 2816 6.7 -> 6.2, 30000 x 4096 21.0 -> 18.7.
 //
 // Stages: whole rows, one bulk copy each (a copy per row costs the requesting warp 60 ns a row); a warp takes 16 rows of one
 // to four super-block columns, the last warp requests the stages and adds the columns' sums in ascending order.
@@ -38,6 +40,16 @@ constexpr int kHalfTiles = 3;        // a CTA with more stages than these takes 
 // next launch at once, 4.4 so), unless the launch is so small that starting the next one is what takes its time
 // (512 x 2048, 4.6 KB a CTA: 2.67 at once, 3.04 with x; 2048 x 1536, 12 KB: 2.68, 2.76; 4096 x 2304, 36 KB: 4.04, 3.99).
 constexpr int kAheadBytes = 80 * 1024, kEarlyBytes = 20 * 1024;
+
+// Q4_K and Q5_K: a block's d, dmin and scales, Q5_K's fifth bits, the nibbles
+struct T4 {
+    static constexpr int kBlock = kQ4KBlock, kQs = 16, kWideRows = 4;
+    static constexpr bool kFifth = false;
+};
+struct T5 {
+    static constexpr int kBlock = 176, kQs = 48, kWideRows = 6;
+    static constexpr bool kFifth = true;
+};
 
 struct MvArgs {
     const uint8_t *w;
@@ -68,7 +80,7 @@ __device__ __forceinline__ void imma(int (&c)[4], uint32_t a0, uint32_t a1, uint
 
 // A lane's share of one row: sub-blocks t and t + 4, with the integers of both levels.
 struct XLane {
-    float k0, k1, sx0, sx1;  // scale / 254 (an odd sub-block's nibbles count sixteen times: / 16) and sum of x
+    float k0, k1, sx0, sx1;  // scale / 254 (Q4_K: an odd sub-block's nibbles count sixteen times: / 16) and sum of x
 };
 __device__ __forceinline__ float scaled(float sc0, float m0, float sc1, float m1, uint32_t dd, int a0, int b0, int a1, int b1, const XLane &x)
 {
@@ -83,6 +95,7 @@ __device__ __forceinline__ float byte_float(uint32_t v, int i)  // 2^23 + byte, 
 }
 
 // kXCols columns of x from c0 on -> two int8 levels, v ~= sc * (a + b / 254), where XFrag reads them
+template <class T>
 __device__ __forceinline__ void split_x(const float (&v)[kXCols], int c0, bool valid, int lane, uint8_t *smem, const MvArgs &P)
 {
     constexpr int kLanes = 32 / kXCols;  // of a sub-block
@@ -111,22 +124,23 @@ __device__ __forceinline__ void split_x(const float (&v)[kXCols], int c0, bool v
     for (int i = 0; i < kXCols / 8; i++) {
         *reinterpret_cast<uint2 *>(to + (chunk & 7) * 64 + 8 * i) = make_uint2(p1[2 * i], p1[2 * i + 1]);
         *reinterpret_cast<uint2 *>(to + (chunk & 7) * 64 + 32 + 8 * i) = make_uint2(p2[2 * i], p2[2 * i + 1]);
-        if (!(chunk & 1)) {
+        if (!T::kFifth && !(chunk & 1)) {
             *reinterpret_cast<uint2 *>(to + 512 + (chunk & 6) * 32 + 8 * i) = make_uint2(__vneg4(p1[2 * i]), __vneg4(p1[2 * i + 1]));
             *reinterpret_cast<uint2 *>(to + 512 + (chunk & 6) * 32 + 32 + 8 * i) = make_uint2(__vneg4(p2[2 * i]), __vneg4(p2[2 * i + 1]));
         }
     }
     if (lane % kLanes == 0) {
-        reinterpret_cast<float *>(smem + P.s1)[chunk] = sc * ((chunk & 1) ? 1.0f / (254.0f * 16.0f) : 1.0f / 254.0f);
+        reinterpret_cast<float *>(smem + P.s1)[chunk] = sc * (!T::kFifth && (chunk & 1) ? 1.0f / (254.0f * 16.0f) : 1.0f / 254.0f);
         reinterpret_cast<float *>(smem + P.sum)[chunk] = sum;
     }
 }
 
 // A lane's levels of one super-block: [half][8 bytes of the lane's 16][word]. The lane's k belong to sub-blocks j (low
 // nibbles) and j + 1 (high nibbles); only the columns of these sub-blocks' levels hold them.
-// low nibbles . x = bytes . x + high nibbles . (-x): one mask a word of weights.
+// Q4_K: low nibbles . x = bytes . x + high nibbles . (-x): one mask a word of weights.
+template <class T>
 struct XFrag {
-    uint4 bytes[2], high[2];
+    uint4 low[2], high[2];
     XLane l;
     __device__ __forceinline__ void load(const uint8_t *smem, const MvArgs &P, int sb, int g, int t)
     {
@@ -134,19 +148,28 @@ struct XFrag {
         const bool is_lo = (g >> 1) == j, is_hi = (g >> 1) == j + 1;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            bytes[h] = *reinterpret_cast<const uint4 *>(smem + (is_lo ? at + (4 * h + j) * 64 : kZero));
-            high[h] = *reinterpret_cast<const uint4 *>(smem + (is_lo ? at + 512 + (4 * h + j) * 32 : is_hi ? at + (4 * h + j) * 64 + 64 : kZero));
+            low[h] = *reinterpret_cast<const uint4 *>(smem + (is_lo ? at + (4 * h + j) * 64 : kZero));
+            high[h] = *reinterpret_cast<const uint4 *>(smem + (!T::kFifth && is_lo ? at + 512 + (4 * h + j) * 32 : is_hi ? at + (4 * h + j) * 64 + 64 : kZero));
         }
         const float *s1 = reinterpret_cast<const float *>(smem + P.s1) + sb * 8 + t, *xs = reinterpret_cast<const float *>(smem + P.sum) + sb * 8 + t;
         l = {s1[0], s1[4], xs[0], xs[4]};
     }
 };
 
+// four nibbles and, from bit i of `bits` on, their fifth bits
+__device__ __forceinline__ uint32_t five(uint32_t w, uint32_t bits, int i)
+{
+    // (a multiplication spreads them: bit k of four goes to bit 8 k + 4)
+    const uint32_t m = i & 4 ? ((bits >> (i & 8)) & 0xF0u) * 0x00204081u : ((bits >> (i & 8)) & 0xFu) * 0x02040810u;
+    return (w & 0x0F0F0F0Fu) | (m & 0x10101010u);
+}
+
 // The lane's part of 16 rows of one super-block: of rows g and g + 8.
-__device__ __forceinline__ void dot16(const uint8_t *pa, const uint8_t *pb, int t, bool turned, const XFrag &x, float &va, float &vb)
+template <class T>
+__device__ __forceinline__ void dot16(const uint8_t *pa, const uint8_t *pb, int t, bool turned, const XFrag<T> &x, float &va, float &vb)
 {
     // 64 bytes of a row over its four lanes; with rows a multiple of 128 bytes apart, the odd ones the other 64 first
-    const int o = 16 + 16 * t + (turned ? 64 : 0), o1 = 16 + 16 * t + (turned ? 0 : 64);
+    const int o = T::kQs + 16 * t + (turned ? 64 : 0), o1 = T::kQs + 16 * t + (turned ? 0 : 64);
     const uint4 a0 = *reinterpret_cast<const uint4 *>(pa + o), b0 = *reinterpret_cast<const uint4 *>(pb + o);
     const uint4 a1 = *reinterpret_cast<const uint4 *>(pa + o1), b1 = *reinterpret_cast<const uint4 *>(pb + o1);
     const uint4 ha = *reinterpret_cast<const uint4 *>(pa), hb = *reinterpret_cast<const uint4 *>(pb);
@@ -155,10 +178,20 @@ __device__ __forceinline__ void dot16(const uint8_t *pa, const uint8_t *pb, int 
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const uint4 u = (h == 0) != turned ? a0 : a1, v = (h == 0) != turned ? b0 : b1;
-        imma(c[h], u.x, v.x, u.y, v.y, x.bytes[h].x, x.bytes[h].y);
-        imma(c[h], u.x & kHi, v.x & kHi, u.y & kHi, v.y & kHi, x.high[h].x, x.high[h].y);
-        imma(c[h], u.z, v.z, u.w, v.w, x.bytes[h].z, x.bytes[h].w);
-        imma(c[h], u.z & kHi, v.z & kHi, u.w & kHi, v.w & kHi, x.high[h].z, x.high[h].w);
+        if (T::kFifth) {
+            const uint2 fa = *reinterpret_cast<const uint2 *>(pa + 16 + 16 * h + 8 * (t >> 1)), fb = *reinterpret_cast<const uint2 *>(pb + 16 + 16 * h + 8 * (t >> 1));
+            const int sh = 16 * (t & 1);
+            const uint32_t al = fa.x >> sh, ah = fa.y >> sh, bl = fb.x >> sh, bh = fb.y >> sh;
+            imma(c[h], five(u.x, al, 0), five(v.x, bl, 0), five(u.y, al, 4), five(v.y, bl, 4), x.low[h].x, x.low[h].y);
+            imma(c[h], five(u.x >> 4, ah, 0), five(v.x >> 4, bh, 0), five(u.y >> 4, ah, 4), five(v.y >> 4, bh, 4), x.high[h].x, x.high[h].y);
+            imma(c[h], five(u.z, al, 8), five(v.z, bl, 8), five(u.w, al, 12), five(v.w, bl, 12), x.low[h].z, x.low[h].w);
+            imma(c[h], five(u.z >> 4, ah, 8), five(v.z >> 4, bh, 8), five(u.w >> 4, ah, 12), five(v.w >> 4, bh, 12), x.high[h].z, x.high[h].w);
+        } else {
+            imma(c[h], u.x, v.x, u.y, v.y, x.low[h].x, x.low[h].y);
+            imma(c[h], u.x & kHi, v.x & kHi, u.y & kHi, v.y & kHi, x.high[h].x, x.high[h].y);
+            imma(c[h], u.z, v.z, u.w, v.w, x.low[h].z, x.low[h].w);
+            imma(c[h], u.z & kHi, v.z & kHi, u.w & kHi, v.w & kHi, x.high[h].z, x.high[h].w);
+        }
     }
     // scales and mins of sub-blocks t and t + 4 of both rows side by side: [scale, min] of row g, [scale, min] of row g + 8
     const uint32_t q = __byte_perm(__byte_perm(ha.y, ha.z, 0x40 + 0x11 * t), __byte_perm(hb.y, hb.z, 0x40 + 0x11 * t), 0x5410);
@@ -169,8 +202,8 @@ __device__ __forceinline__ void dot16(const uint8_t *pa, const uint8_t *pb, int 
 }
 
 // NB: super-blocks a warp takes side by side
-template <int NB>
-__global__ void __launch_bounds__(kMvThreads, NB <= 2 ? 2 : 1) matvec_q4k_mma_kernel(const __grid_constant__ MvArgs P)
+template <class T, int NB>
+__global__ void __launch_bounds__(kMvThreads, NB <= 2 ? 2 : 1) matvec_mma_kernel(const __grid_constant__ MvArgs P)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + kMvStages;
@@ -178,11 +211,11 @@ __global__ void __launch_bounds__(kMvThreads, NB <= 2 ? 2 : 1) matvec_q4k_mma_ke
     const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
     const int cta = blockIdx.x;
     const int first = cta * P.per + min(cta, P.rem), n_rows = P.per + (cta < P.rem ? 1 : 0);
-    const int S = P.stages, pitch = P.bpr * kQ4KBlock;
+    const int S = P.stages, pitch = P.bpr * T::kBlock;
 
     if (warp == kWarps) {
         // ---- requests the stages, adds up their sums ----
-        const uint32_t row_bytes = P.bpr * kQ4KBlock;
+        const uint32_t row_bytes = P.bpr * T::kBlock;
         const uint8_t *w = P.w + (size_t)first * row_bytes;
         const bool leader = elect_lane();
         int req = 0;  // rows requested
@@ -259,7 +292,7 @@ __global__ void __launch_bounds__(kMvThreads, NB <= 2 ? 2 : 1) matvec_q4k_mma_ke
                 told = true;
                 stream::grid_dep_launch();
             }
-            split_x(v, c0, c0 < K, lane, smem, P);
+            split_x<T>(v, c0, c0 < K, lane, smem, P);
         }
     }
     __syncthreads();
@@ -273,13 +306,13 @@ __global__ void __launch_bounds__(kMvThreads, NB <= 2 ? 2 : 1) matvec_q4k_mma_ke
     }
     const bool turned = P.odd & g & 1;
     const bool all = col + (NB - 1) * P.cols < P.bpr;
-    XFrag x[NB];
+    XFrag<T> x[NB];
     int at[NB];  // the warp's super-blocks in a row; a row's last ones may not go round
 #pragma unroll
     for (int n = 0; n < NB; n++) {
         const int sb = min(col + n * P.cols, P.bpr - 1);
         x[n].load(smem, P, sb, g, t);
-        at[n] = sb * kQ4KBlock;
+        at[n] = sb * T::kBlock;
     }
     int slot = 0, phase = 0;
     for (int row = 0; row < n_rows; row += P.rows) {
@@ -290,7 +323,7 @@ __global__ void __launch_bounds__(kMvThreads, NB <= 2 ? 2 : 1) matvec_q4k_mma_ke
             const uint8_t *ra = st + min(g, left - 1) * pitch, *rb = st + min(g + 8, left - 1) * pitch;
             float va[NB], vb[NB];
 #pragma unroll
-            for (int n = 0; n < NB; n++) dot16(ra + at[n], rb + at[n], t, turned, x[n], va[n], vb[n]);
+            for (int n = 0; n < NB; n++) dot16<T>(ra + at[n], rb + at[n], t, turned, x[n], va[n], vb[n]);
 #pragma unroll
             for (int n = 1; n < NB; n++)
                 if (n + 1 < NB || all) {
@@ -312,8 +345,8 @@ __global__ void __launch_bounds__(kMvThreads, NB <= 2 ? 2 : 1) matvec_q4k_mma_ke
     }
 }
 
-// The shared memory of `stages` stages of `rows` rows
-int fit(MvArgs &P, int rows, int stages)
+// The shared memory of `stages` stages of `rows` rows of `row_bytes`
+int fit(MvArgs &P, int row_bytes, int rows, int stages)
 {
     P.rows = rows;
     P.stages = stages;
@@ -321,32 +354,42 @@ int fit(MvArgs &P, int rows, int stages)
     P.sum = P.s1 + P.bpr * 32;
     P.part = P.sum + P.bpr * 32;
     P.stage0 = (P.part + stages * P.cols * rows * 4 + 127) & ~127;
-    P.stage_bytes = rows * P.bpr * kQ4KBlock;
+    P.stage_bytes = rows * row_bytes;
     P.total = P.stage0 + stages * P.stage_bytes;
     return P.total;
 }
 
+template <class T>
+void init()
+{
+    cudaFuncSetAttribute(matvec_mma_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+    cudaFuncSetAttribute(matvec_mma_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+    cudaFuncSetAttribute(matvec_mma_kernel<T, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+    cudaFuncSetAttribute(matvec_mma_kernel<T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+}
+
 }  // namespace
 
-void q4k_mma_init()
+void matvec_mma_init()
 {
     static bool done[kMaxDevices] = {false};
     const int dev = current_device();
     if (done[dev]) return;
-    cudaFuncSetAttribute(matvec_q4k_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
-    cudaFuncSetAttribute(matvec_q4k_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
-    cudaFuncSetAttribute(matvec_q4k_mma_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
-    cudaFuncSetAttribute(matvec_q4k_mma_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWholeSm);
+    init<T4>();
+    init<T5>();
     done[dev] = true;
 }
 
-bool matvec_q4k_mma(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream, const char *where)
+namespace {
+
+template <class T>
+bool launch(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream, const char *where)
 {
     if (n_rows < 1 || n_cols < 256 || n_cols % 256 || n_cols > kMvMaxCols || (reinterpret_cast<uintptr_t>(weights) & 15)) return false;
     // Of wide rows a few per CTA are no better here, with a CTA to an SM: 100 x 4352 4.3 us against 4.0, 500 x 6144 4.8 against
-    // 4.6, but 1025 x 5120 4.4 against 5.0.
-    if (n_cols > 2 * kWarps * 256 && n_rows < 4 * device_sms()) return false;
-    q4k_mma_init();
+    // 4.6, but 1025 x 5120 4.4 against 5.0 (Q5_K: 592 x 4352 5.0 against 4.3, 1025 x 5120 5.1 against 5.3).
+    if (n_cols > 2 * kWarps * 256 && n_rows < T::kWideRows * device_sms()) return false;
+    matvec_mma_init();
     MvArgs P{};
     P.w = static_cast<const uint8_t *>(weights);
     P.x = x;
@@ -354,20 +397,21 @@ bool matvec_q4k_mma(const void *weights, const float *x, float *y, int n_rows, i
     P.bpr = n_cols / 256;
     const int nb = P.bpr <= kWarps ? 1 : P.bpr <= 2 * kWarps ? 2 : P.bpr <= 3 * kWarps ? 3 : 4;
     P.cols = (P.bpr + nb - 1) / nb;
-    P.odd = P.bpr % 8 == 0;
+    const int row_bytes = P.bpr * T::kBlock;
+    P.odd = row_bytes % 128 == 0;
     const int sms = device_sms(), grid = n_rows < sms ? n_rows : sms;
     P.per = n_rows / grid;
     P.rem = n_rows % grid;
     // As few stages of the same size as fit: all of them in half an SM, or a ring in the whole of it. (8192 x 4096, 56 rows a
     // CTA: 7.0 us with three of four stages in half an SM, where the fourth comes behind the next launch's; 6.1 in the whole.)
     const int rows = P.per + (P.rem ? 1 : 0), most = kWarps / P.cols * 16, tiles = (rows + most - 1) / most;
-    if (nb > 2 || tiles > kHalfTiles || fit(P, (rows + tiles - 1) / tiles, tiles) > kHalfSm) {
+    if (nb > 2 || tiles > kHalfTiles || fit(P, row_bytes, (rows + tiles - 1) / tiles, tiles) > kHalfSm) {
         int s = kMvStages;
-        while (s > 3 && fit(P, most, s) > kWholeSm) s--;
-        for (int n = tiles; fit(P, (rows + n - 1) / n, n < s ? n : s) > kWholeSm;) n++;
+        while (s > 3 && fit(P, row_bytes, most, s) > kWholeSm) s--;
+        for (int n = tiles; fit(P, row_bytes, (rows + n - 1) / n, n < s ? n : s) > kWholeSm;) n++;
     }
     P.ahead = P.total <= kHalfSm ? P.stages : P.stage_bytes > kAheadBytes ? 1 : kAheadBytes / P.stage_bytes;
-    P.early = rows * P.bpr * kQ4KBlock <= kEarlyBytes;
+    P.early = rows * row_bytes <= kEarlyBytes;
     P.pdl = stream::pdl_mode();
     P.err = device_error_word();
 
@@ -381,9 +425,20 @@ bool matvec_q4k_mma(const void *weights, const float *x, float *y, int n_rows, i
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = P.pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, nb == 1 ? matvec_q4k_mma_kernel<1> : nb == 2 ? matvec_q4k_mma_kernel<2> : nb == 3 ? matvec_q4k_mma_kernel<3> : matvec_q4k_mma_kernel<4>, P);
+    cudaLaunchKernelEx(&cfg, nb == 1 ? matvec_mma_kernel<T, 1> : nb == 2 ? matvec_mma_kernel<T, 2> : nb == 3 ? matvec_mma_kernel<T, 3> : matvec_mma_kernel<T, 4>, P);
     MB200_CHECK_LAUNCH(where);
     return true;
+}
+
+}  // namespace
+
+bool matvec_q4k_mma(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream, const char *where)
+{
+    return launch<T4>(weights, x, y, n_rows, n_cols, stream, where);
+}
+bool matvec_q5k_mma(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream, const char *where)
+{
+    return launch<T5>(weights, x, y, n_rows, n_cols, stream, where);
 }
 
 }  // namespace mb200

@@ -1,5 +1,5 @@
 // Q8_0 / Q5_K / Q3_K matvecs on the streaming skeleton (other_policies.cuh): for whole 256-column blocks and
-// tensors at the type's alignment. Ragged widths and odd addresses take the row-per-warp kernels of other_types.cu.
+// tensors at the type's alignment (most sizes of Q5_K go to matvec_mma.cu). Ragged widths and odd addresses take the row-per-warp kernels of other_types.cu.
 #include "other_policies.cuh"
 
 namespace mb200 {

@@ -1,7 +1,7 @@
 // Q4_K dequant-matvec family for decode (batch 1), sm_100a: every Q4_K entry
 // point of the reference kernel ABI (plain / +residual / QKV / dual / scaled-add)
 // plus the gate+up+SwiGLU fusion, on the streaming skeleton of
-// stream_matvec.cuh; most sizes of the plain form go to matvec_q4k_mma.cu.
+// stream_matvec.cuh; most sizes of the plain form go to matvec_mma.cu.
 //
 // Arithmetic: the activation vector is split once per CTA into two int8 levels
 // per 32-column group, x ~= s*(q1 + q2/254). Nibbles are masked four at a time
@@ -22,13 +22,13 @@ using stream::Params;
 
 }  // namespace
 
-void q4k_mma_init();
+void matvec_mma_init();
 bool matvec_q4k_mma(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream, const char *where);
 
 void q4k_init()
 {
     stream::init_attrs<Q4>();
-    q4k_mma_init();
+    matvec_mma_init();
 }
 int pdl_enabled() { return stream::pdl_mode(); }
 

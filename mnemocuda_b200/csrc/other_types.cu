@@ -338,6 +338,15 @@ void launch_embed_q3k(const void *table, float *out, const int *token_ptr, int t
              token_ptr, token, hidden, row_bytes);
 }
 
+bool matvec_q5k_mma(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream, const char *where);
+
+// The forms for every width, whose order of sums the decode step keeps
+void q5k_matvec(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream)
+{
+    if (n_rows > 0 && stream_matvec_q5k(weights, x, y, n_rows, n_cols, stream)) return;
+    typed_matvec<Q5K>(weights, x, y, n_rows, n_cols, stream, "cuda_matvec_q5k");
+}
+
 }  // namespace mb200
 
 using namespace mb200;
@@ -352,8 +361,7 @@ void cuda_matvec_q8_0(const void *weights, const float *x, float *y, int n_rows,
 
 void cuda_matvec_q5k(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream)
 {
-    if (n_rows > 0 && stream_matvec_q5k(weights, x, y, n_rows, n_cols, stream)) return;
-    typed_matvec<Q5K>(weights, x, y, n_rows, n_cols, stream, "cuda_matvec_q5k");
+    if (!matvec_q5k_mma(weights, x, y, n_rows, n_cols, stream, "cuda_matvec_q5k")) q5k_matvec(weights, x, y, n_rows, n_cols, stream);
 }
 
 void cuda_matvec_q3k(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream)

@@ -52,6 +52,27 @@ def test_typed_matvec_at_an_odd_address(K, tid, name):
     assert_close_matvec(host(y), y64, ad, name)
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 256), (149, 2048), (148 * 16 + 1, 1792), (5461, 2816), (3000, 768), (148 * 33 + 2, 4096),
+                                       (148 * 6, 4352), (148 * 20 + 3, 6400), (900, 8192)])
+def test_q5k_on_the_tensor_path(K, rows, cols):
+    """Tiles with a row more or less, idle warps, one to four super-blocks a warp, a ring whose slots are used again; x off its
+    16-byte boundary and launches that start beside one another give the same bits."""
+    w, x = synth.typed_matrix(13, 40 + rows, rows, cols), synth.normal_f32(41 + cols, cols + 1)
+    _, y64, ad = oracle.matvec_type(13, w, x[1:], rows, cols, full=True)
+    y = torch.full((3, rows + 1), 5.0, device="cuda")
+    wd, xd = dev(w), dev(x)
+    K.cuda_matvec_q5k(wd, xd[1:], y[0], rows, cols)
+    K.cuda_matvec_q5k(wd, xd[1:].clone(), y[1], rows, cols)
+    before = K.mb200_set_pdl(True)
+    try:
+        for _ in range(3):
+            K.cuda_matvec_q5k(wd, xd[1:], y[2], rows, cols)
+    finally:
+        K.mb200_set_pdl(before)
+    assert_close_matvec(host(y[0][:rows]), y64, ad, f"q5k {rows}x{cols}")
+    assert torch.equal(y[0], y[1]) and torch.equal(y[0], y[2]) and bool((y[:, rows] == 5.0).all())
+
+
 @pytest.mark.parametrize("cols", [512, 300])
 def test_typed_matvec_one_hot_x_reads_single_weights(K, cols):
     """x = e_c picks weight c of every row: a direct check of the unpacking of each bit field, in the streaming
