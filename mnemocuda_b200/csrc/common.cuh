@@ -138,6 +138,10 @@ __device__ __forceinline__ void bulk_g2s(void *dst_smem, const void *src_gmem, u
         : "memory");
 }
 
+// Byte i of v as a float: 2^23 + byte, less 2^23. A byte permute and an addition, where the conversion of a byte runs at a
+// quarter of their rate.
+__device__ __forceinline__ float byte_float(uint32_t v, int i) { return __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440 + i)) - 8388608.0f; }
+
 // ---- Q4_K scale/min pair decode (reference src/kernels.cu:45-53) -------------
 // a,b,c = the three little-endian words of scales[12]; g = 0..3 selects
 // sub-blocks (2g, 2g+1). Returns sc pair / m pair packed as two bytes each.

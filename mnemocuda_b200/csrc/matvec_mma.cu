@@ -89,11 +89,6 @@ __device__ __forceinline__ float scaled(float sc0, float m0, float sc1, float m1
     p = fmaf(sc1, x.k1 * static_cast<float>(a1 * 254 + b1), p);
     return fmaf(d.x, p, -d.y * fmaf(m1, x.sx1, m0 * x.sx0));
 }
-__device__ __forceinline__ float byte_float(uint32_t v, int i)  // 2^23 + byte, less 2^23
-{
-    return __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440 + i)) - 8388608.0f;
-}
-
 // kXCols columns of x from c0 on -> two int8 levels, v ~= sc * (a + b / 254), where XFrag reads them
 template <class T>
 __device__ __forceinline__ void split_x(const float (&v)[kXCols], int c0, bool valid, int lane, uint8_t *smem, const MvArgs &P)

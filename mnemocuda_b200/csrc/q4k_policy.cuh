@@ -77,16 +77,19 @@ struct Q4 {
             i1h = dp4a_us(hi, xr.q1[8 + i], i1h);
             i2h = dp4a_us(hi, xr.q2[8 + i], i2h);
         }
-        uint32_t sc2, m2;
-        q4k_scale_pair(hdr.y, hdr.z, hdr.w, g, sc2, m2);
+        // Scales and mins of the two sub-blocks as the bytes of one word, and floats by byte_float(): half the instructions that
+        // shifts, masks and conversions of each took (the one-launch decode step 1780 -> 1750 us at the 30B shape).
+        const uint32_t sel = 0x5410u + 0x2222u * (g & 1);
+        const uint32_t q6 = __byte_perm(hdr.y, hdr.z, sel), w4 = __byte_perm(hdr.w, hdr.w >> 4, sel);
+        const uint32_t sm = g < 2 ? q6 & 0x3F3F3F3Fu : ((q6 >> 2) & 0x30303030u) | (w4 & 0x0F0F0F0Fu);
         const float2 dd = __half22float2(*reinterpret_cast<const __half2 *>(&hdr.x));
         const float d = dd.x, dmin = dd.y;
         const float il = static_cast<float>(i1l * 254 + i2l);
         const float ih = static_cast<float>(i1h * 254 + i2h);
-        float p = static_cast<float>(sc2 & 0xFFu) * (xr.kl * il);
-        p = fmaf(static_cast<float>(sc2 >> 8), xr.kh * ih, p);
-        float q = static_cast<float>(m2 & 0xFFu) * xr.sxl;
-        q = fmaf(static_cast<float>(m2 >> 8), xr.sxh, q);
+        float p = byte_float(sm, 0) * (xr.kl * il);
+        p = fmaf(byte_float(sm, 1), xr.kh * ih, p);
+        float q = byte_float(sm, 2) * xr.sxl;
+        q = fmaf(byte_float(sm, 3), xr.sxh, q);
         return fmaf(d, p, -dmin * q);
     }
 };

@@ -19,23 +19,23 @@ namespace mb200 {
 namespace {
 
 // 16 bytes starting at any byte address in shared memory -> four words
-__device__ __forceinline__ void lds16(const uint8_t *p, uint32_t (&w)[4])
+// (base: the address rounded down to four bytes, sh: eight times the remainder)
+__device__ __forceinline__ void lds16(uint32_t base, uint32_t sh, uint32_t (&w)[4])
 {
-    const uint32_t a = smem_u32(p);
-    const uint32_t base = a & ~3u;
-    const uint32_t sh = (a & 3u) * 8u;
     uint32_t t[5];
 #pragma unroll
     for (int i = 0; i < 5; i++) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(t[i]) : "r"(base + 4 * i));
 #pragma unroll
     for (int i = 0; i < 4; i++) w[i] = __funnelshift_r(t[i], t[i + 1], sh);
 }
-// 8 bytes -> two words
-__device__ __forceinline__ void lds8(const uint8_t *p, uint32_t &w0, uint32_t &w1)
+__device__ __forceinline__ void lds16(const uint8_t *p, uint32_t (&w)[4])
 {
     const uint32_t a = smem_u32(p);
-    const uint32_t base = a & ~3u;
-    const uint32_t sh = (a & 3u) * 8u;
+    lds16(a & ~3u, (a & 3u) * 8u, w);
+}
+// 8 bytes -> two words
+__device__ __forceinline__ void lds8(uint32_t base, uint32_t sh, uint32_t &w0, uint32_t &w1)
+{
     uint32_t a0, a1, a2;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(a0) : "r"(base));
     asm volatile("ld.shared.u32 %0, [%1+4];" : "=r"(a1) : "r"(base));
@@ -96,12 +96,13 @@ struct Q6 {
     {
         const int hh = sub >> 1, jj = sub & 1;
         uint32_t A[4], B[4], H[4], S[2];
-        lds16(blk + 64 * hh + 16 * jj, A);
-        lds16(blk + 64 * hh + 32 + 16 * jj, B);
-        lds16(blk + 128 + 32 * hh + 16 * jj, H);
-        lds8(blk + 192 + 8 * hh, S[0], S[1]);
+        const uint32_t at = smem_u32(blk), base = at & ~3u, sh = (at & 3u) * 8u;  // the parts lie four bytes apart or more
+        lds16(base + 64 * hh + 16 * jj, sh, A);
+        lds16(base + 64 * hh + 32 + 16 * jj, sh, B);
+        lds16(base + 128 + 32 * hh + 16 * jj, sh, H);
+        lds8(base + 192 + 8 * hh, sh, S[0], S[1]);
         unsigned short d_bits;
-        asm volatile("ld.shared.u16 %0, [%1+208];" : "=h"(d_bits) : "r"(smem_u32(blk)));
+        asm volatile("ld.shared.u16 %0, [%1+208];" : "=h"(d_bits) : "r"(at));
         const float d = __half2float(__ushort_as_half(d_bits));
 
         int i1[4] = {0, 0, 0, 0}, i2[4] = {0, 0, 0, 0};
@@ -123,11 +124,11 @@ struct Q6 {
             i2[3] = dp4a_us(q3, xr.q2[12 + i], i2[3]);
         }
         // scales[8hh + 2g + jj], g = 0..3: bytes jj + {0,2,4,6} of the 8 loaded
-        const uint32_t sh = jj * 8;
-        const int sc0 = static_cast<int8_t>((S[0] >> sh) & 0xFF);
-        const int sc1 = static_cast<int8_t>((S[0] >> (sh + 16)) & 0xFF);
-        const int sc2 = static_cast<int8_t>((S[1] >> sh) & 0xFF);
-        const int sc3 = static_cast<int8_t>((S[1] >> (sh + 16)) & 0xFF);
+        const uint32_t sj = jj * 8;
+        const int sc0 = static_cast<int8_t>((S[0] >> sj) & 0xFF);
+        const int sc1 = static_cast<int8_t>((S[0] >> (sj + 16)) & 0xFF);
+        const int sc2 = static_cast<int8_t>((S[1] >> sj) & 0xFF);
+        const int sc3 = static_cast<int8_t>((S[1] >> (sj + 16)) & 0xFF);
         float acc;
         acc = static_cast<float>(sc0) * fmaf(xr.k[0], static_cast<float>(i1[0] * 254 + i2[0]), -xr.sx32[0]);
         acc = fmaf(static_cast<float>(sc1), fmaf(xr.k[1], static_cast<float>(i1[1] * 254 + i2[1]), -xr.sx32[1]), acc);
