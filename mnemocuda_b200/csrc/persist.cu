@@ -33,8 +33,9 @@
 // several rows per warp in flight instead, thread_id() and cta_id() read anew by every step, and the launch's
 // parameters, divisions already done, in shared memory.
 //
-// Measured, per token: 30B shape at position 4095 (48 layers) 1769 us, 8 layers of the 235B shape at 8191 669 us (layer by layer
-// 3276 / 931); a layer is 35 / 67.5 us. Where a layer's time goes, by clock stamps of warp 0, mean over CTAs and layers, 30B / 235B:
+// Measured, per token: 30B shape at position 4095 (48 layers) 1716 us, 8 layers of the 235B shape at 8191 639 us (layer by layer
+// 3276 / 931; 1763 / 661 before the dot products took their scales by byte permutes). Where a layer's time goes, by clock stamps of
+// warp 0, mean over CTAs and layers, 30B / 235B, taken before that change, when a layer was 35 / 67.5 us (now 34 / 65):
 //   waits for the operation's input (its slowest writer, and 1 us from a store to its readers)   7.8 / 13.6 us
 //   norm, router logit, split into levels                                                        4.3 /  6.0
 //   selection, with the exchange of the logits                                                   2.0 /  1.9
