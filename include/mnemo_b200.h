@@ -49,7 +49,10 @@ extern "C" {
  * called by the engine at load (src/engine.c:1203-1207). Safe to call more than once. */
 void cuda_kernels_init(void);
 
-/* y = W x, W Q4_K [n_rows x n_cols]. Replaces src/kernels.cu:1071-1079 (kernel :66-145). */
+/* y = W x, W Q4_K [n_rows x n_cols]. Replaces src/kernels.cu:1071-1079 (kernel :66-145).
+ * Of this function, cuda_matvec_q5k and cuda_matvec_q6k a row's bits depend on the row, x and n_cols only, not on the other rows of
+ * the call: a tensor split by rows gives what the whole one gives. The forms below (residual, QKV, dual, scaled) and the decode step
+ * add a row's terms in another order than this one where n_cols is a multiple of 256 up to 8192: equal to rounding, not to the bit. */
 void cuda_matvec_q4k(const void *weights, const float *x, float *y, int n_rows, int n_cols,
                      cudaStream_t stream);
 

@@ -16,7 +16,8 @@
 // 4096 x 4096 6.4 -> 4.1, 6144 x 2048 5.1 -> 3.7, 512 x 2048 3.7 -> 2.7, 50000 x 4096 26.5 -> 20.0 (5.7 TB/s);
 // no size of 1 to 50000 rows was slower, with or without dependent launches, and the error against 64 bits is the same.
 // Up to 4096 columns a warp keeps the levels of its one or two super-blocks in registers with two CTAs on an SM; with three
-// or four, up to 8192, a CTA needs the SM's registers for itself: 4096 x 8192 9.3 -> 6.8 us, 2000 x 6144 5.9 -> 5.1. With six
+// or four, up to 8192, a CTA needs the SM's registers for itself and has all of x asked for before it splits any of it (in two rounds one
+// after the other 4096 x 8192 took 6.9 us, 512 x 8192 5.0): 4096 x 8192 9.6 -> 6.5 us, 2048 x 6144 6.1 -> 4.5, 512 x 8192 5.4 -> 4.6. With six
 // (4096 x 12288: 12.3 us against 12.0) and with levels read again for each stage (1000 x 16384: 8.7 against 8.4) it is no faster.
 // Q5_K, with 160 instructions more a unit to put the fifth bits in their places: 8192 x 4096 10.1 -> 8.3 us, 512 x 2048 3.8 -> 2.8,
 // 5461 x 2816 6.7 -> 6.2, 30000 x 4096 21.0 -> 18.7.
@@ -43,11 +44,11 @@ constexpr int kAheadBytes = 80 * 1024, kEarlyBytes = 20 * 1024;
 
 // Q4_K and Q5_K: a block's d, dmin and scales, Q5_K's fifth bits, the nibbles
 struct T4 {
-    static constexpr int kBlock = kQ4KBlock, kQs = 16, kWideRows = 4;
+    static constexpr int kBlock = kQ4KBlock, kQs = 16;
     static constexpr bool kFifth = false;
 };
 struct T5 {
-    static constexpr int kBlock = 176, kQs = 48, kWideRows = 6;
+    static constexpr int kBlock = 176, kQs = 48;
     static constexpr bool kFifth = true;
 };
 
@@ -269,26 +270,29 @@ __global__ void __launch_bounds__(kMvThreads, NB <= 2 ? 2 : 1) matvec_mma_kernel
     {
         const int K = P.bpr * 256;
         const bool vec_ok = (reinterpret_cast<uintptr_t>(P.x) & 15) == 0;
-        bool told = !P.pdl || P.early || static_cast<int>(threadIdx.x) * kXCols >= K;
-        for (int c0 = threadIdx.x * kXCols; c0 - lane * kXCols < K; c0 += kXThreads * kXCols) {
-            float v[kXCols];
+        constexpr int kRounds = NB <= 2 ? 1 : 2, kRound = kXThreads * kXCols;  // all of x is asked for before any of it is split
+        const int c0 = threadIdx.x * kXCols;
+        float v[kRounds][kXCols];
+#pragma unroll
+        for (int n = 0; n < kRounds; n++) {
+            const float *from = P.x + n * kRound + c0;
 #pragma unroll
             for (int i = 0; i < kXCols; i += 4) {
                 float4 q = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                if (c0 < K) {
+                if (n * kRound + c0 < K) {
                     if (vec_ok)
-                        q = __ldcg(reinterpret_cast<const float4 *>(P.x + c0 + i));
+                        q = __ldcg(reinterpret_cast<const float4 *>(from + i));
                     else
-                        q = make_float4(__ldcg(P.x + c0 + i), __ldcg(P.x + c0 + i + 1), __ldcg(P.x + c0 + i + 2), __ldcg(P.x + c0 + i + 3));
+                        q = make_float4(__ldcg(from + i), __ldcg(from + i + 1), __ldcg(from + i + 2), __ldcg(from + i + 3));
                 }
-                v[i] = q.x, v[i + 1] = q.y, v[i + 2] = q.z, v[i + 3] = q.w;
+                v[n][i] = q.x, v[n][i + 1] = q.y, v[n][i + 2] = q.z, v[n][i + 3] = q.w;
             }
-            if (!told && __float_as_uint(v[0]) != 0x7fc12345u) {  // (reads x: not before it has arrived)
-                told = true;
-                stream::grid_dep_launch();
-            }
-            split_x<T>(v, c0, c0 < K, lane, smem, P);
         }
+        // (reads x: not before it has arrived)
+        if (P.pdl && !P.early && c0 < K && __float_as_uint(v[0][0]) != 0x7fc12345u) stream::grid_dep_launch();
+#pragma unroll
+        for (int n = 0; n < kRounds; n++)
+            if (n * kRound + c0 - lane * kXCols < K) split_x<T>(v[n], n * kRound + c0, n * kRound + c0 < K, lane, smem, P);
     }
     __syncthreads();
 
@@ -381,9 +385,12 @@ template <class T>
 bool launch(const void *weights, const float *x, float *y, int n_rows, int n_cols, cudaStream_t stream, const char *where)
 {
     if (n_rows < 1 || n_cols < 256 || n_cols % 256 || n_cols > kMvMaxCols || (reinterpret_cast<uintptr_t>(weights) & 15)) return false;
-    // Of wide rows a few per CTA are no better here, with a CTA to an SM: 100 x 4352 4.3 us against 4.0, 500 x 6144 4.8 against
-    // 4.6, but 1025 x 5120 4.4 against 5.0 (Q5_K: 592 x 4352 5.0 against 4.3, 1025 x 5120 5.1 against 5.3).
-    if (n_cols > 2 * kWarps * 256 && n_rows < T::kWideRows * device_sms()) return false;
+    // By columns alone: the streaming kernel adds in another order, and a row's bits must not depend on how many rows the call has (a
+    // tensor split by rows over ranks gives what the whole one gives). Q4_K is faster here at every width for 700 rows or more and for fewer
+    // no slower but at 4352 columns (512 rows: 4.04 us against 3.93). Q5_K is slower at 4352 and 4608 columns (4.57 against 4.23, 20000
+    // rows 18.0 either way), where the streaming kernel splits x in one round; beyond it is 1.2 to 1.45 times as fast at 1024 to 4096 rows and,
+    // from 6400 columns on, up to 0.5 us slower below 300.
+    if (T::kFifth && n_cols > 2 * kWarps * 256 && n_cols <= 4608) return false;
     matvec_mma_init();
     MvArgs P{};
     P.w = static_cast<const uint8_t *>(weights);

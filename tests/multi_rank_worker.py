@@ -127,18 +127,19 @@ def main():
         assert torch.equal(out, first)
 
     # ---- row-sharded matvec + push all-gather ----
-    rows, cols = 8192, 4096
-    w = torch.empty(rows * (cols // 256) * 144, dtype=torch.uint8, device=dev)
-    K.mb200_fill_q4k(w, rows * cols // 256, 31)
-    rl, rh_ = sharded.row_range(rows, world, rank)
-    rb = (cols // 256) * 144
-    mv = sharded.RowShardedMatvec(w[rl * rb:rh_ * rb], rows, cols, rank, world, "q4k", comm)
-    y = torch.empty(rows, device=dev)
-    mv.forward(xh, y)
-    y_full = torch.empty(rows, device=dev)
-    K.cuda_matvec_q4k(w, xh, y_full, rows, cols)
-    torch.cuda.synchronize()
-    assert torch.equal(y, y_full)  # rows are computed independently: sharding does not change a bit
+    for rows, cols in ((8192, 4096), (4096, 8192)):
+        w = torch.empty(rows * (cols // 256) * 144, dtype=torch.uint8, device=dev)
+        K.mb200_fill_q4k(w, rows * cols // 256, 31)
+        rl, rh_ = sharded.row_range(rows, world, rank)
+        rb = (cols // 256) * 144
+        xw = torch.cat([xh, -0.5 * xh])[:cols].contiguous()
+        mv = sharded.RowShardedMatvec(w[rl * rb:rh_ * rb], rows, cols, rank, world, "q4k", comm)
+        y = torch.empty(rows, device=dev)
+        mv.forward(xw, y)
+        y_full = torch.empty(rows, device=dev)
+        K.cuda_matvec_q4k(w, xw, y_full, rows, cols)
+        torch.cuda.synchronize()
+        assert torch.equal(y, y_full)  # rows are computed independently: sharding does not change a bit
 
     # ---- whole-token decode, model sharded over the ranks, against the unsharded model on every rank ----
     from mnemocuda_b200.decode import DecodeConfig, ResidentModel

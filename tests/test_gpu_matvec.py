@@ -426,3 +426,21 @@ def test_matvec_q4k_on_the_tensor_path(K, rows, cols, pdl):
             assert np.abs(a - b).max() <= 1e-4 * np.abs(b).max()  # two levels: 1.6e-5 of a group's largest |x|, each form
     finally:
         K.mb200_set_pdl(before)
+
+
+@pytest.mark.parametrize("kind", ["q4k", "q5k", "q6k"])
+@pytest.mark.parametrize("cols", [2048, 4096, 4352, 4608, 4864, 6144, 6400, 8192, 8448, 12288])
+def test_bits_of_a_row_do_not_depend_on_the_rows_of_the_call(K, kind, cols):
+    """What splitting a tensor by rows over ranks relies on: the same rows in calls of 1024, 512, 128 and 1 rows, on either side of the widths
+    at which the plain form changes kernels."""
+    rows = 1024
+    gen, call = {"q4k": (synth.q4k_matrix, K.cuda_matvec_q4k), "q6k": (synth.q6k_matrix, K.cuda_matvec_q6k),
+                 "q5k": (lambda *a: synth.typed_matrix(13, *a), K.cuda_matvec_q5k)}[kind]
+    w = dev(gen(5100 + cols, rows, cols).reshape(rows, -1))
+    x = dev(synth.normal_f32(5101 + cols, cols))
+    whole, part = torch.empty(rows, device="cuda"), torch.empty(rows, device="cuda")
+    call(w, x, whole, rows, cols)
+    for n, starts in ((512, (0, 512)), (128, (0, 384, 896)), (1, (8, 1016))):  # (a slice of Q6_K rows on any 2-byte address)
+        for lo in starts:
+            call(w[lo:lo + n], x, part, n, cols)
+            assert torch.equal(part[:n], whole[lo:lo + n]), (n, lo)
