@@ -131,3 +131,43 @@ def test_rows_per_group_and_sums_of_activations(K, counts, H, EFF, down):
         want = (gate / (1 + np.exp(-gate)) * up) @ w2.T
         assert np.all(np.linalg.norm(got[t] - want, axis=1) <= 2e-5 * np.linalg.norm(want, axis=1)), e
     assert K.mb200_device_error() == 0
+
+
+def test_swiglu_between_the_gemms_rounds_as_fp32_does(K):
+    """gate / (1 + exp(-gate)) to one rounding of the sum and one of the quotient: 2^-23 of the value, plus 2^-27 for an exponential off by two
+    units (gate >= 4). Row i of gate and up picks x[i] and x[255], rows of the down projection are unit vectors, scaling is by powers of two,
+    and values whose pair of halves would round once more are left out."""
+    H, EFF, M = 256, 256, 64
+    g, u, d = synth.expert_sizes(H, EFF, 14)
+    gate_up = np.zeros((2 * EFF, synth.Q4K_BLOCK), np.uint8)
+    for row in range(EFF):
+        for r, col in ((row, row), (EFF + row, 255)):
+            sub = col // 32
+            gate_up[r, :2] = np.array([1.0], np.float16).view(np.uint8)
+            gate_up[r, 4 + sub if sub < 4 else 8 + sub] = 1  # scale 1 of this sub-block
+            gate_up[r, 16 + 32 * (sub // 2) + col % 32] = 1 << 4 * (sub & 1)
+    assert np.array_equal(oracle.dequant_q4k(gate_up[:EFF].reshape(-1), EFF, H), np.eye(EFF, dtype=np.float32))
+    down = np.zeros((H, synth.Q6K_BLOCK), np.uint8)
+    down[:, 128:192] = 0xAA  # q - 32 = 0: low nibbles 0, high bits 2
+    down[:, 192:208] = 1
+    down[:, 208:] = np.array([1.0], np.float16).view(np.uint8)
+    for row in range(H):  # q - 32 = 1 in column `row`
+        half, i = row // 128, row % 128
+        down[row, 64 * half + i % 64] |= 1 << 4 * (i // 64)
+    assert np.array_equal(oracle.dequant_q6k(down.reshape(-1), H, EFF), np.eye(H, dtype=np.float32))
+    expert = np.concatenate([gate_up.reshape(-1), down.reshape(-1)])
+    x = np.random.default_rng(9).uniform(4, 15, (M, H)).astype(np.float16)
+    x[:, 255] = 16
+    n = K.mb200_moe_prefill_workspace_bytes(M, 1, H, EFF, 1)
+    ws = torch.empty(n + 256, dtype=torch.uint8, device="cuda")
+    ws = ws[-ws.data_ptr() % 256:]
+    y = torch.empty(M, H, device="cuda")
+    K.mb200_moe_prefill(dev(expert), g + u + d, g, u, 14, 1, 1, H, EFF, dev(x), dev(np.zeros((M, 1), np.int32)),
+                        dev(np.ones((M, 1), np.float32)), None, y, M, 0, ws)
+    gate = x.astype(np.float64)
+    want = gate / (1 + np.exp(-gate))  # times 16 of up, times 1 / 16 on the way through the halves, which the result has back
+    unit = 2.0 ** np.floor(np.log2(want))
+    exact = np.abs(want - want.astype(np.float16)) < 0.99 * 2.0 ** -12 * unit  # what the low half holds has 11 bits
+    err = np.abs(host(y).astype(np.float64) / 16 - want) / want
+    assert exact.sum() > 4000 and err[exact].max() <= 2.0 ** -23 + 2.0 ** -27, (err[exact].max(), exact.sum())
+    assert K.mb200_device_error() == 0
