@@ -70,6 +70,11 @@ struct Cfg {
     static constexpr int kXBytes = kXRows * 128;
     static constexpr int kWBytes = QT == 4 ? kRows * kQ4KBlock : kRows * kQ6Slot;
     static constexpr int kWStages = QT == 6 && BT == 256 && !PAIR ? 2 : 3;
+    // A dequant group takes every second super-block. Barriers of its own for every second round of the ring's stages, so that it waits
+    // for every phase of those it uses: on a stage's one barrier it would miss every second phase, and the parity of the one before the
+    // missed one lets it pass (super-block 4 at once if 2 lands before 1).
+    static constexpr int kWBars = 2 * kWStages;
+    static_assert(kWBars % (kGroups / 2) == 0, "a group meets every phase of the barriers it waits on");
     static constexpr int kOffW = kStages * kXBytes;
     static constexpr int kOffBar = kOffW + kWStages * kWBytes;
     static constexpr int kSmem = kOffBar + 512 + 1024 /* alignment */;
@@ -124,11 +129,12 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
                                                                                 const Params P)
 {
     using C = Cfg<QT, BT, PAIR>;
-    constexpr int S = C::kStages, WS = C::kWStages;
+    constexpr int S = C::kStages, WS = C::kWStages, WB = C::kWBars;
+    static_assert(8 * (3 * S + 2 * WB + 1) + 8 <= 512, "barriers");
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = smem_raw + ((0u - smem_u32(smem_raw)) & 1023u);  // not through an integer: stays a shared-memory pointer
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + C::kOffBar), *empty = full + S;
-    uint64_t *wfull = empty + S, *wempty = wfull + WS, *acc_full = wempty + WS, *pfull = acc_full + 1;
+    uint64_t *wfull = empty + S, *wempty = wfull + WB, *acc_full = wempty + WB, *pfull = acc_full + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(pfull + S);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     const int tid = threadIdx.x, lane = tid & 31, warp = static_cast<int>(warp_uniform(tid >> 5));
@@ -146,7 +152,7 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
             mbar_init(&empty[s], 1);     // tcgen05.commit
             mbar_init(&pfull[s], 1);     // PAIR: the other CTA's stage is full
         }
-        for (int s = 0; s < WS; s++) {
+        for (int s = 0; s < WB; s++) {
             mbar_init(&wfull[s], QT == 4 || P.group ? 1 : 64);  // TMA: the expect_tx arrival; cp.async: every thread of the two warps
             mbar_init(&wempty[s], 8);                // the two groups that share a super-block
         }
@@ -232,21 +238,27 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
     } else if (warp < C::kDq0) {
         // ---- raw weights: 128 rows x one super-block per stage; they never depend on the kernel upstream ----
         if (warp == 2 || !P.group) {
-            int s = 0;
-            uint32_t ph = 1;
+            int s = 0, f = 0, e = 0;  // stage; barrier of this super-block, of the one that had the stage before
+            uint32_t ph = 0;
             for (int b = 0; b < nb; b++) {
-                wait(&wempty[s], ph, abort_flag);
+                if (b >= WS) {
+                    wait(&wempty[e], ph, abort_flag);
+                    if (++e == WB) {
+                        e = 0;
+                        ph ^= 1;
+                    }
+                }
                 __syncwarp();
                 uint8_t *dst = smem + C::kOffW + s * C::kWBytes;
                 if (QT == 4 || P.group) {
                     if (leader) {
-                        mbar_expect_tx(&wfull[s], C::kWBytes);
+                        mbar_expect_tx(&wfull[f], C::kWBytes);
                         if (QT == 4) {
-                            tma_load_2d(dst, &wmap, (b0 + b) * kQ4KBlock, n0, &wfull[s]);  // rows past N arrive as zeros
+                            tma_load_2d(dst, &wmap, (b0 + b) * kQ4KBlock, n0, &wfull[f]);  // rows past N arrive as zeros
                         } else {
                             for (int j = 0; j < P.group; j++)
                                 tma_load_2d(dst + (j * kRows / P.group) * kQ6Slot, &wmap, ((j * P.bpr + b0 + b) * kQ6KBlock) & ~15, n0 / P.group,
-                                            &wfull[s]);
+                                            &wfull[f]);
                         }
                     }
                 } else {
@@ -259,12 +271,10 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
                         blk += (size_t)P.bpr * kQ6KBlock;
                         d += kQ6Pitch;
                     }
-                    cp_async_arrive(&wfull[s]);
+                    cp_async_arrive(&wfull[f]);
                 }
-                if (++s == WS) {
-                    s = 0;
-                    ph ^= 1;
-                }
+                if (++s == WS) s = 0;
+                if (++f == WB) f = 0;
             }
             if (QT == 6 && !P.group) asm volatile("cp.async.wait_all;" ::: "memory");
         }
@@ -298,8 +308,8 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
         for (int j = 0; j < units; j += kGroups) {
             const int G = min(kGroups, units - j), u = j + g;
             if (g >= G) break;
-            const int sb = u >> 1, half = u & 1, ws = sb % WS;
-            wait(&wfull[ws], (sb / WS) & 1, abort_flag);
+            const int sb = u >> 1, half = u & 1, ws = sb % WS, wb = sb % WB;
+            wait(&wfull[wb], (sb / WB) & 1, abort_flag);
             __syncwarp();
             const uint8_t *blk = smem + C::kOffW + ws * C::kWBytes;
             uint32_t o[16];
@@ -310,7 +320,7 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
 #pragma unroll
                 for (int i = 0; i < 4; i++) qv[i] = *reinterpret_cast<const uint4 *>(blk + 16 + 64 * half + 16 * i);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&wempty[ws]);
+                if (lane == 0) mbar_arrive(&wempty[wb]);
                 const float d = __half2float(__ushort_as_half(static_cast<unsigned short>(hdr.x)));
 #pragma unroll
                 for (int c = 0; c < 2; c++) {
@@ -333,7 +343,7 @@ __global__ void __launch_bounds__((Cfg<QT, BT, PAIR>::kThreads), 1) gemm_dense_k
                 RawQ6 raw;
                 if (__any_sync(0xffffffffu, off & 2u)) raw.load<true>(words, off & 2u, half); else raw.load<false>(words, 0, half);
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&wempty[ws]);
+                if (lane == 0) mbar_arrive(&wempty[wb]);
 #pragma unroll
                 for (int c = 0; c < 2; c++) {
                     const int it = 2 * j + c * G + g;

@@ -66,3 +66,37 @@ def test_rows_in_groups_and_splits(K, kind, M, N, Kd):
     assert rel.max() <= 1e-3, rel.max()
     assert bool((guard[M * N:] == 7.0).all())
     assert K.mb200_device_error() == 0
+
+
+@pytest.mark.parametrize("kind,M,N,Kd", [
+    # 64 tokens a tile, 8, 14, 6 and 5 super-blocks a CTA; rows 1, 4, 2 and 8 at a time
+    ("q6k", 8, 8192, 4096), ("q6k", 30, 19000, 3584), ("q6k", 3, 6520, 3072), ("q6k", 1, 2480, 1280), ("q4k", 8, 8192, 4096),
+    ("q6k", 68, 9632, 2048), ("q6k", 65, 4248, 2560), ("q6k", 100, 18944, 2304), ("q4k", 68, 9512, 2048),   # 128
+    ("q6k", 700, 4100, 2048), ("q6k", 268, 6944, 1536), ("q6k", 265, 6440, 1280), ("q4k", 643, 3128, 1536),  # 256
+    ("q6k", 512, 8192, 4096), ("q6k", 130, 9592, 3072), ("q6k", 257, 9472, 2816), ("q4k", 512, 8192, 4096),  # a pair
+])
+def test_weight_stages_used_again(K, kind, M, N, Kd):
+    """More super-blocks a CTA than the ring of raw weights holds, in every form and, for Q6_K, every number of rows that make a tensor map. Rows
+    repeat with a period that no tile divides. Against fp64 products of the weights rounded to fp16: what is left is fp32 accumulation (2e-5
+    at 4096 columns) and weights that round to the other half (5e-6); a super-block taken before it is there would be 0.2."""
+    gen, deq, call = ((synth.q4k_matrix, oracle.dequant_q4k, K.mb200_gemm_q4k_f16) if kind == "q4k" else
+                      (synth.q6k_matrix, oracle.dequant_q6k, K.mb200_gemm_q6k_f16))
+    n = min(N, 509)
+    rows = np.arange(N) % n
+    w = np.ascontiguousarray(gen(2900 + N, n, Kd).reshape(n, -1))
+    w64 = dev(deq(w.reshape(-1), n, Kd).reshape(n, Kd)).half().double()
+    d_w, x = dev(w[rows].reshape(-1)), dev(synth.normal_f16(2901 + M, M * Kd).reshape(M, Kd))
+    assert d_w.data_ptr() % 16 == 0
+    want = (x.double() @ w64.T)[:, torch.from_numpy(rows).cuda()]
+    out = torch.empty(M, N, device="cuda")
+    for pdl in (False, True):
+        before = K.mb200_set_pdl(pdl)
+        try:
+            for _ in range(3):
+                out.fill_(float("nan"))
+                call(d_w, x, out, M, N, Kd)
+                rel = (out.double() - want).norm(dim=1) / want.norm(dim=1)
+                assert float(rel.max()) <= 1e-4, (pdl, float(rel.max()))
+        finally:
+            K.mb200_set_pdl(before)
+    assert K.mb200_device_error() == 0
