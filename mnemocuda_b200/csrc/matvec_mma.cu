@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kMvThreads, NB <= 2 ? 2 : 1) matvec_mma_kernel
             }
             req += rows;
         };
-        if (lane == 0) {
+        if (leader) {  // the lane that arrives on the barriers below, before the CTA's first barrier
             *reinterpret_cast<uint4 *>(smem + kZero) = make_uint4(0u, 0u, 0u, 0u);
             for (int s = 0; s < S; s++) {
                 mbar_init(&full[s], 1);
