@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include "../../include/mnemo_b200.h"
+#include "bounded_wait.cuh"
 
 namespace mb200 {
 
@@ -105,9 +106,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)  //
     return ok != 0;
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) { return mbar_try_wait(smem_u32(bar), parity); }
-// Returns false if the phase did not complete within the iteration budget
-// (each try_wait already blocks for a hardware time slice).
-constexpr uint32_t kWaitBudget = 1u << 16;  // x a few microseconds per try_wait: a fraction of a second
 __device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, uint32_t parity)
 {
     uint32_t ok;
@@ -120,6 +118,8 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, uint32_t parity)
         : "memory");
     return ok != 0;
 }
+// Returns false if the phase did not complete within the iteration budget
+// (each try_wait already blocks for a hardware time slice).
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity)
 {
     for (uint32_t i = 0; i < kWaitBudget; i++)

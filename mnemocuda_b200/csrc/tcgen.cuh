@@ -215,23 +215,13 @@ __device__ __forceinline__ uint64_t desc64(uint32_t lo)
 }
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr) { return desc64(desc_lo(saddr)); }
 
-// Waits inside the GEMMs. A wait that runs out raises the CTA's abort flag and from then on every wait of the CTA returns at
-// once: the roles run through their loops on whatever the buffers hold (all addresses stay in bounds) and the kernel reports
-// the timeout. Nothing is checked on the fast path; a check per step (a shared-memory load and a vote) cost the issuing warp
-// 100 of its 400 cycles per chunk. (try_wait with a time limit sleeps in between: 10 % slower.)
+// Waits inside the GEMMs. After one that ran out (bounded_wait.cuh) the roles run through their loops on whatever the buffers hold (all
+// addresses stay in bounds) and the kernel reports the timeout. (try_wait with a time limit sleeps in between: 10 % slower.)
 // Asking costs issue slots that the dequantising warps need: PATIENT waits (the loaders', which run stages ahead) pause in between.
 template <bool PATIENT = false>
 __device__ __forceinline__ void wait(uint32_t bar, uint32_t parity, volatile int *abort_flag)
 {
-    for (uint32_t i = 0; i < kWaitBudget; i++) {
-#pragma unroll 1
-        for (int j = 0; j < 64; j++) {
-            if (mbar_try_wait(bar, parity)) return;
-            if (PATIENT) __nanosleep(100);
-        }
-        if (*abort_flag) return;
-    }
-    *abort_flag = 1;
+    bounded_wait([=] { return mbar_try_wait(bar, parity); }, [] { if (PATIENT) __nanosleep(100); }, abort_flag);
 }
 template <bool PATIENT = false>
 __device__ __forceinline__ void wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag)
