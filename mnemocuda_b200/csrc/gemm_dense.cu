@@ -414,11 +414,12 @@ void attr()
 }
 
 // CTAs that run at a time when clusters of `s` have to find room in one GPC each: 148, 148, 135, 132, 130, 132, -, 120 for one CTA per SM.
-int clustered_ctas(int s)
+// By size of the cluster, for the current device, which a call asks for once: asking is a call of the runtime.
+const int *clustered_ctas()
 {
     static int known[kMaxDevices][kMaxSplit + 1] = {};
-    int &n = known[current_device()][s];
-    if (n == 0) {
+    int *n = known[current_device()];
+    for (int s = n[kMaxSplit] ? kMaxSplit + 1 : 1; s <= kMaxSplit; s++) {
         attr<4, 64, false>();
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kMaxSplit, 1, s);
@@ -432,7 +433,7 @@ int clustered_ctas(int s)
         cfg.numAttrs = 1;
         int clusters = 0;
         if (cudaOccupancyMaxActiveClusters(&clusters, gemm_dense_kernel<4, 64, false>, &cfg) != cudaSuccess) cudaGetLastError();
-        n = clusters > 0 ? clusters * s : device_sms() / s * s;
+        n[s] = clusters > 0 ? clusters * s : device_sms() / s * s;
     }
     return n;
 }
@@ -452,12 +453,13 @@ Plan plan(int qt, int M, int N, int K)
     } kCost[2][4] = {{{740, 0, 3500}, {780, 1800, 3200}, {1190, 3600, 3600}, {1180, 3600, 3600}},    // Q4_K: 64, 128, 256 tokens, a pair
                      {{810, 0, 4400}, {960, 800, 4600}, {1210, 3100, 5200}, {1200, 3100, 5200}}};  // Q6_K
     const int sms = device_sms(), bpr = K / 256, row_tiles = (N + kRows - 1) / kRows;
+    const int *ctas = clustered_ctas();
     Plan best{256, 1, true};
     long best_cost = -1;
     auto offer = [&](int form, int s) {
         const bool pair = form == 3;
         const int bt = pair ? 256 : 64 << form, rows = pair ? row_tiles + (row_tiles & 1) : row_tiles;
-        const long tiles = (long)rows * ((M + bt - 1) / bt) * s, room = clustered_ctas(pair ? 2 : s);
+        const long tiles = (long)rows * ((M + bt - 1) / bt) * s, room = ctas[pair ? 2 : s];
         if (s > 1 && tiles > room) return;
         const auto &c = kCost[qt == 6][form];
         const long cost = (tiles + room - 1) / room * ((long)(bpr + s - 1) / s * c.sb + c.fixed + c.fill * (tiles < sms ? tiles : sms) / sms) +
@@ -538,7 +540,7 @@ void gemm_init()
     attr<6, 256, false>();
     attr<6, 256, true>();
     (void)encode_tiled();
-    for (int s : {1, 2, 3, 4, 5, 6, 8}) (void)clustered_ctas(s);
+    (void)clustered_ctas();
 }
 
 }  // namespace mb200
