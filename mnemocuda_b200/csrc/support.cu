@@ -787,7 +787,7 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ l
 // mostly, and a warp ranks them. Warps sort 32 candidates each; a key's place among a CTA's 256, then among all, is the number of
 // larger keys in the other sorted lists, by binary search. The walk's three float sums over the nucleus are prefixes of one and the
 // same sequence, so ONE serial chain of additions leaves all of them and the two searches run on all threads.
-// 13.6 us per token at 151936 (28.9 with the maximum in a launch ahead, 32 CTAs that picked by rounds of a warp-wide maximum, a ticket
+// 12.7 us per token at 151936 in a chain of calls, 14 one call at a time; 200064 logits 16.1, 600000 39.7 (27.3, 29.2, 27.5 and 37.1 with the maximum in a launch ahead, 32 CTAs that picked by rounds of a warp-wide maximum, a ticket
 // and a last CTA that sorted). By clock stamps: logits 1 us, maximum 1.3, probabilities 1.7, picking 3.2, sorting 256 2.1, places 1.6,
 // the chain 2.2 (640 additions); three cluster barriers are 2 of it.
 constexpr int kSampleKeep = 8, kSampleCands = 256 * kSampleKeep;
@@ -836,6 +836,8 @@ __device__ __forceinline__ int larger_in(const unsigned long long *list, unsigne
     return before + (list[before] > key);  // the steps add up to LEN - 1: one comparison is left
 }
 
+// MORE: more elements than the registers hold
+template <bool MORE>
 __global__ void __cluster_dims__(kSampleCtas, 1, 1) __launch_bounds__(kSampleThreads)
 sample_top_p_kernel(const float *__restrict__ logits, int n, float temperature, float top_p, unsigned long long seed, int *result)
 {
@@ -866,7 +868,9 @@ sample_top_p_kernel(const float *__restrict__ logits, int n, float temperature, 
     float mx = -1e30f;
 #pragma unroll
     for (int q = 0; q < kSampleHeld; q++) mx = fmaxf(mx, p[q]);
-    for (int q = kSampleHeld; q < count; q++) mx = fmaxf(mx, __ldcg(logits + base + q * kStep));
+    for (int q0 = kSampleHeld; MORE && q0 < count; q0 += 4)
+#pragma unroll
+        for (int j = 0; j < 4; j++) mx = fmaxf(mx, q0 + j < count ? __ldcg(logits + base + (q0 + j) * kStep) : -INFINITY);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (lane == 0) S.smax[warp] = mx;
@@ -900,6 +904,7 @@ sample_top_p_kernel(const float *__restrict__ logits, int n, float temperature, 
         s[q & 3] += p[q];
         if (q < count) consider(p[q], base + q * kStep);
     }
+    // (Without MORE this loop has nothing to do. Left out, the compiler orders what stands above so that 151936 logits take 13.1 instead of 12.7 us.)
     for (int q0 = kSampleHeld; q0 < count; q0 += 4)
 #pragma unroll
         for (int j = 0; j < 4; j++)
@@ -931,30 +936,50 @@ sample_top_p_kernel(const float *__restrict__ logits, int n, float temperature, 
         }
     }
     __syncthreads();
-    // ---- every thread offers its keys from that bound on; where a thread has read more than it holds, its eight largest of them ----
+    // ---- every thread offers its keys from that bound on. Of more elements than the registers hold eight threads may have more of them than
+    // there is room for, then each its eight largest (by as many rounds over its elements, which cost 18 us at 200064 logits, 50 at 600000) ----
     {
         const unsigned long long bound = S.bound[lane];
         const unsigned bound_hi = static_cast<unsigned>(bound >> 32);
-        auto offer = [&](unsigned long long key) { S.offer[lane][atomicAdd(&S.offered[lane], 1)] = key; };
-        if (count <= kSampleHeld) {
+        auto offer = [&](unsigned long long key) {
+            const int at = atomicAdd(&S.offered[lane], 1);
+            if (at < kSampleOffer) S.offer[lane][at] = key;
+        };
+        auto consider = [&](float v, int i) {
+            if (__float_as_uint(v) < bound_hi) return;
+            const unsigned long long key = cand_key(v, i);
+            if (key >= bound) offer(key);
+        };
 #pragma unroll
-            for (int q = 0; q < kSampleHeld; q++)
-                if (q < count && __float_as_uint(p[q]) >= bound_hi) {
-                    const unsigned long long key = cand_key(p[q], base + q * kStep);
-                    if (key >= bound) offer(key);
+        for (int q = 0; q < kSampleHeld; q++)
+            if (q < count) consider(p[q], base + q * kStep);
+        if (MORE) {
+            if (best >= bound)
+                for (int q0 = kSampleHeld; q0 < count; q0 += 4) {
+                    float l[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) l[j] = q0 + j < count ? __ldcg(logits + base + (q0 + j) * kStep) : 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        if (q0 + j < count) consider(prob(l[j]), base + (q0 + j) * kStep);
                 }
-        } else {
-            unsigned long long key = best;
+            __syncthreads();
+            const bool over = S.offered[lane] > kSampleOffer;
+            if (__syncthreads_or(over)) {
+                if (warp == 0 && over) S.offered[lane] = 0;
+                __syncthreads();
+                unsigned long long key = over ? best : 0;
 #pragma unroll 1
-            for (int r = 0; r < kSampleKeep && key != 0 && key >= bound; r++) {
-                offer(key);
-                unsigned long long next = 0;
+                for (int r = 0; r < kSampleKeep && key != 0 && key >= bound; r++) {
+                    offer(key);
+                    unsigned long long next = 0;
 #pragma unroll 1
-                for (int q = 0; q < count; q++) {
-                    const unsigned long long k = cand_key(prob(__ldcg(logits + base + q * kStep)), base + q * kStep);
-                    if (k < key) next = max(next, k);
+                    for (int q = 0; q < count; q++) {
+                        const unsigned long long k = cand_key(prob(__ldcg(logits + base + q * kStep)), base + q * kStep);
+                        if (k < key) next = max(next, k);
+                    }
+                    key = next;
                 }
-                key = next;
             }
         }
     }
@@ -1166,7 +1191,8 @@ void sample_attr()
     static bool done[kMaxDevices] = {false};
     const int dev = current_device();
     if (done[dev]) return;
-    cudaFuncSetAttribute(sample_top_p_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SampleShared));
+    for (auto kernel : {sample_top_p_kernel<false>, sample_top_p_kernel<true>})
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(SampleShared));
     done[dev] = true;
 }
 
@@ -1398,8 +1424,8 @@ void cuda_sample_token(const float *logits, int vocab_size, float temperature, f
     if (vocab_size <= 0) return;
     if (temperature > 0.0f) {
         sample_attr();
-        launch_k(sample_top_p_kernel, dim3(kSampleCtas), dim3(kSampleThreads), sizeof(SampleShared), stream, logits, vocab_size, temperature, top_p,
-                 rng_state, d_result);
+        launch_k(vocab_size > kSampleHeld * kSampleCtas * kSampleThreads ? sample_top_p_kernel<true> : sample_top_p_kernel<false>, dim3(kSampleCtas),
+                 dim3(kSampleThreads), sizeof(SampleShared), stream, logits, vocab_size, temperature, top_p, rng_state, d_result);
         MB200_CHECK_LAUNCH("cuda_sample_token");
         return;
     }

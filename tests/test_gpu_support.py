@@ -213,7 +213,7 @@ def test_sample_token_top_p_degenerate_and_repeat(K):
     assert int(res.item()) == 777
 
 
-@pytest.mark.parametrize("V", [1, 255, 257, 8193, 163840, 163841, 270001])
+@pytest.mark.parametrize("V", [1, 255, 257, 8193, 163840, 163841, 270001, 500003])
 def test_sample_token_top_p_sizes(K, V):
     """One element, a class short of one, the step between rows of the cluster's warps, and what the threads hold and what they read again
     (163840 | 163841). Against the oracle (by the rule above: one state may disagree); and equal logits, where the candidates are the
@@ -242,3 +242,19 @@ def test_kernel_pointer_exports(K):
     lib = _lib.lib()
     ptrs = [lib.cuda_get_rope_kernel_ptr(), lib.cuda_get_f16dual_kernel_ptr(), lib.cuda_get_attn_f16kv_kernel_ptr()]
     assert all(ptrs) and len(set(ptrs)) == 3
+
+
+@pytest.mark.parametrize("V", [163840, 270001])
+@pytest.mark.parametrize("warps", [7, 8, 9])
+def test_sample_token_candidates_of_few_threads(K, V, warps):
+    """Residue classes all of whose large probabilities belong to seven, eight or nine threads (ids 256 warp + class + 8192 q): beyond what
+    the registers hold, more keys than a class has room for. Against the oracle, by the rule above."""
+    logits = (synth.normal_f32(97, V) - 12).astype(np.float32)
+    i = np.arange(V)
+    logits[((i >> 8) % 32 < warps) & (i % 256 < 40)] += 14
+    d_l, res = dev(logits), torch.full((1,), -1, dtype=torch.int32, device="cuda")
+    miss = 0
+    for seed in (int(s) for s in np.random.default_rng(96).integers(1, 2 ** 63, 12)):
+        K.cuda_sample_token(d_l, V, 1.0, 0.95, seed, res)
+        miss += int(res.item()) != oracle.sample_top_p(logits, 1.0, 0.95, seed)
+    assert miss <= 1, miss
