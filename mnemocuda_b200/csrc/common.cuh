@@ -57,15 +57,6 @@ __device__ __forceinline__ float group_sum(float v, int width)
     return v;
 }
 
-__device__ __forceinline__ float h2f_lo(uint32_t packed)
-{
-    return __half2float(__ushort_as_half(static_cast<unsigned short>(packed & 0xFFFFu)));
-}
-__device__ __forceinline__ float h2f_hi(uint32_t packed)
-{
-    return __half2float(__ushort_as_half(static_cast<unsigned short>(packed >> 16)));
-}
-
 // 4 x (u8 * s8) + c, exact.
 __device__ __forceinline__ int dp4a_us(uint32_t a_u8x4, uint32_t b_s8x4, int c)
 {

@@ -31,12 +31,6 @@ __device__ __forceinline__ uint32_t hmul2(uint32_t a, uint32_t b)
     const __half2 r = __hmul2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
     return *reinterpret_cast<const uint32_t *>(&r);
 }
-__device__ __forceinline__ uint32_t hfma2(uint32_t a, uint32_t b, uint32_t c)
-{
-    const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b),
-                              *reinterpret_cast<const __half2 *>(&c));
-    return *reinterpret_cast<const uint32_t *>(&r);
-}
 __device__ __forceinline__ uint32_t hfms2(uint32_t a, uint32_t b, uint32_t c)  // a b - c
 {
     const __half2 r = __hfma2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b),
