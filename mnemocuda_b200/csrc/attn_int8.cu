@@ -2,8 +2,9 @@
 //
 // Grid (KV head x block of 16 query heads, chunk of positions); every K / V byte is read once for all query heads of
 // the block. The cache is 128 + 4 bytes per row, so the kernel is HBM-bound once the arithmetic is on
-// mma.sync.m16n8k16: 64 heads / 4 KV heads / 32768 positions take 16.1 us (5.3 us at the copy rate; 21.4 with eight warps that held a
-// tile ahead in registers, 136 with fp32 FMAs and a five-step warp reduction per position and head), 32 / 8 heads 18.8 (29.4). By clock
+// mma.sync.m16n8k16: 64 heads / 4 KV heads / 32768 positions take 15.0 us in a chain of calls, 15.7 one call at a time (5.3 us at the copy rate; 21.5 and 20.9
+// with eight warps that held a tile ahead in registers, 136 with fp32 FMAs and a five-step warp reduction per position and head), 32 / 8 heads
+// 18.0 in a chain (31.2). By clock
 // stamps, 64 / 4 at 32768: 3 us until q is in fragments (while the first tiles stream), 7.2 the tiles (the MMAs alone are 5), then one
 // after the other the merges of the warps (1.1), the cluster (0.5) and, behind a ticket (1.3), the last CTA (1.2).
 //   * int8 values become fp16 exactly (0x6400 | (v + 128) is 1152 + v); q and the probabilities are carried as

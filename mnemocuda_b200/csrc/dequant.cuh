@@ -67,8 +67,8 @@ __device__ __forceinline__ void int_q4(const uint32_t (&w)[8], const ScaleQ4 &f,
 }
 
 // ---- Q6_K blocks in shared memory ----
-// A block is 210 bytes at a 2-byte alignment: no tensor map fits it and 16-byte copies would have to carry up to 14 bytes of
-// skew. A warp copies the 53 aligned words that hold it (two words per lane; the last word's spare bytes share it with valid
+// A block is 210 bytes at a 2-byte alignment. Groups of rows make a tensor map (encode_q6k_groups); where the address or the number of
+// rows rules that out, a warp copies the 53 aligned words that hold it (two words per lane; the last word's spare bytes share it with valid
 // ones); a row's thread then reads its words, which start 0 or 2 bytes into the first (`skew`).
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void *src)  // 4 bytes, shared <- global, both 4-byte aligned
 {

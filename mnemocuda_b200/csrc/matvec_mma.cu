@@ -11,10 +11,11 @@
 // What bounds it: in a chain of launches, the way from one y to the next x: of 6.1 us at 8192 x 4096, 0.65 from the end of the
 // grid to the next one's wait, 1.3 for x and its levels, 0.5 a stage of 14 rows (a warp's own chain of loads, MMAs and scaling),
 // 0.35 for the last sums; the weights arrive meanwhile. So a CTA whose weights fit takes at most half of an SM (113 KB of
-// shared memory, 112 registers a thread): under programmatic dependent launch the next launch's CTA starts beside it and
+// shared memory, 96 registers a thread, at which Q4_K with two super-blocks a warp spills 4 bytes): under programmatic dependent launch the next launch's CTA starts beside it and
 // has its weights in shared memory when y is done. Chains of 16 launches against the streaming kernel: 8192 x 4096 8.1 -> 6.1 us,
 // 4096 x 4096 6.4 -> 4.1, 6144 x 2048 5.1 -> 3.7, 512 x 2048 3.7 -> 2.7, 50000 x 4096 26.5 -> 20.0 (5.7 TB/s);
-// no size of 1 to 50000 rows was slower, with or without dependent launches, and the error against 64 bits is the same.
+// up to 4096 columns no size of 1 to 50000 rows was slower, with or without dependent launches (wider ones: see launch()), and the error
+// against 64 bits is the same.
 // Up to 4096 columns a warp keeps the levels of its one or two super-blocks in registers with two CTAs on an SM; with three
 // or four, up to 8192, a CTA needs the SM's registers for itself and has all of x asked for before it splits any of it (in two rounds one
 // after the other 4096 x 8192 took 6.9 us, 512 x 8192 5.0): 4096 x 8192 9.6 -> 6.5 us, 2048 x 6144 6.1 -> 4.5, 512 x 8192 5.4 -> 4.6. With six

@@ -787,8 +787,8 @@ __global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ l
 // mostly, and a warp ranks them. Warps sort 32 candidates each; a key's place among a CTA's 256, then among all, is the number of
 // larger keys in the other sorted lists, by binary search. The walk's three float sums over the nucleus are prefixes of one and the
 // same sequence, so ONE serial chain of additions leaves all of them and the two searches run on all threads.
-// 12.7 us per token at 151936 in a chain of calls, 14 one call at a time; 200064 logits 16.1, 600000 39.7 (27.3, 29.2, 27.5 and 37.1 with the maximum in a launch ahead, 32 CTAs that picked by rounds of a warp-wide maximum, a ticket
-// and a last CTA that sorted). By clock stamps: logits 1 us, maximum 1.3, probabilities 1.7, picking 3.2, sorting 256 2.1, places 1.6,
+// 12.7 us per token at 151936 in a chain of calls, 14.0 one call at a time; 200064 logits 16.1, 600000 39.7 (27.3, 29.2, 27.5 and 37.1 with the
+// maximum in a launch ahead, 32 CTAs that picked by rounds of a warp-wide maximum, a ticket and a last CTA that sorted). By clock stamps: logits 1 us, maximum 1.3, probabilities 1.7, picking 3.2, sorting 256 2.1, places 1.6,
 // the chain 2.2 (640 additions); three cluster barriers are 2 of it.
 constexpr int kSampleKeep = 8, kSampleCands = 256 * kSampleKeep;
 constexpr int kSampleCtas = 8, kSampleClasses = 256 / kSampleCtas;  // classes of a CTA: one per lane
